@@ -232,3 +232,126 @@ def tolerance(case):
     if case["kind"] == "projections":
         return "exact"
     return {"rel": 7e-3 if case["act"] == "bf16" else 1.8e-3, "max": 0.07}
+
+
+# ---- the same work in 64 bits, by the definitions and in plain torch -------------------------------------------------
+
+def _rope(x, pos, a):
+    """Rotate-half pairs over the first rope_dim elements; angles as the engine forms them, in 32 bits."""
+    half = a["rope_dim"] // 2
+    freq = torch.tensor([1.0 / a["theta"] ** (2 * i / a["rope_dim"]) for i in range(half)], dtype=torch.float64, device=DEV)
+    ang = (pos.float()[..., None] * freq.float()).double()[..., None, :]
+    lo, hi, c, s = x[..., :half], x[..., half:2 * half], ang.cos(), ang.sin()
+    return torch.cat([lo * c - hi * s, lo * s + hi * c, x[..., 2 * half:]], -1)
+
+
+def _normed(x, w, eps):
+    return x * (x.square().mean(-1, keepdim=True) + eps).rsqrt() * torch.as_tensor(w, device=DEV).double()
+
+
+def _as_cached(x, cache):
+    """A new row as attention sees it, decoded from the cache's format."""
+    if cache == "f32":
+        return x.float().double()
+    f = x.float()
+    if cache == "int8":
+        top = f.abs().amax(-1, keepdim=True)
+        codes = (f * (127.0 / top)).round()
+        return codes.double() * (top / 127.0).double()
+    f = f.unflatten(-1, (-1, 32))
+    d = f.abs().amax(-1, keepdim=True) / 127.0
+    y = f * (1.0 / d)
+    codes = (y.abs() + 0.5).floor() * y.sign()            # ties away from zero
+    return (codes.double() * d.half().double()).flatten(-2)
+
+
+def _cached(kv, cache, b, n):
+    """The first n rows of sequence b, decoded: K and V [n][kv heads][head_dim]."""
+    o, nkv = int(kv.seq_off_host[b]), kv.nkv
+    got = []
+    for pool, scales in ((kv.K, kv.Ks), (kv.V, kv.Vs)):
+        rows = pool[o * nkv * kv.row_bytes:(o + n) * nkv * kv.row_bytes]
+        if cache == "f32":
+            got.append(rows.view(torch.float32).view(n, nkv, kv.hd).double())
+        elif cache == "int8":
+            got.append(rows.view(torch.int8).view(n, nkv, kv.hd).double() * scales[o * nkv:(o + n) * nkv].view(n, nkv, 1).double())
+        else:
+            blocks = rows.view(n, nkv, kv.hd // 32, 34)
+            d = blocks[..., :2].contiguous().view(torch.float16).double()
+            got.append((blocks[..., 2:].contiguous().view(torch.int8).double() * d).flatten(-2))
+    return got
+
+
+def _attend(a, w, kv, cache, b, L, qproj, k, v):
+    """T new tokens of sequence b behind L cached ones: [T][heads x head_dim]."""
+    T, nh, nkv, hd = qproj.shape[0], a["nh"], a["nkv"], a["hd"]
+    pos = torch.arange(L, L + T, device=DEV)
+    q, gate = qproj.double().view(T, nh, 2, hd).unbind(2)
+    q = _rope(_normed(q, w["q_norm_w"], a["eps"]), pos, a)
+    k = _as_cached(_rope(_normed(k.double().view(T, nkv, hd), w["k_norm_w"], a["eps"]), pos, a), cache)
+    v = _as_cached(v.double().view(T, nkv, hd), cache)
+    if L:
+        K, V = _cached(kv, cache, b, L)
+        k, v = torch.cat([K, k]), torch.cat([V, v])
+    out, block = torch.empty(T, nh, hd, dtype=torch.float64, device=DEV), 1024
+    for h in range(nkv):
+        heads = slice(h * nh // nkv, (h + 1) * nh // nkv)
+        for t in range(0, T, block):
+            n = L + min(T, t + block)                     # keys that the last query of the block sees
+            s = q[t:t + block, heads].transpose(0, 1) @ k[:n, h].T * hd ** -0.5
+            s.masked_fill_(torch.arange(n, device=DEV) > pos[t:t + block, None], -math.inf)
+            out[t:t + block, heads] = (s.softmax(-1) @ v[:n, h]).transpose(0, 1)
+    return (out * gate.sigmoid()).flatten(1)
+
+
+def _delta(a, w, S, ring, pos, qkv, x_a, x_b, z):
+    """T tokens of every sequence through one delta-net layer: outputs, states and conv histories behind them."""
+    B, T = qkv.shape[:2]
+    nk, nv, dk, dv, taps = a["nk"], a["nv"], a["dk"], a["dv"], a["conv_k"]
+    f64 = lambda x: torch.as_tensor(x, device=DEV).double()
+    qkv, S, ring, rows = qkv.double(), S.double(), ring.double(), torch.arange(B, device=DEV)
+    before = [ring[rows, (pos.long() + j) % taps] for j in range(1, taps)]         # token t' lies in slot t' % taps
+    x = torch.cat([torch.stack(before, 1), qkv], 1)
+    y = sum(x[:, j:j + T] * f64(w["conv_w"])[:, j] for j in range(taps))
+    y = y * y.sigmoid()
+    for t in range(max(0, T - taps), T):
+        ring[rows, (pos.long() + t) % taps] = qkv[:, t]
+    unit = lambda r: r * (r.square().sum(-1, keepdim=True) + 1e-6).rsqrt()
+    tiled = torch.arange(nv, device=DEV) % nk                                      # the key head of each value head
+    q = unit(y[..., :nk * dk].view(B, T, nk, dk))[:, :, tiled]
+    k = unit(y[..., nk * dk:2 * nk * dk].view(B, T, nk, dk))[:, :, tiled]
+    v = y[..., 2 * nk * dk:].view(B, T, nv, dv)
+    alpha = (f64(w["a_coef"]) * torch.nn.functional.softplus(x_a.double().view(B, T, nv) + f64(w["dt_bias"]))).exp()
+    beta = x_b.double().view(B, T, nv).sigmoid()
+    o = torch.empty(B, T, nv, dv, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        S = S * alpha[:, t, :, None, None]
+        u = beta[:, t, :, None] * (v[:, t] - (S @ k[:, t, :, :, None])[..., 0])
+        S = S + u[..., None] * k[:, t, :, None]
+        o[:, t] = (S @ q[:, t, :, :, None])[..., 0]
+    z = z.double().view(B, T, nv, dv)
+    o = _normed(o * dk ** -0.5, w["norm_w"], a["eps"]) * z * z.sigmoid()
+    return o.view(B, T, nv * dv), S, ring
+
+
+def exact(case, seed):
+    if case["kind"] == "projections":
+        return None                                       # whole numbers up to one f32 sum in a fixed order: compared bit for bit
+    a, state = ARCHS[case["arch"]], prepare(case, seed)
+    if case["kind"] == "full":
+        w, T, inputs = full_weights(a, seed, 3), case["tokens"], state["inputs"]
+        out = [_attend(a, w, state["kv"], case["cache"], b, case["context"], *(x[b] for x in inputs)) for b in range(case["n_seq"])]
+        return torch.stack(out), None, None, None, None
+    if case["kind"] == "linear":
+        return _delta(a, linear_weights(a, seed, 0), state["state"].S, state["state"].conv, state["pos"], *state["inputs"])
+    outs, kept = [], []
+    for i, ((kind, _, s), inputs) in enumerate(zip(state["stack"].layers, state["inputs"])):
+        if kind == "linear":
+            o, S, ring = _delta(a, linear_weights(a, seed, i), s.S, s.conv, state["stack"].pos, *(x[:, None] for x in inputs))
+            outs.append(o[:, 0])
+            kept.append((S, ring))
+        else:
+            w = full_weights(a, seed, i)
+            outs.append(torch.cat([_attend(a, w, s, case["cache"], b, L, *(x[b:b + 1] for x in inputs)) for b, L in enumerate(_contexts(case))]))
+            kept.append((None, None, None, None))
+    return outs, kept
