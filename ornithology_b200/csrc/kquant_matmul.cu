@@ -28,33 +28,16 @@
 // Prompts are walked in passes of 128 tokens (grid.y; the weights are then re-read from L2).  Shapes the tensor copy
 // cannot address (rows that do not start on 16-byte boundaries: Q6_K with n_in not a multiple of 2048) take a plain
 // kernel with the same arithmetic.
-#include <cuda.h>
-#include <cuda_fp16.h>
 #include <math.h>
+#include <stdlib.h>
 
-#include "qproj.cuh"
-#include "tcgen05.cuh"          // the tensor-map encoder entry point, bounded mbarrier waits
+#include "kquant.cuh"
+
+using namespace kq;
 
 namespace {
 
-constexpr int QK = 256;
-
-enum { T_Q4K = 0, T_Q6K = 1, T_Q80 = 2 };
-template <int TYPE> struct Fmt;
-template <> struct Fmt<T_Q4K> { static constexpr int BLOCK = 144, BOX = 144; };
-template <> struct Fmt<T_Q6K> { static constexpr int BLOCK = 210, BOX = 240; };   // 240: rows 60 words apart, no bank conflicts
-template <> struct Fmt<T_Q80> { static constexpr int BLOCK = 272, BOX = 272; };
-
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ void tensor_copy_rows(uint32_t dst, const CUtensorMap *map, int word0, int row0, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(word0), "r"(row0) : "memory");
-}
-
 // d = a . b for one k-step, int32 sums from zero.  k = 32: a = {row g k 0..15 part, row g+8, row g k 16..31 part, row g+8}
 #define ORN_MMA_K32(NAME, TA, TB)                                                                                   \
     __device__ __forceinline__ void NAME(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {           \
@@ -76,37 +59,13 @@ ORN_MMA_K16(mma_k16_s8s8, "s8", "s8")
 ORN_MMA_K16(mma_k16_u8u8, "u8", "u8")
 ORN_MMA_K16(mma_k16_u8s8, "u8", "s8")
 
-typedef const unsigned char *smem_ptr;
-__device__ __forceinline__ uint32_t lds32(smem_ptr p) { return *reinterpret_cast<const uint32_t *>(p); }
 // four bytes from a 2-byte-aligned shared address
 __device__ __forceinline__ uint32_t lds32_any(smem_ptr p) {
     const uint32_t off = (uint32_t)(uintptr_t)p & 3u;
     smem_ptr base = p - off;
     return __funnelshift_r(lds32(base), lds32(base + 4), off * 8);
 }
-__device__ __forceinline__ float f16_bits_to_f32(uint32_t h) { return __half2float(__ushort_as_half((unsigned short)h)); }
 __device__ __forceinline__ int sbyte(uint32_t w, int k) { return (int)(w << (24 - 8 * k)) >> 24; }   // signed byte k of w
-
-// The weight matrices of one launch: projections that read the same activations (attn_qkv, attn_gate, ssm_alpha and
-// ssm_beta of a delta-net layer; attn_q / k / v of a full-attention layer) go as one grid, CTAs cta0[p] .. cta0[p+1]-1
-// belonging to matrix p.
-constexpr int MAX_GROUP = 8;
-struct KqGroup {
-    CUtensorMap map[MAX_GROUP];                   // [n_out rows][row bytes / 4 words] of each matrix
-    void *y[MAX_GROUP];                           // [T][n_out]
-    int n_out[MAX_GROUP];
-    int cta0[MAX_GROUP + 1];
-    int n;
-};
-
-struct KqArgs {
-    const unsigned char *img;                     // [token tiles][nseg] Q8_K images
-    void *y;                                      // [T][n_out]
-    int T, n_out, nseg, out_dtype;
-    int nstage, stage_bytes;                      // shared-memory stages of the tensor-core kernel
-    unsigned int *status;
-};
-
 
 // ---- one super-block of one weight type: rows g and g + 8 of the warp's 16 against MT token tiles ---------------
 // wrow0: shared address of row g's bytes of this super-block (row g + 8 is 8 * BOX further); xs: shared address of
@@ -455,45 +414,13 @@ __global__ void __launch_bounds__(128) k_matmul_kq_plain(const unsigned char *W,
     else act_st((float *)a.y, (size_t)tok * a.n_out + row, total);
 }
 
-// the weight matrix as [n_out rows][row_bytes / 4 words]; one box = box_rows rows x BOX bytes
-template <int TYPE>
-bool weight_map(CUtensorMap *m, const void *W, int n_in, int n_out, int box_rows) {
-    OrnTensorMapEncodeFn enc = orn_tensor_map_encoder();
-    const cuuint64_t row_bytes = (cuuint64_t)n_in / QK * Fmt<TYPE>::BLOCK;
-    if (!enc || ((uintptr_t)W & 15) != 0 || (row_bytes & 15) != 0) return false;
-    cuuint64_t dims[2] = {row_bytes / 4, (cuuint64_t)n_out};
-    cuuint64_t strides[1] = {row_bytes};
-    cuuint32_t box[2] = {Fmt<TYPE>::BOX / 4, (cuuint32_t)box_rows};
-    cuuint32_t es[2] = {1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void *>(W), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 constexpr int SMEM_BUDGET = 200 * 1024;           // dynamic shared memory of one CTA (one CTA per SM: 512 threads)
-
-// what the host knows of a group: the matrices (all of one weight type, one n_in), their outputs
-struct HostGroup {
-    const void *W[MAX_GROUP];
-    void *y[MAX_GROUP];
-    int n_out[MAX_GROUP];
-    int n;
-    int rows_total() const { int r = 0; for (int i = 0; i < n; i++) r += n_out[i]; return r; }
-};
 
 template <int TYPE, int WR, int KS, int MT>
 ornith_status launch_tc(const HostGroup &h, int n_in, int T, KqArgs a, cudaStream_t stream) {
     constexpr int TS = NWARP / (WR * KS), PASS_TOK = 8 * MT * TS, CTA_ROWS = 16 * WR;
     KqGroup g;
-    g.n = h.n;
-    g.cta0[0] = 0;
-    for (int i = 0; i < h.n; i++) {
-        if (!weight_map<TYPE>(&g.map[i], h.W[i], n_in, h.n_out[i], CTA_ROWS)) {
-            orn_record_error("matmul_q: the weight tensor map could not be made");
-            return (ornith_status)ORNITH_ERR_BACKEND;
-        }
-        g.y[i] = h.y[i]; g.n_out[i] = h.n_out[i];
-        g.cta0[i + 1] = g.cta0[i] + (h.n_out[i] + CTA_ROWS - 1) / CTA_ROWS;
-    }
+    if (!fill_group<TYPE>(&g, h, n_in, CTA_ROWS)) return (ornith_status)ORNITH_ERR_BACKEND;
     // tiles of the fullest pass, rounded up to whole groups: a group multiplies all MT of its tiles, so the stage
     // must have room for them (the ones past the pass's last tile hold stale bytes and are never stored)
     const int nt_max = (((T < PASS_TOK ? T : PASS_TOK) + 7) / 8 + MT - 1) / MT * MT;
@@ -554,10 +481,24 @@ ornith_status launch_kq(const HostGroup &h, int n_in, int T, KqArgs a, bool plai
     }
     const int n_out = h.rows_total();
     if (T > 64) {                                 // prompts: passes of 128 tokens; of 64 with fewer rows per CTA for a small matrix
-        const long p128 = (T + 127) / 128, p64 = (T + 63) / 64;
-        if ((n_out + 63) / 64 * p128 >= 100) return launch_tc<TYPE, 4, 1, 4>(h, n_in, T, a, stream);
-        if ((n_out + 63) / 64 * p64 >= 100) return launch_tc<TYPE, 4, 1, 2>(h, n_in, T, a, stream);
-        if ((n_out + 31) / 32 * p64 >= 100) return launch_tc<TYPE, 2, 2, 2>(h, n_in, T, a, stream);
+        const long p128 = (T + 127) / 128, p64 = (T + 63) / 64, r64 = (n_out + 63) / 64;
+        const int shape = r64 * p128 >= 100 ? 0 : r64 * p64 >= 100 ? 1 : (n_out + 31) / 32 * p64 >= 100 ? 2 : 3;
+        if constexpr (TYPE != T_Q80) {
+            // k-quants go to the tcgen05 kernel unless too few of its 128-row tiles exist to fill the GPU.  Microseconds per
+            // super-block and wave here, by shape: fits to 65 .. 777 tokens of 2048 -> 512, 4096 -> 2048, 2048 -> 8192, 8192 -> 4096.
+            // E.g. (mma.sync | tcgen05): Q6_K 8192 -> 4096, 777 tokens 339 | 112 us, 65 tokens 85 | 72; 4096 -> 2048, 100 tokens
+            // 28 | 42; Q4_K 8192 -> 4096, 777 tokens 247 | 168, 128 tokens 57 | 70.
+            static const float q4[4] = {2.1f, 1.7f, 0.95f, 0.95f}, q6[4] = {3.1f, 2.6f, 1.4f, 1.4f};
+            const long ctas = shape == 0 ? r64 * p128 : shape == 1 ? r64 * p64 : shape == 2 ? (n_out + 31) / 32 * p64 : (n_out + 15) / 16 * p64;
+            const float full = shape == 0 && T < 128 ? 0.6f + 0.4f * (float)T / 128.0f : 1.0f;       // a pass with missing tiles
+            int units;
+            const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
+            if (units && tc5 < (float)((ctas + 147) / 148) * full * (TYPE == T_Q4K ? q4 : q6)[shape])
+                return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
+        }
+        if (shape == 0) return launch_tc<TYPE, 4, 1, 4>(h, n_in, T, a, stream);
+        if (shape == 1) return launch_tc<TYPE, 4, 1, 2>(h, n_in, T, a, stream);
+        if (shape == 2) return launch_tc<TYPE, 2, 2, 2>(h, n_in, T, a, stream);
         return launch_tc<TYPE, 1, 4, 2>(h, n_in, T, a, stream);
     }
     if (n_out >= 64 * 100) return launch_wr<TYPE, 4>(h, n_in, T, a, stream);
@@ -568,7 +509,7 @@ ornith_status launch_kq(const HostGroup &h, int n_in, int T, KqArgs a, bool plai
 ornith_status run_group(int wtype, const HostGroup &h, int n_in, const void *image, int T, int out_dtype, cudaStream_t s) {
     KqArgs a;
     a.img = (const unsigned char *)image;
-    a.y = nullptr; a.T = T; a.n_out = 0; a.nseg = n_in / QK; a.out_dtype = out_dtype; a.nstage = 0; a.stage_bytes = 0; a.status = orn_status_word();
+    a.y = nullptr; a.T = T; a.n_out = 0; a.nseg = n_in / QK; a.out_dtype = out_dtype; a.nstage = 0; a.stage_bytes = 0; a.status = orn_status_word(); a.minus_zero = -0.0f;
     const char *e = getenv("ORNITH_CUDA_PROJ_PLAIN");                 // =1: the plain kernel for every shape
     const bool plain = e && e[0] == '1';
     if (wtype == ORNITH_GGML_Q4_K) return launch_kq<T_Q4K>(h, n_in, T, a, plain, s);
