@@ -39,6 +39,27 @@ def test_q8k_blocks_are_the_engines_bytes(oracle):
         assert (got == oracle.q8k_quantize(Xb)).all(), ("bf16", T, n_in)
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_q8k_blocks_of_rows_off_the_16_byte_grid(oracle, dtype):
+    """The quantiser takes 16-byte loads only where the input allows them: the same rows one element further on, with ties
+    between lanes, an infinity and NaNs (which no comparison picks)."""
+    import torch
+    from ornithology_b200 import device as D
+    T, n_in = 11, 512
+    X = bf16_round(_acts(5, T, n_in))
+    X[4, 77] = np.nan
+    X[5, 300] = X[5, 290] = -9.0
+    dt = getattr(torch, dtype)
+    buf = torch.empty(T * n_in + 1, dtype=dt, device="cuda")
+    for off in (0, 1):
+        buf[off:off + T * n_in] = torch.from_numpy(X).cuda().to(dt).flatten()
+        got = D.q8k_quantize(buf[off:off + T * n_in], n_in)
+        ref = oracle.q8k_quantize(X)
+        rows = [t for t in range(T) if t != 4]                     # (the code of a NaN is the conversion instruction's)
+        assert (got[rows] == ref[rows]).all(), (off, dtype)
+        assert (got[4, :, :4] == ref[4, :, :4]).all()              # its block's scale is not
+
+
 @pytest.mark.parametrize("T,n_in,n_out", [(1, 2048, 8192), (64, 2048, 8192), (70, 2048, 520), (5, 512, 40), (8, 4096, 2048)])
 def test_projection_against_the_integer_path(oracle, T, n_in, n_out):
     import torch
