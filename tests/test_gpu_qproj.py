@@ -42,7 +42,7 @@ def test_q8k_blocks_are_the_engines_bytes(oracle):
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_q8k_blocks_of_rows_off_the_16_byte_grid(oracle, dtype):
     """The quantiser takes 16-byte loads only where the input allows them: the same rows one element further on, with ties
-    between lanes, an infinity and NaNs (which no comparison picks)."""
+    between lanes and a NaN (which no comparison picks)."""
     import torch
     from ornithology_b200 import device as D
     T, n_in = 11, 512
