@@ -76,6 +76,14 @@ __device__ __forceinline__ float ex2_fast(float x) { float y; asm("ex2.approx.ft
 __device__ __forceinline__ float rcp_fast(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float silu_fast(float x) { return x * rcp_fast(1.0f + ex2_fast(-1.4426950408889634f * x)); }
 
+// What every kernel of a decode step does first: wait for the kernel in front (whose results it reads and whose inputs it may
+// overwrite), then let the one behind it take its place on the SMs.  A step of one chat is a dozen kernels of a few
+// microseconds; without this each pays its launch latency after the end of the one before.
+__device__ __forceinline__ void dependent_entry() {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
 // Launch `kernel` as a programmatic dependent of the kernel in front of it on the stream: its CTAs may become resident
 // while that kernel still runs.  The kernel must execute griddepcontrol.wait in every CTA before it touches anything a
 // kernel in front of it may write or read, and before it exits.

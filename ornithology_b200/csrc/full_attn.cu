@@ -483,6 +483,7 @@ struct CombineArgs {
 template <typename ACT>
 __global__ void __launch_bounds__(128) k_gqa_combine(CombineArgs a) {
     extern __shared__ float w_s[];                       // [nsplit]
+    dependent_entry();
     __shared__ float red[32];
     const int hd = a.kv.hd, h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
     const int cap = (int)(a.kv.seq_off[b + 1] - a.kv.seq_off[b]);
@@ -508,8 +509,14 @@ __global__ void __launch_bounds__(128) k_gqa_combine(CombineArgs a) {
     ACT *out = (ACT *)a.out + ((size_t)b * a.nh + h) * hd;
     for (int d = tid; d < hd; d += 128) {
         float o = 0.0f;
-        for (int s = 0; s < nlive; s++)
-            if (w_s[s] != 0.0f) o += part[(size_t)s * (hd + 2) + 2 + d] * w_s[s];
+        for (int s0 = 0; s0 < nlive; s0 += 8) {           // eight partials in flight: one at a time paid a memory latency each
+            float v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = s0 + u < nlive ? part[(size_t)(s0 + u) * (hd + 2) + 2 + d] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (s0 + u < nlive && w_s[s0 + u] != 0.0f) o += v[u] * w_s[s0 + u];
+        }
         o *= inv;
         if (gate) o *= sigmoid_f(act_ld(gate, d));
         act_st(out, d, o);
@@ -841,12 +848,10 @@ ornith_status ornith_cuda_full_attn_step(const ornith_cuda_full_layer *l, const 
     CombineArgs c;
     c.kv = d.kv; c.kv_len = kv_len; c.part = part; c.qproj = qproj; c.out = out;
     c.nh = nh; c.nsplit = nsplit_used; c.gated = l->gated; c.tokens_per_split = d.tokens_per_split;
-    dim3 cgrid(nh, B);
-    if (act_dtype == ORNITH_ACT_BF16)
-        k_gqa_combine<__nv_bfloat16><<<cgrid, 128, nsplit_used * sizeof(float), st>>>(c);
-    else
-        k_gqa_combine<float><<<cgrid, 128, nsplit_used * sizeof(float), st>>>(c);
-    return orn_check_launch("k_gqa_combine");
+    const dim3 cgrid(nh, B);
+    const size_t csmem = nsplit_used * sizeof(float);
+    return orn_check(act_dtype == ORNITH_ACT_BF16 ? orn_launch_dependent(k_gqa_combine<__nv_bfloat16>, cgrid, dim3(128), csmem, st, c)
+                                                  : orn_launch_dependent(k_gqa_combine<float>, cgrid, dim3(128), csmem, st, c), "k_gqa_combine");
 }
 
 // The f32 image of the prepared query rows is only read by the kernels other than the tcgen05 one: when that

@@ -145,6 +145,7 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_i8_raw(DecodeArgs a) {
     __shared__ __align__(8) unsigned long long bars[NWARP][2];
     __shared__ int pipe_failed;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    dependent_entry();
     unsigned char *wbase = smem + QS_BYTES + warp * WARP_BYTES;
     uint2 *Q_s = reinterpret_cast<uint2 *>(smem);               // [k-step][lane]
     if (tid == 0) pipe_failed = 0;
@@ -377,6 +378,5 @@ ornith_status launch_gqa_decode_i8_raw(const DecodeArgs &a, int n_seq, cudaStrea
         configured = true;
     }
     dim3 grid(a.kv.nkv * ((a.nh / a.kv.nkv + 7) / 8), a.nsplit, n_seq);
-    k_gqa_decode_i8_raw<<<grid, 128, SMEM_BYTES, st>>>(a);
-    return orn_check_launch("k_gqa_decode_i8_raw");
+    return orn_check(orn_launch_dependent(k_gqa_decode_i8_raw, grid, dim3(128), SMEM_BYTES, st, a), "k_gqa_decode_i8_raw");
 }

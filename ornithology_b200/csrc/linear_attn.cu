@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(256, 2) k_linear_decode_128(LinArgs a) {
     __shared__ __align__(16) float q_s[128], k_s[128], v_s[128];
     __shared__ double redd[32];
     __shared__ float gates[2];
+    dependent_entry();
     const int hv = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int kh = key_head_of(a, hv), qd = a.nk * 128, vd = a.nv * 128, Cc = 2 * qd + vd;
     float *S = a.S + (size_t)b * a.S_stride + (size_t)hv * 128 * 128;
@@ -767,9 +768,8 @@ ornith_status ornith_cuda_linear_attn_step(const ornith_cuda_linear_layer *l, co
         const char *variant = getenv("ORNITH_CUDA_LINEAR_DECODE");
         const bool ring = variant ? variant[0] == 'r' : (long long)n_seq * l->nv > 296;
         if (ring) return launch_linear_decode_ring(x, n_seq, act_dtype, s);
-        if (bf) k_linear_decode_128<__nv_bfloat16><<<grid, 256, 0, s>>>(x);
-        else    k_linear_decode_128<float><<<grid, 256, 0, s>>>(x);
-        return orn_check_launch("k_linear_decode_128");
+        return orn_check(bf ? orn_launch_dependent(k_linear_decode_128<__nv_bfloat16>, grid, dim3(256), 0, s, x)
+                            : orn_launch_dependent(k_linear_decode_128<float>, grid, dim3(256), 0, s, x), "k_linear_decode_128");
     }
     const size_t smem = (size_t)(2 * l->dk + 2 * l->dv) * sizeof(float);
     if (bf) k_linear_decode_generic<__nv_bfloat16><<<grid, 128, smem, s>>>(x);

@@ -308,6 +308,7 @@ ornith_status ornith_cuda_gather_layout(const void *gathered, void *full, int wo
 
 // ---- counters ------------------------------------------------------------------
 __global__ void k_advance(int32_t *c, int n, int delta) {
+    dependent_entry();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) c[i] += delta;
 }
@@ -315,8 +316,7 @@ __global__ void k_advance(int32_t *c, int n, int delta) {
 ornith_status ornith_cuda_advance(int32_t *counters, int n, int delta, void *stream) {
     ORN_TRY(orn_require_device());
     if (n <= 0) return ORNITH_OK;
-    k_advance<<<(n + 255) / 256, 256, 0, as_stream(stream)>>>(counters, n, delta);
-    return orn_check_launch("k_advance");
+    return orn_check(orn_launch_dependent(k_advance, dim3((n + 255) / 256), dim3(256), 0, as_stream(stream), counters, n, delta), "k_advance");
 }
 
 }  // extern "C"
