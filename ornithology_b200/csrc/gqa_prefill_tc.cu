@@ -258,7 +258,13 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
             mbar_arrive(su32(&bars.q_full));
         }
         float m_ref = -INFINITY, l = 0.0f;
+        const size_t tok = (size_t)b * a.T + q0 + row;
+        const ACT *gate = (a.gated && live) ? (const ACT *)a.qproj + tok * a.nh * HD * 2 + (size_t)h * HD * 2 + HD : nullptr;
         for (int j = 0; j < n_tiles; j++) {
+            if (gate && j == max(0, n_tiles - 4)) {            // the epilogue's gate values on their way to L2
+                const char *g0 = reinterpret_cast<const char *>(gate + OCOLS * part);
+                for (int o = 0; o < (int)(OCOLS * sizeof(ACT)); o += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(g0 + o));
+            }
             const int sb = j % NB, key0 = j * BN + COLS * part;
             ok = ok && mbar_wait(su32(&bars.s_full[sb]), (uint32_t)(j / NB) & 1u);
             fence_after();
@@ -327,19 +333,40 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
         ok = ok && mbar_wait(su32(&bars.pv_done[(n_tiles - 1) % NB]), (uint32_t)((n_tiles - 1) / NB) & 1u);
         fence_after();
         const float inv = ok ? 1.0f / l : NAN;
-        const size_t tok = (size_t)b * a.T + q0 + row;
-        const ACT *gate = (a.gated && live) ? (const ACT *)a.qproj + tok * a.nh * HD * 2 + (size_t)h * HD * 2 + HD : nullptr;
         ACT *out = (ACT *)a.out + (tok * a.nh + h) * HD;
+        // 32 columns at a time, the gate of the next 32 requested before this 32 are scaled and stored.  (A thread's row is a
+        // line of its own; element by element, each gate load waits behind the store before it: 128 memory latencies, 70 us of
+        // a CTA that has nothing else to run, which was more than half of a 1000-token prompt.)
+        const bool vec = (((uintptr_t)a.qproj | (uintptr_t)a.out) & 15) == 0;
+        float gt[32];
+        auto load_gate = [&](int c) {
+            if (vec) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) { const float4 v = act_ld4(gate, c + i); gt[i] = v.x; gt[i + 1] = v.y; gt[i + 2] = v.z; gt[i + 3] = v.w; }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; i++) gt[i] = act_ld(gate, c + i);
+            }
+        };
+        if (gate) load_gate(OCOLS * part);
 #pragma unroll 1
         for (int c = OCOLS * part; c < OCOLS * part + OCOLS; c += 32) {
             float o[32];
             tmem_ld32_wait(lane_t + TM_O + c, o);
-            if (live) {
 #pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    float y = o[i] * inv;
-                    if (gate) y *= sigmoid_f(act_ld(gate, c + i));
-                    act_st(out, c + i, y);
+            for (int i = 0; i < 32; i++) o[i] *= inv;
+            if (gate) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) o[i] *= sigmoid_f(gt[i]);
+                if (c + 32 < OCOLS * part + OCOLS) load_gate(c + 32);
+            }
+            if (live) {
+                if (vec) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) act_st4(out, c + i, make_float4(o[i], o[i + 1], o[i + 2], o[i + 3]));
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; i++) act_st(out, c + i, o[i]);
                 }
             }
         }

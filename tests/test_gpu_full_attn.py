@@ -416,3 +416,27 @@ def test_tensor_core_prefill_is_reproducible():
             first = out
         else:
             assert (out == first).all(), rep
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("gated", [True, False])
+def test_prefill_output_off_the_16_byte_grid(dtype, gated):
+    """The tensor-core prefill stores (and reads its gate) 16 bytes at a time where both tensors allow it: an output one
+    element further on takes the element form and must hold the same bits; 300 rows leave a ragged last tile of 128."""
+    import torch
+    from ornithology_b200 import device as D
+    dt = getattr(torch, dtype)
+    g = torch.Generator(device="cuda").manual_seed(7)
+    B, T, nh, nkv, hd = 2, 300, 4, 2, 256
+    w = np.random.default_rng(3).uniform(0.9, 1.1, (2, hd)).astype(np.float32)
+    layer = D.FullLayer(nh, nkv, hd, w[0], w[1], rope_dim=64, theta=1e7, gated=gated)
+    ins = [torch.randn(B, T, n, generator=g, device="cuda").to(dt) for n in (layer.qproj_width, nkv * hd, nkv * hd)]
+    got = []
+    for off in (0, 1):
+        kv = D.KvBatch(D.KV_Q8_0, nkv, hd, [T, T])
+        buf = torch.zeros(B * T * nh * hd + 8, dtype=dt, device="cuda")
+        out = buf[off:off + B * T * nh * hd].view(B, T, nh * hd)
+        D.full_attn_prefill(layer, kv, torch.zeros(B, dtype=torch.int32, device="cuda"), *ins, T, out=out)
+        got.append(out.clone())
+        assert (buf[off + out.numel():] == 0).all() and (off == 0 or buf[0] == 0)
+    assert torch.isfinite(got[0].float()).all() and (got[0] == got[1]).all()
