@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(128) k_conv4_silu_prefill_tma(LinArgs a, const
         tc5::mbar_expect_tx(su32(&bars[stage]), (uint32_t)CT_STAGE);
         tile_copy(su32(smem + stage * CT_STAGE), &map_x, cb * CH, b * a.T + c.t_begin + tt * CT_TOK - 3, su32(&bars[stage]));
     };
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");     // the chunk preparation may take its place behind this grid
     if (tid == 0)
         for (int k = 0; k < CT_NST; k++) {
             const long long tile = (long long)blockIdx.x + (long long)k * gridDim.x;

@@ -132,7 +132,10 @@ __device__ __forceinline__ void block_matvec16(const float *B, int row0, const f
 template <typename ACT>
 __global__ void __launch_bounds__(256, 2) k_delta_prep64(LinArgs a, const float *Y, const float *rqg, const float *rkg,
                                                       const float *la, const float *be, float *AP, float *aux,
-                                                      int n_chunks, int chunk0) {
+                                                      int n_chunks, int chunk0, int refresh) {
+    // A programmatic dependent of the conv in front of it, as the scan is of this kernel (short prompts: four launches of
+    // 8 to 40 us, whose latencies showed)
+    dependent_entry();
     extern __shared__ __align__(16) unsigned char smraw[];
     PrepSmem &sm = *reinterpret_cast<PrepSmem *>(smraw);
     const int chunk = chunk0 + blockIdx.x, kh = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
@@ -140,6 +143,16 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep64(LinArgs a, const float 
     const int qd = a.nk * 128, Cc = 2 * qd + a.nv * 128;
     const int t0 = chunk * C, n = min(C, a.T - t0);
     const size_t tok0 = (size_t)b * a.T + t0;
+
+    // the conv has read the old history for the last time: store the last min(T, conv_k) inputs of the sequence (their own
+    // launch took 2.4 us and a gap of a 512-token prompt's 72)
+    if (refresh && chunk == n_chunks - 1) {
+        const int pos0 = a.pos[b], K = a.conv_k;
+        float *ring = a.conv + (size_t)b * a.conv_stride;
+        const ACT *X = (const ACT *)a.qkv + (size_t)b * a.T * Cc;
+        for (int ch = kh * 256 + tid; ch < Cc; ch += a.nk * 256)
+            for (int t = max(0, a.T - K); t < a.T; t++) ring[(size_t)((pos0 + t) % K) * Cc + ch] = act_ld(X, (size_t)t * Cc + ch);
+    }
 
     for (int e = tid; e < C * 32; e += 256) {             // raw rows (tf32 values); rows past the end are zero
         const int i = e >> 5, c = (e & 31) * 4;
@@ -447,6 +460,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     if (warp == W_TMA) {
         // ================= producer =================
         if (lane == 0) {
+            asm volatile("griddepcontrol.wait;\n" ::: "memory");     // everything that comes through here is written by the kernels in front
             const int yrow0 = b * a.T + c0 * C;                       // first row of this CTA's first chunk
             const size_t blk0 = ((size_t)b * a.nv + hv) * a.n_chunks + c0;
             auto load_kq = [&](int n) {
@@ -1123,14 +1137,25 @@ ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dty
     a.seg_state = (float *)((char *)aux + aux_part(x.nv, n_seq, n_chunks));
     a.seg_raw = (float *)((char *)a.seg_state + seg_state_part(x.nv, n_seq, a.n_seg));
 
-    auto prep = [&](int c_begin, int c_count, cudaStream_t ps) {
+    const int refresh = front != nullptr;                             // (without `front` the caller has refreshed the history)
+    auto prep = [&](int c_begin, int c_count, cudaStream_t ps, bool chained) {
         const dim3 pgrid((unsigned)c_count, (unsigned)x.nk, (unsigned)n_seq);
-        if (bf) k_delta_prep64<__nv_bfloat16><<<pgrid, 256, sizeof(PrepSmem), ps>>>(x, Y, rq, rk, la, be, AP, aux, n_chunks, c_begin);
-        else    k_delta_prep64<float><<<pgrid, 256, sizeof(PrepSmem), ps>>>(x, Y, rq, rk, la, be, AP, aux, n_chunks, c_begin);
+        const float *Yc = Y;
+        if (chained)
+            return orn_check(bf ? orn_launch_dependent(k_delta_prep64<__nv_bfloat16>, pgrid, dim3(256), sizeof(PrepSmem), ps, x, Yc, rq, rk, la, be, AP, aux,
+                                                       n_chunks, c_begin, refresh)
+                                : orn_launch_dependent(k_delta_prep64<float>, pgrid, dim3(256), sizeof(PrepSmem), ps, x, Yc, rq, rk, la, be, AP, aux, n_chunks,
+                                                       c_begin, refresh), "k_delta_prep64");
+        if (bf) k_delta_prep64<__nv_bfloat16><<<pgrid, 256, sizeof(PrepSmem), ps>>>(x, Y, rq, rk, la, be, AP, aux, n_chunks, c_begin, refresh);
+        else    k_delta_prep64<float><<<pgrid, 256, sizeof(PrepSmem), ps>>>(x, Y, rq, rk, la, be, AP, aux, n_chunks, c_begin, refresh);
         return orn_check_launch("k_delta_prep64");
     };
-    auto scan = [&](const ScanArgs &sa, cudaStream_t ss) {
+    auto scan = [&](const ScanArgs &sa, cudaStream_t ss, bool chained) {
         dim3 grid((unsigned)x.nv, (unsigned)n_seq);
+        if (chained)
+            return orn_check(bf ? orn_launch_dependent(k_delta_scan_tc5<__nv_bfloat16, false>, grid, dim3(NTHREADS), SCAN_SMEM, ss, my, mym, map_ap, map_ap32, map_v, sa)
+                                : orn_launch_dependent(k_delta_scan_tc5<float, false>, grid, dim3(NTHREADS), SCAN_SMEM, ss, my, mym, map_ap, map_ap32, map_v, sa),
+                             "k_delta_scan_tc5");
         if (bf) k_delta_scan_tc5<__nv_bfloat16, false><<<grid, NTHREADS, SCAN_SMEM, ss>>>(my, mym, map_ap, map_ap32, map_v, sa);
         else    k_delta_scan_tc5<float, false><<<grid, NTHREADS, SCAN_SMEM, ss>>>(my, mym, map_ap, map_ap32, map_v, sa);
         return orn_check_launch("k_delta_scan_tc5");
@@ -1150,28 +1175,24 @@ ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dty
         const int per = (n_chunks + n_slabs - 1) / n_slabs;
         auto slab = [&](int k, int cb, int cn) -> ornith_status {
             ORN_TRY(front->conv(cb * C, min(x.T, (cb + cn) * C), s));
-            ORN_TRY(prep(cb, cn, s));
+            ORN_TRY(prep(cb, cn, s, false));
             ORN_TRY(orn_check(cudaEventRecord(pipe.front_done[k], s), "slab event record"));
             ORN_TRY(orn_check(cudaStreamWaitEvent(pipe.scan_stream, pipe.front_done[k], 0), "slab event wait"));
             ScanArgs sa = a;
             sa.c_begin = cb; sa.c_count = cn;
-            return scan(sa, pipe.scan_stream);
+            return scan(sa, pipe.scan_stream, false);
         };
         ornith_status st = ORNITH_OK;
         int k = 0;
         for (int cb = 0; cb < n_chunks && st == ORNITH_OK; cb += per, k++) st = slab(k, cb, min(per, n_chunks - cb));
-        if (st == ORNITH_OK) st = front->ring_refresh(s);     // after the conv that reads the old history
         // the caller's stream always rejoins the scan stream, also when a launch failed on the way
         ornith_status join = orn_check(cudaEventRecord(pipe.scans_done, pipe.scan_stream), "slab event record");
         if (join == ORNITH_OK) join = orn_check(cudaStreamWaitEvent(s, pipe.scans_done, 0), "slab event wait");
         return st != ORNITH_OK ? st : join;
     }
-    if (front) {
-        ORN_TRY(front->conv(0, x.T, s));
-        ORN_TRY(front->ring_refresh(s));
-    }
-    ORN_TRY(prep(0, n_chunks, s));
-    if (a.n_seg <= 1) return scan(a, s);
+    if (front) ORN_TRY(front->conv(0, x.T, s));
+    ORN_TRY(prep(0, n_chunks, s, front != nullptr));
+    if (a.n_seg <= 1) return scan(a, s, true);
     // few heads: the runs of the prompt side by side, then the carry over the runs and the finishing pass
     dim3 grid((unsigned)x.nv, (unsigned)n_seq, (unsigned)(2 * a.n_seg - 1));
     if (bf) k_delta_scan_tc5<__nv_bfloat16, true><<<grid, NTHREADS, SCAN_SMEM, s>>>(my, mym, map_ap, map_ap32, map_v, a);

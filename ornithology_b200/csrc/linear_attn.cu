@@ -857,12 +857,6 @@ ornith_status ornith_cuda_linear_attn_prefill(const ornith_cuda_linear_layer *l,
                 else    k_conv4_silu_prefill<float, true, true><<<g, 128, 0, cs>>>(x, Y, rq, rk, t_begin, t_end);
                 return orn_check_launch("k_conv4_silu_prefill");
             };
-            front.ring_refresh = [=](cudaStream_t cs) {
-                dim3 rg((unsigned)((Cc + 255) / 256), n_seq);
-                if (bf) k_conv_ring_refresh<__nv_bfloat16><<<rg, 256, 0, cs>>>(x);
-                else    k_conv_ring_refresh<float><<<rg, 256, 0, cs>>>(x);
-                return orn_check_launch("k_conv_ring_refresh");
-            };
             return launch_linear_prefill_tc5(x, n_seq, act_dtype, Y, rq, rk, nullptr, nullptr, &front, blocks, g_delta_scan_dump, s);
         }
         else if (bf && tc)  k_conv4_silu_prefill<__nv_bfloat16, true, false><<<cgrid, 128, 0, s>>>(x, Y, nullptr, nullptr, 0, T);

@@ -45,7 +45,6 @@ ornith_status launch_linear_prefill_tc(const LinArgs &x, int n_seq, int act_dtyp
 // stream waits for the last scan before the call returns.  front = nullptr: Y, rq and rk are complete already.
 struct TC5Front {
     std::function<ornith_status(int t_begin, int t_end, cudaStream_t)> conv;
-    std::function<ornith_status(cudaStream_t)> ring_refresh;
 };
 // conv_prefill_tma.cu: the conv + SiLU front of that path fed by tensor copies (see there)
 ornith_status launch_conv4_silu_prefill_tma(const LinArgs &x, int n_seq, int act_dtype, float *Y, float *rq, float *rk,
