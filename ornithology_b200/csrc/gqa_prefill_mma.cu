@@ -67,6 +67,7 @@ struct PrefillMmaArgs {
 // ---- decoded f16 image of every cached row the prefill can see: one warp per row -----------
 template <int MODE>
 __global__ void __launch_bounds__(128) k_kv_rows_to_f16(PrefillMmaArgs a) {
+    dependent_entry();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int pos = blockIdx.x * 4 + w, kvh = blockIdx.y, b = blockIdx.z, nkv = a.kv.nkv;
     const int64_t base = a.kv.seq_off[b];
@@ -326,12 +327,9 @@ ornith_status launch_gqa_prefill_mma(const KvView &kv, const int32_t *kv_len, co
     a.Kh = (__half *)kvh_scratch;
     a.Vh = (__half *)((char *)kvh_scratch + half_bytes);
     dim3 cgrid((a.Lp + 3) / 4, kv.nkv, n_seq);
-    switch (kv.mode) {
-    case ORNITH_KV_F32:       k_kv_rows_to_f16<ORNITH_KV_F32><<<cgrid, 128, 0, st>>>(a); break;
-    case ORNITH_KV_INT8_HEAD: k_kv_rows_to_f16<ORNITH_KV_INT8_HEAD><<<cgrid, 128, 0, st>>>(a); break;
-    default:                  k_kv_rows_to_f16<ORNITH_KV_Q8_0><<<cgrid, 128, 0, st>>>(a); break;
-    }
-    ORN_TRY(orn_check_launch("k_kv_rows_to_f16"));
+    auto rows = kv.mode == ORNITH_KV_F32 ? k_kv_rows_to_f16<ORNITH_KV_F32>
+                                         : kv.mode == ORNITH_KV_INT8_HEAD ? k_kv_rows_to_f16<ORNITH_KV_INT8_HEAD> : k_kv_rows_to_f16<ORNITH_KV_Q8_0>;
+    ORN_TRY(orn_check(orn_launch_dependent(rows, cgrid, dim3(128), 0, st, a), "k_kv_rows_to_f16"));
     if (!prefer_mma_sync() && ((uintptr_t)kvh_scratch % 16) == 0)
         return launch_gqa_prefill_tc(kv, kv_len, q_prep, a.Kh, a.Vh, (char *)kvh_scratch + 2 * half_bytes, qproj, out, nh,
                                      T, Lmax, a.Lp, gated, scale, n_seq, bf16_act, st);

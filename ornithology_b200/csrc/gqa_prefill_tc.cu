@@ -126,7 +126,8 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
     const int len0 = a.kv_len[b];
     // tokens that were really appended: the engine stops appending when the cache is full
     const int t_end = min(a.T, max(0, min(cap, a.Lmax) - len0));
-    if (q0 >= t_end) return;
+    // launched as a programmatic dependent of the kernel that writes its f16 images; every CTA waits for that one to end
+    if (q0 >= t_end) { asm volatile("griddepcontrol.wait;\n" ::: "memory"); return; }
     const int rows_here = min(BM, t_end - q0);
     const int kmax = len0 + q0 + rows_here - 1;                // last key any row of the CTA sees
     const int n_tiles = kmax / BN + 1;
@@ -145,6 +146,7 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
                      ::"r"(su32(&tmem_base_s)), "r"((uint32_t)TM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     fence_before();
     __syncthreads();
     fence_after();
@@ -437,12 +439,7 @@ ornith_status launch_gqa_prefill_tc(const KvView &kv, const int32_t *kv_len, con
     // K + V tile pair from L2 per 128 query rows: 137 GB per layer, 7.2 TB/s over the 148 SMs, and that traffic is the bound.
     const char *e = getenv("ORNITH_CUDA_PREFILL_SOFTMAX");
     const int nq = (e && e[0] == '4') ? 4 : 2;
-    if (nq == 4) {
-        if (bf16_act) k_gqa_prefill_tc<__nv_bfloat16, 4><<<grid, (4 * 4 + 6) * 32, SM_BYTES + 1024, st>>>(mq, mk, mv, a);
-        else          k_gqa_prefill_tc<float, 4><<<grid, (4 * 4 + 6) * 32, SM_BYTES + 1024, st>>>(mq, mk, mv, a);
-    } else {
-        if (bf16_act) k_gqa_prefill_tc<__nv_bfloat16, 2><<<grid, (4 * 2 + 6) * 32, SM_BYTES + 1024, st>>>(mq, mk, mv, a);
-        else          k_gqa_prefill_tc<float, 2><<<grid, (4 * 2 + 6) * 32, SM_BYTES + 1024, st>>>(mq, mk, mv, a);
-    }
-    return orn_check_launch("k_gqa_prefill_tc");
+    auto kernel = nq == 4 ? (bf16_act ? k_gqa_prefill_tc<__nv_bfloat16, 4> : k_gqa_prefill_tc<float, 4>)
+                          : (bf16_act ? k_gqa_prefill_tc<__nv_bfloat16, 2> : k_gqa_prefill_tc<float, 2>);
+    return orn_check(orn_launch_dependent(kernel, grid, dim3((unsigned)(4 * nq + 6) * 32), SM_BYTES + 1024, st, mq, mk, mv, a), "k_gqa_prefill_tc");
 }
