@@ -250,9 +250,14 @@ __device__ __forceinline__ void superblock_q80(smem_ptr wrow0, smem_ptr xs, int 
 // round is free and thread 0 refills as far ahead as the stages allow.  The kernel is launched as a programmatic
 // dependent of the quantiser: it starts the weight copies of its first stages at once and waits for the quantiser
 // (griddepcontrol.wait) only before the first copy of an activation image.
+//
+// CTAs per SM: one, with all of its shared memory, but two for Q8_0 where no super-block split needs the stages (KS = 1) and the
+// registers allow it (MT = 2).  A group of projections rarely has a multiple of 148 row tiles: 64 tokens of 2048 -> 12352
+// (193 tiles) 31 -> 25 us, of a shape with 128 tiles unchanged
 constexpr int NWARP = 16, MAX_STAGES = 16;
+template <int TYPE, int KS, int MT> constexpr int CTAS_PER_SM = TYPE == T_Q80 && KS == 1 && MT == 2 ? 2 : 1;
 template <int TYPE, int WR, int KS, int MT>
-__global__ void __launch_bounds__(NWARP * 32, 1) k_matmul_kq(KqArgs a, const __grid_constant__ KqGroup grp) {
+__global__ void __launch_bounds__(NWARP * 32, (CTAS_PER_SM<TYPE, KS, MT>)) k_matmul_kq(KqArgs a, const __grid_constant__ KqGroup grp) {
     constexpr int BLOCK = Fmt<TYPE>::BLOCK, BOX = Fmt<TYPE>::BOX, CTA_ROWS = 16 * WR, WBYTES = CTA_ROWS * BOX, TS = NWARP / (WR * KS);
     static_assert(WR * KS * TS == NWARP, "the warps split rows x super-blocks x token tiles");
     extern __shared__ unsigned char smem_raw[];
@@ -414,7 +419,7 @@ __global__ void __launch_bounds__(128) k_matmul_kq_plain(const unsigned char *W,
     else act_st((float *)a.y, (size_t)tok * a.n_out + row, total);
 }
 
-constexpr int SMEM_BUDGET = 200 * 1024;           // dynamic shared memory of one CTA (one CTA per SM: 512 threads)
+constexpr int SMEM_BUDGET = 200 * 1024;           // dynamic shared memory of the CTAs of an SM
 
 template <int TYPE, int WR, int KS, int MT>
 ornith_status launch_tc(const HostGroup &h, int n_in, int T, KqArgs a, cudaStream_t stream) {
@@ -426,7 +431,8 @@ ornith_status launch_tc(const HostGroup &h, int n_in, int T, KqArgs a, cudaStrea
     const int nt_max = (((T < PASS_TOK ? T : PASS_TOK) + 7) / 8 + MT - 1) / MT * MT;
     a.stage_bytes = (int)align_up((size_t)CTA_ROWS * Fmt<TYPE>::BOX + (size_t)nt_max * ORN_Q8K_IMG_BYTES, 128);
     const int terms = KS > 1 ? 2 * NWARP * 32 * MT * 4 * (int)sizeof(float) : 0;
-    int nstage = (SMEM_BUDGET - 128 - terms) / a.stage_bytes;
+    constexpr int BUDGET = CTAS_PER_SM<TYPE, KS, MT> == 1 ? SMEM_BUDGET : 110 * 1024;
+    int nstage = (BUDGET - 128 - terms) / a.stage_bytes;
     if (nstage > MAX_STAGES) nstage = MAX_STAGES;
     if (nstage > a.nseg) nstage = a.nseg;
     if (nstage < KS && nstage < a.nseg) {         // a round reads KS stages at once
