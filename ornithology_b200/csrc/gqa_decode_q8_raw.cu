@@ -224,6 +224,14 @@ __device__ __forceinline__ int block_scan128(int v, int *wt, int *total) {
     return incl + add;
 }
 
+// Range length: an equal share, but no shorter than this many tiles, by the longest context the call allows.  The last CTA
+// of a sequence merges its partials alone: more than 16 of them are not worth a range below 16 tiles (four per warp), nor
+// more than 32 a range below 1/32 of the context; below 8 tiles (two per warp) the fixed work of a piece is all there is.
+__host__ __device__ __forceinline__ int range_floor(int tiles) {
+    const int w16 = (tiles + 15) / 16, w32 = (tiles + 31) / 32, w = w16 < 8 ? 8 : (w16 > 16 ? 16 : w16);
+    return w > w32 ? w : w32;
+}
+
 // BALANCED = false: one CTA per (head group, split of tokens_per_split tokens, sequence); grid (groups, nsplit, n_seq).
 // BALANCED = true:  grid (groups, ranges).  The 16-token tiles of all sequences, laid end to end, are cut into
 //   gridDim.y ranges of equal length (found on the device from kv_len: the host never learns the contexts), and a
@@ -282,9 +290,7 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
             if (b0 == 0) { mine_n = n; mine_incl = incl; }           // kept for the search below when the batch is one pass
             total += t;
         }
-        // range length: an equal share, but no shorter than 16 tiles nor than 1/32 of the longest context the call
-        // allows (the last CTA of a sequence merges its partials alone; past ~32 of them that outweighs the gain)
-        const int floor_w = max(16, ((a.max_len + TILE - 1) / TILE + 31) / 32);
+        const int floor_w = range_floor((a.max_len + TILE - 1) / TILE);
         W = max((total + (int)gridDim.y - 1) / (int)gridDim.y, floor_w);
         pos = (int)blockIdx.y * W;
         range_end = min(total, pos + W);
@@ -603,13 +609,36 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
         // Partials of other SMs are read past L1.  Four partials' rows are in flight per thread at a time.
         const int h = tid >> 4, q = tid & 15;
         if (h < G) {
+            // the gate first: its loads, one per stored element, would each wait behind the store before (6 us of a merge)
+            const size_t head = (size_t)b * a.nh + (size_t)head0 + h;
+            float2 gate[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const size_t at = head * HD * 2 + HD + 2 * (q + 16 * k);
+                gate[k] = make_float2(0.0f, 0.0f);
+                if (a.gated)
+                    gate[k] = a.act_dtype == ORNITH_ACT_BF16
+                                  ? make_float2(act_ld((const __nv_bfloat16 *)a.qproj, at), act_ld((const __nv_bfloat16 *)a.qproj, at + 1))
+                                  : make_float2(act_ld((const float *)a.qproj, at), act_ld((const float *)a.qproj, at + 1));
+            }
             const unsigned hm = 0xffffu << (lane & 16);           // this half-warp (the other half may belong to no head)
             const float *ph = part_g + (size_t)slot0 * (HD + 2) + h * part_stride;   // first partial of head h
-            float M = -INFINITY;
-            for (int s = q; s < nlive; s += 16) {
+            const float2 ml0 = q < nlive ? __ldcg(reinterpret_cast<const float2 *>(ph + (size_t)q * (HD + 2))) : make_float2(0.0f, 0.0f);
+            float M = ml0.y > 0.0f ? ml0.x : -INFINITY;
+            for (int s = q + 16; s < nlive; s += 16) {
                 const float2 ml = __ldcg(reinterpret_cast<const float2 *>(ph + (size_t)s * (HD + 2)));
                 if (ml.y > 0.0f) M = fmaxf(M, ml.x);
             }
+            float2 v[4][8];                                           // four partials' rows; the first four do not wait for the maximum
+            auto load_rows = [&](int s) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const float2 *o2 = reinterpret_cast<const float2 *>(ph + (size_t)min(s + u, nlive - 1) * (HD + 2) + 2);
+#pragma unroll
+                    for (int k = 0; k < 8; k++) v[u][k] = __ldcg(o2 + q + 16 * k);           // dims 2 (q + 16 k), +1
+                }
+            };
+            load_rows(0);
 #pragma unroll
             for (int sft = 8; sft >= 1; sft >>= 1) M = fmaxf(M, __shfl_xor_sync(hm, M, sft, 16));
             float lsum = 0.0f;
@@ -618,20 +647,17 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
             for (int k = 0; k < 8; k++) acc[k] = make_float2(0.0f, 0.0f);
             for (int s0 = 0; s0 < nlive; s0 += 16) {
                 const int s = s0 + q;
-                const float2 ml = s < nlive ? __ldcg(reinterpret_cast<const float2 *>(ph + (size_t)s * (HD + 2))) : make_float2(0.0f, 0.0f);
+                const float2 ml = s0 == 0 ? ml0 : s < nlive ? __ldcg(reinterpret_cast<const float2 *>(ph + (size_t)s * (HD + 2))) : make_float2(0.0f, 0.0f);
                 const float w = (ml.y > 0.0f) ? expf(ml.x - M) : 0.0f;
                 lsum += ml.y * w;
                 const int n = min(16, nlive - s0);
                 for (int i0 = 0; i0 < n; i0 += 4) {
-                    float2 v[4][8];
                     float wi[4];
+                    if (s0 + i0 > 0) load_rows(s0 + i0);
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         wi[u] = __shfl_sync(hm, w, (i0 + u) & 15, 16);
                         if (i0 + u >= n) wi[u] = 0.0f;
-                        const float2 *o2 = reinterpret_cast<const float2 *>(ph + (size_t)(s0 + min(i0 + u, n - 1)) * (HD + 2) + 2);
-#pragma unroll
-                        for (int k = 0; k < 8; k++) v[u][k] = __ldcg(o2 + q + 16 * k);       // dims 2 (q + 16 k), +1
                     }
 #pragma unroll
                     for (int u = 0; u < 4; u++)
@@ -644,21 +670,14 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
 #pragma unroll
             for (int sft = 8; sft >= 1; sft >>= 1) lsum += __shfl_xor_sync(hm, lsum, sft, 16);
             const float inv = 1.0f / lsum;
-            const size_t head = (size_t)b * a.nh + (size_t)head0 + h;
 #pragma unroll
-            for (int k = 0; k < 8; k++)
-#pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int d = 2 * (q + 16 * k) + e;
-                    float o = (e ? acc[k].y : acc[k].x) * inv;
-                    if (a.act_dtype == ORNITH_ACT_BF16) {
-                        if (a.gated) o *= sigmoid_f(act_ld((const __nv_bfloat16 *)a.qproj, head * HD * 2 + HD + d));
-                        act_st((__nv_bfloat16 *)a.out, head * HD + d, o);
-                    } else {
-                        if (a.gated) o *= sigmoid_f(act_ld((const float *)a.qproj, head * HD * 2 + HD + d));
-                        act_st((float *)a.out, head * HD + d, o);
-                    }
-                }
+            for (int k = 0; k < 8; k++) {
+                float2 o = make_float2(acc[k].x * inv, acc[k].y * inv);
+                if (a.gated) { o.x *= sigmoid_f(gate[k].x); o.y *= sigmoid_f(gate[k].y); }
+                const size_t at = head * HD + 2 * (q + 16 * k);
+                if (a.act_dtype == ORNITH_ACT_BF16) { act_st((__nv_bfloat16 *)a.out, at, o.x); act_st((__nv_bfloat16 *)a.out, at + 1, o.y); }
+                else { act_st((float *)a.out, at, o.x); act_st((float *)a.out, at + 1, o.y); }
+            }
         }
     }
 }
@@ -700,7 +719,7 @@ bool q8_rows_map(CUtensorMap *m, const void *pool, int nkv) {
 // the batch is too small for ranges of at least floor_w tiles (same rule as in the kernel)
 static int balanced_ranges(int nkv, int nh, int n_seq, int max_len) {
     const int X = nkv * ((nh / nkv + 7) / 8);
-    const long long tiles = (max_len + TILE - 1) / TILE, floor_w = (tiles + 31) / 32 > 16 ? (tiles + 31) / 32 : 16;
+    const long long tiles = (max_len + TILE - 1) / TILE, floor_w = range_floor((int)tiles);
     const long long by_work = ((long long)n_seq * tiles + floor_w - 1) / floor_w, cap = 592 / X > 0 ? 592 / X : 1;
     return (int)(by_work < cap ? (by_work > 0 ? by_work : 1) : cap);
 }

@@ -440,3 +440,35 @@ def test_prefill_output_off_the_16_byte_grid(dtype, gated):
         got.append(out.clone())
         assert (buf[off + out.numel():] == 0).all() and (off == 0 or buf[0] == 0)
     assert torch.isfinite(got[0].float()).all() and (got[0] == got[1]).all()
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("lens", [(62,), (63,), (64,), (127, 128), (255, 256, 257), (511, 15, 512), (1100,), (2047, 40)])
+def test_short_context_splits(oracle, mode, lens):
+    """Contexts around the edges of the short splits (64 tokens and up) and of the short ranges of the Q8_0 schedule (8 to
+    16 tiles of 16): the last row of a split, the first of the next, sequences that end in an earlier split."""
+    import torch
+    from ornithology_b200 import device as D
+    layer = full_case(9)
+    dl = device_full(layer)
+    dm, om = _modes(mode)
+    B, top = len(lens), max(lens)
+    kv = D.KvBatch(dm, layer.nkv, layer.hd, [n + 2 for n in lens])
+    kvd = layer.nkv * layer.hd
+    rng = np.random.default_rng(sum(lens))
+    K = rng.standard_normal((B, top, kvd)).astype(np.float32)
+    V = rng.standard_normal((B, top, kvd)).astype(np.float32)
+    for b, n in enumerate(lens):                          # sequence by sequence: the append of the others is a full cache's no-op
+        at = torch.tensor([0 if i == b else lens[i] + 2 for i in range(B)], dtype=torch.int32, device="cuda")
+        k = torch.zeros(B, n, kvd, device="cuda"); k[b] = torch.from_numpy(K[b, :n]).cuda()
+        v = torch.zeros(B, n, kvd, device="cuda"); v[b] = torch.from_numpy(V[b, :n]).cuda()
+        D.kv_append(dl, kv, at, k, v, T=n)
+    kv_len = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    QP, K1, V1 = full_inputs(77, layer, B)
+    out = D.full_attn_step(dl, kv, kv_len, torch.from_numpy(QP).cuda(), torch.from_numpy(K1).cuda(), torch.from_numpy(V1).cuda()).cpu().numpy()
+    qp = np.zeros((top, QP.shape[1]), np.float32)
+    for b, n in enumerate(lens):
+        okv = oracle.kv(n + 2, layer.nkv, layer.hd, om)
+        oracle.full_attn_prefill(layer, okv, 0, qp[:n].copy(), K[b, :n].copy(), V[b, :n].copy())
+        ref = oracle.full_attn_step(layer, okv, n, QP[b], K1[b], V1[b])
+        assert rel_err(out[b], ref) < TOL, (b, n)
