@@ -90,9 +90,11 @@ bool fill_group(KqGroup *g, const HostGroup &h, int n_in, int cta_rows) {
     return true;
 }
 
-// Q4_K and Q6_K prompts on the tcgen05 tensor cores (kquant_prefill_tc5.cu): what the product would take there, in
-// microseconds per super-block, and how many units a CTA should own (0: too large for that kernel); and the launch
+// Prompts on the tcgen05 tensor cores (kquant_prefill_tc5.cu, q80_tc5.cu): what the product would take there, in
+// microseconds per super-block, and how many units of tokens a CTA should own (0: too large for that kernel); and the launch
 template <int TYPE> float kq_tc5_cost(const HostGroup &h, int T, int *units);
 template <int TYPE> ornith_status launch_kq_tc5(const HostGroup &h, int n_in, int T, const KqArgs &a, int units, cudaStream_t stream);
+template <> float kq_tc5_cost<T_Q80>(const HostGroup &h, int T, int *units);
+template <> ornith_status launch_kq_tc5<T_Q80>(const HostGroup &h, int n_in, int T, const KqArgs &a, int units, cudaStream_t stream);
 
 }  // namespace kq

@@ -252,8 +252,8 @@ __device__ __forceinline__ void superblock_q80(smem_ptr wrow0, smem_ptr xs, int 
 // (griddepcontrol.wait) only before the first copy of an activation image.
 //
 // CTAs per SM: one, with all of its shared memory, but two for Q8_0 where no super-block split needs the stages (KS = 1) and the
-// registers allow it (MT = 2).  A group of projections rarely has a multiple of 148 row tiles: 64 tokens of 2048 -> 12352
-// (193 tiles) 31 -> 25 us, of a shape with 128 tiles unchanged
+// registers allow it (MT = 2).  A group of projections rarely has a multiple of 148 row tiles:
+// with 193 of them the eight launches of a 35B group of four layers, 64 tokens, take 181 -> 173 us; shapes of 128 tiles are unchanged.
 constexpr int NWARP = 16, MAX_STAGES = 16;
 template <int TYPE, int KS, int MT> constexpr int CTAS_PER_SM = TYPE == T_Q80 && KS == 1 && MT == 2 ? 2 : 1;
 template <int TYPE, int WR, int KS, int MT>
@@ -489,24 +489,31 @@ ornith_status launch_kq(const HostGroup &h, int n_in, int T, KqArgs a, bool plai
     if (T > 64) {                                 // prompts: passes of 128 tokens; of 64 with fewer rows per CTA for a small matrix
         const long p128 = (T + 127) / 128, p64 = (T + 63) / 64, r64 = (n_out + 63) / 64;
         const int shape = r64 * p128 >= 100 ? 0 : r64 * p64 >= 100 ? 1 : (n_out + 31) / 32 * p64 >= 100 ? 2 : 3;
-        if constexpr (TYPE != T_Q80) {
-            // k-quants go to the tcgen05 kernel unless too few of its 128-row tiles exist to fill the GPU.  Microseconds per
-            // super-block and wave here, by shape: fits to 65 .. 777 tokens of 2048 -> 512, 4096 -> 2048, 2048 -> 8192, 8192 -> 4096.
-            // E.g. (mma.sync | tcgen05): Q6_K 8192 -> 4096, 777 tokens 339 | 112 us, 65 tokens 85 | 72; 4096 -> 2048, 100 tokens
-            // 28 | 42; Q4_K 8192 -> 4096, 777 tokens 247 | 168, 128 tokens 57 | 70.
-            static const float q4[4] = {2.1f, 1.7f, 0.95f, 0.95f}, q6[4] = {3.1f, 2.6f, 1.4f, 1.4f};
-            const long ctas = shape == 0 ? r64 * p128 : shape == 1 ? r64 * p64 : shape == 2 ? (n_out + 31) / 32 * p64 : (n_out + 15) / 16 * p64;
-            const float full = shape == 0 && T < 128 ? 0.6f + 0.4f * (float)T / 128.0f : 1.0f;       // a pass with missing tiles
-            int units;
-            const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
-            if (units && tc5 < (float)((ctas + 147) / 148) * full * (TYPE == T_Q4K ? q4 : q6)[shape])
-                return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
-        }
+        // The tcgen05 kernels, unless too few of their 128-row tiles exist to fill the GPU.  Microseconds per super-block and
+        // wave here, by shape: fits to 65 .. 777 tokens of 2048 -> 512, 4096 -> 2048, 2048 -> 8192, 8192 -> 4096.
+        // E.g. (mma.sync | tcgen05, us): Q6_K 8192 -> 4096, 777 tokens 339 | 112, 65 tokens 85 | 72; 4096 -> 2048, 100 tokens
+        // 28 | 42; Q4_K 8192 -> 4096, 777 tokens 247 | 168, 128 tokens 57 | 70; Q8_0 8192 -> 4096, 777 tokens 261 | 183, 128 tokens
+        // 56 | 63.
+        static const float per_sb[3][4] = {{2.1f, 1.7f, 0.95f, 0.95f}, {3.1f, 2.6f, 1.4f, 1.4f}, {2.3f, 1.55f, 0.95f, 0.95f}};   // T_Q4K, T_Q6K, T_Q80
+        const long ctas = shape == 0 ? r64 * p128 : shape == 1 ? r64 * p64 : shape == 2 ? (n_out + 31) / 32 * p64 : (n_out + 15) / 16 * p64;
+        const float full = shape == 0 && T < 128 ? 0.6f + 0.4f * (float)T / 128.0f : 1.0f;       // a pass with missing tiles
+        const float here = (float)((ctas + 147) / 148) * full * per_sb[TYPE][shape];
+        int units;
+        const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
+        if (units && tc5 < here) return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
         if (shape == 0) return launch_tc<TYPE, 4, 1, 4>(h, n_in, T, a, stream);
         if (shape == 1) return launch_tc<TYPE, 4, 1, 2>(h, n_in, T, a, stream);
         if (shape == 2) return launch_tc<TYPE, 2, 2, 2>(h, n_in, T, a, stream);
         return launch_tc<TYPE, 1, 4, 2>(h, n_in, T, a, stream);
     }
+    // 33-64 tokens of Q8_0: where the 64-row tiles of the kernel here make an uneven second wave and the 128-row ones do not
+    // (2048 -> 12352, 64 tokens: 25 -> 20 us; 2048 -> 8192 stays: 16 against 20)
+    if constexpr (TYPE == T_Q80)
+        if (T > 32 && n_out >= 64 * 100) {
+            int units;
+            const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
+            if (units && tc5 < 1.25f * (float)(((n_out + 63) / 64 + 147) / 148)) return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
+        }
     if (n_out >= 64 * 100) return launch_wr<TYPE, 4>(h, n_in, T, a, stream);
     if (n_out >= 32 * 100) return launch_wr<TYPE, 2>(h, n_in, T, a, stream);
     return launch_wr<TYPE, 1>(h, n_in, T, a, stream);

@@ -144,23 +144,25 @@ def test_integer_projection_is_bit_exact(oracle, monkeypatch, wtype, T, n_in, n_
             assert (plain.view(np.uint32) == ref.view(np.uint32)).all(), "plain kernel"
 
 
-# (type, tokens, n_in, n_out): units of 64 (Q4_K) or 128 (Q6_K) tokens and tiles of 128 rows, one past and one short of them;
-# one super-block, two, an odd number; 1 to 4 units per CTA, and more tiles than CTAs (both token orders of a row tile)
+# (type, tokens, n_in, n_out): units of 64 (Q4_K) or 128 (Q6_K) tokens, tiles of 64 or 128 tokens (Q8_0), and tiles of 128 rows,
+# one past and one short of them; one super-block, two, an odd number; 1 to 4 units per CTA, and more tiles than CTAs
 TC5_SHAPES = [("q4_k", 200, 256, 8200), ("q4_k", 129, 768, 8193), ("q4_k", 192, 512, 16000), ("q4_k", 193, 1280, 16001),
               ("q4_k", 256, 512, 16000), ("q4_k", 600, 512, 16070), ("q4_k", 1000, 256, 20000),
               ("q6_k", 65, 2048, 8192), ("q6_k", 128, 2048, 8200), ("q6_k", 257, 2048, 8193), ("q6_k", 300, 2048, 12300),
-              ("q6_k", 521, 2048, 12303), ("q6_k", 200, 4096, 4096)]
+              ("q6_k", 521, 2048, 12303), ("q6_k", 200, 4096, 4096),
+              ("q8_0", 33, 256, 12353), ("q8_0", 64, 768, 12800), ("q8_0", 65, 256, 12352), ("q8_0", 80, 512, 12300), ("q8_0", 129, 768, 8193),
+              ("q8_0", 400, 512, 4100), ("q8_0", 777, 256, 8200), ("q8_0", 1000, 512, 12000)]
 
 
 @pytest.mark.parametrize("wtype,T,n_in,n_out", TC5_SHAPES)
 def test_prompt_projection_on_tcgen05_is_bit_exact(oracle, monkeypatch, wtype, T, n_in, n_out):
-    """The kernel that prompts of Q4_K and Q6_K weights take, with random block bytes (every code, scale and minimum, so the
+    """The kernels that prompts take, with random block bytes (every code, scale and minimum, so the
     two int8 planes of code x scale reach both ends of their ranges), against the plain kernel bit for bit, and its first
     and last rows against the engine's integer path."""
     import torch
     from oracle import oracle as O
     from ornithology_b200 import device as D
-    wt = {"q4_k": O.GGML_Q4_K, "q6_k": O.GGML_Q6_K}[wtype]
+    wt = {"q4_k": O.GGML_Q4_K, "q6_k": O.GGML_Q6_K, "q8_0": O.GGML_Q8_0}[wtype]
     X = _acts(T, T, n_in)
     X[3, :256] = np.where(np.arange(256) % 2, 1.0, -1.0)              # codes at both ends
     W = _random_rows(3 * T + wt, wt, n_out, n_in)
