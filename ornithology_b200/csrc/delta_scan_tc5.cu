@@ -97,35 +97,46 @@ __device__ __forceinline__ void mma_tf32_sync(float (&d)[4], const float (&a)[4]
 }
 __device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
+// Multiply-adds in pairs (two per issued instruction, each rounded as a single one is): the preparation waits for its
+// shared-memory loads and dependent chains with two CTAs per SM, so every instruction it does not issue shows:
+// with the history spread over the grid, 6 prompts of 777 tokens, 35B, 264 -> 246 us in all, 267 tokens x 8, 397B, 222 -> 215.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float sum2(f32x2 v) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a + b; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
 // (I + L)^-1 of a 32x32 strictly lower block by forward substitution; lane = column.  Four partial sums per
 // row: the rows form one dependent chain, and a single accumulator would make it 496 multiply-adds long.
+// (L is stored with zeros on and above the diagonal, and a row not yet solved counts as zero.)
 __device__ __forceinline__ void inv_unit_lower(const float *Mb, int lane, float (&x)[32]) {
+    float nx[32];                                         // -x
+#pragma unroll
+    for (int i = 0; i < 32; i++) nx[i] = 0.0f;
 #pragma unroll
     for (int i = 0; i < 32; i++) {
-        float a0 = (i == lane) ? 1.0f : 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+        f32x2 a01 = pack2((i == lane) ? 1.0f : 0.0f, 0.0f), a23 = 0;
 #pragma unroll
         for (int l4 = 0; l4 < (i + 3) / 4; l4++) {
             const float4 m = *reinterpret_cast<const float4 *>(Mb + i * LDB + 4 * l4);
-            if (4 * l4 + 0 < i) a0 -= m.x * x[4 * l4 + 0];
-            if (4 * l4 + 1 < i) a1 -= m.y * x[4 * l4 + 1];
-            if (4 * l4 + 2 < i) a2 -= m.z * x[4 * l4 + 2];
-            if (4 * l4 + 3 < i) a3 -= m.w * x[4 * l4 + 3];
+            a01 = fma2(pack2(m.x, m.y), pack2(nx[4 * l4], nx[4 * l4 + 1]), a01);
+            if (4 * l4 + 2 < i) a23 = fma2(pack2(m.z, m.w), pack2(nx[4 * l4 + 2], nx[4 * l4 + 3]), a23);
         }
-        x[i] = (a0 + a1) + (a2 + a3);
+        x[i] = sum2(a01) + sum2(a23);
+        nx[i] = -x[i];
     }
 }
 // y[i] = sum_l B[row0 + i][l] x[l] for 16 rows of a 32x32 block in shared memory, x in registers
 __device__ __forceinline__ void block_matvec16(const float *B, int row0, const float (&x)[32], float (&y)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; i++) {
-        float a0 = 0.0f, a1 = 0.0f;
+        f32x2 a = 0;
 #pragma unroll
         for (int l4 = 0; l4 < 8; l4++) {
             const float4 m = *reinterpret_cast<const float4 *>(B + (row0 + i) * LDB + 4 * l4);
-            a0 = fmaf(m.x, x[4 * l4], a0); a1 = fmaf(m.y, x[4 * l4 + 1], a1);
-            a0 = fmaf(m.z, x[4 * l4 + 2], a0); a1 = fmaf(m.w, x[4 * l4 + 3], a1);
+            a = fma2(pack2(m.x, m.y), pack2(x[4 * l4], x[4 * l4 + 1]), a);
+            a = fma2(pack2(m.z, m.w), pack2(x[4 * l4 + 2], x[4 * l4 + 3]), a);
         }
-        y[i] = a0 + a1;
+        y[i] = sum2(a);
     }
 }
 
@@ -146,12 +157,18 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep64(LinArgs a, const float 
 
     // the conv has read the old history for the last time: store the last min(T, conv_k) inputs of the sequence (their own
     // launch took 2.4 us and a gap of a 512-token prompt's 72)
-    if (refresh && chunk == n_chunks - 1) {
-        const int pos0 = a.pos[b], K = a.conv_k;
+    if (refresh && chunk0 + (int)gridDim.x == n_chunks) {
+        const int pos0 = a.pos[b];
         float *ring = a.conv + (size_t)b * a.conv_stride;
         const ACT *X = (const ACT *)a.qkv + (size_t)b * a.T * Cc;
-        for (int ch = kh * 256 + tid; ch < Cc; ch += a.nk * 256)
-            for (int t = max(0, a.T - K); t < a.T; t++) ring[(size_t)((pos0 + t) % K) * Cc + ch] = act_ld(X, (size_t)t * Cc + ch);
+        for (int ch = ((int)blockIdx.x * a.nk + kh) * 256 + tid; ch < Cc; ch += (int)gridDim.x * a.nk * 256) {
+            float v[4];                                   // (conv_k is 4 on this path)
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = a.T - 4 + i >= 0 ? act_ld(X, (size_t)(a.T - 4 + i) * Cc + ch) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                if (a.T - 4 + i >= 0) ring[(size_t)((pos0 + a.T - 4 + i) & 3) * Cc + ch] = v[i];
+        }
     }
 
     for (int e = tid; e < C * 32; e += 256) {             // raw rows (tf32 values); rows past the end are zero
