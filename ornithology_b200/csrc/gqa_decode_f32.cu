@@ -86,9 +86,13 @@ __global__ void __launch_bounds__(128, 3) k_gqa_decode_f32_tc(DecodeArgs a) {
         return;
     }
     // ---- query group -> shared memory, tf32; rows of heads the group does not have are zero
-    for (int e = tid; e < 8 * HD; e += 128) {
-        const int h = e >> 8, d = e & 255;
-        Q_s[h * LDQ + d] = (h < G) ? tf32r(a.q_prep[((size_t)b * a.nh + (size_t)head0 + h) * HD + d]) : 0.0f;
+    {   // all 16 loads before the first store: one behind the other they were 5 us of a 22 us launch
+        float qv[16];
+        const float *q = a.q_prep + ((size_t)b * a.nh + (size_t)head0) * HD + tid;
+#pragma unroll
+        for (int i = 0; i < 16; i++) qv[i] = (i >> 1) < G ? q[i * 128] : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; i++) Q_s[(i >> 1) * LDQ + (i & 1) * 128 + tid] = tf32r(qv[i]);
     }
     // staging slots: zero once (skipped tail rows must stay finite), one mbarrier per slot
     for (int i = lane; i < WARP_BYTES / 16; i += 32) reinterpret_cast<uint4 *>(Kt)[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -182,7 +186,9 @@ __global__ void __launch_bounds__(128, 3) k_gqa_decode_f32_tc(DecodeArgs a) {
     }
     if (j == 0) { m_s[warp][g] = m_run; l_s[warp][g] = l_run; }
     __syncthreads();
-    for (int h = 0; h < G; h++) {
+#pragma unroll                                                        // the heads' loads and stores overlap
+    for (int h = 0; h < 8; h++) {
+        if (h >= G) break;
         float M = -INFINITY;
 #pragma unroll
         for (int w = 0; w < NWARP; w++) if (l_s[w][h] > 0.0f) M = fmaxf(M, m_s[w][h]);

@@ -338,7 +338,9 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_i8_raw(DecodeArgs a) {
         l_s[warp][2 * j] = lA; l_s[warp][2 * j + 1] = lB;
     }
     __syncthreads();
-    for (int h = 0; h < G; h++) {
+#pragma unroll                                                        // the heads' loads and stores overlap
+    for (int h = 0; h < 8; h++) {
+        if (h >= G) break;
         float M = -INFINITY;
 #pragma unroll
         for (int w = 0; w < NWARP; w++) if (l_s[w][h] > 0.0f) M = fmaxf(M, m_s[w][h]);
