@@ -17,6 +17,7 @@ struct DecodeArgs {
     void *out;
     int gated, act_dtype;
     int n_seq, max_len;                  // batch size and the call's bound on any context after the append
+    int range_floor;                     // balanced schedule: the fewest tiles of a range (gqa_decode_range_floor)
     int piece_cost;                      // balanced schedule: tiles charged per sequence for the fixed work of a piece
     unsigned int *status;                // device status word (a bounded wait that gave up sets ORN_WAIT_DECODE), or NULL
 };
@@ -34,7 +35,9 @@ ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a, int n_seq, cudaStrea
 // length found on the device instead of a grid of fixed splits), and then how many partial slots per head its
 // scratch needs: a.nsplit = gqa_decode_q8_raw_slots(...) and a.part laid out [head][slot][hd + 2].
 bool gqa_decode_q8_raw_balanced(const KvView &kv, int nh);
-int gqa_decode_q8_raw_slots(int nkv, int nh, int n_seq, int max_len);
+int gqa_decode_q8_raw_slots(int nkv, int nh, int n_seq, int max_len, int range_floor);
+// the fewest tiles of a range: the long ones need the fewest partials, the short ones spread small batches further
+int gqa_decode_range_floor(int max_len, bool short_ranges);
 
 // The same for int8-per-head rows (gqa_decode_i8_raw.cu), up to 8 query heads per KV head.
 bool gqa_decode_i8_raw_supported(const KvView &kv, int nh);

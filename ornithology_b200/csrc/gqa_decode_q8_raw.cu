@@ -224,14 +224,6 @@ __device__ __forceinline__ int block_scan128(int v, int *wt, int *total) {
     return incl + add;
 }
 
-// Range length: an equal share, but no shorter than this many tiles, by the longest context the call allows.  The last CTA
-// of a sequence merges its partials alone: more than 16 of them are not worth a range below 16 tiles (four per warp), nor
-// more than 32 a range below 1/32 of the context; below 8 tiles (two per warp) the fixed work of a piece is all there is.
-__host__ __device__ __forceinline__ int range_floor(int tiles) {
-    const int w16 = (tiles + 15) / 16, w32 = (tiles + 31) / 32, w = w16 < 8 ? 8 : (w16 > 16 ? 16 : w16);
-    return w > w32 ? w : w32;
-}
-
 // BALANCED = false: one CTA per (head group, split of tokens_per_split tokens, sequence); grid (groups, nsplit, n_seq).
 // BALANCED = true:  grid (groups, ranges).  The 16-token tiles of all sequences, laid end to end, are cut into
 //   gridDim.y ranges of equal length (found on the device from kv_len: the host never learns the contexts), and a
@@ -290,8 +282,8 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
             if (b0 == 0) { mine_n = n; mine_incl = incl; }           // kept for the search below when the batch is one pass
             total += t;
         }
-        const int floor_w = range_floor((a.max_len + TILE - 1) / TILE);
-        W = max((total + (int)gridDim.y - 1) / (int)gridDim.y, floor_w);
+        // range length: an equal share, but no shorter than the floor (see gqa_decode_range_floor)
+        W = max((total + (int)gridDim.y - 1) / (int)gridDim.y, a.range_floor);
         pos = (int)blockIdx.y * W;
         range_end = min(total, pos + W);
         if (pos >= total) { asm volatile("griddepcontrol.wait;\n" ::: "memory"); return; }
@@ -717,14 +709,23 @@ bool q8_rows_map(CUtensorMap *m, const void *pool, int nkv) {
 
 // ranges of the balanced schedule: one per resident CTA of a head-group column (4 CTAs on each of 148 SMs), fewer when
 // the batch is too small for ranges of at least floor_w tiles (same rule as in the kernel)
-static int balanced_ranges(int nkv, int nh, int n_seq, int max_len) {
+static int balanced_ranges(int nkv, int nh, int n_seq, int max_len, int floor_w) {
     const int X = nkv * ((nh / nkv + 7) / 8);
-    const long long tiles = (max_len + TILE - 1) / TILE, floor_w = range_floor((int)tiles);
+    const long long tiles = (max_len + TILE - 1) / TILE;
     const long long by_work = ((long long)n_seq * tiles + floor_w - 1) / floor_w, cap = 592 / X > 0 ? 592 / X : 1;
     return (int)(by_work < cap ? (by_work > 0 ? by_work : 1) : cap);
 }
-int gqa_decode_q8_raw_slots(int nkv, int nh, int n_seq, int max_len) {
-    return balanced_ranges(nkv, nh, n_seq, max_len) + n_seq;
+// By the longest context the call allows.  The last CTA of a sequence merges its partials alone: past ~32 of them that
+// outweighs the gain of a shorter range.  Short ranges: 16 tiles (four per warp) are halved while at most 16 partials
+// result; below 8 tiles (two per warp) the fixed work of a piece is all there is.  33 sequences of up to 115 tokens, 35B,
+// eight layers: 287 us at 16 tiles, 260 at 8.
+int gqa_decode_range_floor(int max_len, bool short_ranges) {
+    const int tiles = (max_len + TILE - 1) / TILE, w16 = (tiles + 15) / 16, w32 = (tiles + 31) / 32;
+    const int w = !short_ranges || w16 > 16 ? 16 : (w16 < 8 ? 8 : w16);
+    return w > w32 ? w : w32;
+}
+int gqa_decode_q8_raw_slots(int nkv, int nh, int n_seq, int max_len, int range_floor) {
+    return balanced_ranges(nkv, nh, n_seq, max_len, range_floor) + n_seq;
 }
 
 ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a_in, int n_seq, cudaStream_t st, bool *merged) {
@@ -757,7 +758,7 @@ ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a_in, int n_seq, cudaSt
     if (piece_cost < 0) { const char *e = getenv("ORNITH_CUDA_DECODE_PIECE_COST"); piece_cost = e ? atoi(e) : 4; if (piece_cost < 0 || piece_cost > 15) piece_cost = 4; }
     a.piece_cost = piece_cost;
     dim3 grid(X, a.nsplit, n_seq);
-    if (balanced) grid = dim3(X, balanced_ranges(a.kv.nkv, a.nh, n_seq, a.max_len), 1);
+    if (balanced) grid = dim3(X, balanced_ranges(a.kv.nkv, a.nh, n_seq, a.max_len, a.range_floor), 1);
     // may start while the append kernel in front of it still runs: it waits (griddepcontrol.wait) before it reads that kernel's output
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = dim3(128); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = st;

@@ -472,3 +472,35 @@ def test_short_context_splits(oracle, mode, lens):
         oracle.full_attn_prefill(layer, okv, 0, qp[:n].copy(), K[b, :n].copy(), V[b, :n].copy())
         ref = oracle.full_attn_step(layer, okv, n, QP[b], K1[b], V1[b])
         assert rel_err(out[b], ref) < TOL, (b, n)
+
+
+def test_scratch_of_the_long_ranges_is_still_enough():
+    """A Q8_0 step whose scratch holds the partials of 16-tile ranges but not of the shorter ones a small batch prefers runs
+    with the long ones; one partial less is refused."""
+    import ctypes as C
+    import torch
+    from ornithology_b200 import _lib, device as D
+    layer = full_case(9)
+    dl = device_full(layer)
+    B, n = 25, 70
+    kv = D.KvBatch(D.KV_Q8_0, layer.nkv, layer.hd, [n + 2] * B)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    kvd = layer.nkv * layer.hd
+    D.kv_append(dl, kv, torch.zeros(B, dtype=torch.int32, device="cuda"), rnd(B, n, kvd), rnd(B, n, kvd), T=n)
+    kv_len = torch.full((B,), n, dtype=torch.int32, device="cuda")
+    ins = [rnd(B, dl.qproj_width), rnd(B, kvd), rnd(B, kvd)]
+    ref = D.full_attn_step(dl, kv, kv_len, *ins, max_len=n + 2)
+    tiles, up = (n + 2 + 15) // 16, lambda b: (b + 255) // 256 * 256
+    slots = (B * tiles + 15) // 16 + B                    # ranges of 16 tiles, and one per sequence
+    need = up(B * layer.nh * layer.hd * 4) + up(B * layer.nh * 4) + up(layer.nh * slots * (layer.hd + 2) * 4)
+    scr = torch.empty(need, dtype=torch.uint8, device="cuda")
+    out = torch.empty_like(ref)
+    p = lambda t: C.c_void_p(t.data_ptr())
+
+    def step(nbytes):
+        return _lib.load().ornith_cuda_full_attn_step(C.byref(dl.c), C.byref(kv.c), p(kv_len), None, *[p(x) for x in ins], p(out), D.ACT_F32, n + 2,
+                                                      p(scr), nbytes, D._stream())
+    assert step(need) == 0
+    assert rel_err(out.cpu().numpy(), ref.cpu().numpy()) < 1e-3          # the same sums in another order, f16 operands
+    assert step(need - 256) != 0
