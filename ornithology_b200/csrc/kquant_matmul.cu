@@ -25,7 +25,8 @@
 //                8 minimums of a row as an unsigned A operand, the sums split into low (unsigned) and high (signed)
 //                bytes as two B operands: two more MMAs per tile instead of 32 multiply-adds per thread.
 //
-// Prompts are walked in passes of 128 tokens (grid.y; the weights are then re-read from L2).  Shapes the tensor copy
+// Prompts whose 128-row tiles fill the GPU go to the tcgen05 kernels (kquant_prefill_tc5.cu, q80_tc5.cu; the rule is in
+// launch_kq); the others are walked in passes of 128 tokens here (grid.y; the weights are then re-read from L2).  Shapes the tensor copy
 // cannot address (rows that do not start on 16-byte boundaries: Q6_K with n_in not a multiple of 2048) take a plain
 // kernel with the same arithmetic.
 #include <math.h>
