@@ -19,8 +19,8 @@
 // What bounds it: the issue slots of the workers.  A super-block of 128 rows x 256 tokens (Q6_K, H = 2) takes about 6100
 // cycles: 2000 to unpack, 2000 for each of two drains; its MMAs take 2048 of the tensor pipe.  More tokens per CTA would
 // share the unpacking further, but the totals already take half of the register file.
-// Measured (us, mma.sync kernel -> this one): Q6_K 4096 tokens 2048 -> 8192 821 -> 224, 777 tokens 4096 -> 20608 806 -> 288 and
-// 8192 -> 4096 339 -> 112; Q4_K 602 -> 328, 594 -> 367, 247 -> 168.
+// Measured (us, mma.sync kernel -> this one): Q6_K 4096 tokens 2048 -> 8192 821 -> 224, 777 tokens 4096 -> 20608 806 -> 283 and
+// 8192 -> 4096 339 -> 111; Q4_K 602 -> 326, 594 -> 360, 247 -> 167.
 // Tried: one weight stage (the copy's latency showed: 262 instead of 224 us); one tile per CTA instead of persistent CTAs (239);
 // 16 columns per tensor-memory load (spills); int32 -> float by exponent bias instead of the conversion (no faster).
 // The image of 8 tokens x 256 codes holds 8 x 16-byte core matrices in order, so it is a B operand as it lies (K-major,
@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
                 const Tile t = tile_of<NS, H>(grp, a.T, idx);
                 for (int s = 0; s < nseg; s++, n++) {
                     if (n >= 2) {                                     // the rows that had this stage are unpacked
-                        ok = tc5::mbar_wait(tc5::su32(&bars.w_free[n & 1]), (uint32_t)((n - 2) >> 1) & 1u);
+                        ok = tc5::mbar_wait_parked(tc5::su32(&bars.w_free[n & 1]), (uint32_t)((n - 2) >> 1) & 1u);
                         if (!ok) break;
                         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                     }
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
                 for (int s = 0; s < nseg && ok; s++)
                     for (int h = 0; h < t.nh; h++) {
                         if (round > 0) {                              // the unit that had this stage is drained
-                            ok = tc5::mbar_wait(tc5::su32(&bars.x_free[st]), (uint32_t)(round - 1) & 1u);
+                            ok = tc5::mbar_wait_parked(tc5::su32(&bars.x_free[st]), (uint32_t)(round - 1) & 1u);
                             if (!ok) break;
                             asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                         }
@@ -241,11 +241,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
             const Tile t = tile_of<NS, H>(grp, a.T, idx);
             const int n_last = (t.n_tok - (t.nh - 1) * NS + 15) & ~15;
             for (int s = 0; s < nseg && ok; s++, n_sb++) {
-                ok = tc5::mbar_wait(tc5::su32(&bars.a_full), (uint32_t)n_sb & 1u);
+                ok = tc5::mbar_wait_parked(tc5::su32(&bars.a_full), (uint32_t)n_sb & 1u);
                 for (int h = 0; h < t.nh && ok; h++, u++) {
                     const int slot = u & 1;
-                    ok = tc5::mbar_wait(tc5::su32(&bars.x_full[st]), (uint32_t)round & 1u);
-                    if (ok && u >= 2) ok = tc5::mbar_wait(tc5::su32(&bars.d_free[slot]), (uint32_t)((u >> 1) - 1) & 1u);
+                    ok = tc5::mbar_wait_parked(tc5::su32(&bars.x_full[st]), (uint32_t)round & 1u);
+                    if (ok && u >= 2) ok = tc5::mbar_wait_parked(tc5::su32(&bars.d_free[slot]), (uint32_t)((u >> 1) - 1) & 1u);
                     if (!ok) break;
                     tc5::fence_after();
                     const int n = h == t.nh - 1 ? n_last : NS;

@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
                 const Tile t = tile_of<NS, 1>(grp, a.T, idx);
                 for (int s = 0; s < nseg; s++, n++) {
                     if (n >= 2) {                                     // the rows that had this stage are unpacked
-                        ok = tc5::mbar_wait(tc5::su32(&bars.w_free[n & 1]), (uint32_t)((n - 2) >> 1) & 1u);
+                        ok = tc5::mbar_wait_parked(tc5::su32(&bars.w_free[n & 1]), (uint32_t)((n - 2) >> 1) & 1u);
                         if (!ok) break;
                         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                     }
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
                 const int nt = (t.n_tok + 7) / 8;
                 for (int s = 0; s < nseg; s++, n++) {
                     if (n >= 2) {                                     // the super-block that had this stage is drained
-                        ok = tc5::mbar_wait(tc5::su32(&bars.x_free[n & 1]), (uint32_t)((n - 2) >> 1) & 1u);
+                        ok = tc5::mbar_wait_parked(tc5::su32(&bars.x_free[n & 1]), (uint32_t)((n - 2) >> 1) & 1u);
                         if (!ok) break;
                         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
                     }
@@ -135,13 +135,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
                 const Tile t = tile_of<NS, 1>(grp, a.T, idx);
                 const uint32_t id = idesc_i8(true, (t.n_tok + 15) & ~15);
                 for (int s = 0; s < nseg && ok; s++, n++) {
-                    ok = tc5::mbar_wait(tc5::su32(&bars.a_full[n & 1]), (uint32_t)(n >> 1) & 1u) &&
+                    ok = tc5::mbar_wait_parked(tc5::su32(&bars.a_full[n & 1]), (uint32_t)(n >> 1) & 1u) &&
                          tc5::mbar_wait(tc5::su32(&bars.x_full[n & 1]), (uint32_t)(n >> 1) & 1u);
                     const uint64_t A = desc_plain(tc5::su32(smem + (n & 1) * PLANE), 128, QK * 8);
                     const uint64_t B = desc_plain(tc5::su32(smem + S::O_X + (n & 1) * S::XSTAGE), 128, S::XB);
                     for (int v = 0; v < U && ok; v++, u++) {
                         const int slot = u & 1;
-                        if (u >= 2) ok = tc5::mbar_wait(tc5::su32(&bars.d_free[slot]), (uint32_t)((u >> 1) - 1) & 1u);
+                        if (u >= 2) ok = tc5::mbar_wait_parked(tc5::su32(&bars.d_free[slot]), (uint32_t)((u >> 1) - 1) & 1u);
                         if (!ok) break;
                         tc5::fence_after();
 #pragma unroll
