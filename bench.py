@@ -478,7 +478,7 @@ def run_projections(dev, n_tok=64, cpu=True):
             D.matmul_q(w, None, out=op, image=ip, T=Tp)
     mp = graph_ms(prompt_pass)
     prompt = {"shape": "attn_qkv 2048 -> 8192, q8_0", "tokens": Tp, "us": mp * 1e3, "tops": 2.0 * Tp * 2048 * 8192 / (mp * 1e-3) / 1e12,
-              "note": "int8 mma.sync with int32 sums (exact); integer multiply-adds per sub-block scale share the issue slots"}
+              "note": "tcgen05 int8 products with int32 sums (exact), drained, scaled and added in f32 block by block"}
     out = {"workload": f"integer-path projections of one delta-net layer (Q8_0) and one full-attention layer (Q6_K), {n_tok} tokens, bf16",
            "per_layer": res, "per_projection": per, "prompt": prompt, "total_us": tot_ms * 1e3, "total_weight_bytes": tot_bytes,
            "launches": launches,
