@@ -31,9 +31,15 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
+# The current stream without a Stream object around it, where this build of torch has the two private functions for it.
+_raw_stream, _current_device = (getattr(torch._C, n, None) for n in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+
+
 def _stream():
-    """The current device's current stream, without building a Stream object around it."""
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    """The current device's current stream."""
+    if _raw_stream is None or _current_device is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 _ACTS = {torch.float32: ACT_F32, torch.bfloat16: ACT_BF16}

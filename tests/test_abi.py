@@ -64,6 +64,21 @@ def test_no_cpu_fallback_without_a_gpu(lib):
     attn.kv_free(c)
 
 
+def test_stream_of_a_torch_build_without_the_private_functions(monkeypatch):
+    """The stream handed to the library comes from two private functions of torch where they exist, else from the public call."""
+    import importlib.util
+    import types
+    import torch
+    import ornithology_b200
+    for name in ("_cuda_getCurrentRawStream", "_cuda_getDevice"):
+        monkeypatch.delattr(torch._C, name, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda *a: types.SimpleNamespace(cuda_stream=1234))
+    spec = importlib.util.spec_from_file_location("ornithology_b200._device_again", os.path.join(ornithology_b200.__path__[0], "device.py"))
+    again = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(again)
+    assert again._stream() == 1234
+
+
 def test_decode_scratch_follows_the_batch(lib):
     """Host-side sizing only (no GPU work).  The size query does not see the cache, so it covers both schedules:
     the grid of splits (finer splits, hence more partials per head, when the batch is too small to fill the GPU;
