@@ -38,6 +38,16 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm(
 // into one fused operation whatever their rounding is said to be (seen as last-bit differences), so the product is a fused
 // multiply-add onto -0, which the compiler does not know to be -0.
 __device__ __forceinline__ f32x2 mul2_apart(f32x2 a, f32x2 b, f32x2 minus_zero) { return fma2(a, b, minus_zero); }
+// Before a worker reads the activation scales of an image by plain loads: the barrier of the copy that wrote them, whose
+// completion makes them visible.  The image was complete before its products were issued, which this thread has seen done, so
+// one poll is enough; were it not there, the scales become NaN (of `tiles` x 8 tokens) and the status word says so.
+__device__ __forceinline__ void see_image(uint32_t x_full, uint32_t parity, unsigned char *scales, int tiles, int tile_bytes, unsigned int *status) {
+    if (tc5::mbar_try(x_full, parity)) return;
+#pragma unroll 1
+    for (int i = 0; i < 8 * tiles; i++) reinterpret_cast<float *>(scales + (i >> 3) * tile_bytes)[i & 7] = NAN;
+    tc5::report_timeout(status, ORN_WAIT_DECODE);
+}
+
 // A tile is 128 rows of one matrix x H NS tokens; persistent CTAs walk tiles blockIdx.x, + gridDim.x, .. with the token tiles of
 // the same rows next to one another (they share the weight bytes in L2).  Every role walks the same tiles with its counters
 // running on, so the copies and products of a tile start while the one before it is drained and stored.

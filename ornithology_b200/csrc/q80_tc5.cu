@@ -223,7 +223,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
                 }
                 if (!ok) break;
                 if (mine) {
-                    const unsigned char *xs = smem + S::O_X + (n & 1) * S::XSTAGE + cg * (COLS / 8) * S::XB + ORN_Q8K_IMG_D;
+                    unsigned char *xs = smem + S::O_X + (n & 1) * S::XSTAGE + cg * (COLS / 8) * S::XB + ORN_Q8K_IMG_D;
+                    see_image(tc5::su32(&bars.x_full[n & 1]), (uint32_t)(n >> 1) & 1u, xs, COLS / 8, S::XB, a.status);
 #pragma unroll
                     for (int i = 0; i < COLS / 2; i++) {
                         const float2 y = *reinterpret_cast<const float2 *>(xs + i / 4 * S::XB + (i & 3) * 8);

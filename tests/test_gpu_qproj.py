@@ -178,6 +178,28 @@ def test_prompt_projection_on_tcgen05_is_bit_exact(oracle, monkeypatch, wtype, T
         assert (np.ascontiguousarray(got[:, rows].cpu().numpy()).view(np.uint32) == ref.view(np.uint32)).all()
 
 
+@pytest.mark.parametrize("wtype,T,n_in,n_out", [("q4_k", 600, 1024, 20000), ("q6_k", 300, 2048, 20000), ("q8_0", 400, 1024, 20000)])
+def test_activation_scales_follow_their_image_stage(monkeypatch, wtype, T, n_in, n_out):
+    """The tcgen05 kernels keep two to five activation images in flight, and their workers read the scales out of an image by
+    plain loads.  Every (token, super-block) has a power of two of its own here and every CTA walks several tiles, so a scale
+    of the image that held the stage before is off by a factor; two inputs in turn, launch behind launch."""
+    import torch
+    from oracle import oracle as O
+    from ornithology_b200 import device as D
+    wt = {"q4_k": O.GGML_Q4_K, "q6_k": O.GGML_Q6_K, "q8_0": O.GGML_Q8_0}[wtype]
+    g = np.random.default_rng(T)
+    xs = []
+    for _ in range(2):
+        X = g.standard_normal((T, n_in // 256, 256)) * 2.0 ** g.integers(-20, 21, (T, n_in // 256, 1))
+        xs.append(torch.from_numpy(X.reshape(T, n_in).astype(np.float32)).cuda())
+    w = D.QWeight(wt, _random_rows(T, wt, n_out, n_in), n_in)
+    got = [D.matmul_q(w, xs[i & 1]) for i in range(6)]
+    monkeypatch.setenv("ORNITH_CUDA_PROJ_PLAIN", "1")
+    plain = [D.matmul_q(w, x) for x in xs]
+    for i, y in enumerate(got):
+        assert (y.view(torch.int32) == plain[i & 1].view(torch.int32)).all(), i
+
+
 def test_projections_sharing_one_image(oracle):
     """One quantisation of the input, three products against it (what the engine does for attn_qkv / attn_gate /
     ssm_alpha of a layer): each equals the integer path bit for bit."""
