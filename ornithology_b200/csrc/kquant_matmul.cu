@@ -252,9 +252,11 @@ __device__ __forceinline__ void superblock_q80(smem_ptr wrow0, smem_ptr xs, int 
 // dependent of the quantiser: it starts the weight copies of its first stages at once and waits for the quantiser
 // (griddepcontrol.wait) only before the first copy of an activation image.
 //
-// CTAs per SM: one, with all of its shared memory, but two for Q8_0 where no super-block split needs the stages (KS = 1) and the
-// registers allow it (MT = 2).  A group of projections rarely has a multiple of 148 row tiles:
-// with 193 of them the eight launches of a 35B group of four layers, 64 tokens, take 181 -> 173 us; shapes of 128 tiles are unchanged.
+// CTAs per SM: one, with all of its shared memory, but two for Q8_0 where no super-block split needs the stages (KS = 1), the
+// registers allow it (MT = 2) and the grid has more CTAs than the GPU has SMs.  A group of projections rarely has a multiple of
+// 148 row tiles: with 193 of them the eight launches of a 35B group of four layers, 64 tokens, take 181 -> 173 us.  With 148 CTAs or
+// fewer a second one on an SM only leaves another SM idle: quantiser and product of 2048 -> 8192, 64 tokens, 24.6 us paired, 16.8
+// alone; 8192 -> 4096, 100 tokens, 88.7 and 56.8.
 constexpr int NWARP = 16, MAX_STAGES = 16;
 template <int TYPE, int KS, int MT> constexpr int CTAS_PER_SM = TYPE == T_Q80 && KS == 1 && MT == 2 ? 2 : 1;
 template <int TYPE, int WR, int KS, int MT>
@@ -420,7 +422,10 @@ __global__ void __launch_bounds__(128) k_matmul_kq_plain(const unsigned char *W,
     else act_st((float *)a.y, (size_t)tok * a.n_out + row, total);
 }
 
-constexpr int SMEM_BUDGET = 200 * 1024;           // dynamic shared memory of the CTAs of an SM
+constexpr int SMS = 148;
+constexpr int SMEM_BUDGET = 200 * 1024;           // dynamic shared memory of a CTA that has an SM to itself
+constexpr int PAIR_BUDGET = 110 * 1024;           // of one of two
+constexpr int SOLO_SMEM = 116 * 1024;             // what leaves no room for a second one
 
 template <int TYPE, int WR, int KS, int MT>
 ornith_status launch_tc(const HostGroup &h, int n_in, int T, KqArgs a, cudaStream_t stream) {
@@ -432,8 +437,9 @@ ornith_status launch_tc(const HostGroup &h, int n_in, int T, KqArgs a, cudaStrea
     const int nt_max = (((T < PASS_TOK ? T : PASS_TOK) + 7) / 8 + MT - 1) / MT * MT;
     a.stage_bytes = (int)align_up((size_t)CTA_ROWS * Fmt<TYPE>::BOX + (size_t)nt_max * ORN_Q8K_IMG_BYTES, 128);
     const int terms = KS > 1 ? 2 * NWARP * 32 * MT * 4 * (int)sizeof(float) : 0;
-    constexpr int BUDGET = CTAS_PER_SM<TYPE, KS, MT> == 1 ? SMEM_BUDGET : 110 * 1024;
-    int nstage = (BUDGET - 128 - terms) / a.stage_bytes;
+    const long long ctas = (long long)g.cta0[h.n] * ((T + PASS_TOK - 1) / PASS_TOK);
+    const bool solo = CTAS_PER_SM<TYPE, KS, MT> == 1 || ctas <= SMS;
+    int nstage = ((solo ? SMEM_BUDGET : PAIR_BUDGET) - 128 - terms) / a.stage_bytes;
     if (nstage > MAX_STAGES) nstage = MAX_STAGES;
     if (nstage > a.nseg) nstage = a.nseg;
     if (nstage < KS && nstage < a.nseg) {         // a round reads KS stages at once
@@ -441,7 +447,7 @@ ornith_status launch_tc(const HostGroup &h, int n_in, int T, KqArgs a, cudaStrea
         return (ornith_status)ORNITH_ERR_BACKEND;
     }
     a.nstage = nstage;
-    const int smem = nstage * a.stage_bytes + terms + 128;
+    const int need = nstage * a.stage_bytes + terms + 128, smem = solo && need < SOLO_SMEM ? SOLO_SMEM : need;
     static bool opted[ORN_MAX_DEVICES] = {};
     bool &have = opted[orn_device_index()];
     if (!have) {
