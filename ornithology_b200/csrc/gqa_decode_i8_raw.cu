@@ -145,7 +145,6 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_i8_raw(DecodeArgs a) {
     __shared__ __align__(8) unsigned long long bars[NWARP][2];
     __shared__ int pipe_failed;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    dependent_entry();
     unsigned char *wbase = smem + QS_BYTES + warp * WARP_BYTES;
     uint2 *Q_s = reinterpret_cast<uint2 *>(smem);               // [k-step][lane]
     if (tid == 0) pipe_failed = 0;
@@ -380,5 +379,9 @@ ornith_status launch_gqa_decode_i8_raw(const DecodeArgs &a, int n_seq, cudaStrea
         configured = true;
     }
     dim3 grid(a.kv.nkv * ((a.nh / a.kv.nkv + 7) / 8), a.nsplit, n_seq);
-    return orn_check(orn_launch_dependent(k_gqa_decode_i8_raw, grid, dim3(128), SMEM_BYTES, st, a), "k_gqa_decode_i8_raw");
+    // Launched plainly, behind the append kernel's end, and not releasing the combine kernel early: CTAs that start while the
+    // append still runs land unevenly on the SMs (2 sequences x 16000, 35B, group of four layers: 57.3 us so, 53.4 plain), and
+    // a combine grid waiting beside them slows a full wave (9 x 16000: 100.0 us with both, 96.9 with the release alone, 91.7 plain).
+    k_gqa_decode_i8_raw<<<grid, 128, SMEM_BYTES, st>>>(a);
+    return orn_check_launch("k_gqa_decode_i8_raw");
 }
