@@ -715,7 +715,7 @@ static size_t step_need(const ornith_cuda_full_layer *l, int n_seq, int max_len,
     size_t rows = (size_t)n_seq * l->n_heads * nsplit;
     if (path != PATH_SPLIT_TC && l->n_kv_heads > 0 && l->n_heads % l->n_kv_heads == 0) {
         const size_t bal = (size_t)l->n_heads * gqa_decode_q8_raw_slots(l->n_kv_heads, l->n_heads, n_seq, max_len,
-                                                                         gqa_decode_range_floor(max_len, short_ranges));
+                                                                         gqa_decode_range_floor(l->n_kv_heads, l->n_heads, n_seq, max_len, short_ranges));
         rows = path == PATH_BALANCED ? bal : (bal > rows ? bal : rows);
     }
     return align_up((size_t)n_seq * l->n_heads * l->head_dim * sizeof(float), 256) +
@@ -827,7 +827,7 @@ ornith_status ornith_cuda_full_attn_step(const ornith_cuda_full_layer *l, const 
     d.nh = nh; d.scale = attn_scale(l);
     d.group_ctr = group_ctr; d.qproj = qproj; d.out = out; d.gated = l->gated; d.act_dtype = act_dtype;
     d.n_seq = B; d.max_len = max_len; d.status = nullptr; d.piece_cost = 0;
-    d.range_floor = gqa_decode_range_floor(max_len, short_ranges);
+    d.range_floor = path == PATH_BALANCED ? gqa_decode_range_floor(l->n_kv_heads, nh, B, max_len, short_ranges) : 0;
     bool merged = false;
     int nsplit_used;
     if (gqa_decode_q8_mma_supported(d.kv, nh) && !force_generic_decode()) {

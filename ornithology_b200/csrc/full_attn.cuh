@@ -37,7 +37,7 @@ ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a, int n_seq, cudaStrea
 bool gqa_decode_q8_raw_balanced(const KvView &kv, int nh);
 int gqa_decode_q8_raw_slots(int nkv, int nh, int n_seq, int max_len, int range_floor);
 // the fewest tiles of a range: the long ones need the fewest partials, the short ones spread small batches further
-int gqa_decode_range_floor(int max_len, bool short_ranges);
+int gqa_decode_range_floor(int nkv, int nh, int n_seq, int max_len, bool short_ranges);
 
 // The same for int8-per-head rows (gqa_decode_i8_raw.cu), up to 8 query heads per KV head.
 bool gqa_decode_i8_raw_supported(const KvView &kv, int nh);

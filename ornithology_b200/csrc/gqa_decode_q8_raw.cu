@@ -717,12 +717,15 @@ static int balanced_ranges(int nkv, int nh, int n_seq, int max_len, int floor_w)
 }
 // By the longest context the call allows.  The last CTA of a sequence merges its partials alone: past ~32 of them that
 // outweighs the gain of a shorter range.  Short ranges: 16 tiles (four per warp) are halved while at most 16 partials
-// result; below 8 tiles (two per warp) the fixed work of a piece is all there is.  33 sequences of up to 115 tokens, 35B,
-// eight layers: 287 us at 16 tiles, 260 at 8.
-int gqa_decode_range_floor(int max_len, bool short_ranges) {
-    const int tiles = (max_len + TILE - 1) / TILE, w16 = (tiles + 15) / 16, w32 = (tiles + 31) / 32;
-    const int w = !short_ranges || w16 > 16 ? 16 : (w16 < 8 ? 8 : w16);
-    return w > w32 ? w : w32;
+// result (below 8 tiles, two per warp, the fixed work of a piece is all there is), and only while the long ones give fewer
+// than 100 CTAs.  224 batches of 1 to 64 sequences of 25 to 3000 tokens, 35B, one group of four layers, time with long ranges /
+// with short ones by CTAs of the long form: below 40 1.08, 40 to 60 1.06, 60 to 100 1.04; from 100 up 0.997 to 1.013 in the
+// mean and single batches down to 0.92 (20 sequences of 3000: 107.5 us long, 113.7 short).
+int gqa_decode_range_floor(int nkv, int nh, int n_seq, int max_len, bool short_ranges) {
+    const int tiles = (max_len + TILE - 1) / TILE, w16 = (tiles + 15) / 16, w32 = (tiles + 31) / 32, w_long = w32 > 16 ? w32 : 16;
+    const int X = nkv * ((nh / nkv + 7) / 8);
+    if (!short_ranges || w16 > 16 || X * balanced_ranges(nkv, nh, n_seq, max_len, w_long) >= 100) return w_long;
+    return w16 < 8 ? 8 : w16;
 }
 int gqa_decode_q8_raw_slots(int nkv, int nh, int n_seq, int max_len, int range_floor) {
     return balanced_ranges(nkv, nh, n_seq, max_len, range_floor) + n_seq;

@@ -104,6 +104,12 @@ def test_decode_scratch_follows_the_batch(lib):
     # 8 sequences x 16k: 576-token splits -> 29, below the CUDA-core path's 33 -> 264 rows; balanced: 249 + 8
     assert abs(rows(8, 16448) - max(8 * 33, balanced(8, 16448))) < 0.1
     assert lib.ornith_cuda_full_attn_step_scratch(C.byref(layer), 0, 100) == 0
+    # the short ranges (8 tiles and up, at most 16 per sequence) of a batch whose 16-tile ranges give fewer than 100 CTAs
+    # (two head-group columns), and the 16-tile ranges of one that reaches them
+    for n_seq, max_len, floor_w in ((12, 864, 8), (64, 180, 8), (33, 180, 8), (33, 564, 16), (16, 1564, 16), (20, 3064, 16)):
+        ranges = lambda w: -(-n_seq * -(-max_len // 16) // w)
+        assert (2 * ranges(16) < 100) == (floor_w == 8)
+        assert abs(rows(n_seq, max_len) - (ranges(floor_w) + n_seq)) < 0.1, (n_seq, max_len)
 
 
 def test_product_does_not_touch_the_oracle():
