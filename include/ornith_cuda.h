@@ -473,6 +473,10 @@ typedef struct {
 } ornith_cuda_qproj;
 ornith_status ornith_cuda_matmul_q_group(const ornith_cuda_qproj *projs, int n, int n_in,
                                          const void *image, int T, int out_dtype, void *stream);
+/* Host only, no GPU needed: the tokens of a tile where a launch of these n matrices (rows of n_out[i] outputs, one type,
+ * 16-byte-aligned weights, n <= 8) runs on the tcgen05 kernels; 0 where another kernel serves it; -1 for arguments that
+ * have no integer path. */
+int ornith_cuda_matmul_q_tile_tokens(int wtype, int n_in, const int *n_out, int n, int T);
 
 /* ---- host-fed layer calls over device-resident state -------------------------
  * For an engine whose projections still run on the host: one object holds the state of all

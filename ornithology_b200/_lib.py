@@ -125,6 +125,7 @@ SYMBOLS = {
     "ornith_cuda_q8k_image": (_I, [vp, _I, _I, _I, vp, _SZ, vp]),
     "ornith_cuda_matmul_q_image": (_I, [_I, vp, _I, _I, vp, _I, vp, _I, vp]),
     "ornith_cuda_matmul_q_group": (_I, [vp, _I, _I, vp, _I, _I, vp]),
+    "ornith_cuda_matmul_q_tile_tokens": (_I, [_I, _I, vp, _I, _I]),
     "ornith_cuda_engine_new": (vp, [_I, _I, _I, _I, _I, _I, _I, _F, _F, _I, _I, _I, _I, _I]),
     "ornith_cuda_engine_free": (None, [vp]),
     "ornith_cuda_engine_full_layer": (_I, [vp, _I, vp, vp]),

@@ -90,6 +90,8 @@ bool fill_group(KqGroup *g, const HostGroup &h, int n_in, int cta_rows) {
     return true;
 }
 
+constexpr int TC5_UNIT[3] = {64, 128, 64};        // tokens of a unit of the tcgen05 kernels, by weight type
+
 // Prompts on the tcgen05 tensor cores (kquant_prefill_tc5.cu, q80_tc5.cu): what the product would take there, in
 // microseconds per super-block, and how many units of tokens a CTA should own (0: too large for that kernel); and the launch
 template <int TYPE> float kq_tc5_cost(const HostGroup &h, int T, int *units);

@@ -26,7 +26,7 @@
 //                bytes as two B operands: two more MMAs per tile instead of 32 multiply-adds per thread.
 //
 // Prompts whose 128-row tiles fill the GPU go to the tcgen05 kernels (kquant_prefill_tc5.cu, q80_tc5.cu; the rule is in
-// launch_kq); the others are walked in passes of 128 tokens here (grid.y; the weights are then re-read from L2).  Shapes the tensor copy
+// tc5_units); the others are walked in passes of 128 tokens here (grid.y; the weights are then re-read from L2).  Shapes the tensor copy
 // cannot address (rows that do not start on 16-byte boundaries: Q6_K with n_in not a multiple of 2048) take a plain
 // kernel with the same arithmetic.
 #include <math.h>
@@ -479,10 +479,47 @@ ornith_status launch_wr(const HostGroup &h, int n_in, int T, KqArgs a, cudaStrea
     return launch_tc<TYPE, WR, 4 / WR, 2>(h, n_in, T, a, stream);
 }
 
+// The mma.sync kernel's shape for a prompt (T > 64): passes of 128 tokens; of 64 with fewer rows per CTA for a small matrix
+int prompt_shape(int n_out, int T) {
+    const long p128 = (T + 127) / 128, p64 = (T + 63) / 64, r64 = (n_out + 63) / 64;
+    return r64 * p128 >= 100 ? 0 : r64 * p64 >= 100 ? 1 : (n_out + 31) / 32 * p64 >= 100 ? 2 : 3;
+}
+
+// Units of tokens per CTA on the tcgen05 kernels, or 0: the mma.sync kernel is the faster one.
+template <int TYPE>
+int tc5_units(const HostGroup &h, int T) {
+    const int n_out = h.rows_total();
+    int units = 0;
+    if (T > 64) {
+        // The tcgen05 kernels, unless too few of their 128-row tiles exist to fill the GPU.  Microseconds per super-block and
+        // wave here, by shape: fits to 65 .. 777 tokens of 2048 -> 512, 4096 -> 2048, 2048 -> 8192, 8192 -> 4096.
+        // E.g. (mma.sync | tcgen05, us): Q6_K 8192 -> 4096, 777 tokens 339 | 112, 65 tokens 85 | 72; 4096 -> 2048, 100 tokens
+        // 28 | 42; Q4_K 8192 -> 4096, 777 tokens 247 | 168, 128 tokens 57 | 70; Q8_0 8192 -> 4096, 777 tokens 261 | 183, 128 tokens
+        // 56 | 63.
+        static const float per_sb[3][4] = {{2.1f, 1.7f, 0.95f, 0.95f}, {3.1f, 2.6f, 1.4f, 1.4f}, {2.3f, 1.55f, 0.95f, 0.95f}};   // T_Q4K, T_Q6K, T_Q80
+        const long p128 = (T + 127) / 128, p64 = (T + 63) / 64, r64 = (n_out + 63) / 64;
+        const int shape = prompt_shape(n_out, T);
+        const long ctas = shape == 0 ? r64 * p128 : shape == 1 ? r64 * p64 : shape == 2 ? (n_out + 31) / 32 * p64 : (n_out + 15) / 16 * p64;
+        const float full = shape == 0 && T < 128 ? 0.6f + 0.4f * (float)T / 128.0f : 1.0f;       // a pass with missing tiles
+        const float here = (float)((ctas + 147) / 148) * full * per_sb[TYPE][shape];
+        const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
+        return tc5 < here ? units : 0;
+    }
+    // 33-64 tokens of Q8_0: where the 64-row tiles of the mma.sync kernel make an uneven second wave and the 128-row ones do not
+    // (2048 -> 12352, 64 tokens: 25 -> 20 us; 2048 -> 8192 stays: 16 against 20)
+    if constexpr (TYPE == T_Q80)
+        if (T > 32 && n_out >= 64 * 100) {
+            const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
+            return tc5 < 1.25f * (float)(((n_out + 63) / 64 + 147) / 148) ? units : 0;
+        }
+    return 0;
+}
+
+template <int TYPE> bool rows_aligned(int n_in) { return ((size_t)n_in / QK * Fmt<TYPE>::BLOCK & 15) == 0; }
+
 template <int TYPE>
 ornith_status launch_kq(const HostGroup &h, int n_in, int T, KqArgs a, bool plain, cudaStream_t stream) {
-    const size_t row_bytes = (size_t)n_in / QK * Fmt<TYPE>::BLOCK;
-    bool tc = !plain && (row_bytes & 15) == 0 && orn_tensor_map_encoder();
+    bool tc = !plain && rows_aligned<TYPE>(n_in) && orn_tensor_map_encoder();
     for (int i = 0; i < h.n; i++) tc = tc && ((uintptr_t)h.W[i] & 15) == 0;
     if (!tc) {                                    // the plain kernel, matrix by matrix
         for (int i = 0; i < h.n; i++) {
@@ -492,39 +529,22 @@ ornith_status launch_kq(const HostGroup &h, int n_in, int T, KqArgs a, bool plai
         }
         return ORNITH_OK;
     }
+    if (const int units = tc5_units<TYPE>(h, T)) return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
     const int n_out = h.rows_total();
-    if (T > 64) {                                 // prompts: passes of 128 tokens; of 64 with fewer rows per CTA for a small matrix
-        const long p128 = (T + 127) / 128, p64 = (T + 63) / 64, r64 = (n_out + 63) / 64;
-        const int shape = r64 * p128 >= 100 ? 0 : r64 * p64 >= 100 ? 1 : (n_out + 31) / 32 * p64 >= 100 ? 2 : 3;
-        // The tcgen05 kernels, unless too few of their 128-row tiles exist to fill the GPU.  Microseconds per super-block and
-        // wave here, by shape: fits to 65 .. 777 tokens of 2048 -> 512, 4096 -> 2048, 2048 -> 8192, 8192 -> 4096.
-        // E.g. (mma.sync | tcgen05, us): Q6_K 8192 -> 4096, 777 tokens 339 | 112, 65 tokens 85 | 72; 4096 -> 2048, 100 tokens
-        // 28 | 42; Q4_K 8192 -> 4096, 777 tokens 247 | 168, 128 tokens 57 | 70; Q8_0 8192 -> 4096, 777 tokens 261 | 183, 128 tokens
-        // 56 | 63.
-        static const float per_sb[3][4] = {{2.1f, 1.7f, 0.95f, 0.95f}, {3.1f, 2.6f, 1.4f, 1.4f}, {2.3f, 1.55f, 0.95f, 0.95f}};   // T_Q4K, T_Q6K, T_Q80
-        const long ctas = shape == 0 ? r64 * p128 : shape == 1 ? r64 * p64 : shape == 2 ? (n_out + 31) / 32 * p64 : (n_out + 15) / 16 * p64;
-        const float full = shape == 0 && T < 128 ? 0.6f + 0.4f * (float)T / 128.0f : 1.0f;       // a pass with missing tiles
-        const float here = (float)((ctas + 147) / 148) * full * per_sb[TYPE][shape];
-        int units;
-        const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
-        if (units && tc5 < here) return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
+    if (T > 64) {
+        const int shape = prompt_shape(n_out, T);
         if (shape == 0) return launch_tc<TYPE, 4, 1, 4>(h, n_in, T, a, stream);
         if (shape == 1) return launch_tc<TYPE, 4, 1, 2>(h, n_in, T, a, stream);
         if (shape == 2) return launch_tc<TYPE, 2, 2, 2>(h, n_in, T, a, stream);
         return launch_tc<TYPE, 1, 4, 2>(h, n_in, T, a, stream);
     }
-    // 33-64 tokens of Q8_0: where the 64-row tiles of the kernel here make an uneven second wave and the 128-row ones do not
-    // (2048 -> 12352, 64 tokens: 25 -> 20 us; 2048 -> 8192 stays: 16 against 20)
-    if constexpr (TYPE == T_Q80)
-        if (T > 32 && n_out >= 64 * 100) {
-            int units;
-            const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
-            if (units && tc5 < 1.25f * (float)(((n_out + 63) / 64 + 147) / 148)) return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
-        }
     if (n_out >= 64 * 100) return launch_wr<TYPE, 4>(h, n_in, T, a, stream);
     if (n_out >= 32 * 100) return launch_wr<TYPE, 2>(h, n_in, T, a, stream);
     return launch_wr<TYPE, 1>(h, n_in, T, a, stream);
 }
+
+template <int TYPE>
+int tile_tokens(const HostGroup &h, int n_in, int T) { return rows_aligned<TYPE>(n_in) ? TC5_UNIT[TYPE] * tc5_units<TYPE>(h, T) : 0; }
 
 ornith_status run_group(int wtype, const HostGroup &h, int n_in, const void *image, int T, int out_dtype, cudaStream_t s) {
     KqArgs a;
@@ -548,6 +568,20 @@ size_t ornith_cuda_matmul_q_scratch(int wtype, int T, int n_in) {
 }
 
 static bool kq_type_ok(int wtype) { return wtype == ORNITH_GGML_Q4_K || wtype == ORNITH_GGML_Q6_K || wtype == ORNITH_GGML_Q8_0; }
+
+// Host only: which kernel the products of a group take, for the tests of the dispatch
+int ornith_cuda_matmul_q_tile_tokens(int wtype, int n_in, const int *n_out, int n, int T) {
+    if (!kq_type_ok(wtype) || n_in <= 0 || n_in % QK || !n_out || n <= 0 || n > MAX_GROUP || T <= 0) return -1;
+    HostGroup h;
+    h.n = n;
+    for (int i = 0; i < n; i++) {
+        if (n_out[i] <= 0) return -1;
+        h.W[i] = nullptr; h.y[i] = nullptr; h.n_out[i] = n_out[i];
+    }
+    if (wtype == ORNITH_GGML_Q4_K) return tile_tokens<T_Q4K>(h, n_in, T);
+    if (wtype == ORNITH_GGML_Q6_K) return tile_tokens<T_Q6K>(h, n_in, T);
+    return tile_tokens<T_Q80>(h, n_in, T);
+}
 
 ornith_status ornith_cuda_q8k_image(const void *x, int act_dtype, int T, int n_in, void *image, size_t image_bytes, void *stream) {
     ORN_TRY(orn_require_device());

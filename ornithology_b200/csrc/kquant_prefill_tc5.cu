@@ -36,8 +36,8 @@ using namespace kq_tc5;
 
 template <int TYPE> struct Tc5Fmt;
 // NS tokens per unit; two slots of NACC accumulators of NS columns fill the 512 columns
-template <> struct Tc5Fmt<T_Q6K> { static constexpr int NACC = 2, NS = 128, XB = ORN_Q8K_IMG_LO, AMIN = 0; };
-template <> struct Tc5Fmt<T_Q4K> { static constexpr int NACC = 4, NS = 64, XB = ORN_Q8K_IMG_BYTES, AMIN = ROWS * 32; };
+template <> struct Tc5Fmt<T_Q6K> { static constexpr int NACC = 2, NS = TC5_UNIT[T_Q6K], XB = ORN_Q8K_IMG_LO, AMIN = 0; };
+template <> struct Tc5Fmt<T_Q4K> { static constexpr int NACC = 4, NS = TC5_UNIT[T_Q4K], XB = ORN_Q8K_IMG_BYTES, AMIN = ROWS * 32; };
 
 template <int TYPE, int H> struct Tc5Smem {       // byte offsets; every part a multiple of 128
     using F = Tc5Fmt<TYPE>;

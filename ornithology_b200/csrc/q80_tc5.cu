@@ -276,7 +276,7 @@ ornith_status launch_ns(const HostGroup &h, int n_in, int T, const KqArgs &a, cu
 
 namespace kq {
 
-// units: tokens of a tile / 64.  Microseconds per super-block and wave, from 8192 -> 4096: 1.9 for 64 tokens, 3.2 for 128.
+// units: tokens of a tile / TC5_UNIT.  Microseconds per super-block and wave, from 8192 -> 4096: 1.9 for 64 tokens, 3.2 for 128.
 template <>
 float kq_tc5_cost<T_Q80>(const HostGroup &h, int T, int *units) {
     long long row_tiles = 0;
@@ -290,7 +290,7 @@ float kq_tc5_cost<T_Q80>(const HostGroup &h, int T, int *units) {
 }
 template <>
 ornith_status launch_kq_tc5<T_Q80>(const HostGroup &h, int n_in, int T, const KqArgs &a, int units, cudaStream_t stream) {
-    return units == 1 ? launch_ns<64>(h, n_in, T, a, stream) : launch_ns<128>(h, n_in, T, a, stream);
+    return units == 1 ? launch_ns<TC5_UNIT[T_Q80]>(h, n_in, T, a, stream) : launch_ns<2 * TC5_UNIT[T_Q80]>(h, n_in, T, a, stream);
 }
 
 }  // namespace kq

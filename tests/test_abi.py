@@ -138,6 +138,16 @@ def test_projection_sizing_and_no_gpu_behaviour(lib):
     assert lib.ornith_cuda_matmul_q_scratch(8, 8, 300) == 0
     assert lib.ornith_cuda_matmul_q_scratch(8, 0, 2048) == 0
     assert C.sizeof(_lib.CudaQproj) == 32 and _lib.CudaQproj.n_out.offset == 16 and _lib.CudaQproj.y.offset == 24
+    # the dispatch of prompts, host only: the tile of every case that the GPU tests send to the tcgen05 kernels, each instantiation
+    # of them among these, and shapes that stay with the other kernels
+    from tests.test_gpu_qproj import TC5_CASES, tile_tokens
+    for wtype, T, n_in, n_outs, tile in TC5_CASES:
+        assert tile_tokens(wtype, n_in, n_outs, T) == tile, (wtype, T, n_in, n_outs)
+    for wtype, tiles in (("q4_k", {64, 128, 192, 256}), ("q6_k", {128, 256}), ("q8_0", {64, 128})):
+        assert {c[4] for c in TC5_CASES if c[0] == wtype} == tiles == {c[4] for c in TC5_CASES if c[0] == wtype and len(c[3]) > 1}
+    for wtype, T, n_in, n_outs in (("q4_k", 64, 512, [16000]), ("q6_k", 300, 2304, [12300]), ("q6_k", 100, 4096, [2048]), ("q8_0", 64, 2048, [8192])):
+        assert tile_tokens(wtype, n_in, n_outs, T) == 0
+    assert tile_tokens("q8_0", 300, [64], 100) == -1 and tile_tokens("q8_0", 512, [64, 0], 100) == -1
     if not torch.cuda.is_available():
         p = _lib.CudaQproj(8, None, 64, None)
         assert lib.ornith_cuda_matmul_q_group(C.byref(p), 1, 2048, None, 4, 0, None) != 0

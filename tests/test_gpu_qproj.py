@@ -144,38 +144,50 @@ def test_integer_projection_is_bit_exact(oracle, monkeypatch, wtype, T, n_in, n_
             assert (plain.view(np.uint32) == ref.view(np.uint32)).all(), "plain kernel"
 
 
-# (type, tokens, n_in, n_out): units of 64 (Q4_K) or 128 (Q6_K) tokens, tiles of 64 or 128 tokens (Q8_0), and tiles of 128 rows,
-# one past and one short of them; one super-block, two, an odd number; 1 to 4 units per CTA, and more tiles than CTAs
-TC5_SHAPES = [("q4_k", 200, 256, 8200), ("q4_k", 129, 768, 8193), ("q4_k", 192, 512, 16000), ("q4_k", 193, 1280, 16001),
-              ("q4_k", 256, 512, 16000), ("q4_k", 600, 512, 16070), ("q4_k", 1000, 256, 20000),
-              ("q6_k", 65, 2048, 8192), ("q6_k", 128, 2048, 8200), ("q6_k", 257, 2048, 8193), ("q6_k", 300, 2048, 12300),
-              ("q6_k", 521, 2048, 12303), ("q6_k", 200, 4096, 4096),
-              ("q8_0", 33, 256, 12353), ("q8_0", 64, 768, 12800), ("q8_0", 65, 256, 12352), ("q8_0", 80, 512, 12300), ("q8_0", 129, 768, 8193),
-              ("q8_0", 400, 512, 4100), ("q8_0", 777, 256, 8200), ("q8_0", 1000, 512, 12000)]
+# (type, tokens, n_in, rows of the matrices, tokens of a tile): tiles of 64 to 256 tokens (Q4_K: 1 to 4 units of 64; Q6_K: 1 and 2 of 128;
+# Q8_0: 64 and 128), one past and one short of them; row counts around multiples of 128; one super-block, two, an odd number; more
+# tiles than CTAs; groups whose matrices end inside a tile of rows.  tests/test_abi.py pins the tiles without a GPU.
+TC5_CASES = [("q4_k", 200, 256, (8200,), 128), ("q4_k", 129, 768, (8193,), 128), ("q4_k", 192, 512, (16000,), 192), ("q4_k", 193, 1280, (16001,), 256),
+             ("q4_k", 256, 512, (16000,), 256), ("q4_k", 600, 512, (16070,), 128), ("q4_k", 1000, 256, (20000,), 256), ("q4_k", 129, 256, (19000,), 64),
+             ("q6_k", 65, 2048, (8192,), 128), ("q6_k", 128, 2048, (8200,), 128), ("q6_k", 257, 2048, (8193,), 256), ("q6_k", 300, 2048, (12300,), 128),
+             ("q6_k", 521, 2048, (12303,), 256), ("q6_k", 200, 4096, (4096,), 128),
+             ("q8_0", 33, 256, (12353,), 64), ("q8_0", 64, 768, (12800,), 64), ("q8_0", 65, 256, (12352,), 128), ("q8_0", 80, 512, (12300,), 128),
+             ("q8_0", 129, 768, (8193,), 128), ("q8_0", 400, 512, (4100,), 128), ("q8_0", 777, 256, (8200,), 64), ("q8_0", 1000, 512, (12000,), 128),
+             ("q4_k", 129, 256, (19000, 130, 4097, 32), 64), ("q4_k", 600, 512, (12000, 4070, 1, 127), 128), ("q4_k", 192, 512, (16000, 40, 90), 192),
+             ("q4_k", 200, 256, (8200, 32, 129, 4100), 256), ("q6_k", 128, 2048, (8200, 40, 513), 128), ("q6_k", 257, 2048, (8193, 40, 513), 256),
+             ("q8_0", 64, 512, (8192, 4096, 32, 32), 64), ("q8_0", 129, 768, (8193, 100, 40), 128), ("q8_0", 400, 512, (4100, 513, 1), 64)]
+WTYPES = {"q8_0": 8, "q4_k": 12, "q6_k": 14}
 
 
-@pytest.mark.parametrize("wtype,T,n_in,n_out", TC5_SHAPES)
-def test_prompt_projection_on_tcgen05_is_bit_exact(oracle, monkeypatch, wtype, T, n_in, n_out):
+def tile_tokens(wtype, n_in, n_outs, T):
+    """Tokens of a tile of this launch on the tcgen05 kernels, 0 where another kernel serves it (host only)."""
+    from ornithology_b200 import _lib
+    rows = np.array(n_outs, np.int32)
+    return _lib.load().ornith_cuda_matmul_q_tile_tokens(WTYPES[wtype], n_in, rows.ctypes.data, len(n_outs), T)
+
+
+@pytest.mark.parametrize("wtype,T,n_in,n_outs,tile", TC5_CASES)
+def test_prompt_projection_on_tcgen05_is_bit_exact(oracle, monkeypatch, wtype, T, n_in, n_outs, tile):
     """The kernels that prompts take, with random block bytes (every code, scale and minimum, so the
-    two int8 planes of code x scale reach both ends of their ranges), against the plain kernel bit for bit, and its first
-    and last rows against the engine's integer path."""
+    two int8 planes of code x scale reach both ends of their ranges), against the plain kernel bit for bit, and the first
+    and last rows of every matrix against the engine's integer path; f32 and bf16 outputs."""
     import torch
-    from oracle import oracle as O
     from ornithology_b200 import device as D
-    wt = {"q4_k": O.GGML_Q4_K, "q6_k": O.GGML_Q6_K, "q8_0": O.GGML_Q8_0}[wtype]
+    assert tile_tokens(wtype, n_in, n_outs, T) == tile
+    wt = WTYPES[wtype]
     X = _acts(T, T, n_in)
     X[3, :256] = np.where(np.arange(256) % 2, 1.0, -1.0)              # codes at both ends
-    W = _random_rows(3 * T + wt, wt, n_out, n_in)
-    w, x = D.QWeight(wt, W, n_in), torch.from_numpy(X).cuda()
-    got = D.matmul_q(w, x)
-    gotb = D.matmul_q(w, x, out=torch.empty(T, n_out, dtype=torch.bfloat16, device="cuda"))
+    Ws = [_random_rows(3 * T + wt + 5 * i, wt, n, n_in) for i, n in enumerate(n_outs)]
+    ws, image = [D.QWeight(wt, W, n_in) for W in Ws], D.q8k_image(torch.from_numpy(X).cuda(), n_in)
+    got, gotb = D.matmul_q_group(ws, image, T), D.matmul_q_group(ws, image, T, out_dtype=torch.bfloat16)
     monkeypatch.setenv("ORNITH_CUDA_PROJ_PLAIN", "1")
-    plain = D.matmul_q(w, x)
-    assert (got.view(torch.int32) == plain.view(torch.int32)).all()
-    assert (gotb == plain.to(torch.bfloat16)).all()
-    for rows in (slice(0, 8), slice(n_out - 8, n_out)):
-        ref = oracle.matmul_q(wt, np.ascontiguousarray(W[rows]), n_in, X)
-        assert (np.ascontiguousarray(got[:, rows].cpu().numpy()).view(np.uint32) == ref.view(np.uint32)).all()
+    for W, w, y, yb in zip(Ws, ws, got, gotb):
+        plain = D.matmul_q(w, None, image=image, T=T)
+        assert (y.view(torch.int32) == plain.view(torch.int32)).all()
+        assert (yb == plain.to(torch.bfloat16)).all()
+        for rows in (slice(0, 8), slice(max(0, w.n_out - 8), w.n_out)):
+            ref = oracle.matmul_q(wt, np.ascontiguousarray(W[rows]), n_in, X)
+            assert (np.ascontiguousarray(y[:, rows].cpu().numpy()).view(np.uint32) == ref.view(np.uint32)).all()
 
 
 @pytest.mark.parametrize("wtype,T,n_in,n_out", [("q4_k", 600, 1024, 20000), ("q6_k", 300, 2048, 20000), ("q8_0", 400, 1024, 20000)])
