@@ -38,14 +38,13 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm(
 // into one fused operation whatever their rounding is said to be (seen as last-bit differences), so the product is a fused
 // multiply-add onto -0, which the compiler does not know to be -0.
 __device__ __forceinline__ f32x2 mul2_apart(f32x2 a, f32x2 b, f32x2 minus_zero) { return fma2(a, b, minus_zero); }
-// Before a worker reads the activation scales of an image by plain loads: the barrier of the copy that wrote them, whose
-// completion makes them visible.  The image was complete before its products were issued, which this thread has seen done, so
-// one poll is enough; were it not there, the scales become NaN (of `tiles` x 8 tokens) and the status word says so.
-__device__ __forceinline__ void see_image(uint32_t x_full, uint32_t parity, unsigned char *scales, int tiles, int tile_bytes, unsigned int *status) {
-    if (tc5::mbar_try(x_full, parity)) return;
-#pragma unroll 1
-    for (int i = 0; i < 8 * tiles; i++) reinterpret_cast<float *>(scales + (i >> 3) * tile_bytes)[i & 7] = NAN;
-    tc5::report_timeout(status, ORN_WAIT_DECODE);
+// The products of a unit are issued: one arrival when they are complete, and one of the issuing lane itself.  The lane has seen
+// the unit's image arrive (the completion of a bulk copy makes it visible to whoever observes it), so its own arrival, a release,
+// passes the image on to the workers, which acquire this barrier before they read the activation scales by plain loads.
+constexpr int MMA_DONE_ARRIVALS = 2;
+__device__ __forceinline__ void mma_issued(uint32_t mma_done) {
+    tc5::mbar_arrive(mma_done);
+    tc5::mma_commit(mma_done);
 }
 
 // A tile is 128 rows of one matrix x H NS tokens; persistent CTAs walk tiles blockIdx.x, + gridDim.x, .. with the token tiles of

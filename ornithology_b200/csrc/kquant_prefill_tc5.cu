@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
         for (int i = 0; i < 2; i++) {
             tc5::mbar_init(tc5::su32(&bars.w_full[i]), 1);
             tc5::mbar_init(tc5::su32(&bars.w_free[i]), NWORK);
-            tc5::mbar_init(tc5::su32(&bars.mma_done[i]), 1);
+            tc5::mbar_init(tc5::su32(&bars.mma_done[i]), MMA_DONE_ARRIVALS);
             tc5::mbar_init(tc5::su32(&bars.d_free[i]), NWORK);
         }
         for (int i = 0; i < S::NX; i++) {
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
                         mma_i8_ss(d + 2 * NS, a_min, desc_plain(xu + ORN_Q8K_IMG_LO, 128, F::XB), idesc_i8(false, n), 0);
                         mma_i8_ss(d + 3 * NS, a_min, desc_plain(xu + ORN_Q8K_IMG_HI, 128, F::XB), id, 0);
                     }
-                    tc5::mma_commit(tc5::su32(&bars.mma_done[slot]));
+                    mma_issued(tc5::su32(&bars.mma_done[slot]));
                     if (++st == S::NX) { st = 0; round++; }
                 }
             }
@@ -280,18 +280,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
             if (ok) ok = __all_sync(0xffffffffu, tc5::mbar_wait(tc5::su32(bar), parity));
         };
         const f32x2 mz = pack2(a.minus_zero, a.minus_zero);
-        unsigned du = 0;                                              // number of the next unit to drain; its image is in stage du % NX
+        int st = 0, du = 0;                                           // image stage and number of the next unit to drain
         auto drain = [&](auto HI, int n, int n_tok) {                 // a unit of super-block n (counted over all tiles)
             constexpr int h = decltype(HI)::value;
-            const unsigned slot = du & 1, round = du / S::NX, st = du - round * S::NX;
-            wait_all(&bars.mma_done[slot], (du >> 1) & 1u);
+            const int slot = du & 1;
+            wait_all(&bars.mma_done[slot], (uint32_t)(du >> 1) & 1u);
             if (!ok) return;
             tc5::fence_after();
             if (h * NS + cg * COLS < n_tok) {
                 const float *sc = scales + (n & 3) * (S::NSCALE * ROWS) + q * 32 + lane;
                 const f32x2 dw = pack2(sc[0], sc[0]), dmw = F::AMIN ? pack2(-sc[ROWS], -sc[ROWS]) : 0;      // (-yd) dmw = yd (-dmw)
-                unsigned char *xu = smem + S::O_X + st * S::XUNIT + cg * (COLS / 8) * F::XB + ORN_Q8K_IMG_D;
-                see_image(tc5::su32(&bars.x_full[st]), round & 1u, xu, COLS / 8, F::XB, a.status);
+                const unsigned char *xu = smem + S::O_X + st * S::XUNIT + cg * (COLS / 8) * F::XB + ORN_Q8K_IMG_D;
                 const uint32_t t0 = tq + slot * (F::NACC * NS);
 #pragma unroll
                 for (int c = 0; c < COLS; c += 8) {                   // 8 columns = one image tile (16 at a time spill registers)
@@ -321,6 +320,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
                 tc5::mbar_arrive(tc5::su32(&bars.d_free[slot]));
                 tc5::mbar_arrive(tc5::su32(&bars.x_free[st]));
             }
+            if (++st == S::NX) st = 0;
             du++;
         };
         auto drain_last = [&](int n, int n_tok) {                     // the last unit of super-block n, which is one of a tile of n_tok tokens
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
 #pragma unroll
                 for (int i = 0; i < COLS / 2; i++) tot[h][i] = 0;
             for (int s = 0; s < nseg; s++, n++) {
-                if (s > 0) wait_all(&bars.mma_done[du & 1], (du >> 1) & 1u);       // the planes are free: the last unit of n - 1 is multiplied
+                if (s > 0) wait_all(&bars.mma_done[du & 1], (uint32_t)(du >> 1) & 1u);       // the planes are free: the last unit of n - 1 is multiplied
                 wait_all(&bars.w_full[n & 1], (uint32_t)(n >> 1) & 1u);
                 if (!ok) break;
                 const int row = warp * 8 + g;

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
             tc5::mbar_init(tc5::su32(&bars.a_full[i]), NWORK);
             tc5::mbar_init(tc5::su32(&bars.x_full[i]), 1);
             tc5::mbar_init(tc5::su32(&bars.x_free[i]), NWORK);
-            tc5::mbar_init(tc5::su32(&bars.mma_done[i]), 1);
+            tc5::mbar_init(tc5::su32(&bars.mma_done[i]), MMA_DONE_ARRIVALS);
             tc5::mbar_init(tc5::su32(&bars.d_free[i]), NWORK);
         }
         tc5::mbar_init_fence();
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
 #pragma unroll
                         for (int i = 0; i < BU; i++)                  // a block is two core matrices along K: 256 bytes
                             mma_i8_ss(tmem + slot * 256 + i * NS, A + 16 * (v * BU + i), B + 16 * (v * BU + i), id, 0);
-                        tc5::mma_commit(tc5::su32(&bars.mma_done[slot]));
+                        mma_issued(tc5::su32(&bars.mma_done[slot]));
                     }
                 }
             }
@@ -223,8 +223,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
                 }
                 if (!ok) break;
                 if (mine) {
-                    unsigned char *xs = smem + S::O_X + (n & 1) * S::XSTAGE + cg * (COLS / 8) * S::XB + ORN_Q8K_IMG_D;
-                    see_image(tc5::su32(&bars.x_full[n & 1]), (uint32_t)(n >> 1) & 1u, xs, COLS / 8, S::XB, a.status);
+                    const unsigned char *xs = smem + S::O_X + (n & 1) * S::XSTAGE + cg * (COLS / 8) * S::XB + ORN_Q8K_IMG_D;
 #pragma unroll
                     for (int i = 0; i < COLS / 2; i++) {
                         const float2 y = *reinterpret_cast<const float2 *>(xs + i / 4 * S::XB + (i & 3) * 8);
