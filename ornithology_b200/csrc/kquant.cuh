@@ -91,6 +91,7 @@ bool fill_group(KqGroup *g, const HostGroup &h, int n_in, int cta_rows) {
 }
 
 constexpr int TC5_UNIT[3] = {64, 128, 64};        // tokens of a unit of the tcgen05 kernels, by weight type
+constexpr float TC5_START[3] = {2.4f, 3.5f, 2.6f};   // microseconds that a launch of them takes beside its super-blocks
 
 // Prompts on the tcgen05 tensor cores (kquant_prefill_tc5.cu, q80_tc5.cu): what the product would take there, in
 // microseconds per super-block, and how many units of tokens a CTA should own (0: too large for that kernel); and the launch

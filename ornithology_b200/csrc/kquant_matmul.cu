@@ -487,23 +487,25 @@ int prompt_shape(int n_out, int T) {
 
 // Units of tokens per CTA on the tcgen05 kernels, or 0: the mma.sync kernel is the faster one.
 template <int TYPE>
-int tc5_units(const HostGroup &h, int T) {
+int tc5_units(const HostGroup &h, int nseg, int T) {
     const int n_out = h.rows_total();
     int units = 0;
     if (T > 64) {
-        // The tcgen05 kernels, unless too few of their 128-row tiles exist to fill the GPU.  Microseconds per super-block and
-        // wave here, by shape: fits to 65 .. 777 tokens of 2048 -> 512, 4096 -> 2048, 2048 -> 8192, 8192 -> 4096.
-        // E.g. (mma.sync | tcgen05, us): Q6_K 8192 -> 4096, 777 tokens 339 | 112, 65 tokens 85 | 72; 4096 -> 2048, 100 tokens
-        // 28 | 42; Q4_K 8192 -> 4096, 777 tokens 247 | 168, 128 tokens 57 | 70; Q8_0 8192 -> 4096, 777 tokens 261 | 183, 128 tokens
-        // 56 | 63.
-        static const float per_sb[3][4] = {{2.1f, 1.7f, 0.95f, 0.95f}, {3.1f, 2.6f, 1.4f, 1.4f}, {2.3f, 1.55f, 0.95f, 0.95f}};   // T_Q4K, T_Q6K, T_Q80
-        const long p128 = (T + 127) / 128, p64 = (T + 63) / 64, r64 = (n_out + 63) / 64;
-        const int shape = prompt_shape(n_out, T);
-        const long ctas = shape == 0 ? r64 * p128 : shape == 1 ? r64 * p64 : shape == 2 ? (n_out + 31) / 32 * p64 : (n_out + 15) / 16 * p64;
-        const float full = shape == 0 && T < 128 ? 0.6f + 0.4f * (float)T / 128.0f : 1.0f;       // a pass with missing tiles
-        const float here = (float)((ctas + 147) / 148) * full * per_sb[TYPE][shape];
+        // The tcgen05 kernels, unless too few of their 128-row tiles exist to fill the GPU or too few super-blocks to pay for
+        // their start.  Microseconds per super-block and wave here, by shape, fitted with theirs (kq_tc5_cost) to 16 matrices from
+        // 2048 -> 32 to 4096 -> 20608 and 13 token counts from 65 to 2048.  A last wave that holds nothing but CTAs of the last
+        // pass costs what that pass's tokens cost, not a whole wave; a pass of the first shape walks its tokens 32 at a time.
+        // E.g. (mma.sync | tcgen05, us): Q6_K 8192 -> 4096, 777 tokens 339 | 112, 65 tokens 87 | 70; 2048 -> 1024, 129 tokens
+        // 17 | 24; Q4_K 8192 -> 4096, 777 tokens 247 | 168, 128 tokens 58 | 67; Q8_0 8192 -> 4096, 777 tokens 261 | 183, 128 tokens
+        // 58 | 65; 256 -> 8192, 128 tokens 6.6 | 7.4.
+        static const float per_sb[3][4] = {{2.6f, 1.7f, 0.95f, 0.95f}, {3.6f, 2.65f, 1.62f, 1.2f}, {2.75f, 1.7f, 0.95f, 0.95f}};   // T_Q4K, T_Q6K, T_Q80
+        const int shape = prompt_shape(n_out, T), pass = shape == 0 ? 128 : 64, cta_rows = shape == 3 ? 16 : shape == 2 ? 32 : 64;
+        const long rows = (n_out + cta_rows - 1) / cta_rows, passes = (T + pass - 1) / pass, ctas = rows * passes, rest = ctas % 148;
+        float waves = (float)((ctas + 147) / 148);
+        if (passes > 1 && ctas > 148 && rest > 0 && rest <= rows) waves += 0.45f + 0.42f * (float)(T - (passes - 1) * pass) / (float)pass - 1.0f;
+        if (shape == 0 && T < 128) waves *= 0.25f * (float)((T + 31) / 32);
         const float tc5 = kq_tc5_cost<TYPE>(h, T, &units);
-        return tc5 < here ? units : 0;
+        return tc5 + TC5_START[TYPE] / (float)nseg < waves * per_sb[TYPE][shape] ? units : 0;
     }
     // 33-64 tokens of Q8_0: where the 64-row tiles of the mma.sync kernel make an uneven second wave and the 128-row ones do not
     // (2048 -> 12352, 64 tokens: 25 -> 20 us; 2048 -> 8192 stays: 16 against 20)
@@ -529,7 +531,7 @@ ornith_status launch_kq(const HostGroup &h, int n_in, int T, KqArgs a, bool plai
         }
         return ORNITH_OK;
     }
-    if (const int units = tc5_units<TYPE>(h, T)) return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
+    if (const int units = tc5_units<TYPE>(h, a.nseg, T)) return launch_kq_tc5<TYPE>(h, n_in, T, a, units, stream);
     const int n_out = h.rows_total();
     if (T > 64) {
         const int shape = prompt_shape(n_out, T);
@@ -544,7 +546,7 @@ ornith_status launch_kq(const HostGroup &h, int n_in, int T, KqArgs a, bool plai
 }
 
 template <int TYPE>
-int tile_tokens(const HostGroup &h, int n_in, int T) { return rows_aligned<TYPE>(n_in) ? TC5_UNIT[TYPE] * tc5_units<TYPE>(h, T) : 0; }
+int tile_tokens(const HostGroup &h, int n_in, int T) { return rows_aligned<TYPE>(n_in) ? TC5_UNIT[TYPE] * tc5_units<TYPE>(h, n_in / QK, T) : 0; }
 
 ornith_status run_group(int wtype, const HostGroup &h, int n_in, const void *image, int T, int out_dtype, cudaStream_t s) {
     KqArgs a;

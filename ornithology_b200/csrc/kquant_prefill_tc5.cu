@@ -421,7 +421,7 @@ float kq_tc5_cost(const HostGroup &h, int T, int *units) {
     if (row_tiles * ((T + NS - 1) / NS) > (1 << 30)) return best;
     for (int H = 1; H <= HMAX; H++) {
         const long long tiles = row_tiles * ((T + H * NS - 1) / (H * NS));
-        const float cost = (float)((tiles + SMS - 1) / SMS * (1 + H)) * (TYPE == T_Q6K ? 1.15f : 0.98f);
+        const float cost = (float)((tiles + SMS - 1) / SMS * (1 + H)) * (TYPE == T_Q6K ? 1.10f : 0.98f);
         if (*units == 0 || cost < best) { *units = H; best = cost; }
     }
     return best;

@@ -145,7 +145,8 @@ def test_projection_sizing_and_no_gpu_behaviour(lib):
         assert tile_tokens(wtype, n_in, n_outs, T) == tile, (wtype, T, n_in, n_outs)
     for wtype, tiles in (("q4_k", {64, 128, 192, 256}), ("q6_k", {128, 256}), ("q8_0", {64, 128})):
         assert {c[4] for c in TC5_CASES if c[0] == wtype} == tiles == {c[4] for c in TC5_CASES if c[0] == wtype and len(c[3]) > 1}
-    for wtype, T, n_in, n_outs in (("q4_k", 64, 512, [16000]), ("q6_k", 300, 2304, [12300]), ("q6_k", 100, 4096, [2048]), ("q8_0", 64, 2048, [8192])):
+    for wtype, T, n_in, n_outs in (("q4_k", 64, 512, [16000]), ("q6_k", 300, 2304, [12300]), ("q6_k", 100, 4096, [2048]), ("q8_0", 64, 2048, [8192]),
+                                   ("q6_k", 300, 2048, [512]), ("q6_k", 129, 2048, [1024]), ("q8_0", 128, 256, [8192]), ("q8_0", 80, 2048, [8192])):
         assert tile_tokens(wtype, n_in, n_outs, T) == 0
     assert tile_tokens("q8_0", 300, [64], 100) == -1 and tile_tokens("q8_0", 512, [64, 0], 100) == -1
     if not torch.cuda.is_available():

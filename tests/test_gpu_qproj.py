@@ -147,15 +147,15 @@ def test_integer_projection_is_bit_exact(oracle, monkeypatch, wtype, T, n_in, n_
 # (type, tokens, n_in, rows of the matrices, tokens of a tile): tiles of 64 to 256 tokens (Q4_K: 1 to 4 units of 64; Q6_K: 1 and 2 of 128;
 # Q8_0: 64 and 128), one past and one short of them; row counts around multiples of 128; one super-block, two, an odd number; more
 # tiles than CTAs; groups whose matrices end inside a tile of rows.  tests/test_abi.py pins the tiles without a GPU.
-TC5_CASES = [("q4_k", 200, 256, (8200,), 128), ("q4_k", 129, 768, (8193,), 128), ("q4_k", 192, 512, (16000,), 192), ("q4_k", 193, 1280, (16001,), 256),
+TC5_CASES = [("q4_k", 400, 256, (8200,), 256), ("q4_k", 129, 768, (8193,), 128), ("q4_k", 192, 512, (16000,), 192), ("q4_k", 193, 1280, (16001,), 256),
              ("q4_k", 256, 512, (16000,), 256), ("q4_k", 600, 512, (16070,), 128), ("q4_k", 1000, 256, (20000,), 256), ("q4_k", 129, 256, (19000,), 64),
              ("q6_k", 65, 2048, (8192,), 128), ("q6_k", 128, 2048, (8200,), 128), ("q6_k", 257, 2048, (8193,), 256), ("q6_k", 300, 2048, (12300,), 128),
              ("q6_k", 521, 2048, (12303,), 256), ("q6_k", 200, 4096, (4096,), 128),
-             ("q8_0", 33, 256, (12353,), 64), ("q8_0", 64, 768, (12800,), 64), ("q8_0", 65, 256, (12352,), 128), ("q8_0", 80, 512, (12300,), 128),
-             ("q8_0", 129, 768, (8193,), 128), ("q8_0", 400, 512, (4100,), 128), ("q8_0", 777, 256, (8200,), 64), ("q8_0", 1000, 512, (12000,), 128),
+             ("q8_0", 33, 256, (12353,), 64), ("q8_0", 64, 768, (12800,), 64), ("q8_0", 65, 1024, (12352,), 128), ("q8_0", 100, 768, (12300,), 128),
+             ("q8_0", 129, 1280, (8193,), 128), ("q8_0", 400, 512, (4100,), 128), ("q8_0", 777, 256, (8200,), 64), ("q8_0", 1000, 512, (12000,), 128),
              ("q4_k", 129, 256, (19000, 130, 4097, 32), 64), ("q4_k", 600, 512, (12000, 4070, 1, 127), 128), ("q4_k", 192, 512, (16000, 40, 90), 192),
-             ("q4_k", 200, 256, (8200, 32, 129, 4100), 256), ("q6_k", 128, 2048, (8200, 40, 513), 128), ("q6_k", 257, 2048, (8193, 40, 513), 256),
-             ("q8_0", 64, 512, (8192, 4096, 32, 32), 64), ("q8_0", 129, 768, (8193, 100, 40), 128), ("q8_0", 400, 512, (4100, 513, 1), 64)]
+             ("q4_k", 200, 768, (8200, 32, 129, 4100), 256), ("q6_k", 128, 2048, (8200, 40, 513), 128), ("q6_k", 257, 2048, (8193, 40, 513), 256),
+             ("q8_0", 64, 512, (8192, 4096, 32, 32), 64), ("q8_0", 129, 1280, (8193, 100, 40), 128), ("q8_0", 400, 512, (4100, 513, 1), 64)]
 WTYPES = {"q8_0": 8, "q4_k": 12, "q6_k": 14}
 
 
