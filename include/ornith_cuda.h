@@ -446,7 +446,8 @@ ornith_status ornith_cuda_matmul_q8_0(const void *W, int n_in, int n_out, const 
  * n_in/256 super-blocks (144 / 210 / 272 bytes); wtype: the GGUF type id.  Rows that start on 16-byte
  * boundaries (always for Q4_K and Q8_0; Q6_K when n_in is a multiple of 2048) and a 16-byte-aligned W take the
  * tensor-core kernel, any other shape a plain kernel with the same result.  scratch: 256-byte aligned,
- * ornith_cuda_matmul_q_scratch bytes.  Any T: a prompt is walked in passes of 128 tokens inside one launch. */
+ * ornith_cuda_matmul_q_scratch bytes.  Any T, one launch: prompts whose tiles of 128 rows fill the GPU run on the
+ * tcgen05 tensor cores (tiles of 64 to 256 tokens), others in passes of 64 or 128 tokens on mma.sync. */
 enum { ORNITH_GGML_Q8_0 = 8, ORNITH_GGML_Q4_K = 12, ORNITH_GGML_Q6_K = 14 };   /* src/ornith_gguf.h:24-30 */
 size_t ornith_cuda_matmul_q_scratch(int wtype, int T, int n_in);
 ornith_status ornith_cuda_matmul_q(int wtype, const void *W, int n_in, int n_out, const void *x,

@@ -76,9 +76,21 @@ __device__ __forceinline__ float ex2_fast(float x) { float y; asm("ex2.approx.ft
 __device__ __forceinline__ float rcp_fast(float x) { float y; asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
 __device__ __forceinline__ float silu_fast(float x) { return x * rcp_fast(1.0f + ex2_fast(-1.4426950408889634f * x)); }
 
-// What every kernel of a decode step does first: wait for the kernel in front (whose results it reads and whose inputs it may
-// overwrite), then let the one behind it take its place on the SMs.  A step of one chat is a dozen kernels of a few
-// microseconds; without this each pays its launch latency after the end of the one before.
+// ---- pairs of f32: two operations per issued instruction, each rounded as a single one is
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpack2(f32x2 v, float *a, float *b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(*a), "=f"(*b) : "l"(v)); }
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) { f32x2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
+// What most kernels of the chains do first: wait for the kernel in front (whose results they read and whose inputs they may
+// overwrite), then let the one behind take its place on the SMs.  A step of one chat is a dozen kernels of a few
+// microseconds; without this each pays its launch latency after the end of the one before.  Not so, on purpose:
+// k_gqa_decode_q8_raw and k_linear_decode_ring release the kernel behind them at once (it must wait before all else) and
+// wait themselves only before they read what the kernel in front wrote; k_conv4_silu_prefill_tma, itself launched plainly,
+// releases at once too; the projection kernels, the tcgen05 scan and the tcgen05 GQA prefill wait only where they first touch
+// such data and release nothing before their end; the f32 and int8 decode kernels are launched plainly.
 __device__ __forceinline__ void dependent_entry() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");

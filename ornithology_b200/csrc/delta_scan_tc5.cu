@@ -99,11 +99,8 @@ __device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 6
 
 // Multiply-adds in pairs (two per issued instruction, each rounded as a single one is): the preparation waits for its
 // shared-memory loads and dependent chains with two CTAs per SM, so every instruction it does not issue shows:
-// with the history spread over the grid, 6 prompts of 777 tokens, 35B, 264 -> 246 us in all, 267 tokens x 8, 397B, 222 -> 215.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ float sum2(f32x2 v) { float a, b; asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); return a + b; }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+// 6 prompts of 777 tokens, 35B, 252 -> 246 us.
+__device__ __forceinline__ float sum2(f32x2 v) { float a, b; unpack2(v, &a, &b); return a + b; }
 
 // (I + L)^-1 of a 32x32 strictly lower block by forward substitution; lane = column.  Four partial sums per
 // row: the rows form one dependent chain, and a single accumulator would make it 496 multiply-adds long.
@@ -144,7 +141,7 @@ template <typename ACT>
 __global__ void __launch_bounds__(256, 2) k_delta_prep64(LinArgs a, const float *Y, const float *rqg, const float *rkg,
                                                       const float *la, const float *be, float *AP, float *aux,
                                                       int n_chunks, int chunk0, int refresh) {
-    // A programmatic dependent of the conv in front of it, as the scan is of this kernel (short prompts: four launches of
+    // A programmatic dependent of the conv in front of it, as the scan is of this kernel (short prompts: three launches of
     // 8 to 40 us, whose latencies showed)
     dependent_entry();
     extern __shared__ __align__(16) unsigned char smraw[];

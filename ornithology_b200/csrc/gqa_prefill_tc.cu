@@ -337,8 +337,8 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
         const float inv = ok ? 1.0f / l : NAN;
         ACT *out = (ACT *)a.out + (tok * a.nh + h) * HD;
         // 32 columns at a time, the gate of the next 32 requested before this 32 are scaled and stored.  (A thread's row is a
-        // line of its own; element by element, each gate load waits behind the store before it: 128 memory latencies, 70 us of
-        // a CTA that has nothing else to run, which was more than half of a 1000-token prompt.)
+        // line of its own; element by element, each gate load waits behind the store before it: 128 memory latencies at the end of
+        // a CTA that has nothing else to run.  1000 tokens behind 3001 cached ones, 35B, 139 -> 91 us; 32768 tokens, 397B, 19.2 -> 16.0 ms.)
         const bool vec = (((uintptr_t)a.qproj | (uintptr_t)a.out) & 15) == 0;
         float gt[32];
         auto load_gate = [&](int c) {

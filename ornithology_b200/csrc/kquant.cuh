@@ -1,4 +1,4 @@
-// kquant.cuh — what the two integer-projection kernels share (kquant_matmul.cu: mma.sync; kquant_prefill_tc5.cu: tcgen05):
+// kquant.cuh — what the integer-projection kernels share (kquant_matmul.cu: mma.sync; kquant_prefill_tc5.cu, q80_tc5.cu: tcgen05):
 // the weight formats, the matrices of one launch, the tensor map of a weight matrix.
 #pragma once
 #include <cuda.h>

@@ -38,11 +38,13 @@ ornith_status launch_linear_prefill_tc(const LinArgs &x, int n_seq, int act_dtyp
 // rounded to tf32 (k_conv4_silu_prefill does that); work = linear_prefill_tc5_work_bytes() bytes;
 // la = be = nullptr: the gates are computed from the layer's a / b inputs.
 //
-// With a front (the causal conv of a token range and the refresh of the conv history, as launches the caller
-// provides) and one wave of heads or less, the prompt is cut into slabs and pipelined: conv + chunk preparation
+// With a front (the causal conv of a token range, as a launch the caller provides) the chunk preparation that ends the
+// prompt also stores the new conv history, behind the conv's last read of the old one; the caller must not store it too.
+// With a front and one wave of heads or less, the prompt is cut into slabs and pipelined: conv + chunk preparation
 // of slab k + 1 run on the caller's stream while slab k is scanned on a second, high-priority stream, so the
 // SMs the scan leaves idle (one CTA per head) do the memory-bound passes.  Events order the slabs; the caller's
-// stream waits for the last scan before the call returns.  front = nullptr: Y, rq and rk are complete already.
+// stream waits for the last scan before the call returns.  front = nullptr: Y, rq and rk are complete already, and the
+// caller has stored the new conv history.
 struct TC5Front {
     std::function<ornith_status(int t_begin, int t_end, cudaStream_t)> conv;
 };
