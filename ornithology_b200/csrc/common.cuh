@@ -90,7 +90,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm(
 // k_gqa_decode_q8_raw and k_linear_decode_ring release the kernel behind them at once (it must wait before all else) and
 // wait themselves only before they read what the kernel in front wrote; k_conv4_silu_prefill_tma, itself launched plainly,
 // releases at once too; the projection kernels, the tcgen05 scan and the tcgen05 GQA prefill wait only where they first touch
-// such data and release nothing before their end; the f32 and int8 decode kernels are launched plainly.
+// such data and release nothing before their end; the int8 decode kernel is launched plainly.
 __device__ __forceinline__ void dependent_entry() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");

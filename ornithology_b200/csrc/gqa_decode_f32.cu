@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(128, 3) k_gqa_decode_f32_tc(DecodeArgs a) {
     __shared__ __align__(8) unsigned long long bars[NWARP][2];
     __shared__ int pipe_failed;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, j = lane & 3;
+    dependent_entry();
     float *Q_s = reinterpret_cast<float *>(smem);                        // [8 heads][LDQ] tf32
     float *Kt = reinterpret_cast<float *>(smem + QS_BYTES + warp * WARP_BYTES), *Vt = Kt + TILE * LDKT;
     if (tid == 0) pipe_failed = 0;
@@ -227,8 +228,5 @@ ornith_status launch_gqa_decode_f32_tc(const DecodeArgs &a, int n_seq, cudaStrea
         configured = true;
     }
     dim3 grid(a.kv.nkv * ((a.nh / a.kv.nkv + 7) / 8), a.nsplit, n_seq);
-    // Launched plainly, behind the append kernel's end, and not releasing the combine kernel early (as the int8 kernel, see there):
-    // 4 sequences x 4096, 35B, group of four layers, 51.4 us as a programmatic dependent, 48.1 plain; 9 x 16000 164.6 and 160.9.
-    k_gqa_decode_f32_tc<<<grid, 128, SMEM_BYTES, st>>>(a);
-    return orn_check_launch("k_gqa_decode_f32_tc");
+    return orn_check(orn_launch_dependent(k_gqa_decode_f32_tc, grid, dim3(128), SMEM_BYTES, st, a), "k_gqa_decode_f32_tc");
 }
