@@ -434,9 +434,10 @@ ornith_status launch_gqa_prefill_tc(const KvView &kv, const int32_t *kv_len, con
         configured = true;
     }
     dim3 grid((T + BM - 1) / BM, nh, n_seq);
-    // softmax threads per query row: 2 (default) or 4.  Measured at 32768 tokens x 32 heads: 19.1 ms with 2, 19.8 ms
-    // with 4 (back to back under the power cap, before the epilogue's gate was loaded ahead; 15.6 ms with 2 since): the softmax is not what bounds the kernel.  Every CTA pulls a 64 KB
-    // K + V tile pair from L2 per 128 query rows: 137 GB per layer, 7.2 TB/s over the 148 SMs, and that traffic is the bound.
+    // softmax threads per query row: 2 (default) or 4.  32768 tokens x 32 heads, back to back under the power cap: 19.1 ms with 2 and
+    // 19.8 with 4 while the epilogue still loaded its gate element by element; 15.3 to 16.0 ms with 2 since, 4 not measured again.
+    // Every CTA pulls a 64 KB K + V tile pair from L2 per 128 query rows, 137 GB per layer, which is 8.6 to 9.0 TB/s over the 148
+    // SMs at these times: more than the 7.2 TB/s that once looked like the bound.
     const char *e = getenv("ORNITH_CUDA_PREFILL_SOFTMAX");
     const int nq = (e && e[0] == '4') ? 4 : 2;
     auto kernel = nq == 4 ? (bf16_act ? k_gqa_prefill_tc<__nv_bfloat16, 4> : k_gqa_prefill_tc<float, 4>)
