@@ -434,8 +434,8 @@ ornith_status launch_gqa_prefill_tc(const KvView &kv, const int32_t *kv_len, con
         configured = true;
     }
     dim3 grid((T + BM - 1) / BM, nh, n_seq);
-    // softmax threads per query row: 2 (default) or 4.  32768 tokens x 32 heads, back to back under the power cap: 19.1 ms with 2 and
-    // 19.8 with 4 while the epilogue still loaded its gate element by element; 15.3 to 16.0 ms with 2 since, 4 not measured again.
+    // softmax threads per query row: 2 (default) or 4.  In turn, back to back: 32768 tokens x 32 heads under the power cap 15.8 and
+    // 16.6 ms with 2, 16.8 and 17.2 with 4; 1000 tokens behind 3001, 16 heads, 82 us with 2, 89 with 4.
     // Every CTA pulls a 64 KB K + V tile pair from L2 per 128 query rows, 137 GB per layer, which is 8.6 to 9.0 TB/s over the 148
     // SMs at these times: more than the 7.2 TB/s that once looked like the bound.
     const char *e = getenv("ORNITH_CUDA_PREFILL_SOFTMAX");
