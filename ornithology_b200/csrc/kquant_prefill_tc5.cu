@@ -17,7 +17,8 @@
 //   1 MMA lane    per unit 8 k-steps x 2 planes.  Two accumulator slots: a unit is multiplied while the one before
 //                 it is drained; the unit left over from a super-block is drained after the next one is unpacked.
 // What bounds it: the issue slots of the workers.  A super-block of 128 rows x 256 tokens (Q6_K, H = 2) takes about 6100
-// cycles: 2000 to unpack, 2000 for each of two drains; its MMAs take 2048 of the tensor pipe.  More tokens per CTA would
+// cycles, 7800 with its share of a CTA's start and stores in a launch of 16: 2000 to unpack, 2000 for each of two drains; its
+// MMAs take 2048 of the tensor pipe.  More tokens per CTA would
 // share the unpacking further, but the totals already take half of the register file.
 // Measured (us, mma.sync kernel -> this one): Q6_K 4096 tokens 2048 -> 8192 821 -> 224, 777 tokens 4096 -> 20608 806 -> 283 and
 // 8192 -> 4096 339 -> 111; Q4_K 602 -> 326, 594 -> 360, 247 -> 167.

@@ -10,8 +10,8 @@
 // The roles and the walk over the tiles are those of kquant_prefill_tc5.cu.  Per super-block (8 blocks) a worker copies the
 // codes of its row group out of the 34-byte blocks into core-matrix order (one plane, two stages: the next super-block is
 // unpacked before this one is drained), then drains units of BU blocks, NS tokens wide (BU NS = 256 columns, two slots).
-// What bounds it: the drain's issue slots and the latencies between them (a super-block of 128 x 128 takes about 6000 cycles,
-// 2300 of them issue; its MMAs take 512 of the tensor pipe).  Measured (us, mma.sync kernel -> this one): 2048 -> 8192, 128
+// What bounds it: the drain's issue slots and the latencies between them (a super-block of 128 x 128 takes about 6600 cycles, in
+// which a scheduler issues 4700 times; its MMAs take 512 of the tensor pipe).  Measured (us, mma.sync kernel -> this one): 2048 -> 8192, 128
 // tokens 24 -> 20, 2048 tokens 319 -> 198; 4096 -> 20608, 777 tokens 625 -> 410, 2048 tokens 1538 -> 951.
 #include "kq_tc5.cuh"
 
