@@ -14,8 +14,7 @@
 //   warps 9-11  scores    one lane each issues S_j = Q K_j^T (16 x tcgen05.mma M128 N64 K16) for
 //                         the tiles j = 0, 1, 2 (mod 3) into its own score buffer
 //   warp 12     values    one lane issues O += P_j V_j (4 x M128 N256 K16)
-//                         Several issuing threads because one thread issues at most one MMA per
-//                         64-96 cycles, several times what an N = 64 product occupies the pipe;
+//                         Several issuing threads because one that waits for its score buffer holds back nobody else;
 //                         three score buffers so that the chain issue -> softmax -> value product
 //                         -> next issue of a buffer spans three tiles.
 //   warps 0-7   softmax   two threads per query row (= TMEM lane), 32 of the 64 scores each:
@@ -155,7 +154,7 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
 
     if (warp == W_K) {
         // ================= producer =================
-        if (lane == 0) {
+        if (elect_one()) {
             // dims 128..255 of the query tile stay in shared memory (two 64-dim slabs)
             mbar_expect_tx(su32(&bars.q_full), 32768u);
             const int qrow = (b * a.nh + h) * a.T + q0;
@@ -174,7 +173,7 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
         // ================= producer of the V tiles =================
         // its own lane: a V stage is released late (after the value product of its tile), and
         // waiting for that must not hold back the K tiles, which the score MMAs need much earlier
-        if (lane == 0) {
+        if (elect_one()) {
             const int krow = (b * a.nkv + kvh) * a.Lp;
             for (int j = 0; j < n_tiles; j++) {
                 const int sv = j % NSV;
@@ -187,12 +186,10 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
         }
     } else if (warp >= W_QK && warp < W_QK + 3) {
         // ================= score MMAs: warp 9 + e issues the tiles j = e (mod 3) =================
-        // One thread cannot issue tcgen05.mma faster than one per ~64-96 cycles, two to three times
-        // the 32 cycles an M128 N64 K16 product occupies the pipe; several issuing threads overlap.
         // With three score buffers the chain issue -> softmax -> value product -> next issue of a
         // buffer spans three tiles.  Dims 0..127 of Q are a tensor-memory operand, dims 128..255 a
         // shared-memory one (512 columns: output 256, scores 3 x 64, query 64).
-        if (lane == 0) {
+        if (elect_one()) {
             const int e = warp - W_QK;
             const uint32_t idesc_qk = (1u << 4) | (8u << 17) | (8u << 24);                 // f16 x f16 -> f32, N 64, M 128
             ok = mbar_wait(su32(&bars.q_full), 0);
@@ -219,7 +216,7 @@ __global__ void __launch_bounds__((4 * NQ + 6) * 32, 1) k_gqa_prefill_tc(const _
         }
     } else if (warp == W_PV) {
         // ================= value MMAs =================
-        if (lane == 0) {
+        if (elect_one()) {
             const uint32_t idesc_pv = (1u << 4) | (1u << 16) | (32u << 17) | (8u << 24);   // B MN-major, N 256, M 128
             for (int j = 0; j < n_tiles && ok; j++) {
                 const int st = j % NSV, sb = j % NB;

@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
 
     if (warp == W_COPY) {
         // ---- weight bytes, two super-blocks ahead of the workers -------------------------------------------------
-        if (lane == 0) {
+        if (tc5::elect_one()) {
             int n = 0;                                                // super-blocks copied
             for (int idx = blockIdx.x; idx < n_tiles && ok; idx += gridDim.x) {
                 const Tile t = tile_of<NS, H>(grp, a.T, idx);
@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
         }
     } else if (warp == X_COPY) {
         // ---- activation images, unit by unit ---------------------------------------------------------------------
-        if (lane == 0) {
+        if (tc5::elect_one()) {
             asm volatile("griddepcontrol.wait;\n" ::: "memory");     // they come from the kernel in front
             int st = 0, round = 0, issued = 0;
             for (int idx = blockIdx.x; idx < n_tiles && ok; idx += gridDim.x) {
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_kq_tc5(KqArgs a, int n_t
         }
     } else if (warp == W_MMA) {
         // ---- MMA issue ---------------------------------------------------------------------------------------
-        if (lane == 0) {
+        if (tc5::elect_one()) {
             const uint32_t A = tc5::su32(smem), X = tc5::su32(smem + S::O_X);
             const uint64_t a_hi = desc_plain(A, 128, QK * 8), a_lo = desc_plain(A + PLANE, 128, QK * 8), a_min = desc_plain(A + S::O_AMIN, 128, 256);
             int u = 0, st = 0, round = 0, n_sb = 0;

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
 
     if (warp == W_COPY) {
         // ---- weight bytes, two super-blocks ahead of the workers -------------------------------------------------
-        if (lane == 0) {
+        if (tc5::elect_one()) {
             int n = 0;                                                // super-blocks copied
             for (int idx = blockIdx.x; idx < n_tiles && ok; idx += gridDim.x) {
                 const Tile t = tile_of<NS, 1>(grp, a.T, idx);
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
         }
     } else if (warp == X_COPY) {
         // ---- activation images ---------------------------------------------------------------------------------------
-        if (lane == 0) {
+        if (tc5::elect_one()) {
             asm volatile("griddepcontrol.wait;\n" ::: "memory");     // they come from the kernel in front
             int n = 0;
             for (int idx = blockIdx.x; idx < n_tiles && ok; idx += gridDim.x) {
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_matmul_q80_tc5(KqArgs a, int n_
         }
     } else if (warp == W_MMA) {
         // ---- MMA issue -----------------------------------------------------------------------------------------------
-        if (lane == 0) {
+        if (tc5::elect_one()) {
             int u = 0, n = 0;
             for (int idx = blockIdx.x; idx < n_tiles && ok; idx += gridDim.x) {
                 const Tile t = tile_of<NS, 1>(grp, a.T, idx);
