@@ -6,23 +6,26 @@
 // The pass is a stream: read the projected activations once, write the f32 image Y once.  With plain loads a thread
 // can keep about a hundred bytes in flight, and with the registers that takes the SM holds too few warps to cover the
 // memory latency (the kernel sat at 0.56 of the HBM rate, waiting on its loads).  Here the loads are tensor copies
-// into shared memory, three stages per CTA and four CTAs per SM, so an SM keeps about 200 KB in flight whatever the
+// into shared memory, two stages per CTA and six CTAs per SM (three and four left the SM 16 warps, too few to cover the special-function
+// chains: 512 tokens of the 35B layer 54.4 -> 51.6 us), so an SM keeps about 200 KB in flight whatever the
 // register count; the threads only read shared memory, compute and store.
 //
 // Tile: 32 tokens (+ the 3 tokens of history in front of them) x 512 bytes of channels (256 bf16 or 128 f32).  A warp
 // owns 128 adjacent channels (one q or k head when the channel is a q/k channel, so the sums of squares of a head
 // are warp sums) and a run of 16 (bf16) or 8 (f32) tokens, which it walks with a sliding window of 4 rows.  The
 // first tile of a sequence takes its history from the conv ring instead.  Same arithmetic as k_conv4_silu_prefill's
-// tensor-core form: fused multiply-adds in tap order, hardware-exponential SiLU, q/k rounded to tf32.
+// tensor-core form: fused multiply-adds in tap order, hardware-exponential SiLU, v times its write gate, all rounded to tf32.
 #include <cuda.h>
 #include <cuda_bf16.h>
+
+#include <type_traits>
 
 #include "linear_attn.cuh"
 #include "tcgen05.cuh"          // the tensor-map encoder entry point, bounded mbarrier waits
 
 namespace {
 
-constexpr int CT_TOK = 32, CT_ROWS = CT_TOK + 3, CT_ROWB = 512, CT_STAGE = CT_ROWS * CT_ROWB, CT_NST = 3;
+constexpr int CT_TOK = 32, CT_ROWS = CT_TOK + 3, CT_ROWB = 512, CT_STAGE = CT_ROWS * CT_ROWB, CT_NST = 2, CT_CTAS = 6;
 constexpr int CT_SMEM = CT_NST * CT_STAGE + 128;
 
 __device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -48,7 +51,7 @@ struct ConvTmaArgs {
 };
 
 template <typename ACT>
-__global__ void __launch_bounds__(128) k_conv4_silu_prefill_tma(LinArgs a, const __grid_constant__ CUtensorMap map_x, ConvTmaArgs c) {
+__global__ void __launch_bounds__(128, CT_CTAS) k_conv4_silu_prefill_tma(LinArgs a, const __grid_constant__ CUtensorMap map_x, ConvTmaArgs c) {
     constexpr int CH = CT_ROWB / (int)sizeof(ACT);        // channels of a tile: 256 (bf16) or 128 (f32)
     constexpr int SPAN = CH / 128, GROUPS = 4 / SPAN, TPT = CT_TOK / GROUPS;   // warps across the channels; token runs; tokens per thread
     extern __shared__ unsigned char smem_raw[];
@@ -91,12 +94,21 @@ __global__ void __launch_bounds__(128) k_conv4_silu_prefill_tma(LinArgs a, const
             for (int q = 0; q < 4; q++) w[q] = *reinterpret_cast<const float4 *>(a.conv_w + (size_t)(ch + q) * 4);
             float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
             if (a.conv_b) bias = *reinterpret_cast<const float4 *>(a.conv_b + ch);
-            float4 x0, x1, x2;
+            // Two channels to a register pair: multiply-adds, scalings and additions go in pairs, each rounded as a single one is.
+            // (The kernel is bound by issue and special-function slots when it shares the GPU with the scan of the slab before.)
+            f32x2 wt[4][2];                               // wt[tap][pair]
+            wt[0][0] = pack2(w[0].x, w[1].x); wt[0][1] = pack2(w[2].x, w[3].x);
+            wt[1][0] = pack2(w[0].y, w[1].y); wt[1][1] = pack2(w[2].y, w[3].y);
+            wt[2][0] = pack2(w[0].z, w[1].z); wt[2][1] = pack2(w[2].z, w[3].z);
+            wt[3][0] = pack2(w[0].w, w[1].w); wt[3][1] = pack2(w[2].w, w[3].w);
+            const f32x2 bias2[2] = {pack2(bias.x, bias.y), pack2(bias.z, bias.w)};
+            f32x2 x0[2], x1[2], x2[2];
+            auto pairs = [](float4 v, f32x2 (&x)[2]) { x[0] = pack2(v.x, v.y); x[1] = pack2(v.z, v.w); };
             const int tfirst = t0 + grp * TPT;            // this thread's first token
             if (tfirst >= 3) {
-                x0 = ld_row4(rows, ch_local, (const ACT *)nullptr);
-                x1 = ld_row4(rows + CT_ROWB, ch_local, (const ACT *)nullptr);
-                x2 = ld_row4(rows + 2 * CT_ROWB, ch_local, (const ACT *)nullptr);
+                pairs(ld_row4(rows, ch_local, (const ACT *)nullptr), x0);
+                pairs(ld_row4(rows + CT_ROWB, ch_local, (const ACT *)nullptr), x1);
+                pairs(ld_row4(rows + 2 * CT_ROWB, ch_local, (const ACT *)nullptr), x2);
             } else {                                      // the start of the sequence: the history is the conv ring's
                 const int pos0 = a.pos[b];
                 const float *ring = a.conv + (size_t)b * a.conv_stride;
@@ -107,49 +119,76 @@ __global__ void __launch_bounds__(128) k_conv4_silu_prefill_tma(LinArgs a, const
                     h[i] = t >= 0 ? ld_row4(rows + i * CT_ROWB, ch_local, (const ACT *)nullptr)
                                   : *reinterpret_cast<const float4 *>(ring + (size_t)(((pos0 + t) % 4 + 4) % 4) * Cc + ch);
                 }
-                x0 = h[0]; x1 = h[1]; x2 = h[2];
+                pairs(h[0], x0); pairs(h[1], x1); pairs(h[2], x2);
             }
             const bool qk = ch < 2 * qd;                  // warp-uniform: a warp covers 128 channels = one head
-            float *Yp = c.Y + ((size_t)b * a.T + tfirst) * Cc + ch;
+            // v channels leave as beta v, what the chunk's products take, rounded to tf32: lane i has the write gate of token i
+            float beta = 0.0f;
+            if (!qk && lane < TPT && tfirst + lane < a.T)
+                beta = sigmoid_f(act_ld((const ACT *)a.b, ((size_t)b * a.T + tfirst + lane) * a.nv + (ch - 2 * qd) / 128));
+            // the tokens of this thread, kinds of channels and whole or ragged runs apart: a test per token ends a basic block per
+            // token, and the special-function chains of neighbouring tokens then no longer overlap
+            auto run = [&](auto qk_t, auto whole_t) {
+                constexpr bool QK = decltype(qk_t)::value, WHOLE = decltype(whole_t)::value;
+                float *Yp = c.Y + ((size_t)b * a.T + tfirst) * Cc + ch;
+                const unsigned char *xp = rows + 3 * CT_ROWB;
+                int left = c.t_end - tfirst;
 #pragma unroll
-            for (int i8 = 0; i8 < TPT; i8 += 8) {
-                float ss[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float4 x3 = ld_row4(rows + (i8 + i + 3) * CT_ROWB, ch_local, (const ACT *)nullptr);
-                    float4 y;
-#define ORN_TAP(F, Q) y.F = silu_fast(fmaf(w[Q].w, x3.F, fmaf(w[Q].z, x2.F, fmaf(w[Q].y, x1.F, fmaf(w[Q].x, x0.F, bias.F)))))
-                    ORN_TAP(x, 0); ORN_TAP(y, 1); ORN_TAP(z, 2); ORN_TAP(w, 3);
-#undef ORN_TAP
-                    if (qk) { y.x = tf32_round(y.x); y.y = tf32_round(y.y); y.z = tf32_round(y.z); y.w = tf32_round(y.w); }
-                    if (tfirst + i8 + i < c.t_end) *reinterpret_cast<float4 *>(Yp + (size_t)(i8 + i) * Cc) = y;
-                    ss[i] = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
-                    x0 = x1; x1 = x2; x2 = x3;
-                }
-                if (qk) {
-                    // sums over the 32 lanes for 8 tokens: token i ends up in lanes i, i + 8, i + 16, i + 24
+                for (int i8 = 0; i8 < TPT; i8 += 8) {
+                    float ss[8];
 #pragma unroll
                     for (int i = 0; i < 8; i++) {
-                        ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 16);
-                        ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 8);
+                        f32x2 x3[2], y2[2];
+                        pairs(ld_row4(xp + (i8 + i) * CT_ROWB, ch_local, (const ACT *)nullptr), x3);
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {     // taps in order, then SiLU (silu_fast on a pair)
+                            const f32x2 v = fma2(wt[3][h], x3[h], fma2(wt[2][h], x2[h], fma2(wt[1][h], x1[h], fma2(wt[0][h], x0[h], bias2[h]))));
+                            float e0, e1;
+                            unpack2(mul2(pack2(-1.4426950408889634f, -1.4426950408889634f), v), &e0, &e1);
+                            unpack2(add2(pack2(1.0f, 1.0f), pack2(ex2_fast(e0), ex2_fast(e1))), &e0, &e1);
+                            y2[h] = mul2(v, pack2(rcp_fast(e0), rcp_fast(e1)));
+                            x0[h] = x1[h]; x1[h] = x2[h]; x2[h] = x3[h];
+                        }
+                        if (!QK) {
+                            const float bt = __shfl_sync(0xffffffffu, beta, i8 + i);
+                            y2[0] = mul2(y2[0], pack2(bt, bt));
+                            y2[1] = mul2(y2[1], pack2(bt, bt));
+                        }
+                        float4 y;
+                        unpack2(y2[0], &y.x, &y.y);
+                        unpack2(y2[1], &y.z, &y.w);
+                        y.x = tf32_round(y.x); y.y = tf32_round(y.y); y.z = tf32_round(y.z); y.w = tf32_round(y.w);
+                        if (WHOLE || i8 + i < left) *reinterpret_cast<float4 *>(Yp) = y;
+                        Yp += Cc;
+                        if (QK) ss[i] = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
                     }
+                    if (QK) {
+                        // sums over the 32 lanes for 8 tokens: token i ends up in lanes i, i + 8, i + 16, i + 24
 #pragma unroll
-                    for (int off = 4; off >= 1; off >>= 1) {
-                        const bool up = (lane & off) != 0;
+                        for (int i = 0; i < 8; i++) {
+                            ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 16);
+                            ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 8);
+                        }
 #pragma unroll
-                        for (int i = 0; i < off; i++) {
-                            const float send = up ? ss[i] : ss[i + off], keep = up ? ss[i + off] : ss[i];
-                            ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                        for (int off = 4; off >= 1; off >>= 1) {
+                            const bool up = (lane & off) != 0;
+#pragma unroll
+                            for (int i = 0; i < off; i++) {
+                                const float send = up ? ss[i] : ss[i + off], keep = up ? ss[i + off] : ss[i];
+                                ss[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                            }
+                        }
+                        if (lane < 8 && i8 + lane < left) {
+                            const bool is_k = ch >= qd;
+                            const int kh = (is_k ? ch - qd : ch) / 128;
+                            (is_k ? c.rk : c.rq)[((size_t)b * a.T + tfirst + i8 + lane) * a.nk + kh] = 1.0f / sqrtf(ss[0] + 1e-6f);
                         }
                     }
-                    const int t = tfirst + i8 + lane;
-                    if (lane < 8 && t < c.t_end) {
-                        const bool is_k = ch >= qd;
-                        const int kh = (is_k ? ch - qd : ch) / 128;
-                        (is_k ? c.rk : c.rq)[((size_t)b * a.T + t) * a.nk + kh] = 1.0f / sqrtf(ss[0] + 1e-6f);
-                    }
                 }
-            }
+            };
+            const bool whole = tfirst + TPT <= c.t_end;
+            if (qk) { if (whole) run(std::true_type{}, std::true_type{}); else run(std::true_type{}, std::false_type{}); }
+            else    { if (whole) run(std::false_type{}, std::true_type{}); else run(std::false_type{}, std::false_type{}); }
         }
         __syncthreads();                                  // every warp is done with this stage
         if (tid == 0 && !failed) {
@@ -194,7 +233,7 @@ ornith_status launch_t(const LinArgs &x, int n_seq, float *Y, float *rq, float *
     c.n_cblk = (Cc + CH - 1) / CH; c.n_ttile = (t_end - t_begin + CT_TOK - 1) / CT_TOK; c.status = orn_status_word();
     const long long tiles = (long long)c.n_cblk * c.n_ttile * n_seq;
     if (tiles >= (1ll << 31)) return ORNITH_OK;
-    const int grid = (int)(tiles < 4ll * n_sm ? tiles : 4ll * n_sm);
+    const int grid = (int)(tiles < (long long)CT_CTAS * n_sm ? tiles : (long long)CT_CTAS * n_sm);
     k_conv4_silu_prefill_tma<ACT><<<grid, 128, CT_SMEM, s>>>(x, map, c);
     *handled = true;
     return orn_check_launch("k_conv4_silu_prefill_tma");
@@ -202,7 +241,7 @@ ornith_status launch_t(const LinArgs &x, int n_seq, float *Y, float *rq, float *
 
 }  // namespace
 
-// conv + SiLU of tokens t_begin .. t_end - 1 of every sequence into Y, q/k rounded to tf32, inverse norms into rq / rk.
+// conv + SiLU of tokens t_begin .. t_end - 1 of every sequence into Y (q, k and beta v, rounded to tf32), inverse norms into rq / rk.
 // *handled = false (and ORNITH_OK) when the shape cannot be addressed by a tensor copy: the caller takes the plain kernel.
 ornith_status launch_conv4_silu_prefill_tma(const LinArgs &x, int n_seq, int act_dtype, float *Y, float *rq, float *rk,
                                             int t_begin, int t_end, cudaStream_t s, bool *handled) {

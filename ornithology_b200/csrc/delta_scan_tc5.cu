@@ -1,5 +1,5 @@
 // delta_scan_tc5.cu — gated delta-net prefill scan for dk = dv = 128 on the 5th-generation
-// tensor cores: operands staged by TMA, tcgen05.mma (tf32) with the recurrent state and every
+// tensor cores: operands staged by bulk copies, tcgen05.mma (tf32) with the recurrent state and every
 // intermediate of the chunk in tensor memory.
 //
 // Reference behaviour being replaced: the chunked scan of ornith_delta_prefill
@@ -10,40 +10,29 @@
 // inverse norms rk_i, rq_i, G_i the running sum of the log-decay inside the chunk, p_i = exp(G_i),
 // Gamma_ij = exp(G_i - G_j), w_j = Gamma_63,j:
 //   M = diag(beta) strictLower(Gamma o Khat Khat^T),  A = (I + M)^-1,  P = lower(Gamma o Qhat Khat^T)
-//   T = diag(beta) V - diag(beta p rk) (K S^T)
-//   U = A T
+//   U = A (beta V) + A' (K S^T),  A' = -A diag(beta p rk)
 //   O = diag(p rq) (Q S^T) + P U
 //   S <- p_63 S + sum_j (w_j rk_j u_j) k_j^T
 // (Khat, Qhat the normalised rows; the norms are folded into the per-token factors so that the
-// tensor cores read the K / Q tiles straight from the conv output.)  A, P and the per-token
-// factors do not depend on the state: k_delta_prep64 produces them for all chunks at once.
+// tensor cores read the K / Q tiles straight from the conv output; its v channels are stored as beta V.)  A, A', P and
+// the per-token factors do not depend on the state: k_delta_prep produces them for all chunks at once.
 //
 // k_delta_scan_tc5, one CTA per (value head, sequence), keeps everything transposed, dv on the
 // 128 tensor-memory lanes:
-//   KS^T | QS^T = S [K ; Q]^T     M128 N128 K128   A operand = the state itself (tensor memory)
-//   U^T  = T^T A^T                M128 N64  K64    A operand = T^T (tensor memory)
+//   (K S^T)^T = S K^T             M128 N64  K128   A operand = the state itself (tensor memory)
+//   (Q S^T)^T = S Q^T             M128 N64  K128   the same
+//   U^T  = (beta V)^T A^T + (K S^T)^T A'^T   M128 N64 K64 twice   A operands = the beta V tile (shared memory, MN-major) and
+//                                                the accumulator K S^T as it is
+//   S'  = p_63 S + (w rk U)^T K   M128 N128 K64    A operand = (w rk U)^T; B = the K tile, MN-major
 //   (PU)^T = U^T P^T              M128 N64  K64    A operand = U^T
-//   S   += (w rk U)^T K           M128 N128 K64    accumulator = the state; B = the K tile, MN-major
 // so the fp32 state never leaves tensor memory during a prompt: it is the accumulator of the
 // update and, read as tf32 (low mantissa bits ignored), the A operand of the next chunk.
-//   warp 16    one lane issues the TMA loads: the K | Q tile (64 KiB, two buffers), a second copy of the K rows
-//              for the state update (an MN-major tf32 operand must lie in 32-byte swizzle atoms, a K-major one in
-//              16-byte atoms, so one image cannot serve both), A and P (lower triangles only), the V rows, factors
-//   warp 17    one lane issues the tcgen05.mma of the dependency chain (KS | QS, U, state update)
-//   warp 18    one lane issues (P U)^T, which nothing on the chain waits for
-//   warps 0-7  chain epilogues, two threads per lane (32 tokens each): T from KS and V, the decay sweep of S
-//              (while U^T is computed), U -> tf32 U and w rk U
-//   warps 8-15 output epilogue, off the dependency chain: O, per-token RMSNorm over the head (transpose-reduce
-//              by shuffles), SiLU(z) gate, store; z is requested one chunk ahead
-// All warps keep the 96 registers of the launch (no setmaxnreg: the issuing warps run three different roles, and
-// that instruction must be executed identically by all four warps of a warpgroup).
-// Every wait is bounded in time; a wait that gives up is reported through the device status word and poisons
-// the outputs.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <math.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "linear_attn.cuh"
 #include "tcgen05.cuh"
@@ -53,13 +42,19 @@ using namespace tc5;
 
 constexpr int C = 64;                                   // tokens per chunk
 constexpr float LOG2E_F = 1.4426950408889634f;
-constexpr int AUX_FLOATS = 5 * C;                       // beta | beta p rk | w rk | p rq | p_63 (first word)
-constexpr uint32_t AUX_BYTES = AUX_FLOATS * 4;
-// A and P are lower triangular.  Stored per block as four dense pieces of 32 columns: A columns 0..31 (64 rows),
-// A columns 32..63 of rows 32..63 (32 rows), then the same for P: 192 rows of 32 floats.
-constexpr int AP_ROWS = 192, AP_A1 = 64, AP_P0 = 96, AP_P1 = 160;
-constexpr int AP_FLOATS = AP_ROWS * 32;
-constexpr uint32_t AP_BYTES = AP_FLOATS * 4;
+// What the preparation leaves for one (value head, chunk), in the layouts the scan's copies need: every part is one
+// contiguous bulk copy.
+//   A, A', P   lower triangular: columns 0..31 of 64 rows, then columns 32..63 of rows 32..63; rows of 128 bytes, 128-byte swizzle
+//           (a K-major B operand)
+//   factors    w rk (64), p rq (64), p_63
+constexpr int REC_A = 0, REC_AK = 12288, REC_P = 24576, REC_F = 36864, REC_BYTES = 37632;
+constexpr uint32_t TRI_BYTES = 12288, FAC_BYTES = 2 * C * 4 + 16;
+// The tensor core drops the 13 low mantissa bits of the state and of K S^T when it reads them, which takes 2^-11 / (2 ln 2) =
+// 3.52e-4 off a value on average (mantissas spread evenly over their logarithm).  A' and p rq scale that back.
+constexpr float S_DROP = 1.0f + 3.52e-4f;
+static_assert(REC_F + (int)FAC_BYTES <= REC_BYTES && REC_BYTES % 256 == 0, "record layout");
+// float index of element (i, l) of such a triangle
+__device__ __forceinline__ int tri_at(int i, int l) { return (l & 32) * 64 + (i - (l & 32)) * 32 + (((((l & 31) >> 2) ^ (i & 7)) << 2) | (l & 3)); }
 
 // Round to tf32 (nearest, ties away from zero; finite inputs) with integer arithmetic: cvt.rna.tf32.f32 runs at
 // the special-function rate, a sixteenth of this.  tf32r gives a clean tf32 value (low 13 mantissa bits zero) for
@@ -68,93 +63,190 @@ constexpr uint32_t AP_BYTES = AP_FLOATS * 4;
 __device__ __forceinline__ float tf32r(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
 __device__ __forceinline__ float tf32q(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
 
-// =============================================================================
-// state-independent part: one CTA per (chunk, key head, sequence), 256 threads
-// =============================================================================
-constexpr int LDK = 132;                                // K / Q rows: stride = 4 mod 32 keeps MMA fragments conflict-free
-constexpr int LDG = 65;
-constexpr int LDB = 36;                                 // 32x32 blocks, rows 16-byte aligned
-
-struct PairSmem {                                       // one value head in flight per pair of warps
-    float M11[32 * LDB], M21[32 * LDB], M22[32 * LDB];  // blocks of M = beta_i Gamma_il khat_i.khat_l (l < i)
-    float A22[32 * LDB];
-    float g[C], be[C];
-};
-struct PrepSmem {
-    union {
-        struct { float Ks[C * LDK], Qs[C * LDK]; } t;   // dead once the Gram matrices exist
-        PairSmem pair[4];
-    } u;
-    float GK[C * LDG], GQ[C * LDG];                     // khat_i.khat_l, qhat_i.khat_l for l <= i
-    float rk[C], rq[C];
-};
-
 __device__ __forceinline__ void mma_tf32_sync(float (&d)[4], const float (&a)[4], float b0, float b1) {
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])),
           "r"(__float_as_uint(a[3])), "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
 }
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
-// Multiply-adds in pairs (two per issued instruction, each rounded as a single one is): the preparation waits for its
-// shared-memory loads and dependent chains with two CTAs per SM, so every instruction it does not issue shows:
-// 6 prompts of 777 tokens, 35B, 252 -> 246 us.
-__device__ __forceinline__ float sum2(f32x2 v) { float a, b; unpack2(v, &a, &b); return a + b; }
+// =============================================================================
+// state-independent part: one CTA per (chunk, key head, sequence), 256 threads
+// =============================================================================
+//   gates     of up to four value heads, a thread per (head, token), while the K and Q rows are on their way
+//   Gram      K K^T and Q K^T, lower triangle, tf32 mma.sync, kept in the accumulators for all value heads
+//   M, P      from the accumulators: P to the record, M over the K and Q rows
+//   A         blocked inverse, in f32: the 32 x 32 diagonal blocks of all heads by substitution, a warp each (a lane per column), then the
+//             block below, four warps to a head, by two products
+// What the former kernel spent its 25k to 35k cycles a chunk on was waiting: shared-memory loads behind stores that might alias them,
+// a broadcast load to every two multiply-adds, gate inputs and rows fetched one dependent load after the other.  Here the
+// loads of a phase are issued together and nothing but M goes through shared memory: 22k to 27k cycles, two CTAs to an SM; 4096 tokens of
+// 64 heads 85 -> 68 us.  It is bound by latency (issue 0.4, shared-memory pipe 0.5).  Measured and not kept: the products of the
+// inverse on the tensor cores in three tf32 terms (60 us, but A then differs in the last places from what f32 gives); three
+// CTAs to an SM (75 us, spills); persistent CTAs that request the next item's rows early (71 us).
+//
+// M has rows of 16-byte pieces; piece c of row r lies at c ^ f(r), f = the three low bits of r in reverse order: a fragment's stores and
+// the reads along rows and down columns stay clear of bank conflicts.  Row offsets that are multiples of 8 leave f alone: a lane's
+// addresses differ by constants.
+__device__ __forceinline__ constexpr int swz(int r) { return ((r & 1) << 2) | (r & 2) | ((r >> 2) & 1); }
+__device__ __forceinline__ void ldmatrix_x4(float (&r)[4], uint32_t addr) {
+    uint32_t x[4];
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(addr) : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; i++) r[i] = __uint_as_float(x[i]);
+}
 
-// (I + L)^-1 of a 32x32 strictly lower block by forward substitution; lane = column.  Four partial sums per
-// row: the rows form one dependent chain, and a single accumulator would make it 496 multiply-adds long.
-// (L is stored with zeros on and above the diagonal, and a row not yet solved counts as zero.)
-__device__ __forceinline__ void inv_unit_lower(const float *Mb, int lane, float (&x)[32]) {
-    float nx[32];                                         // -x
+constexpr int HB = 4;                                   // value heads of a batch
+struct PrepSmem {
+    union {
+        struct { float K[C * 128], Q[C * 128]; } t;     // as copied: 4 slabs of 32 dims x 64 rows of 128 bytes, 128-byte swizzle; dead once the Gram matrices exist
+        float M[HB][C * C];
+    } u;
+    float g[HB][C], be[HB][C], tot[HB], gend[HB], rk[C], rq[C];
+};
+
+constexpr int PREP_SMEM = (int)sizeof(PrepSmem) + 1024; // + alignment slack
+
+__device__ __forceinline__ void team_sync(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+
+// Diagonal block q of (I + M)^-1, 32 x 32, over that of M, by a warp, by forward substitution, lane = column.  M is strictly lower
+// triangular inside its 16 x 16 diagonal blocks (zeros elsewhere in them).  Four partial sums per row: the rows form one dependent
+// chain, and a single accumulator would make it 496 multiply-adds long.  (A row not yet solved counts as zero.)
+__device__ __forceinline__ void invert_diagonal(float *M, int q, int lane) {
+    float *B = M + 32 * q * 64 + 32 * q;                  // the block's first piece is number 8 q
+    float nx[32];                                         // - the solution
 #pragma unroll
     for (int i = 0; i < 32; i++) nx[i] = 0.0f;
 #pragma unroll
     for (int i = 0; i < 32; i++) {
-        f32x2 a01 = pack2((i == lane) ? 1.0f : 0.0f, 0.0f), a23 = 0;
+        f32x2 a01 = pack2(i == lane ? 1.0f : 0.0f, 0.0f), a23 = 0;
 #pragma unroll
         for (int l4 = 0; l4 < (i + 3) / 4; l4++) {
-            const float4 m = *reinterpret_cast<const float4 *>(Mb + i * LDB + 4 * l4);
+            const float4 m = *reinterpret_cast<const float4 *>(B + i * 64 + ((l4 ^ swz(i)) << 2));
             a01 = fma2(pack2(m.x, m.y), pack2(nx[4 * l4], nx[4 * l4 + 1]), a01);
             if (4 * l4 + 2 < i) a23 = fma2(pack2(m.z, m.w), pack2(nx[4 * l4 + 2], nx[4 * l4 + 3]), a23);
         }
-        x[i] = sum2(a01) + sum2(a23);
-        nx[i] = -x[i];
+        float s0, s1, s2, s3;
+        unpack2(a01, &s0, &s1);
+        unpack2(a23, &s2, &s3);
+        nx[i] = -((s0 + s1) + (s2 + s3));
     }
-}
-// y[i] = sum_l B[row0 + i][l] x[l] for 16 rows of a 32x32 block in shared memory, x in registers
-__device__ __forceinline__ void block_matvec16(const float *B, int row0, const float (&x)[32], float (&y)[16]) {
+    __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
+    for (int i = 0; i < 32; i++) B[i * 64 + (((lane >> 2) ^ swz(i)) << 2) + (lane & 3)] = -nx[i];
+}
+
+// rows 8 q .. of the product of the 32 x 32 blocks at L (rows, 16 bytes at a time) and at R (lane = column): y[i] = sum_l L[8 q + i][l] R[l][lane]
+__device__ __forceinline__ void block_rows(const float *L, const float *R, int q, int lane, float (&y)[8]) {
+    float x[32];
+    const int c3 = lane >> 2, c0 = lane & 3;
+#pragma unroll
+    for (int l = 0; l < 32; l++) x[l] = R[l * 64 + ((c3 ^ swz(l)) << 2) + c0];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
         f32x2 a = 0;
 #pragma unroll
         for (int l4 = 0; l4 < 8; l4++) {
-            const float4 m = *reinterpret_cast<const float4 *>(B + (row0 + i) * LDB + 4 * l4);
+            const float4 m = *reinterpret_cast<const float4 *>(L + (8 * q + i) * 64 + ((l4 ^ swz(i)) << 2));
             a = fma2(pack2(m.x, m.y), pack2(x[4 * l4], x[4 * l4 + 1]), a);
             a = fma2(pack2(m.z, m.w), pack2(x[4 * l4 + 2], x[4 * l4 + 3]), a);
         }
-        y[i] = sum2(a);
+        float s0, s1;
+        unpack2(a, &s0, &s1);
+        y[i] = s0 + s1;
     }
 }
+// The block below the diagonal ones, [[A11, 0], [-A22 M21 A11, A22]], over M21, by the four warps of a team (q = warp of the team, bar = the
+// team's barrier), by rows.  The product M21 A11 takes the place above the diagonal blocks, which nothing else uses.
+__device__ __forceinline__ void invert_below(float *M, int q, int lane, int bar) {
+    float y[8];
+    float *M21 = M + 32 * 64, *A22 = M21 + 32, *T = M + 32;
+    const int c3 = lane >> 2, c0 = lane & 3;
+    block_rows(M21, M, q, lane, y);
+#pragma unroll
+    for (int i = 0; i < 8; i++) T[(8 * q + i) * 64 + ((c3 ^ swz(i)) << 2) + c0] = y[i];
+    team_sync(bar);
+    block_rows(A22, T, q, lane, y);
+#pragma unroll
+    for (int i = 0; i < 8; i++) M21[(8 * q + i) * 64 + ((c3 ^ swz(i)) << 2) + c0] = -y[i];
+    team_sync(bar);
+}
+
+struct PrepArgs64 {
+    const float *Y, *rq, *rk, *la, *be;   // la, be: log-decay and write gate, or nullptr (made here from the layer's inputs)
+    unsigned char *rec;                   // records [n_seq * nv][rec_chunks]
+    int n_chunks, chunk0, rec_chunks, refresh;
+    unsigned int *status;
+};
 
 template <typename ACT>
-__global__ void __launch_bounds__(256, 2) k_delta_prep64(LinArgs a, const float *Y, const float *rqg, const float *rkg,
-                                                      const float *la, const float *be, float *AP, float *aux,
-                                                      int n_chunks, int chunk0, int refresh) {
+__global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ CUtensorMap map_y, LinArgs a, PrepArgs64 p) {
     // A programmatic dependent of the conv in front of it, as the scan is of this kernel (short prompts: three launches of
     // 8 to 40 us, whose latencies showed)
     dependent_entry();
     extern __shared__ __align__(16) unsigned char smraw[];
-    PrepSmem &sm = *reinterpret_cast<PrepSmem *>(smraw);
-    const int chunk = chunk0 + blockIdx.x, kh = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    __shared__ unsigned long long rows_in;
+    PrepSmem &sm = *reinterpret_cast<PrepSmem *>(smraw + ((0u - su32(smraw)) & 1023u));
+    const int chunk = p.chunk0 + blockIdx.x, kh = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int g = lane >> 2, j = lane & 3;
-    const int qd = a.nk * 128, Cc = 2 * qd + a.nv * 128;
+    const int qd = a.nk * 128, Cc = 2 * qd + a.nv * 128, nvk = a.nv / a.nk;
     const int t0 = chunk * C, n = min(C, a.T - t0);
     const size_t tok0 = (size_t)b * a.T + t0;
+    auto head_of = [&](int m) { return a.head_map == ORNITH_HEADMAP_GROUPED ? kh * nvk + m : kh + m * a.nk; };
 
+    if (tid == 0) {                                       // (asked for by the threads, 16 bytes each, the requests alone took 2500 cycles)
+        mbar_init(su32(&rows_in), 1);
+        mbar_init_fence();
+        mbar_expect_tx(su32(&rows_in), 65536u);
+        for (int sl = 0; sl < 4; sl++) {
+            tma_load_2d(su32(sm.u.t.K) + sl * 8192, &map_y, qd + kh * 128 + 32 * sl, (int)tok0, su32(&rows_in));
+            tma_load_2d(su32(sm.u.t.Q) + sl * 8192, &map_y, kh * 128 + 32 * sl, (int)tok0, su32(&rows_in));
+        }
+    }
+    if (tid < C) {
+        sm.rk[tid] = tid < n ? p.rk[(tok0 + tid) * a.nk + kh] : 0.0f;
+        sm.rq[tid] = tid < n ? p.rq[(tok0 + tid) * a.nk + kh] : 0.0f;
+    }
+    // gates of the heads m0 .. m0 + 3: thread (head, token); running sums of the log-decay over the chunk
+    const int gh = tid >> 6, pt = tid & 63;
+    float bpk = 0.0f;                                     // -beta p rk of the thread's (head, token)
+    auto gates = [&](int m0) {
+        float gg = 0.0f, bb = 0.0f;
+        if (m0 + gh < nvk && pt < n) {
+            const int hv = head_of(m0 + gh);
+            const size_t i = (tok0 + pt) * a.nv + hv;
+            if (p.la) { gg = p.la[i]; bb = p.be[i]; }
+            else {                                        // reference: decay_alpha, src/ornith_rforward.c:282-284
+                const float xa = act_ld((const ACT *)a.a, i), xb = act_ld((const ACT *)a.b, i), ac = a.a_coef[hv], dt = a.dt_bias[hv];
+                gg = ac * softplus_f(xa + dt);
+                bb = sigmoid_f(xb);
+            }
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const float up = __shfl_up_sync(0xffffffffu, gg, o);
+            if (lane >= o) gg += up;
+        }
+        if (pt == 31) sm.tot[gh] = gg;
+        __syncthreads();
+        if (pt >= 32) gg += sm.tot[gh];
+        if (pt == C - 1) sm.gend[gh] = gg;
+        sm.g[gh][pt] = gg;
+        sm.be[gh][pt] = bb;
+        __syncthreads();
+        if (m0 + gh < nvk) {
+            float *f = reinterpret_cast<float *>(p.rec + (((size_t)b * a.nv + head_of(m0 + gh)) * p.rec_chunks + blockIdx.x) * REC_BYTES + REC_F);
+            const float gend = sm.gend[gh], pp = expf(gg);
+            f[pt] = expf(gend - gg) * sm.rk[pt];
+            f[C + pt] = pp * sm.rq[pt] * S_DROP;
+            if (pt < 4) f[2 * C + pt] = expf(gend);
+            bpk = -bb * pp * sm.rk[pt] * (S_DROP * S_DROP);
+        }
+    };
+    gates(0);
     // the conv has read the old history for the last time: store the last min(T, conv_k) inputs of the sequence (their own
     // launch took 2.4 us and a gap of a 512-token prompt's 72)
-    if (refresh && chunk0 + (int)gridDim.x == n_chunks) {
+    if (p.refresh && p.chunk0 + (int)gridDim.x == p.n_chunks) {
         const int pos0 = a.pos[b];
         float *ring = a.conv + (size_t)b * a.conv_stride;
         const ACT *X = (const ACT *)a.qkv + (size_t)b * a.T * Cc;
@@ -167,178 +259,184 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep64(LinArgs a, const float 
                 if (a.T - 4 + i >= 0) ring[(size_t)((pos0 + a.T - 4 + i) & 3) * Cc + ch] = v[i];
         }
     }
+    if (!mbar_wait(su32(&rows_in), 0u)) report_timeout(p.status, ORN_WAIT_DELTA_SCAN);
 
-    for (int e = tid; e < C * 32; e += 256) {             // raw rows (tf32 values); rows past the end are zero
-        const int i = e >> 5, c = (e & 31) * 4;
-        float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
-        if (i < n) {
-            const float *y = Y + (tok0 + i) * Cc + kh * 128 + c;
-            q = *reinterpret_cast<const float4 *>(y);
-            k = *reinterpret_cast<const float4 *>(y + qd);
-        }
-        *reinterpret_cast<float4 *>(&sm.u.t.Qs[i * LDK + c]) = q;
-        *reinterpret_cast<float4 *>(&sm.u.t.Ks[i * LDK + c]) = k;
-    }
-    if (tid < C) {
-        sm.rk[tid] = tid < n ? rkg[(tok0 + tid) * a.nk + kh] : 0.0f;
-        sm.rq[tid] = tid < n ? rqg[(tok0 + tid) * a.nk + kh] : 0.0f;
-    }
-    __syncthreads();
-    {   // Gram tiles on or below the diagonal: warps 0-3 K K^T, warps 4-7 Q K^T; 16 rows each
-        const int which = w >> 2, mt = w & 3, ntn = 2 * mt + 2;
-        float acc[8][4];
+    // Gram tiles: warp w has the rows 16 mt .. of K and of Q and up to three groups of 8 columns from nt0 on (20 such groups lie on
+    // or below the diagonal)
+    const int mt = w < 3 ? 3 : w < 5 ? 2 : w < 7 ? 1 : 0, nt0 = w == 1 || w == 4 ? 3 : w == 2 ? 6 : w == 6 ? 2 : 0,
+              cnt = w == 2 || w >= 5 ? 2 : 3;
+    float gk[3][4] = {}, gq[3][4] = {};
+    {
+        const uint32_t ka = su32(sm.u.t.K) + (uint32_t)(16 * mt + (lane & 15)) * 128, kb = su32(sm.u.t.K) + (uint32_t)(8 * nt0 + (lane & 7)) * 128;
+        const uint32_t fa = (uint32_t)(((lane >> 4) ^ (lane & 7)) << 4), fb = (uint32_t)(((lane >> 3) ^ (lane & 7)) << 4);
 #pragma unroll
-        for (int t = 0; t < 8; t++)
+        for (int s2 = 0; s2 < 8; s2++) {                  // two k-steps of 8
+            float qa[2][4], kf[2][4];
 #pragma unroll
-            for (int x = 0; x < 4; x++) acc[t][x] = 0.0f;
-        const float *Am = (which ? sm.u.t.Qs : sm.u.t.Ks) + 16 * mt * LDK;
-#pragma unroll 2
-        for (int k0 = 0; k0 < 128; k0 += 8) {
-            float af[4];
-            af[0] = Am[g * LDK + k0 + j];
-            af[1] = Am[(g + 8) * LDK + k0 + j];
-            af[2] = Am[g * LDK + k0 + j + 4];
-            af[3] = Am[(g + 8) * LDK + k0 + j + 4];
-#pragma unroll
-            for (int t = 0; t < 8; t++) {
-                if (t < ntn) {
-                    const float *kr = sm.u.t.Ks + (8 * t + g) * LDK + k0 + j;
-                    mma_tf32_sync(acc[t], af, kr[0], kr[4]);
-                }
+            for (int x = 0; x < 2; x++) {
+                const uint32_t at = ka + (s2 >> 1) * 8192 + (((4 * (s2 & 1) + 2 * x) << 4) ^ fa);
+                ldmatrix_x4(kf[x], at);
+                ldmatrix_x4(qa[x], at + C * 128 * 4);
             }
-        }
-        float *G = which ? sm.GQ : sm.GK;
-        const float *rrow = which ? sm.rq : sm.rk;
+            const uint32_t bt = kb + (s2 >> 1) * 8192 + (((s2 & 1) << 6) ^ fb);
 #pragma unroll
-        for (int t = 0; t < 8; t++)
-            if (t < ntn) {
+            for (int t = 0; t < 3; t++)
+                if (t < cnt) {
+                    float r[4];
+                    ldmatrix_x4(r, bt + t * 1024);
+                    mma_tf32_sync(gk[t], kf[0], r[0], r[1]);
+                    mma_tf32_sync(gq[t], qa[0], r[0], r[1]);
+                    mma_tf32_sync(gk[t], kf[1], r[2], r[3]);
+                    mma_tf32_sync(gq[t], qa[1], r[2], r[3]);
+                }
+        }
+        if (n < C) {                                      // rows past the end are another sequence's: whatever they hold, they count as zero
+#pragma unroll
+            for (int t = 0; t < 3; t++)
+#pragma unroll
+                for (int x = 0; x < 4; x++)
+                    if (16 * mt + g + 8 * (x >> 1) >= n || 8 * (nt0 + t) + 2 * j + (x & 1) >= n) gk[t][x] = gq[t][x] = 0.0f;
+        }
+        // the norms of both rows
+        const float k0 = sm.rk[16 * mt + g], k1 = sm.rk[16 * mt + g + 8], q0 = sm.rq[16 * mt + g], q1 = sm.rq[16 * mt + g + 8];
+#pragma unroll
+        for (int t = 0; t < 3; t++)
+            if (t < cnt) {
+                const float2 rl = *reinterpret_cast<const float2 *>(&sm.rk[8 * (nt0 + t) + 2 * j]);
+                gk[t][0] = gk[t][0] * k0 * rl.x; gk[t][1] = gk[t][1] * k0 * rl.y; gk[t][2] = gk[t][2] * k1 * rl.x; gk[t][3] = gk[t][3] * k1 * rl.y;
+                gq[t][0] = gq[t][0] * q0 * rl.x; gq[t][1] = gq[t][1] * q0 * rl.y; gq[t][2] = gq[t][2] * q1 * rl.x; gq[t][3] = gq[t][3] * q1 * rl.y;
+            }
+    }
+
+    for (int m0 = 0; m0 < nvk; m0 += HB) {
+        const int heads = min(HB, nvk - m0);
+        auto rec_of = [&](int h) { return p.rec + (((size_t)b * a.nv + head_of(m0 + h)) * p.rec_chunks + blockIdx.x) * REC_BYTES; };
+        if (m0 > 0) gates(m0);
+        __syncthreads();                                  // K and Q, or the A of the heads before, have been read for the last time
+        // M and P from the Gram accumulators
+        const int i0 = 16 * mt + g, i1 = i0 + 8;
+        float *m_at[3];                                   // this lane's elements of M (head 0) and P: rows i0; eight rows on, the swizzle is the same
+        int p_at[3];
+#pragma unroll
+        for (int t = 0; t < 3; t++) {
+            const int l = 8 * (nt0 + t) + 2 * j, pc = l >> 2;
+            m_at[t] = sm.u.M[0] + i0 * 64 + ((((pc & 7) ^ swz(g)) | (pc & 8)) << 2) + (l & 3);
+            p_at[t] = tri_at(i0, l);
+        }
+#pragma unroll 1
+        for (int h = 0; h < heads; h++) {
+            const float g0 = sm.g[h][i0], g1 = sm.g[h][i1], b0 = sm.be[h][i0], b1 = sm.be[h][i1];
+            float *Pg = reinterpret_cast<float *>(rec_of(h) + REC_P);
+            auto tile = [&](int t, auto diag_t) {
+                constexpr bool diag = decltype(diag_t)::value;        // a group of columns that meets the diagonal
+                const int l = 8 * (nt0 + t) + 2 * j;
+                const float2 gl = *reinterpret_cast<const float2 *>(&sm.g[h][l]);
+                float e[4] = {(g0 - gl.x) * LOG2E_F, (g0 - gl.y) * LOG2E_F, (g1 - gl.x) * LOG2E_F, (g1 - gl.y) * LOG2E_F}, mm[4], pp[4];
 #pragma unroll
                 for (int x = 0; x < 4; x++) {
-                    const int i = 16 * mt + g + 8 * (x >> 1), l = 8 * t + 2 * j + (x & 1);
-                    G[i * LDG + l] = acc[t][x] * rrow[i] * sm.rk[l];
+                    const int i = x < 2 ? i0 : i1, c = l + (x & 1);
+                    if (diag && c > i) e[x] = -INFINITY;              // (above it the decay would grow)
+                    e[x] = ex2_fast(e[x]);
+                    mm[x] = (x < 2 ? b0 : b1) * e[x] * gk[t][x];
+                    pp[x] = tf32q(e[x] * gq[t][x]);
+                    if (diag && c >= i) mm[x] = 0.0f;
+                    if (diag && c > i) pp[x] = 0.0f;
                 }
-            }
-    }
-    __syncthreads();                                      // the tiles are dead: the pair buffers alias them
-    const int nvk = a.nv / a.nk, pr = w >> 1, wl = w & 1, pt = tid & 63;
-    PairSmem &ps = sm.u.pair[pr];
-    for (int m = pr; m < nvk; m += 4) {                   // one pair of warps per value head of this key head
-        const int hv = a.head_map == ORNITH_HEADMAP_GROUPED ? kh * nvk + m : kh + m * a.nk;
-        const size_t blk = ((size_t)b * a.nv + hv) * n_chunks + chunk;
-        float *Ag = AP + blk * AP_FLOATS, *ax = aux + blk * AUX_FLOATS;
-        float gg = 0.0f, bb = 0.0f;                       // thread pt = token pt: log-decay and write gate
-        if (pt < n) {
-            if (la) { gg = la[(tok0 + pt) * a.nv + hv]; bb = be[(tok0 + pt) * a.nv + hv]; }
-            else {                                        // reference: decay_alpha, src/ornith_rforward.c:282-284
-                gg = a.a_coef[hv] * softplus_f(act_ld((const ACT *)a.a, (tok0 + pt) * a.nv + hv) + a.dt_bias[hv]);
-                bb = sigmoid_f(act_ld((const ACT *)a.b, (tok0 + pt) * a.nv + hv));
-            }
-        }
+                float *m = m_at[t] + h * (C * C), *P = Pg + p_at[t];
+                *reinterpret_cast<float2 *>(m) = make_float2(mm[0], mm[1]);
+                *reinterpret_cast<float2 *>(m + 512) = make_float2(mm[2], mm[3]);
+                *reinterpret_cast<float2 *>(P) = make_float2(pp[0], pp[1]);
+                *reinterpret_cast<float2 *>(P + 256) = make_float2(pp[2], pp[3]);
+            };
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float up = __shfl_up_sync(0xffffffffu, gg, o);
-            if (lane >= o) gg += up;
-        }
-        if (wl == 0) ps.g[pt] = gg;
-        ps.be[pt] = bb;
-        pair_sync(1 + pr);
-        if (wl == 1) { gg += ps.g[31]; ps.g[pt] = gg; }
-        pair_sync(1 + pr);
-        const float gend = ps.g[C - 1], pp = expf(gg);
-        ax[pt] = bb;
-        ax[C + pt] = bb * pp * sm.rk[pt];
-        ax[2 * C + pt] = expf(gend - gg) * sm.rk[pt];
-        ax[3 * C + pt] = pp * sm.rq[pt];
-        ax[4 * C + pt] = expf(gend);
-        // thread pt = column l of M and P; rows 0..31 concern the first warp of the pair only (columns 32.. are zero there)
-        if (wl == 0) {
-#pragma unroll 8
-            for (int i = 0; i < 32; i++) {
-                const float gam = (pt <= i) ? ex2_fast((ps.g[i] - gg) * LOG2E_F) : 0.0f;
-                ps.M11[i * LDB + pt] = (pt < i) ? ps.be[i] * gam * sm.GK[i * LDG + pt] : 0.0f;
-                Ag[(AP_P0 + i) * 32 + pt] = (pt <= i) ? tf32r(gam * sm.GQ[i * LDG + pt]) : 0.0f;
-            }
-#pragma unroll 8
-            for (int i = 32; i < C; i++) {                // pt < 32 <= i: below the diagonal throughout
-                const float gam = ex2_fast((ps.g[i] - gg) * LOG2E_F);
-                ps.M21[(i - 32) * LDB + pt] = ps.be[i] * gam * sm.GK[i * LDG + pt];
-                Ag[(AP_P0 + i) * 32 + pt] = tf32r(gam * sm.GQ[i * LDG + pt]);
-            }
-        } else {
-#pragma unroll 8
-            for (int i = 32; i < C; i++) {
-                const float gam = (pt <= i) ? ex2_fast((ps.g[i] - gg) * LOG2E_F) : 0.0f;
-                ps.M22[(i - 32) * LDB + pt - 32] = (pt < i) ? ps.be[i] * gam * sm.GK[i * LDG + pt] : 0.0f;
-                Ag[(AP_P1 + i - 32) * 32 + pt - 32] = (pt <= i) ? tf32r(gam * sm.GQ[i * LDG + pt]) : 0.0f;
+            for (int t = 0; t < 3; t++)
+                if (t < cnt) {
+                    if (((nt0 + t) >> 1) == mt) tile(t, std::true_type{});
+                    else tile(t, std::false_type{});
+                }
+            // the records' rows are whole: zeros right of the diagonal blocks of rows 0..15 (columns 16..31) and 32..47 (48..63)
+            if (w == 7 || w == 5) {
+                float *P = Pg + (lane >> 1) * 32 + (w == 5 ? 2048 : 0);
+#pragma unroll
+                for (int x = 0; x < 2; x++) *reinterpret_cast<float4 *>(P + (((4 + 2 * (lane & 1) + x) ^ ((lane >> 1) & 7)) << 2)) = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         }
-        pair_sync(1 + pr);
-        // A = (I + M)^-1 = [[A11, 0], [-A22 M21 A11, A22]]; lane = column.  The two diagonal blocks are inverted by one
-        // warp each; the two products of the off-diagonal block are split by rows between the warps.
-        float x[32];
-        if (wl == 0) {
-            inv_unit_lower(ps.M11, lane, x);
+        __syncthreads();
+        sm.be[gh][pt] = bpk;                              // (beta has been read for the last time)
+        if ((w >> 1) < heads) invert_diagonal(sm.u.M[w >> 1], w & 1, lane);
+        __syncthreads();
+#pragma unroll 1
+        for (int h = w >> 2; h < heads; h += 2) {         // two teams of four warps
+            float *M = sm.u.M[h];
+            invert_below(M, w & 3, lane, 1 + (w >> 2));
+            // A and -A diag(beta p rk), rounded to tf32: columns 0..31 of the rows 16 x .., then columns 32..63 of rows 32 + 16 (x - 4) ..
+            const int t = tid & 127, pc = t & 7, r = t >> 3;
+            const float *ms = M + r * 64 + ((pc ^ swz(r & 7)) << 2);
+            float *Ag = reinterpret_cast<float *>(rec_of(h) + REC_A) + r * 32 + ((pc ^ (r & 7)) << 2);
+            const float4 s0 = *reinterpret_cast<const float4 *>(&sm.be[h][4 * pc]), s1 = *reinterpret_cast<const float4 *>(&sm.be[h][32 + 4 * pc]);
 #pragma unroll
-            for (int i = 0; i < 32; i++) { Ag[i * 32 + lane] = tf32r(x[i]); ps.M11[i * LDB + lane] = x[i]; }   // A11 over M11
-        } else {
-            inv_unit_lower(ps.M22, lane, x);
-#pragma unroll
-            for (int i = 0; i < 32; i++) { Ag[(AP_A1 + i) * 32 + lane] = tf32r(x[i]); ps.A22[i * LDB + lane] = x[i]; }
+            for (int x = 0; x < 6; x++) {
+                const float4 v = *reinterpret_cast<const float4 *>(ms + (x < 4 ? x * 1024 : (x - 2) * 1024 + 32)), s = x < 4 ? s0 : s1;
+                *reinterpret_cast<float4 *>(Ag + x * 512) = make_float4(tf32q(v.x), tf32q(v.y), tf32q(v.z), tf32q(v.w));
+                *reinterpret_cast<float4 *>(Ag + x * 512 + (REC_AK - REC_A) / 4) = make_float4(tf32q(v.x * s.x), tf32q(v.y * s.y), tf32q(v.z * s.z), tf32q(v.w * s.w));
+            }
         }
-        pair_sync(1 + pr);
-        {
-            float y[16];
-#pragma unroll
-            for (int l = 0; l < 32; l++) x[l] = ps.M11[l * LDB + lane];          // column `lane` of A11
-            block_matvec16(ps.M21, 16 * wl, x, y);                               // rows 16 wl .. of M21 A11
-            pair_sync(1 + pr);                                                   // M22 has been read for the last time
-#pragma unroll
-            for (int i = 0; i < 16; i++) ps.M22[(16 * wl + i) * LDB + lane] = y[i];   // B = M21 A11 over M22
-            pair_sync(1 + pr);
-#pragma unroll
-            for (int l = 0; l < 32; l++) x[l] = ps.M22[l * LDB + lane];          // column `lane` of B
-            block_matvec16(ps.A22, 16 * wl, x, y);
-#pragma unroll
-            for (int i = 0; i < 16; i++) Ag[(32 + 16 * wl + i) * 32 + lane] = tf32r(-y[i]);
-        }
-        pair_sync(1 + pr);                                // the pair buffers are reused by the next head
     }
 }
 
 // =============================================================================
-// sequential part: one CTA per (value head, sequence), 18 warps
+// sequential part: one CTA per (value head, sequence)
 // =============================================================================
-constexpr int W_TMA = 24, W_MMA = 25, W_PU = 26, NTHREADS = 27 * 32;
-constexpr int TM_S = 0, TM_KQ = 128, TM_TU = 384, TM_U = 448, TM_COLS = 512;   // tensor-memory columns
-// Shared memory.  The K | Q tile is needed first in a chunk and is double-buffered; the operands of the
-// later products (second K copy for the state update, A, P) have one buffer each, refilled as soon as
-// the product that reads them is complete, which is most of a chunk period before their next use.
-constexpr int SM_KQ = 0;                 // 2 x [4 slabs of 32 dims x (64 K rows, then 64 Q rows) x 128 bytes]
-constexpr int SM_KM = 131072;            // the K tile again, laid out for the state update (see below)
-// A and P are lower triangular: of their second slab (columns 32..63) only rows 32..63 exist, and the
-// products that read it are issued for those 32 rows only
-constexpr int SM_A = 163840;             // slab 0: 64 rows x 32 columns (8 KiB); slab 1: rows 32..63 (4 KiB)
-constexpr int SM_P = 176128;
-constexpr int SM_V = 188416;             // [64 tokens][128] f32 rows of V, not swizzled
-constexpr int SM_AUX = 221184;           // 2 x per-token factors for the chain epilogues
-constexpr int SM_AUX2 = SM_AUX + 2 * (int)AUX_BYTES;   // one more copy for the output epilogue (freed later)
-constexpr int SCAN_SMEM = SM_AUX2 + (int)AUX_BYTES + 1024;   // + alignment slack
-constexpr uint32_t TX_KQ = 65536 + AUX_BYTES, TX_KM = 32768, TX_A = 12288, TX_P = 12288 + AUX_BYTES, TX_V = 32768;
+//   warps 0-7   chain: the decayed copy of the state, then U as the operands of the two products behind it; two threads per lane (row
+//               of S)
+//   warps 8-23  output, off the chain: O, per-token RMSNorm over the head, SiLU(z) gate, store
+//   warp 24     one lane issues the copies of the chunk's operands: one buffer each, refilled as soon as the product that reads it is
+//               complete, which is most of a chunk before its next use.  K and beta V rows that serve as MN-major operands come in
+//               32-byte swizzle atoms (a K-major tf32 operand must lie in 16-byte atoms, so K is copied twice)
+//   warp 25     one lane issues the tcgen05.mma of the chain and Q S^T
+//   warp 26     one lane issues those of P U: behind the state update in one stream they kept the issuing lane from the next chunk
+//   warp 27     one lane issues the copies of z and of the outputs, and asks L2 for what comes two chunks later
+// Tensor memory, 512 columns: two states of 128 (chunk n reads number n & 1; the other takes the decayed copy and then the
+// update), K S^T / w rk U, the accumulator and then operand U, Q S^T, P U.
+// A product that reads what an earlier product of another shape accumulated (the state, K S^T) is only issued after a wait on that
+// one's commit: the pipe does not order them, and issued back to back the read came too early.
+// What bounds it: the chain of a chunk, K S^T (530 cycles), its commit, A' K S^T (260), its commit, the pass over U (about 600), the
+// update (530), its commit; Q S^T, beta V's product and P U run beside those waits, and the copies, one period ahead, take up to 1.7 us
+// when the passes in front of the next slab share the memory.  4.0k to 4.3k cycles a chunk (64 chunks x 64 heads alone 220 -> 145 us; with
+// T = beta V - (beta p rk) K S^T made by the chain warps between the first two products 5.5k, with z loaded by the output warps 6.2k).
+// The output warps have as long for a chunk.  So they read their tiles as 16 x 256-bit fragments, a thread holding 4 rows of 4 tokens
+// (the sum of squares over the head is three shuffle levels on 4 values; as one row of 16 tokens it was five levels on 16),
+// arithmetic goes in pairs, and z and bf16 outputs pass through shared memory by tensor copies, read and written as transposed
+// 8 x 8 matrices (TILE; when z or out is not 16-byte aligned the threads load and store them): loaded by the threads one chunk
+// ahead, z held up each chunk's shuffles for 1300 to 2000 cycles.
+// Every wait is bounded in time; a wait that gives up is reported through the device status word and poisons the outputs.
+constexpr int W_TMA = 24, W_MMA = 25, W_PU = 26, W_IO = 27, NTHREADS = 28 * 32;
+constexpr int TM_S = 0, TM_X = 256, TM_U = 320, TM_QS = 384, TM_PU = 448, TM_COLS = 512;   // tensor-memory columns
+constexpr int NFAC = 4;
+constexpr int SM_K = 0, SM_V = 32768, SM_Q = 65536, SM_KM = 98304;
+// the two A tiles whole (64 x 64): their upper right quarter is zeroed once and never written again
+constexpr int SM_AV = 131072, SM_AK = SM_AV + 16384, SM_P = SM_AK + 16384;
+constexpr int SM_F = SM_P + (int)TRI_BYTES;             // NFAC x factors
+constexpr int SM_Z = (SM_F + NFAC * (int)FAC_BYTES + 1023) / 1024 * 1024;   // z of a chunk: 64 x 128 activations (bf16 or f32)
+constexpr int SM_O = SM_Z + 16384;                      // bf16 outputs of a chunk on their way out (f32 ones are stored by the threads)
+constexpr int SCAN_SMEM = SM_Z + 32768 + 1024;          // + alignment slack
+static_assert(SCAN_SMEM + 4096 <= 227 * 1024, "with the static part: the shared memory of an SM");
 
+enum { B_K, B_V, B_AK, B_Q, B_KM, B_P, NBUF };          // operand buffers (B_V: beta V and A)
 struct ScanBars {
-    unsigned long long full_kq[2], empty_kq[2], kq_done[2], pu_done[2], o_read[2], red[2][4];
-    unsigned long long full_km, empty_km, full_a, empty_a, full_p, empty_p, full_v, empty_v, t_ready, u_done, u_ready, s_final;
+    unsigned long long full[NBUF], empty[NBUF], full_f[NFAC], red[2][4], o_full[4], o_free[4];
+    unsigned long long ks_done, u_done, wu_ready, u_ready, s_done, pu_done, qs_done, o_read, full_z, empty_z;
 };
 
 struct ScanArgs {
-    const float *Y, *aux;
+    const unsigned char *rec;
     float *S;
     long long S_stride;
     const void *z;
     void *out;
     const float *norm_w;
     int nk, nv, head_map, T, n_chunks;
-    int c_begin, c_count;                // the chunks one launch of the sequential form scans (a slab of the prompt)
+    int c_begin, c_count, rec_chunks;    // the chunks one launch of the sequential form scans (a slab of the prompt); records per head
     float out_scale, eps;
     // Segment-parallel form (n_seg > 1; for few heads): the prompt is cut into n_seg runs of seg_chunks chunks that
     // are scanned at the same time by different CTAs (grid.z = 2 n_seg - 1).  The state enters the recurrence
@@ -352,10 +450,7 @@ struct ScanArgs {
     float *seg_state;                    // [n_seq * nv][3 n_seg][128][128]: slot 3j: S0 (j = 0: end state of run 0), 3j+1: Phi, 3j+2: S_in
     float *seg_raw;                      // [2][n_seq * nv][T][128] f32: o0, then qt
     unsigned int *status;
-    long long *trace;                    // bring-up aid: clock64 stamps of CTA (0, 0), [role][chunk][8]
-    float *dbg;                          // bring-up aid: first chunk's KS, U, QS, PU and the state after it (nullptr in production)
 };
-constexpr int DBG_FLOATS = 4 * 128 * 64 + 128 * 128;
 
 // MN-major tf32 operand: rows of 128 bytes along N, groups of 4 k, 32-byte swizzle atoms
 // (the only shared-memory layout the tensor core accepts for a transposed 32-bit operand)
@@ -379,25 +474,30 @@ __device__ __forceinline__ uint32_t ld_raw(const __nv_bfloat16 *p, size_t i) { r
 __device__ __forceinline__ float cvt_raw(const float *, uint32_t r) { return __uint_as_float(r); }
 __device__ __forceinline__ float cvt_raw(const __nv_bfloat16 *, uint32_t r) { return __uint_as_float(r << 16); }
 
-// D[dv][i] = sum_j X[dv][j] L[i][j] with L lower triangular (X in tensor memory at column x, L in shared memory
-// at l): j < 32 feeds all 64 rows i of L, j >= 32 only rows 32..63
-__device__ __forceinline__ void issue_tri(uint32_t d, uint32_t x, uint32_t l) {
-    constexpr uint32_t ID_64 = idesc(2, 64, false), ID_32 = idesc(2, 32, false);
-#pragma unroll
-    for (int ks = 0; ks < 4; ks++) mma_tf32_ts(d, x + 8 * ks, smem_desc(l + ks * 32, 16, 1024), ID_64, ks > 0);
-#pragma unroll
-    for (int ks = 0; ks < 4; ks++) mma_tf32_ts(d + 32, x + 32 + 8 * ks, smem_desc(l + 8192 + ks * 32, 16, 1024), ID_32, 1u);
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
+// this thread's stores to shared memory, seen by the tensor copy a thread issues after a barrier
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// four 8 x 8 matrices of 16-bit values, transposed: lane l names row l & 7 of matrix l >> 3 and holds of each the rows 2 (l & 3), + 1 at
+// column l >> 2
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t (&r)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 
-template <typename ACT, bool SEG>
+template <typename ACT, bool SEG, bool TILE>
 __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_constant__ CUtensorMap map_y,
                                                                const __grid_constant__ CUtensorMap map_ym,
-                                                               const __grid_constant__ CUtensorMap map_ap,
-                                                               const __grid_constant__ CUtensorMap map_ap32,
-                                                               const __grid_constant__ CUtensorMap map_v, ScanArgs a) {
+                                                               const __grid_constant__ CUtensorMap map_z,
+                                                               const __grid_constant__ CUtensorMap map_o, ScanArgs a) {
     extern __shared__ unsigned char smraw[];
     __shared__ ScanBars bars;
-    __shared__ float red[2][4][4][16];                    // [chunk parity][group of 16 tokens][lane quarter][token]
+    __shared__ __align__(16) float red[2][4][16][4];                    // [chunk parity][group of 16 tokens][token][lane quarter]
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hv = blockIdx.x, b = blockIdx.y;
@@ -413,21 +513,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     unsigned char *gbase = smraw + (base - su32(smraw));
 
     if (tid == 0) {
-        for (int s = 0; s < 2; s++) {
-            mbar_init(su32(&bars.full_kq[s]), 1); mbar_init(su32(&bars.empty_kq[s]), 9);
-            mbar_init(su32(&bars.kq_done[s]), 1); mbar_init(su32(&bars.pu_done[s]), 1);
-            mbar_init(su32(&bars.o_read[s]), 512);
-            for (int g = 0; g < 4; g++) mbar_init(su32(&bars.red[s][g]), 128);
-        }
-        mbar_init(su32(&bars.full_km), 1); mbar_init(su32(&bars.empty_km), 1);
-        mbar_init(su32(&bars.full_a), 1); mbar_init(su32(&bars.empty_a), 1);
-        mbar_init(su32(&bars.full_p), 1); mbar_init(su32(&bars.empty_p), 17);
-        mbar_init(su32(&bars.full_v), 1); mbar_init(su32(&bars.empty_v), 8);
-        mbar_init(su32(&bars.t_ready), 256); mbar_init(su32(&bars.u_done), 1);
-        mbar_init(su32(&bars.u_ready), 256); mbar_init(su32(&bars.s_final), 1);
+        for (int s = 0; s < NBUF; s++) { mbar_init(su32(&bars.full[s]), 1); mbar_init(su32(&bars.empty[s]), 1); }
+        for (int s = 0; s < NFAC; s++) mbar_init(su32(&bars.full_f[s]), 1);
+        for (int s = 0; s < 2; s++)
+            for (int g = 0; g < 4; g++) mbar_init(su32(&bars.red[s][g]), 4);
+        for (int g = 0; g < 4; g++) { mbar_init(su32(&bars.o_full[g]), 4); mbar_init(su32(&bars.o_free[g]), 1); }
+        mbar_init(su32(&bars.ks_done), 1); mbar_init(su32(&bars.u_done), 1);
+        mbar_init(su32(&bars.wu_ready), 8); mbar_init(su32(&bars.u_ready), 8); mbar_init(su32(&bars.s_done), 1);
+        mbar_init(su32(&bars.pu_done), 1); mbar_init(su32(&bars.qs_done), 1); mbar_init(su32(&bars.o_read), 16);
+        mbar_init(su32(&bars.full_z), 1); mbar_init(su32(&bars.empty_z), 16);
         mbar_init_fence();
     }
     if (warp == W_MMA) tmem_alloc(&tmem_slot, TM_COLS);
+    for (int e = tid; e < 512; e += NTHREADS)             // rows 0..31, columns 32..63 of both A tiles
+        *reinterpret_cast<float4 *>(gbase + (e < 256 ? SM_AV : SM_AK) + 8192 + (e & 255) * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+    fence_async();
     fence_before();
     __syncthreads();
     fence_after();
@@ -439,20 +539,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
         Sout = a.seg_state + (((size_t)b * a.nv + hv) * 3 * a.n_seg + 3 * seg + (kind == 2 ? 1 : 0)) * (128 * 128);
         if (kind) raw = a.seg_raw + ((size_t)(kind - 1) * gridDim.y * a.nv + (size_t)b * a.nv + hv) * (size_t)a.T * 128;
     }
-    // lane quarter and token (column) half of an epilogue thread
+    // lane quarter and token (column) half of a chain thread
     const int qtr = warp & 3, half = (warp >> 2) & 1, row = 32 * qtr + lane;
     const uint32_t lane_t = tmem + ((uint32_t)(32 * qtr) << 16);
-#ifdef ORNITH_SCAN_TRACE
-    float *dbg = a.dbg ? a.dbg + (size_t)(b * a.nv + hv) * DBG_FLOATS : nullptr;
-#else
-    constexpr float *dbg = nullptr;
-#endif
-    long long *trace = (a.trace && hv == 0 && b == 0) ? a.trace : nullptr;
-#ifdef ORNITH_SCAN_TRACE
-#define TR(role, n, pt) do { if (trace && (n) < 64) trace[((role) * 64 + (n)) * 8 + (pt)] = clock64(); } while (0)
-#else
-#define TR(role, n, pt) do { (void)trace; } while (0)
-#endif
 
     if (warp < 8) {                                       // the state goes to tensor memory: S[r][c] in lane r, column c
 #pragma unroll 1
@@ -473,381 +562,383 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
 
     if (warp == W_TMA) {
         // ================= producer =================
-        if (lane == 0) {
+        if (elect_one()) {
             asm volatile("griddepcontrol.wait;\n" ::: "memory");     // everything that comes through here is written by the kernels in front
-            const int yrow0 = b * a.T + c0 * C;                       // first row of this CTA's first chunk
-            const size_t blk0 = ((size_t)b * a.nv + hv) * a.n_chunks + c0;
-            auto load_kq = [&](int n) {
-                const int s = n & 1;
-                if (n >= 2 && !mbar_wait(su32(&bars.empty_kq[s]), (uint32_t)((n >> 1) - 1) & 1u)) return false;
-                const uint32_t dst = base + SM_KQ + s * 65536, bar = su32(&bars.full_kq[s]);
-                mbar_expect_tx(bar, TX_KQ);
-                for (int sl = 0; sl < 4; sl++) {
-                    tma_load_2d(dst + sl * 16384, &map_y, qd + kh * 128 + 32 * sl, yrow0 + n * C, bar);        // K rows
-                    tma_load_2d(dst + sl * 16384 + 8192, &map_y, kh * 128 + 32 * sl, yrow0 + n * C, bar);      // Q rows
-                }
-                bulk_load(base + SM_AUX + s * AUX_BYTES, a.aux + (blk0 + n) * AUX_FLOATS, AUX_BYTES, bar);
-                return true;
-            };
-            auto load_a = [&](int n) {
-                if (n >= 1 && !mbar_wait(su32(&bars.empty_a), (uint32_t)(n - 1) & 1u)) return false;
-                mbar_expect_tx(su32(&bars.full_a), TX_A);
-                tma_load_2d(base + SM_A, &map_ap, 0, (int)((blk0 + n) * AP_ROWS), su32(&bars.full_a));
-                tma_load_2d(base + SM_A + 8192, &map_ap32, 0, (int)((blk0 + n) * AP_ROWS) + AP_A1, su32(&bars.full_a));
-                return true;
-            };
-            auto load_v = [&](int n) {
-                if (n >= 1 && !mbar_wait(su32(&bars.empty_v), (uint32_t)(n - 1) & 1u)) return false;
-                mbar_expect_tx(su32(&bars.full_v), TX_V);
-                tma_load_2d(base + SM_V, &map_v, 2 * qd + hv * 128, yrow0 + n * C, su32(&bars.full_v));
-                return true;
-            };
-            auto load_km = [&](int n) {
-                if (n >= 1 && !mbar_wait(su32(&bars.empty_km), (uint32_t)(n - 1) & 1u)) return false;
-                mbar_expect_tx(su32(&bars.full_km), TX_KM);
-                for (int sl = 0; sl < 4; sl++)              // [64 tokens][128 dims]: 4 slabs of 32 dims, 32-byte swizzle atoms
-                    tma_load_2d(base + SM_KM + sl * 8192, &map_ym, qd + kh * 128 + 32 * sl, yrow0 + n * C, su32(&bars.full_km));
-                return true;
-            };
-            auto load_p = [&](int n) {
-                if (n >= 1 && !mbar_wait(su32(&bars.empty_p), (uint32_t)(n - 1) & 1u)) return false;
-                mbar_expect_tx(su32(&bars.full_p), TX_P);
-                tma_load_2d(base + SM_P, &map_ap, 0, (int)((blk0 + n) * AP_ROWS) + AP_P0, su32(&bars.full_p));
-                tma_load_2d(base + SM_P + 8192, &map_ap32, 0, (int)((blk0 + n) * AP_ROWS) + AP_P1, su32(&bars.full_p));
-                bulk_load(base + SM_AUX2, a.aux + (blk0 + n) * AUX_FLOATS, AUX_BYTES, su32(&bars.full_p));
-                return true;
-            };
-            // issue order = the order in which the buffers come free in the steady state
-            ok = load_kq(0) && load_v(0) && load_a(0) && load_km(0);
-            if (ok && N > 1) ok = load_kq(1);
-            for (int m = 0; m < N && ok; m++) {
-                TR(3, m, 0);
-                if (m + 1 < N) ok = load_v(m + 1);
-                if (ok) ok = load_p(m);
-                TR(3, m, 1);
-                if (ok && m + 1 < N) ok = load_a(m + 1);
-                TR(3, m, 2);
-                if (ok && m + 2 < N) ok = load_kq(m + 2);
-                TR(3, m, 3);
-                if (ok && m + 1 < N) ok = load_km(m + 1);
-                TR(3, m, 4);
+            const int yrow0 = b * a.T + c0 * C;                       // row of this CTA's first token
+            const unsigned char *rec0 = a.rec + (((size_t)b * a.nv + hv) * a.rec_chunks + (SEG ? c0 : 0)) * (size_t)REC_BYTES;
+            for (int n = 0; n < N && ok; n++) {
+                const unsigned char *r = rec0 + (size_t)n * REC_BYTES;
+                const int y = yrow0 + n * C;
+                auto refill = [&](int s, uint32_t bytes) {                // the buffer is free: its next contents are announced
+                    if (n >= 1) ok = ok && mbar_wait_parked(su32(&bars.empty[s]), (uint32_t)(n - 1) & 1u);
+                    if (ok) mbar_expect_tx(su32(&bars.full[s]), bytes);
+                    return ok;
+                };
+                auto rows = [&](int dst, const CUtensorMap *map, int x, int s) {
+                    for (int sl = 0; sl < 4; sl++) tma_load_2d(base + dst + sl * 8192, map, x + 32 * sl, y, su32(&bars.full[s]));
+                };
+                auto part = [&](int dst, int off, uint32_t bytes, int s) { bulk_load(base + dst, r + off, bytes, su32(&bars.full[s])); };
+                if (!refill(B_K, 32768u)) break;
+                rows(SM_K, &map_y, qd + kh * 128, B_K);
+                // (the readers of the factors of chunk n - 4 are done: K S^T of chunk n - 1 was behind them)
+                mbar_expect_tx(su32(&bars.full_f[n % NFAC]), FAC_BYTES);
+                bulk_load(base + SM_F + n % NFAC * FAC_BYTES, r + REC_F, FAC_BYTES, su32(&bars.full_f[n % NFAC]));
+                if (!refill(B_V, 32768u + TRI_BYTES)) break;
+                rows(SM_V, &map_ym, 2 * qd + hv * 128, B_V);
+                part(SM_AV, REC_A, 8192u, B_V);
+                part(SM_AV + 8192 + 4096, REC_A + 8192, 4096u, B_V);
+                if (!refill(B_AK, TRI_BYTES)) break;
+                part(SM_AK, REC_AK, 8192u, B_AK);
+                part(SM_AK + 8192 + 4096, REC_AK + 8192, 4096u, B_AK);
+                if (!refill(B_Q, 32768u)) break;
+                rows(SM_Q, &map_y, kh * 128, B_Q);
+                if (!refill(B_KM, 32768u)) break;
+                rows(SM_KM, &map_ym, qd + kh * 128, B_KM);
+                if (!refill(B_P, TRI_BYTES)) break;
+                part(SM_P, REC_P, TRI_BYTES, B_P);
             }
         }
     } else if (warp == W_MMA) {
         // ================= every tcgen05.mma =================
-        if (lane == 0) {
-            constexpr uint32_t ID_KQ = idesc(2, 128, false), ID_SU = idesc(2, 128, true);
-            fence_after();
+        if (elect_one()) {
+            constexpr uint32_t ID_64 = idesc(2, 64, false), ID_SU = idesc(2, 128, true), ID_V = ID_64 | (1u << 15);
+            auto full = [&](int s, int n) { return mbar_wait(su32(&bars.full[s]), (uint32_t)n & 1u); };
+            auto empty = [&](int s) { mma_commit(su32(&bars.empty[s])); };
+            auto times_state = [&](uint32_t d, uint32_t S, uint32_t tile) {       // D[dv][token] = sum_dk S[dv][dk] tile[token][dk]
+#pragma unroll
+                for (int ks = 0; ks < 16; ks++) mma_tf32_ts(d, S + 8 * ks, smem_desc(tile + (ks >> 2) * 8192 + (ks & 3) * 32, 16, 1024), ID_64, ks > 0);
+            };
+            // what a product needs beside the result it follows is waited for ahead of that result
             for (int n = 0; n < N; n++) {
-                const int s = n & 1;
-                const uint32_t kqs = base + SM_KQ + s * 65536, kq = tmem + TM_KQ + 128 * s;
-                ok = mbar_wait(su32(&bars.full_kq[s]), (uint32_t)(n >> 1) & 1u);
-                // this KS | QS buffer holds the output tiles of chunk n-2 until the output epilogue has read them
-                if (ok && n >= 2) ok = mbar_wait(su32(&bars.o_read[s]), (uint32_t)((n >> 1) - 1) & 1u);
+                const uint32_t S = tmem + TM_S + 128 * (n & 1), S2 = tmem + TM_S + 128 * ((n & 1) ^ 1);
+                ok = full(B_K, n) && full(B_V, n) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u));
                 if (!ok) break;
-                TR(0, n, 0);
+                fence_after();
+                times_state(tmem + TM_X, S, base + SM_K);                         // (K S^T)^T
+                mma_commit(su32(&bars.ks_done));
+                empty(B_K);
+                // U^T = (beta V)^T A^T + (K S^T)^T A'^T; U of the chunk before is an operand no more
+                ok = n == 0 || mbar_wait(su32(&bars.pu_done), (uint32_t)(n - 1) & 1u);
+                if (!ok) break;
+                const bool with_v = !(SEG && kind == 2);
+                if (with_v) {
+#pragma unroll
+                    for (int ks = 0; ks < 8; ks++)
+                        mma_tf32_ss(tmem + TM_U, smem_desc_mn32(base + SM_V + ks * 1024, 8192, 512),
+                                    smem_desc(base + SM_AV + (ks >> 2) * 8192 + (ks & 3) * 32, 16, 1024), ID_V, ks > 0);
+                }
+                empty(B_V);
+                ok = full(B_AK, n) && mbar_wait(su32(&bars.ks_done), (uint32_t)n & 1u);
+                if (!ok) break;
                 fence_after();
 #pragma unroll
-                for (int ks = 0; ks < 16; ks++)           // KS^T | QS^T = S [K ; Q]^T
-                    mma_tf32_ts(kq, tmem + TM_S + 8 * ks, smem_desc(kqs + (ks >> 2) * 16384 + (ks & 3) * 32, 16, 1024), ID_KQ, ks > 0);
-                mma_commit(su32(&bars.kq_done[s]));
-                mma_commit(su32(&bars.empty_kq[s]));
-                TR(0, n, 1);
-                // U^T of this chunk overwrites the U^T that (P U)^T of the previous chunk reads (issued by warp 18)
-                if (n >= 1) ok = mbar_wait(su32(&bars.pu_done[s ^ 1]), (uint32_t)((n - 1) >> 1) & 1u);
-                if (!ok) break;
-                TR(0, n, 3);
-                ok = mbar_wait(su32(&bars.full_a), (uint32_t)n & 1u) && mbar_wait(su32(&bars.t_ready), (uint32_t)n & 1u);
-                if (!ok) break;
-                TR(0, n, 4);
-                fence_after();
-                issue_tri(tmem + TM_U, tmem + TM_TU, base + SM_A);   // U^T = T^T A^T
+                for (int ks = 0; ks < 8; ks++)
+                    mma_tf32_ts(tmem + TM_U, tmem + TM_X + 8 * ks, smem_desc(base + SM_AK + (ks >> 2) * 8192 + (ks & 3) * 32, 16, 1024), ID_64,
+                                ks > 0 || with_v);
                 mma_commit(su32(&bars.u_done));
-                mma_commit(su32(&bars.empty_a));
-                TR(0, n, 5);
-                ok = mbar_wait(su32(&bars.full_km), (uint32_t)n & 1u) && mbar_wait(su32(&bars.u_ready), (uint32_t)n & 1u);
+                empty(B_AK);
+                // the tiles Q S^T and P U of the chunk before have been read
+                ok = full(B_Q, n) && (n == 0 || mbar_wait(su32(&bars.o_read), (uint32_t)(n - 1) & 1u));
                 if (!ok) break;
-                TR(0, n, 6);
+                fence_after();
+                times_state(tmem + TM_QS, S, base + SM_Q);                        // (Q S^T)^T, while the chain warps work on U
+                mma_commit(su32(&bars.qs_done));
+                empty(B_Q);
+                ok = full(B_KM, n) && mbar_wait(su32(&bars.wu_ready), (uint32_t)n & 1u);
+                if (!ok) break;
                 fence_after();
 #pragma unroll
-                for (int ks = 0; ks < 8; ks++)            // S += (w rk U)^T K, the K tile read MN-major
-                    mma_tf32_ts(tmem + TM_S, tmem + TM_TU + 8 * ks, smem_desc_mn32(base + SM_KM + ks * 1024, 8192, 512), ID_SU, 1u);
-                mma_commit(su32(&bars.empty_km));
-                TR(0, n, 7);
+                for (int ks = 0; ks < 8; ks++)            // S' += (w rk U)^T K, the K tile read MN-major
+                    mma_tf32_ts(S2, tmem + TM_X + 8 * ks, smem_desc_mn32(base + SM_KM + ks * 1024, 8192, 512), ID_SU, 1u);
+                mma_commit(su32(&bars.s_done));
+                empty(B_KM);
             }
-            mma_commit(su32(&bars.s_final));
+        }
+    } else if (warp == W_PU) {
+        // ================= (P U)^T =================
+        // P is lower triangular (layout: tri_at), rows 0..31 need tokens j < 32 only
+        if (elect_one()) {
+            constexpr uint32_t ID_32 = idesc(2, 32, false);
+            for (int n = 0; n < N; n++) {
+                ok = mbar_wait_parked(su32(&bars.full[B_P]), (uint32_t)n & 1u) && (n == 0 || mbar_wait_parked(su32(&bars.o_read), (uint32_t)(n - 1) & 1u)) &&
+                     mbar_wait_parked(su32(&bars.u_ready), (uint32_t)n & 1u);
+                if (!ok) break;
+                fence_after();
+#pragma unroll
+                for (int ks = 0; ks < 4; ks++) mma_tf32_ts(tmem + TM_PU, tmem + TM_U + 8 * ks, smem_desc(base + SM_P + ks * 32, 16, 1024), ID_32, ks > 0);
+#pragma unroll
+                for (int ks = 0; ks < 8; ks++)
+                    mma_tf32_ts(tmem + TM_PU + 32, tmem + TM_U + 8 * ks,
+                                smem_desc(base + SM_P + (ks < 4 ? 4096 + ks * 32 : 8192 + (ks - 4) * 32), 16, 1024), ID_32, ks > 0);
+                mma_commit(su32(&bars.pu_done));
+                mma_commit(su32(&bars.empty[B_P]));
+            }
         }
     } else if (warp < 8) {
-        // ================= chain epilogues: T, decay sweep, U =================
-        const float *Vs = reinterpret_cast<const float *>(gbase + SM_V) + 32 * half * 128 + row;   // Vs[i * 128] = V[token 32 half + i][row]
-        for (int n = 0; n < N && ok; n++) {
-            const int s = n & 1;
-            const float *aux = reinterpret_cast<const float *>(gbase + SM_AUX + s * AUX_BYTES);
-            ok = mbar_wait(su32(&bars.full_kq[s]), (uint32_t)(n >> 1) & 1u) && mbar_wait(su32(&bars.full_v), (uint32_t)n & 1u) &&
-                 mbar_wait(su32(&bars.kq_done[s]), (uint32_t)(n >> 1) & 1u);
+        // ================= chain: the decayed state, U =================
+        const uint32_t X = lane_t + TM_X + 32 * half, U = lane_t + TM_U + 32 * half;
+        for (int n = 0; n < N; n++) {
+            const float *fac = reinterpret_cast<const float *>(gbase + SM_F + (n % NFAC) * FAC_BYTES);
+            const uint32_t S = lane_t + TM_S + 128 * (n & 1) + 64 * half, S2 = lane_t + TM_S + 128 * ((n & 1) ^ 1) + 64 * half;
+            ok = mbar_wait(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u));
             if (!ok) break;
-            if (tid == 0) TR(1, n, 0);
             fence_after();
             float x[32];
-            if (dbg && n == 1) {                                         // the state after the first update (before this chunk's decay)
+            {   // the other state = p_63 S, while the tensor core reads S (the update is accumulated onto it)
+                const float pend = fac[2 * C];
+                const f32x2 p2 = pack2(pend, pend);
 #pragma unroll 1
                 for (int cc = 0; cc < 2; cc++) {
-                    tmem_ld32_wait(lane_t + TM_S + 64 * half + 32 * cc, x);
+                    tmem_ld32_wait(S + 32 * cc, x);
 #pragma unroll
-                    for (int i = 0; i < 32; i++) dbg[4 * 128 * 64 + row * 128 + 64 * half + 32 * cc + i] = x[i];
+                    for (int i = 0; i < 32; i += 2) { const f32x2 y = mul2(p2, pack2(x[i], x[i + 1])); unpack2(y, &x[i], &x[i + 1]); }
+                    tmem_st32(S2 + 32 * cc, x);
                 }
             }
-            tmem_ld32_wait(lane_t + TM_KQ + 128 * s + 32 * half, x);          // KS^T
-            if (tid == 0) TR(4, n, 0);
-            if (dbg && n == 0) {
-#pragma unroll
-                for (int i = 0; i < 32; i++) dbg[row * 64 + 32 * half + i] = x[i];
-            }
-#pragma unroll
-            for (int hh = 0; hh < 4; hh++) {                             // T = beta v - (beta p rk) KS, 8 tokens at a time
-                float v[8];
-#pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = (SEG && kind == 2) ? 0.0f : Vs[(8 * hh + i) * 128];
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    const float4 be4 = *reinterpret_cast<const float4 *>(aux + 32 * half + 8 * hh + 4 * i);
-                    const float4 bp4 = *reinterpret_cast<const float4 *>(aux + C + 32 * half + 8 * hh + 4 * i);
-                    const int k = 8 * hh + 4 * i;
-                    x[k] = tf32q(fmaf(-bp4.x, x[k], be4.x * v[4 * i]));
-                    x[k + 1] = tf32q(fmaf(-bp4.y, x[k + 1], be4.y * v[4 * i + 1]));
-                    x[k + 2] = tf32q(fmaf(-bp4.z, x[k + 2], be4.z * v[4 * i + 2]));
-                    x[k + 3] = tf32q(fmaf(-bp4.w, x[k + 3], be4.w * v[4 * i + 3]));
-                }
-            }
-            if (tid == 0) TR(4, n, 1);
-            tmem_st32(lane_t + TM_TU + 32 * half, x);                    // T^T
-            tmem_wait_st();
-            if (tid == 0) TR(4, n, 2);
-            fence_before();
-            mbar_arrive(su32(&bars.t_ready));
-            if (tid == 0) TR(1, n, 1);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(su32(&bars.empty_v));             // this warp has read its V rows
-            if (tid == 0) TR(1, n, 2);
-            {   // S *= p_63 while the tensor core computes U^T (nothing reads S until the update)
-                const float pend = aux[4 * C];
-#pragma unroll 1
-                for (int cc = 0; cc < 2; cc++) {
-                    tmem_ld32_wait(lane_t + TM_S + 64 * half + 32 * cc, x);
-#pragma unroll
-                    for (int i = 0; i < 32; i++) x[i] *= pend;
-                    tmem_st32(lane_t + TM_S + 64 * half + 32 * cc, x);
-                }
-            }
-            if (tid == 0) TR(1, n, 3);
             ok = mbar_wait(su32(&bars.u_done), (uint32_t)n & 1u);
             if (!ok) break;
-            if (tid == 0) TR(1, n, 4);
             fence_after();
-            tmem_ld32_wait(lane_t + TM_U + 32 * half, x);                     // U^T
-            if (tid == 0) TR(4, n, 3);
-            if (dbg && n == 0) {
+            tmem_ld32_wait(U, x);                                        // U^T
+            fac += 32 * half;
+            // (w rk U)^T over (K S^T)^T first: the state update waits for it
 #pragma unroll
-                for (int i = 0; i < 32; i++) dbg[128 * 64 + row * 64 + 32 * half + i] = x[i];
-            }
-#pragma unroll
-            for (int hh = 0; hh < 4; hh++) {                             // (w rk U)^T over T^T, 8 tokens at a time
+            for (int hh = 0; hh < 4; hh++) {                             // 8 tokens at a time
                 float f[8];
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
-                    const float4 w4 = *reinterpret_cast<const float4 *>(aux + 2 * C + 32 * half + 8 * hh + 4 * i);   // w rk
-                    f[4 * i] = tf32q(w4.x * x[8 * hh + 4 * i]); f[4 * i + 1] = tf32q(w4.y * x[8 * hh + 4 * i + 1]);
-                    f[4 * i + 2] = tf32q(w4.z * x[8 * hh + 4 * i + 2]); f[4 * i + 3] = tf32q(w4.w * x[8 * hh + 4 * i + 3]);
+                    const float4 w4 = *reinterpret_cast<const float4 *>(fac + 8 * hh + 4 * i);   // w rk
+                    const float *t = x + 8 * hh + 4 * i;
+                    const f32x2 t0 = mul2(pack2(w4.x, w4.y), pack2(t[0], t[1])), t1 = mul2(pack2(w4.z, w4.w), pack2(t[2], t[3]));
+                    unpack2(t0, f + 4 * i, f + 4 * i + 1);
+                    unpack2(t1, f + 4 * i + 2, f + 4 * i + 3);
                 }
-                tmem_st8(lane_t + TM_TU + 32 * half + 8 * hh, f);
+#pragma unroll
+                for (int i = 0; i < 8; i++) f[i] = tf32q(f[i]);
+                tmem_st8(X + 8 * hh, f);
             }
+            tmem_wait_st();
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(su32(&bars.wu_ready));
 #pragma unroll
             for (int i = 0; i < 32; i++) x[i] = tf32q(x[i]);
-            if (tid == 0) TR(4, n, 4);
-            tmem_st32(lane_t + TM_U + 32 * half, x);                     // tf32 U^T over the accumulator
+            tmem_st32(U, x);                                             // tf32 U^T over the accumulator
             tmem_wait_st();
-            if (tid == 0) TR(4, n, 5);
             fence_before();
-            mbar_arrive(su32(&bars.u_ready));
-            if (tid == 0) TR(1, n, 5);
             __syncwarp();
-            if (lane == 0) mbar_arrive(su32(&bars.empty_kq[s]));         // this warp has read its factors
+            if (lane == 0) mbar_arrive(su32(&bars.u_ready));
         }
-        ok = ok && mbar_wait(su32(&bars.s_final), 0u);
+        ok = ok && mbar_wait(su32(&bars.s_done), (uint32_t)(N - 1) & 1u);
         fence_after();
 #pragma unroll 1
         for (int cc = 0; cc < 2; cc++) {                                 // the state goes home
             float x[32];
-            tmem_ld32_wait(lane_t + TM_S + 64 * half + 32 * cc, x);
+            tmem_ld32_wait(lane_t + TM_S + 128 * (N & 1) + 64 * half + 32 * cc, x);
             float4 *dst = reinterpret_cast<float4 *>(Sout + (size_t)row * 128 + 64 * half + 32 * cc);
 #pragma unroll
             for (int i = 0; i < 8; i++)
                 dst[i] = ok ? make_float4(x[4 * i], x[4 * i + 1], x[4 * i + 2], x[4 * i + 3]) : make_float4(NAN, NAN, NAN, NAN);
         }
-    } else if (warp < 24) {
-        // ================= output epilogue =================
-        // 16 warps: lane quarter qtr, group grp of 16 tokens
-        const int grp = (warp - 8) >> 2;
-        const float nwr = a.norm_w[row];
-        const size_t zoff = (size_t)b * a.T * vd + (size_t)hv * 128 + row;
+    } else if (warp < W_TMA) {
+        // ================= output =================
+        // 16 warps: lane quarter qtr, group grp of 16 tokens.  A thread (g, j) has the rows 8 k + g of the quarter (k = 0..3) and the
+        // tokens 8 m + 2 j + c of the group (m, c = 0, 1): value 8 m + 2 k + c
+        constexpr bool TILE_O = TILE && sizeof(ACT) == 2;
+        const int grp = (warp - 8) >> 2, g = lane >> 2, j = lane & 3;
+        float nw[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) nw[k] = a.norm_w[32 * qtr + 8 * k + g];
         const ACT *zp = (const ACT *)a.z;
         ACT *op = (ACT *)a.out;
-        const float *aux = reinterpret_cast<const float *>(gbase + SM_AUX2) + 3 * C + 16 * grp;       // p rq of this group's tokens
-        const uint32_t t_qs = lane_t + TM_KQ + 64 + 16 * grp, t_pu = lane_t + TM_KQ + 16 * grp;
-        // z of this thread's 16 outputs of a chunk is requested one chunk ahead and stays in these registers until it
-        // is used: the loads (DRAM latency, 2 bytes per lane) would otherwise be exposed in every chunk.  The output
-        // tiles are read from tensor memory twice (for the sum of squares, then for the store) instead of being kept.
-        uint32_t zr[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++)
-            zr[i] = (!(SEG && kind) && c0 * C + 16 * grp + i < a.T) ? ld_raw(zp, zoff + (size_t)(c0 * C + 16 * grp + i) * vd) : 0u;
+        const size_t gofs = ((size_t)b * a.T + 2 * j) * vd + (size_t)hv * 128 + 32 * qtr + g;       // + (token of the group's first) vd + 8 k + ..
+        const uint32_t t_qs = lane_t + TM_QS + 16 * grp, t_pu = lane_t + TM_PU + 16 * grp;
+        // z and the outputs in shared memory: rows of 128 bytes per token, 128-byte swizzle, 64 (bf16) or 32 (f32) channels to a
+        // tile of 8 KiB: the 16-byte pieces of a row change places by its number modulo 8.  bf16: the address of the 8 x 8 matrix row
+        // this lane names (matrix lane >> 3 = channels 8 (lane >> 3) .., row = token lane & 7); f32: this thread's element, k = c = 0
+        const uint32_t zoff = sizeof(ACT) == 2
+            ? (qtr >> 1) * 8192 + (16 * grp + (lane & 7)) * 128 + (((4 * (qtr & 1) + (lane >> 3)) ^ (lane & 7)) * 16)
+            : qtr * 8192 + (16 * grp + 2 * j) * 128 + ((g >> 2) ^ (2 * j)) * 16 + (g & 3) * 4;
         int n = 0;
-        if (SEG && kind) {
-            // raw outputs p rq QS + P U of a run scanned from zero / from the identity: no norm, no gate
-            for (; n < N; n++) {
-                const int s = n & 1, tok = (c0 + n) * C + 16 * grp;
-                ok = mbar_wait(su32(&bars.full_p), (uint32_t)n & 1u) && mbar_wait(su32(&bars.pu_done[s]), (uint32_t)(n >> 1) & 1u);
-                if (!ok) break;
-                fence_after();
-                float q[16], x[16];
-                tmem_ld16x2_wait(t_qs + 128 * s, q, t_pu + 128 * s, x);
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const float4 p4 = *reinterpret_cast<const float4 *>(aux + 4 * i);
-                    x[4 * i] = fmaf(p4.x, q[4 * i], x[4 * i]); x[4 * i + 1] = fmaf(p4.y, q[4 * i + 1], x[4 * i + 1]);
-                    x[4 * i + 2] = fmaf(p4.z, q[4 * i + 2], x[4 * i + 2]); x[4 * i + 3] = fmaf(p4.w, q[4 * i + 3], x[4 * i + 3]);
-                }
-                fence_before();
-                mbar_arrive(su32(&bars.o_read[s]));
-                __syncwarp();
-                if (lane == 0) mbar_arrive(su32(&bars.empty_p));
-#pragma unroll
-                for (int i = 0; i < 16; i++)
-                    if (tok + i < a.T) raw[(size_t)(tok + i) * 128 + row] = x[i];
-            }
-            n = N;                                                       // nothing to poison: the finishing kernel reads the status
-        }
         for (; n < N; n++) {
             const int s = n & 1, tok = (c0 + n) * C + 16 * grp;
-            if (tid == 256) TR(2, n, 0);
-            // the gate factors of this chunk, while the tensor core still works on it: norm weight x SiLU(z), in place
+            float zr[16];
+            if (!(SEG && kind)) {
+                // the gate factors of this chunk, while the tensor core still works on it: norm weight x SiLU(z)
+                if (TILE) {
+                    ok = mbar_wait_parked(su32(&bars.full_z), (uint32_t)n & 1u);
+                    if (!ok) break;
 #pragma unroll
-            for (int h8 = 0; h8 < 2; h8++) {
+                    for (int m = 0; m < 2; m++) {
+                        if (sizeof(ACT) == 2) {
+                            uint32_t r[4];
+                            ldmatrix_x4_trans(r, base + SM_Z + zoff + m * 1024);
 #pragma unroll
-                for (int i = 0; i < 8; i++) zr[8 * h8 + i] = __float_as_uint(nwr * silu_fast(cvt_raw(zp, zr[8 * h8 + i])));
-                asm volatile("" ::: "memory");                           // keeps the two batches apart (registers)
-            }
-            ok = mbar_wait(su32(&bars.full_p), (uint32_t)n & 1u) && mbar_wait(su32(&bars.pu_done[s]), (uint32_t)(n >> 1) & 1u);
-            if (!ok) break;
-            if (tid == 256) TR(2, n, 1);
-            fence_after();
-            {
-                float x[16];
+                            for (int k = 0; k < 4; k++) { zr[8 * m + 2 * k] = __uint_as_float(r[k] << 16); zr[8 * m + 2 * k + 1] = __uint_as_float(r[k] & 0xFFFF0000u); }
+                        } else {
 #pragma unroll
-                for (int h8 = 0; h8 < 2; h8++) {                         // 8 tokens at a time: O = p rq QS + P U, squared
-                    float q[8], y[8];
-                    tmem_ld8x2_wait(t_qs + 128 * s + 8 * h8, q, t_pu + 128 * s + 8 * h8, y);   // QS^T, (P U)^T
-                    if (dbg && n == 0) {
-#pragma unroll
-                        for (int i = 0; i < 8; i++) {
-                            dbg[2 * 128 * 64 + row * 64 + 16 * grp + 8 * h8 + i] = q[i];
-                            dbg[3 * 128 * 64 + row * 64 + 16 * grp + 8 * h8 + i] = y[i];
+                            for (int i = 0; i < 8; i++)
+                                zr[8 * m + i] = *reinterpret_cast<const float *>(gbase + SM_Z + ((zoff ^ ((i >> 1) * 32)) ^ ((i & 1) * 16)) + (i & 1) * 128 + m * 1024);
                         }
                     }
-#pragma unroll
-                    for (int i = 0; i < 2; i++) {
-                        const float4 p4 = *reinterpret_cast<const float4 *>(aux + 8 * h8 + 4 * i);
-                        y[4 * i] = fmaf(p4.x, q[4 * i], y[4 * i]); y[4 * i + 1] = fmaf(p4.y, q[4 * i + 1], y[4 * i + 1]);
-                        y[4 * i + 2] = fmaf(p4.z, q[4 * i + 2], y[4 * i + 2]); y[4 * i + 3] = fmaf(p4.w, q[4 * i + 3], y[4 * i + 3]);
-                    }
-#pragma unroll
-                    for (int i = 0; i < 8; i++) x[8 * h8 + i] = y[i] * y[i];
-                }
-                // sum of squares over the 32 rows of this warp: token t of the 16 ends up in lanes t and t + 16
-#pragma unroll
-                for (int i = 0; i < 16; i++) x[i] += __shfl_xor_sync(0xffffffffu, x[i], 16);
-#pragma unroll
-                for (int off = 8; off >= 1; off >>= 1) {
-                    const bool up = (lane & off) != 0;
-#pragma unroll
-                    for (int k = 0; k < off; k++) {
-                        const float send = up ? x[k] : x[k + off], keep = up ? x[k + off] : x[k];
-                        x[k] = keep + __shfl_xor_sync(0xffffffffu, send, off);
-                    }
-                }
-                if (lane < 16) red[s][grp][qtr][lane] = x[0];
-            }
-            if (tid == 256) TR(2, n, 2);
-            mbar_arrive(su32(&bars.red[s][grp]));
-            if (tid == 256) TR(2, n, 3);
-            ok = mbar_wait(su32(&bars.red[s][grp]), (uint32_t)(n >> 1) & 1u);
-            if (!ok) break;
-            if (tid == 256) TR(2, n, 4);
-            const int tl = lane & 15;
-            const float ss = a.out_scale * a.out_scale *
-                             ((red[s][grp][0][tl] + red[s][grp][1][tl]) + (red[s][grp][2][tl] + red[s][grp][3][tl]));
-            const float inv = rsqrtf(ss * (1.0f / 128.0f) + a.eps) * a.out_scale;   // of token tl
-#pragma unroll
-            for (int ps = 0; ps < 2; ps++) {                             // 8 tokens at a time
-                float q[8], x[8];
-                tmem_ld8x2_wait(t_qs + 128 * s + 8 * ps, q, t_pu + 128 * s + 8 * ps, x);
-#pragma unroll
-                for (int i = 0; i < 2; i++) {
-                    const float4 p4 = *reinterpret_cast<const float4 *>(aux + 8 * ps + 4 * i);
-                    x[4 * i] = fmaf(p4.x, q[4 * i], x[4 * i]); x[4 * i + 1] = fmaf(p4.y, q[4 * i + 1], x[4 * i + 1]);
-                    x[4 * i + 2] = fmaf(p4.z, q[4 * i + 2], x[4 * i + 2]); x[4 * i + 3] = fmaf(p4.w, q[4 * i + 3], x[4 * i + 3]);
-                }
-                if (ps == 1) {                                           // both tiles and the factors have been read for the last time
-                    fence_before();
-                    mbar_arrive(su32(&bars.o_read[s]));
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(su32(&bars.empty_p));
-                }
-                // Whole groups of 8 tokens take the path without per-token bounds checks: a conditional store per token
-                // would end a basic block per token and keep the independent chains (shuffle, exp, reciprocal) from
-                // overlapping.
-                const size_t o0 = zoff + (size_t)(tok + 8 * ps) * vd;
-#pragma unroll
-                for (int i = 0; i < 8; i++) x[i] *= __shfl_sync(0xffffffffu, inv, 8 * ps + i) * __uint_as_float(zr[8 * ps + i]);
-                if (tok + 8 * ps + 8 <= a.T) {
-#pragma unroll
-                    for (int i = 0; i < 8; i++) act_st(op, o0 + (size_t)i * vd, x[i]);
+                    if (lane == 0) mbar_arrive(su32(&bars.empty_z));
                 } else {
 #pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        if (tok + 8 * ps + i < a.T) act_st(op, o0 + (size_t)i * vd, x[i]);
+                    for (int i = 0; i < 16; i++) {
+                        const int k = (i >> 1) & 3, t = tok + 8 * (i >> 3) + (i & 1);
+                        zr[i] = t + 2 * j < a.T ? cvt_raw(zp, ld_raw(zp, gofs + (size_t)t * vd + 8 * k)) : 0.0f;
+                    }
                 }
-                if (tok + C + 8 * ps + 8 <= a.T) {                       // the same tokens of the next chunk
 #pragma unroll
-                    for (int i = 0; i < 8; i++) zr[8 * ps + i] = ld_raw(zp, o0 + (size_t)(C + i) * vd);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        zr[8 * ps + i] = (tok + C + 8 * ps + i < a.T) ? ld_raw(zp, o0 + (size_t)(C + i) * vd) : 0u;
+                for (int i = 0; i < 16; i += 2) {
+                    const f32x2 z2 = pack2(zr[i], zr[i + 1]), e2 = mul2(z2, pack2(-LOG2E_F, -LOG2E_F));
+                    float e0, e1;
+                    unpack2(e2, &e0, &e1);
+                    unpack2(add2(pack2(ex2_fast(e0), ex2_fast(e1)), pack2(1.0f, 1.0f)), &e0, &e1);
+                    const float w = nw[(i >> 1) & 3];
+                    unpack2(mul2(mul2(z2, pack2(w, w)), pack2(rcp_fast(e0), rcp_fast(e1))), &zr[i], &zr[i + 1]);
                 }
             }
-            if (tid == 256) TR(2, n, 5);
+            ok = mbar_wait_parked(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && mbar_wait_parked(su32(&bars.qs_done), (uint32_t)n & 1u) &&
+                 mbar_wait_parked(su32(&bars.pu_done), (uint32_t)n & 1u);
+            if (!ok) break;
+            fence_after();
+            float x[16];                                                 // O = p rq QS + P U
+            {
+                const float *pq = reinterpret_cast<const float *>(gbase + SM_F + (n % NFAC) * FAC_BYTES) + C + 16 * grp + 2 * j;
+                float q[16];
+                tmem_ld_16x256_wait(t_qs, q, t_pu, x);
+                const float2 pa = *reinterpret_cast<const float2 *>(pq), pb = *reinterpret_cast<const float2 *>(pq + 8);
+                const float back = SEG && kind == 2 && n == 0 ? 1.0f / S_DROP : 1.0f;        // (the identity loses nothing when read)
+                const f32x2 p2[2] = {pack2(pa.x * back, pa.y * back), pack2(pb.x * back, pb.y * back)};
+#pragma unroll
+                for (int i = 0; i < 16; i += 2) unpack2(fma2(p2[i >> 3], pack2(q[i], q[i + 1]), pack2(x[i], x[i + 1])), &x[i], &x[i + 1]);
+            }
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(su32(&bars.o_read));              // the tensor core may overwrite both tiles
+            if (SEG && kind) {                                           // raw outputs of a run scanned from zero / from the identity: no norm, no gate
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int k = (i >> 1) & 3, t = tok + 8 * (i >> 3) + 2 * j + (i & 1);
+                    if (t < a.T) raw[(size_t)t * 128 + 32 * qtr + 8 * k + g] = x[i];
+                }
+                continue;
+            }
+            {
+                // sum of squares: over the thread's rows, then over the 8 lanes of a j; lane (bit 4 = m, bit 3 = c, j) ends up with token
+                // 8 m + 2 j + c of the group
+                f32x2 s0 = 0, s1 = 0;
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const f32x2 a0 = pack2(x[2 * k], x[2 * k + 1]), a1 = pack2(x[8 + 2 * k], x[8 + 2 * k + 1]);
+                    s0 = fma2(a0, a0, s0);
+                    s1 = fma2(a1, a1, s1);
+                }
+                float v00, v01, v10, v11;
+                unpack2(s0, &v00, &v01);
+                unpack2(s1, &v10, &v11);
+                const bool hm = lane & 16, hc = lane & 8;
+                float a0 = hm ? v10 : v00, a1 = hm ? v11 : v01;
+                a0 += __shfl_xor_sync(0xffffffffu, hm ? v00 : v10, 16);
+                a1 += __shfl_xor_sync(0xffffffffu, hm ? v01 : v11, 16);
+                float b0 = hc ? a1 : a0;
+                b0 += __shfl_xor_sync(0xffffffffu, hc ? a0 : a1, 8);
+                b0 += __shfl_xor_sync(0xffffffffu, b0, 4);
+                if ((lane & 4) == 0) red[s][grp][8 * (lane >> 4) + 2 * j + ((lane >> 3) & 1)][qtr] = b0;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(su32(&bars.red[s][grp]));
+            ok = mbar_wait_parked(su32(&bars.red[s][grp]), (uint32_t)(n >> 1) & 1u);
+            if (!ok) break;
+            const float4 r4 = *reinterpret_cast<const float4 *>(&red[s][grp][8 * (lane >> 4) + 2 * j + ((lane >> 3) & 1)][0]);
+            const float ss = a.out_scale * a.out_scale * ((r4.x + r4.y) + (r4.z + r4.w));
+            const float inv = rsqrtf(ss * (1.0f / 128.0f) + a.eps) * a.out_scale;   // of this lane's token
+            f32x2 i2[2];
+#pragma unroll
+            for (int m = 0; m < 2; m++) i2[m] = pack2(__shfl_sync(0xffffffffu, inv, 16 * m + j), __shfl_sync(0xffffffffu, inv, 16 * m + 8 + j));
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) unpack2(mul2(mul2(pack2(x[i], x[i + 1]), i2[i >> 3]), pack2(zr[i], zr[i + 1])), &x[i], &x[i + 1]);
+            if (TILE_O) {
+                if (n >= 1) ok = mbar_wait_parked(su32(&bars.o_free[grp]), (uint32_t)(n - 1) & 1u);     // the group's rows of the chunk before have left
+                if (!ok) break;
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+                    uint32_t r[4];
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const __nv_bfloat162 o2 = __floats2bfloat162_rn(x[8 * m + 2 * k], x[8 * m + 2 * k + 1]);
+                        r[k] = *reinterpret_cast<const uint32_t *>(&o2);
+                    }
+                    stmatrix_x4_trans(base + SM_O + zoff + m * 1024, r);
+                }
+                fence_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(su32(&bars.o_full[grp]));
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; i++) {
+                    const int k = (i >> 1) & 3, t = tok + 8 * (i >> 3) + (i & 1);
+                    if (t + 2 * j < a.T) act_st(op, gofs + (size_t)t * vd + 8 * k, x[i]);
+                }
+            }
         }
-        for (; n < N; n++) {                                             // a wait gave up: poison what was not written
-            const int tok = n * C + 16 * grp;
-            for (int i = 0; i < 16; i++)
-                if (tok + i < a.T) act_st(op, zoff + (size_t)(tok + i) * vd, NAN);
+        for (; n < N && !(SEG && kind); n++) {                           // a wait gave up: poison what was not written
+            const int tok = (c0 + n) * C + 16 * grp;
+            for (int i = 0; i < 16; i++) {
+                const int kk = (i >> 1) & 3, t = tok + 8 * (i >> 3) + (i & 1);
+                if (t + 2 * j < a.T) act_st(op, gofs + (size_t)t * vd + 8 * kk, NAN);
+            }
         }
     }
-    else {
-        // ================= (P U)^T, issued apart from the chain =================
-        // Its operand U^T is ready at the same moment as the state update's; a thread of its own keeps these
-        // eight instructions out of the issue stream the next chunk waits for.
-        if (warp == W_PU && lane == 0) {
-            fence_after();
-            for (int n = 0; n < N; n++) {
-                ok = mbar_wait(su32(&bars.full_p), (uint32_t)n & 1u) && mbar_wait(su32(&bars.u_ready), (uint32_t)n & 1u);
-                if (!ok) break;
-                fence_after();
-                issue_tri(tmem + TM_KQ + 128 * (n & 1), tmem + TM_U, base + SM_P);   // over the KS columns of the chunk
-                mma_commit(su32(&bars.pu_done[n & 1]));
-                mma_commit(su32(&bars.empty_p));
+    if (warp == W_IO) {
+        // ================= z, outputs, L2 =================
+        if (elect_one()) {
+            asm volatile("griddepcontrol.wait;\n" ::: "memory");
+            constexpr int TZ = (int)sizeof(ACT), CZ = 128 / TZ;           // tiles of z: their number, their channels
+            const bool out = TILE && !(SEG && kind);
+            const unsigned char *rec0 = a.rec + (((size_t)b * a.nv + hv) * a.rec_chunks + (SEG ? c0 : 0)) * (size_t)REC_BYTES;
+            auto l2_2d = [&](int x, int y) {
+                asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&map_ym), "r"(x), "r"(y) : "memory");
+            };
+            auto ahead = [&](int n) {                                     // (K and Q rows are shared by the value heads of a key head)
+                if (n >= N) return;
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rec0 + (size_t)n * REC_BYTES), "r"((uint32_t)REC_BYTES) : "memory");
+                for (int sl = 0; sl < 4; sl++) l2_2d(2 * qd + hv * 128 + 32 * sl, b * a.T + (c0 + n) * C);
+                if (out)
+                    for (int t = 0; t < TZ; t++)
+                        asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                                     ::"l"(&map_z), "r"(hv * 128 + t * CZ), "r"((c0 + n) * C), "r"(b) : "memory");
+            };
+            auto load_z = [&](int n) {
+                mbar_expect_tx(su32(&bars.full_z), (uint32_t)(C * 128 * TZ));
+                for (int t = 0; t < TZ; t++)
+                    tma_load_3d(base + SM_Z + t * 8192, &map_z, hv * 128 + t * CZ, (c0 + n) * C, b, su32(&bars.full_z));
+            };
+            ahead(1);
+            if (out) load_z(0);
+            for (int n = 0; n < N && ok; n++) {
+                ahead(n + 2);
+                if (!out) { ok = mbar_wait_parked(su32(&bars.ks_done), (uint32_t)n & 1u); continue; }      // (no faster than the scan)
+                ok = mbar_wait_parked(su32(&bars.empty_z), (uint32_t)n & 1u);
+                if (ok && n + 1 < N) load_z(n + 1);
+                if (TZ == 2 && ok) {
+                    for (int g = 0; g < 4 && ok; g++) {
+                        ok = mbar_wait_parked(su32(&bars.o_full[g]), (uint32_t)n & 1u);
+                        const int tok = (c0 + n) * C + 16 * g;
+                        if (ok && tok < a.T) {                           // (rows past T are left out by the copy)
+#pragma unroll
+                            for (int hf = 0; hf < 2; hf++)
+                                asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
+                                             ::"l"(&map_o), "r"(base + SM_O + hf * 8192 + g * 2048), "r"(hv * 128 + hf * 64), "r"(tok), "r"(b) : "memory");
+                        }
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    for (int g = 0; g < 4; g++) mbar_arrive(su32(&bars.o_free[g]));
+                }
             }
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");    // shared memory outlives the copies
         }
     }
     if (!ok) report_timeout(a.status, ORN_WAIT_DELTA_SCAN);
@@ -855,6 +946,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     __syncthreads();
     if (warp == W_MMA) tmem_dealloc(tmem, TM_COLS);
 }
+
 
 // =============================================================================
 // segment-parallel form: carrying the state over the runs, and the finishing pass
@@ -999,18 +1091,23 @@ __global__ void __launch_bounds__(128, 2) k_delta_seg_finish(ScanArgs a) {
     }
 }
 
-// How many runs the prompt is cut into: only when the heads alone would leave most SMs idle (2 P - 1 CTAs per
-// head), with at least 8 chunks per run.  ORNITH_CUDA_DELTA_SEGMENTS=<n> forces a count (1 = off).
+// How many runs the prompt is cut into: only when the heads alone would leave most SMs idle (2 P - 1 CTAs per head), with at least 16
+// chunks per run, and not into two: every run but the first is scanned twice and finished by two more kernels.  us, one run | the
+// best cut: 32 heads x 4096 tokens 219 | 245, 8192 402 | 427; 16 heads x 1024 tokens 60 | 97, 4096 187 | 190, 8192 350 | 296;
+// 8 heads x 2048 92 | 110, 4096 166 | 146, 32768 1206 | 527.  ORNITH_CUDA_DELTA_SEGMENTS=<n> forces a count (1 = off).
 int delta_seg_plan(int nv, int n_seq, int n_chunks, int *seg_chunks) {
     int p = 1;
     const char *e = getenv("ORNITH_CUDA_DELTA_SEGMENTS");
-    if (e && e[0]) p = atoi(e);
-    else {
+    if (e && e[0]) {
+        p = atoi(e);
+        if (p > n_chunks / 8) p = n_chunks / 8;
+    } else {
         const int heads = nv * n_seq;
-        if (heads <= 37) p = (148 / heads + 1) / 2;                  // 2 p - 1 <= 148 / heads
+        if (heads <= 29) p = (148 / heads + 1) / 2;                  // 2 p - 1 <= 148 / heads
         if (p > 16) p = 16;
+        if (p > n_chunks / 16) p = n_chunks / 16;
+        if (p == 2) p = 1;
     }
-    if (p > n_chunks / 8) p = n_chunks / 8;
     if (p < 1) p = 1;
     int sc = (n_chunks + p - 1) / p;
     p = (n_chunks + sc - 1) / sc;                                     // no empty run
@@ -1018,48 +1115,81 @@ int delta_seg_plan(int nv, int n_seq, int n_chunks, int *seg_chunks) {
     return p;
 }
 
-// [rows][cols] f32, boxes of box_cols columns x box_rows rows; swz 0: no swizzle, 1: 128-byte swizzle, 2: the same with 32-byte atoms
-ornith_status f32_rows_map(CUtensorMap *m, const void *basep, uint64_t cols, uint64_t rows, uint32_t box_rows, int swz, uint32_t box_cols = 32) {
+// [rows][cols] f32, boxes of 32 columns x box_rows rows; 128-byte swizzle, in 16-byte or in 32-byte atoms
+ornith_status f32_rows_map(CUtensorMap *m, const void *basep, uint64_t cols, uint64_t rows, uint32_t box_rows, bool atom32) {
     OrnTensorMapEncodeFn enc = orn_tensor_map_encoder();
     if (!enc) { orn_record_error("delta scan: cuTensorMapEncodeTiled is not available"); return (ornith_status)ORNITH_ERR_BACKEND; }
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
-    cuuint32_t box[2] = {box_cols, box_rows};
+    cuuint32_t box[2] = {32, box_rows};
     cuuint32_t es[2] = {1, 1};
     const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(basep), dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           swz == 2 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : (swz == 1 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE),
+                           atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) { orn_record_error("delta scan: cuTensorMapEncodeTiled failed (%d)", (int)r); return (ornith_status)ORNITH_ERR_BACKEND; }
+    return ORNITH_OK;
+}
+
+// [n_seq][T][width] activations: boxes of 128 bytes of channels x `rows` tokens of one sequence, 128-byte swizzle
+ornith_status act_rows_map(CUtensorMap *m, const void *basep, bool bf, uint64_t width, uint64_t T, uint64_t n_seq, uint32_t rows) {
+    OrnTensorMapEncodeFn enc = orn_tensor_map_encoder();
+    if (!enc) { orn_record_error("delta scan: cuTensorMapEncodeTiled is not available"); return (ornith_status)ORNITH_ERR_BACKEND; }
+    const uint64_t row = width * (bf ? 2 : 4);
+    cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)T, (cuuint64_t)n_seq};
+    cuuint64_t strides[2] = {(cuuint64_t)row, (cuuint64_t)(row * T)};
+    cuuint32_t box[3] = {bf ? 64u : 32u, rows, 1};
+    cuuint32_t es[3] = {1, 1, 1};
+    const CUresult r = enc(m, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(basep), dims, strides, box, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { orn_record_error("delta scan: cuTensorMapEncodeTiled failed (%d)", (int)r); return (ornith_status)ORNITH_ERR_BACKEND; }
     return ORNITH_OK;
 }
 
 }  // namespace
 
-static size_t ap_part(int nv, int n_seq, int n_chunks) { return align_up((size_t)n_seq * nv * n_chunks * AP_BYTES, 256); }
-static size_t aux_part(int nv, int n_seq, int n_chunks) { return align_up((size_t)n_seq * nv * n_chunks * AUX_BYTES, 256); }
+// How a prompt is cut: into runs scanned side by side (n_seg > 1), or into slabs of `per` chunks, whose records take `slots`
+// places in turn.
+struct DeltaPlan { int n_chunks, n_seg, seg_chunks, per, slots; };
 
-static size_t seg_state_part(int nv, int n_seq, int n_seg) { return n_seg > 1 ? align_up((size_t)n_seq * nv * 3 * n_seg * 128 * 128 * 4, 256) : 0; }
-static size_t seg_raw_part(int nv, int n_seq, int T, int n_seg) { return n_seg > 1 ? align_up((size_t)2 * n_seq * nv * T * 128 * 4, 256) : 0; }
+static int slab_plan(int heads, int n_chunks, int n_seg);
+
+static DeltaPlan delta_plan(int nv, int n_seq, int T) {
+    DeltaPlan p;
+    p.n_chunks = (T + C - 1) / C;
+    const int units = nv * n_seq;
+    p.n_seg = delta_seg_plan(nv, n_seq, p.n_chunks, &p.seg_chunks);
+    p.per = p.n_chunks;
+    p.slots = 1;
+    if (p.n_seg > 1) return p;
+    const int n = slab_plan(units, p.n_chunks, p.n_seg);
+    if (n > 1) {                                                      // the pipeline: one slab is scanned while the next is prepared
+        p.per = (p.n_chunks + n - 1) / n;
+        p.slots = 2;
+    }
+    return p;
+}
+
+static size_t rec_part(const DeltaPlan &p, int units) { return align_up((size_t)p.slots * units * p.per * REC_BYTES, 256); }
+static size_t seg_state_part(int units, int n_seg) { return n_seg > 1 ? align_up((size_t)units * 3 * n_seg * 128 * 128 * 4, 256) : 0; }
+static size_t seg_raw_part(int units, int T, int n_seg) { return n_seg > 1 ? align_up((size_t)2 * units * T * 128 * 4, 256) : 0; }
 
 size_t linear_prefill_tc5_work_bytes(int nk, int nv, int n_seq, int T) {
-    const int n_chunks = (T + C - 1) / C;
     (void)nk;
-    int sc;
-    const int n_seg = delta_seg_plan(nv, n_seq, n_chunks, &sc);
-    return ap_part(nv, n_seq, n_chunks) + aux_part(nv, n_seq, n_chunks) + seg_state_part(nv, n_seq, n_seg) + seg_raw_part(nv, n_seq, T, n_seg);
+    const DeltaPlan p = delta_plan(nv, n_seq, T);
+    const int units = nv * n_seq;
+    return rec_part(p, units) + seg_state_part(units, p.n_seg) + seg_raw_part(units, T, p.n_seg);
 }
-size_t linear_prefill_tc5_dump_floats() { return DBG_FLOATS; }
-
-namespace {
 
 // The second stream and the events of the slab pipeline, one set per device.  The lock covers one call's
 // launches: a wait takes the event's state at the moment it is enqueued, so the next call may re-record.
-constexpr int MAX_SLABS = 16;
+static constexpr int MAX_SLABS = 16;
+namespace {
 struct SlabPipe {
     std::mutex lock;
     cudaStream_t scan_stream = nullptr;
-    cudaEvent_t front_done[MAX_SLABS] = {}, scans_done = nullptr;
+    cudaEvent_t front_done[MAX_SLABS] = {}, scan_done[MAX_SLABS] = {};
 };
 SlabPipe g_slab_pipe[ORN_MAX_DEVICES];
 
@@ -1069,17 +1199,22 @@ ornith_status slab_pipe_ready(SlabPipe &p) {
     ORN_TRY(orn_check(cudaDeviceGetStreamPriorityRange(&least, &greatest), "stream priority range"));
     cudaStream_t st = nullptr;
     ORN_TRY(orn_check(cudaStreamCreateWithPriority(&st, cudaStreamNonBlocking, greatest), "delta scan stream"));
-    for (int i = 0; i < MAX_SLABS; i++) ORN_TRY(orn_check(cudaEventCreateWithFlags(&p.front_done[i], cudaEventDisableTiming), "slab event"));
-    ORN_TRY(orn_check(cudaEventCreateWithFlags(&p.scans_done, cudaEventDisableTiming), "slab event"));
+    for (int i = 0; i < MAX_SLABS; i++) {
+        ORN_TRY(orn_check(cudaEventCreateWithFlags(&p.front_done[i], cudaEventDisableTiming), "slab event"));
+        ORN_TRY(orn_check(cudaEventCreateWithFlags(&p.scan_done[i], cudaEventDisableTiming), "slab event"));
+    }
     p.scan_stream = st;
     return ORNITH_OK;
 }
+}  // namespace
 
-// slabs of the prompt: 48 chunks or more each, at most 8; 1 = no pipeline (ORNITH_CUDA_DELTA_SLABS overrides)
-int slab_plan(int heads, int n_chunks, int n_seg) {
+// Slabs of the prompt; 1 = no pipeline (ORNITH_CUDA_DELTA_SLABS overrides).  The scan of up to half as many heads as SMs leaves the
+// passes in front of it room; each slab costs a start of the scan.  us at 1 | 2 | 3 | 4 | 8 slabs: 64 heads x 4096 tokens 257 | 268 | 274 |
+// 278 | 315, 8192 490 | 465 | 473 | 495 | 515, 16384 948 | 885 | 903 | 920 | 986, 32768 1925 | 1750 | 1755 | 1725 | 1877; 32 heads x 8192
+// 414 | 402 | 405 | 427, 16384 801 | 747 | 731 | 714; 128 heads x 8192 790 | 824 | 934 | 961 | 1029.
+static int slab_plan(int heads, int n_chunks, int n_seg) {
     if (n_seg > 1 || heads > 148) return 1;
-    int n = n_chunks / 48;                                            // a slab costs about 25 us of start-up and hand-over
-    if (n > 8) n = 8;
+    int n = heads <= 74 ? min(4, 1 + n_chunks / 128) : 1;
     const char *e = getenv("ORNITH_CUDA_DELTA_SLABS");
     if (e && e[0]) n = atoi(e);
     if (n > MAX_SLABS) n = MAX_SLABS;
@@ -1087,130 +1222,136 @@ int slab_plan(int heads, int n_chunks, int n_seg) {
     return n < 1 ? 1 : n;
 }
 
-}  // namespace
-
 // frees the current device's scan stream and events (the next long prefill makes new ones); the device is idle
 ornith_status release_delta_slab_pipe() {
     SlabPipe &p = g_slab_pipe[orn_device_index()];
     std::lock_guard<std::mutex> hold(p.lock);
     if (!p.scan_stream) return ORNITH_OK;
-    for (int i = 0; i < MAX_SLABS; i++) { if (p.front_done[i]) (void)cudaEventDestroy(p.front_done[i]); p.front_done[i] = nullptr; }
-    if (p.scans_done) (void)cudaEventDestroy(p.scans_done);
-    p.scans_done = nullptr;
+    for (int i = 0; i < MAX_SLABS; i++) {
+        for (cudaEvent_t *e : {&p.front_done[i], &p.scan_done[i]}) { if (*e) (void)cudaEventDestroy(*e); *e = nullptr; }
+    }
     const cudaError_t e = cudaStreamDestroy(p.scan_stream);
     p.scan_stream = nullptr;
     return orn_check(e, "delta scan stream destroy");
 }
 
+using ScanKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ScanArgs);
+static ScanKernel scan_kernel(bool bf, bool seg, bool tile) {
+    static const ScanKernel k[8] = {k_delta_scan_tc5<float, false, false>, k_delta_scan_tc5<__nv_bfloat16, false, false>,
+                                    k_delta_scan_tc5<float, true, false>,  k_delta_scan_tc5<__nv_bfloat16, true, false>,
+                                    k_delta_scan_tc5<float, false, true>,  k_delta_scan_tc5<__nv_bfloat16, false, true>,
+                                    k_delta_scan_tc5<float, true, true>,   k_delta_scan_tc5<__nv_bfloat16, true, true>};
+    return k[bf + 2 * seg + 4 * tile];
+}
+
 ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dtype, const float *Y, const float *rq,
                                         const float *rk, const float *la, const float *be, const TC5Front *front,
-                                        float *work, float *dbg, cudaStream_t s) {
-    extern long long *g_delta_scan_trace;
-    const int n_chunks = (x.T + C - 1) / C;
-    const size_t n_blocks = (size_t)n_seq * x.nv * n_chunks;
-    const int Cc = 2 * x.nk * 128 + x.nv * 128;
-    if ((size_t)n_seq * x.T >= (1u << 31) || n_blocks * AP_ROWS >= (1u << 31)) {
+                                        float *work, cudaStream_t s) {
+    const int Cc = 2 * x.nk * 128 + x.nv * 128, units = x.nv * n_seq;
+    if ((size_t)n_seq * x.T >= (1u << 31)) {
         orn_record_error("delta scan: %d sequences x %d tokens exceed the tensor-map coordinates", n_seq, x.T);
         return ORNITH_ERR_UNSUPPORTED;
     }
-    float *AP = work, *aux = (float *)((char *)work + ap_part(x.nv, n_seq, n_chunks));
+    const DeltaPlan p = delta_plan(x.nv, n_seq, x.T);
     static bool configured_dev[ORN_MAX_DEVICES] = {};
     bool &configured = configured_dev[orn_device_index()];
     if (!configured) {
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_delta_prep64<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PrepSmem)),
-                          "delta prep smem opt-in"));
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_delta_prep64<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PrepSmem)),
-                          "delta prep smem opt-in"));
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_delta_scan_tc5<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM),
-                          "delta scan smem opt-in"));
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_delta_scan_tc5<__nv_bfloat16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM),
-                          "delta scan smem opt-in"));
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_delta_scan_tc5<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM),
-                          "delta scan smem opt-in"));
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_delta_scan_tc5<__nv_bfloat16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM),
-                          "delta scan smem opt-in"));
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_delta_seg_finish<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinSmem)),
-                          "delta finish smem opt-in"));
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_delta_seg_finish<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinSmem)),
-                          "delta finish smem opt-in"));
+        const auto opt_in = [](auto *k, size_t smem, const char *what) {
+            return orn_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), what);
+        };
+        ORN_TRY(opt_in(k_delta_prep<float>, PREP_SMEM, "delta prep smem opt-in"));
+        ORN_TRY(opt_in(k_delta_prep<__nv_bfloat16>, PREP_SMEM, "delta prep smem opt-in"));
+        for (int v = 0; v < 8; v++) ORN_TRY(opt_in(scan_kernel(v & 1, v & 2, v & 4), SCAN_SMEM, "delta scan smem opt-in"));
+        ORN_TRY(opt_in(k_delta_seg_finish<float>, sizeof(FinSmem), "delta finish smem opt-in"));
+        ORN_TRY(opt_in(k_delta_seg_finish<__nv_bfloat16>, sizeof(FinSmem), "delta finish smem opt-in"));
         configured = true;
     }
     const bool bf = act_dtype == ORNITH_ACT_BF16;
-    CUtensorMap my, mym, map_ap, map_ap32, map_v;
-    ORN_TRY(f32_rows_map(&my, Y, (uint64_t)Cc, (uint64_t)n_seq * x.T, C, 1));
-    ORN_TRY(f32_rows_map(&mym, Y, (uint64_t)Cc, (uint64_t)n_seq * x.T, C, 2));
-    ORN_TRY(f32_rows_map(&map_v, Y, (uint64_t)Cc, (uint64_t)n_seq * x.T, C, 0, 128));
-    ORN_TRY(f32_rows_map(&map_ap, AP, 32, n_blocks * AP_ROWS, C, 1));
-    ORN_TRY(f32_rows_map(&map_ap32, AP, 32, n_blocks * AP_ROWS, 32, 1));
+    // z and the outputs travel by tensor copies where their rows lie on 16-byte boundaries (the row length always is a multiple)
+    const bool tile = ((uintptr_t)x.z % 16) == 0 && ((uintptr_t)x.out % 16) == 0;
+    CUtensorMap my, mym, mz, mo;
+    ORN_TRY(f32_rows_map(&my, Y, (uint64_t)Cc, (uint64_t)n_seq * x.T, C, false));
+    ORN_TRY(f32_rows_map(&mym, Y, (uint64_t)Cc, (uint64_t)n_seq * x.T, C, true));
+    mz = mo = my;
+    if (tile) {
+        ORN_TRY(act_rows_map(&mz, x.z, bf, (uint64_t)x.nv * 128, (uint64_t)x.T, (uint64_t)n_seq, C));
+        ORN_TRY(act_rows_map(&mo, x.out, bf, (uint64_t)x.nv * 128, (uint64_t)x.T, (uint64_t)n_seq, 16));
+    }
+    unsigned char *rec = (unsigned char *)work;
+    const size_t slot_bytes = (size_t)units * p.per * REC_BYTES;
     ScanArgs a;
-    a.Y = Y; a.aux = aux; a.S = x.S; a.S_stride = x.S_stride; a.z = x.z; a.out = x.out; a.norm_w = x.norm_w;
-    a.nk = x.nk; a.nv = x.nv; a.head_map = x.head_map; a.T = x.T; a.n_chunks = n_chunks;
-    a.c_begin = 0; a.c_count = n_chunks;
-    a.out_scale = x.out_scale; a.eps = x.eps; a.status = orn_status_word(); a.dbg = dbg; a.trace = g_delta_scan_trace;
-    a.n_seg = delta_seg_plan(x.nv, n_seq, n_chunks, &a.seg_chunks);
-    a.seg_state = (float *)((char *)aux + aux_part(x.nv, n_seq, n_chunks));
-    a.seg_raw = (float *)((char *)a.seg_state + seg_state_part(x.nv, n_seq, a.n_seg));
+    a.rec = rec; a.S = x.S; a.S_stride = x.S_stride; a.z = x.z; a.out = x.out; a.norm_w = x.norm_w;
+    a.nk = x.nk; a.nv = x.nv; a.head_map = x.head_map; a.T = x.T; a.n_chunks = p.n_chunks;
+    a.c_begin = 0; a.c_count = p.n_chunks; a.rec_chunks = p.per;
+    a.out_scale = x.out_scale; a.eps = x.eps; a.status = orn_status_word();
+    a.n_seg = p.n_seg; a.seg_chunks = p.seg_chunks;
+    a.seg_state = (float *)((char *)work + rec_part(p, units));
+    a.seg_raw = (float *)((char *)a.seg_state + seg_state_part(units, p.n_seg));
 
-    const int refresh = front != nullptr;                             // (without `front` the caller has refreshed the history)
-    auto prep = [&](int c_begin, int c_count, cudaStream_t ps, bool chained) {
-        const dim3 pgrid((unsigned)c_count, (unsigned)x.nk, (unsigned)n_seq);
-        const float *Yc = Y;
+    // the records of the chunks cb .. cb + cn - 1, into a slot.  With a front the launch that ends the prompt also stores the
+    // new history (without one the caller has done that)
+    auto prep = [&](int cb, int cn, int slot, bool chained) {
+        PrepArgs64 pa;
+        pa.Y = Y; pa.rq = rq; pa.rk = rk; pa.la = la; pa.be = be;
+        pa.rec = rec + slot * slot_bytes;
+        pa.n_chunks = p.n_chunks; pa.chunk0 = cb; pa.rec_chunks = p.per; pa.refresh = front != nullptr; pa.status = orn_status_word();
+        const dim3 pgrid((unsigned)cn, (unsigned)x.nk, (unsigned)n_seq);
         if (chained)
-            return orn_check(bf ? orn_launch_dependent(k_delta_prep64<__nv_bfloat16>, pgrid, dim3(256), sizeof(PrepSmem), ps, x, Yc, rq, rk, la, be, AP, aux,
-                                                       n_chunks, c_begin, refresh)
-                                : orn_launch_dependent(k_delta_prep64<float>, pgrid, dim3(256), sizeof(PrepSmem), ps, x, Yc, rq, rk, la, be, AP, aux, n_chunks,
-                                                       c_begin, refresh), "k_delta_prep64");
-        if (bf) k_delta_prep64<__nv_bfloat16><<<pgrid, 256, sizeof(PrepSmem), ps>>>(x, Y, rq, rk, la, be, AP, aux, n_chunks, c_begin, refresh);
-        else    k_delta_prep64<float><<<pgrid, 256, sizeof(PrepSmem), ps>>>(x, Y, rq, rk, la, be, AP, aux, n_chunks, c_begin, refresh);
-        return orn_check_launch("k_delta_prep64");
+            return orn_check(bf ? orn_launch_dependent(k_delta_prep<__nv_bfloat16>, pgrid, dim3(256), PREP_SMEM, s, my, x, pa)
+                                : orn_launch_dependent(k_delta_prep<float>, pgrid, dim3(256), PREP_SMEM, s, my, x, pa), "k_delta_prep");
+        if (bf) k_delta_prep<__nv_bfloat16><<<pgrid, 256, PREP_SMEM, s>>>(my, x, pa);
+        else    k_delta_prep<float><<<pgrid, 256, PREP_SMEM, s>>>(my, x, pa);
+        return orn_check_launch("k_delta_prep");
     };
-    auto scan = [&](const ScanArgs &sa, cudaStream_t ss, bool chained) {
+    auto scan = [&](int cb, int cn, int slot, cudaStream_t ss, bool chained) {
+        ScanArgs sa = a;
+        sa.rec = rec + slot * slot_bytes; sa.c_begin = cb; sa.c_count = cn;
         dim3 grid((unsigned)x.nv, (unsigned)n_seq);
         if (chained)
-            return orn_check(bf ? orn_launch_dependent(k_delta_scan_tc5<__nv_bfloat16, false>, grid, dim3(NTHREADS), SCAN_SMEM, ss, my, mym, map_ap, map_ap32, map_v, sa)
-                                : orn_launch_dependent(k_delta_scan_tc5<float, false>, grid, dim3(NTHREADS), SCAN_SMEM, ss, my, mym, map_ap, map_ap32, map_v, sa),
-                             "k_delta_scan_tc5");
-        if (bf) k_delta_scan_tc5<__nv_bfloat16, false><<<grid, NTHREADS, SCAN_SMEM, ss>>>(my, mym, map_ap, map_ap32, map_v, sa);
-        else    k_delta_scan_tc5<float, false><<<grid, NTHREADS, SCAN_SMEM, ss>>>(my, mym, map_ap, map_ap32, map_v, sa);
+            return orn_check(orn_launch_dependent(scan_kernel(bf, false, tile), grid, dim3(NTHREADS), SCAN_SMEM, ss, my, mym, mz, mo, sa), "k_delta_scan_tc5");
+        scan_kernel(bf, false, tile)<<<grid, NTHREADS, SCAN_SMEM, ss>>>(my, mym, mz, mo, sa);
         return orn_check_launch("k_delta_scan_tc5");
     };
 
-    // two runs per head (30-37 heads) lose to the slab pipeline on a long prompt: 2.41 against 2.07 ms for 32 heads x
-    // 32768 tokens (the finishing pass costs more than the halved chain saves); three runs or more win (16 heads: 1.72
-    // against 1.99 ms)
-    const char *seg_env = getenv("ORNITH_CUDA_DELTA_SEGMENTS");
-    if (front && a.n_seg == 2 && !(seg_env && seg_env[0]) && slab_plan(x.nv * n_seq, n_chunks, 1) >= 2) a.n_seg = 1;
-    const int n_slabs = front ? slab_plan(x.nv * n_seq, n_chunks, a.n_seg) : 1;
-    if (n_slabs > 1) {
+    if (front && p.slots == 2) {
         // front of slab k + 1 on the caller's stream beside the scan of slab k on the scan stream
         SlabPipe &pipe = g_slab_pipe[orn_device_index()];
         std::lock_guard<std::mutex> hold(pipe.lock);
         ORN_TRY(slab_pipe_ready(pipe));
-        const int per = (n_chunks + n_slabs - 1) / n_slabs;
-        auto slab = [&](int k, int cb, int cn) -> ornith_status {
+        int k = 0, forked = -1;                                       // forked: the last slab whose scan was enqueued
+        auto slab = [&](int cb, int cn) -> ornith_status {
             ORN_TRY(front->conv(cb * C, min(x.T, (cb + cn) * C), s));
-            ORN_TRY(prep(cb, cn, s, false));
+            if (k >= 2) ORN_TRY(orn_check(cudaStreamWaitEvent(s, pipe.scan_done[k - 2], 0), "slab event wait"));     // its records' place is free
+            ORN_TRY(prep(cb, cn, k & 1, false));
             ORN_TRY(orn_check(cudaEventRecord(pipe.front_done[k], s), "slab event record"));
             ORN_TRY(orn_check(cudaStreamWaitEvent(pipe.scan_stream, pipe.front_done[k], 0), "slab event wait"));
-            ScanArgs sa = a;
-            sa.c_begin = cb; sa.c_count = cn;
-            return scan(sa, pipe.scan_stream, false);
+            forked = k;
+            ORN_TRY(scan(cb, cn, k & 1, pipe.scan_stream, false));
+            return orn_check(cudaEventRecord(pipe.scan_done[k], pipe.scan_stream), "slab event record");
         };
         ornith_status st = ORNITH_OK;
-        int k = 0;
-        for (int cb = 0; cb < n_chunks && st == ORNITH_OK; cb += per, k++) st = slab(k, cb, min(per, n_chunks - cb));
+        for (int cb = 0; cb < p.n_chunks && st == ORNITH_OK; cb += p.per, k++) st = slab(cb, min(p.per, p.n_chunks - cb));
         // the caller's stream always rejoins the scan stream, also when a launch failed on the way
-        ornith_status join = orn_check(cudaEventRecord(pipe.scans_done, pipe.scan_stream), "slab event record");
-        if (join == ORNITH_OK) join = orn_check(cudaStreamWaitEvent(s, pipe.scans_done, 0), "slab event wait");
+        ornith_status join = ORNITH_OK;
+        if (forked >= 0) {
+            if (st != ORNITH_OK) join = orn_check(cudaEventRecord(pipe.scan_done[forked], pipe.scan_stream), "slab event record");
+            if (join == ORNITH_OK) join = orn_check(cudaStreamWaitEvent(s, pipe.scan_done[forked], 0), "slab event wait");
+        }
         return st != ORNITH_OK ? st : join;
     }
     if (front) ORN_TRY(front->conv(0, x.T, s));
-    ORN_TRY(prep(0, n_chunks, s, front != nullptr));
-    if (a.n_seg <= 1) return scan(a, s, true);
+    if (p.n_seg <= 1) {
+        for (int cb = 0; cb < p.n_chunks; cb += p.per) {              // (more than one slab: the scan of one before the preparation of the next)
+            const int cn = min(p.per, p.n_chunks - cb);
+            ORN_TRY(prep(cb, cn, 0, front != nullptr && cb == 0));
+            ORN_TRY(scan(cb, cn, 0, s, true));
+        }
+        return ORNITH_OK;
+    }
     // few heads: the runs of the prompt side by side, then the carry over the runs and the finishing pass
+    ORN_TRY(prep(0, p.n_chunks, 0, front != nullptr));
     dim3 grid((unsigned)x.nv, (unsigned)n_seq, (unsigned)(2 * a.n_seg - 1));
-    if (bf) k_delta_scan_tc5<__nv_bfloat16, true><<<grid, NTHREADS, SCAN_SMEM, s>>>(my, mym, map_ap, map_ap32, map_v, a);
-    else    k_delta_scan_tc5<float, true><<<grid, NTHREADS, SCAN_SMEM, s>>>(my, mym, map_ap, map_ap32, map_v, a);
+    scan_kernel(bf, true, tile)<<<grid, NTHREADS, SCAN_SMEM, s>>>(my, mym, mz, mo, a);
     ORN_TRY(orn_check_launch("k_delta_scan_tc5 (runs)"));
     k_delta_seg_carry<<<dim3((unsigned)x.nv, (unsigned)n_seq, 16), 128, 0, s>>>(a);
     ORN_TRY(orn_check_launch("k_delta_seg_carry"));

@@ -421,6 +421,9 @@ __global__ void __launch_bounds__(128) k_conv4_silu_prefill(LinArgs a, float *Y,
 #undef ORN_CONV4
         if (FAST && ch < 2 * qd) {                        // q and k feed tf32 tensor-core products: round once, here
             y.x = tf32_rna(y.x); y.y = tf32_rna(y.y); y.z = tf32_rna(y.z); y.w = tf32_rna(y.w);
+        } else if (NORMS) {                               // the tcgen05 scan's v channels: beta v, rounded to tf32
+            const float bt = sigmoid_f(act_ld((const ACT *)a.b, ((size_t)b * a.T + t0 + i) * a.nv + (ch - 2 * qd) / 128));
+            y.x = tf32_rna(bt * y.x); y.y = tf32_rna(bt * y.y); y.z = tf32_rna(bt * y.z); y.w = tf32_rna(bt * y.w);
         }
         *reinterpret_cast<float4 *>(Y + ((size_t)b * a.T + t0 + i) * Cc + ch) = y;
         if (NORMS) ss[i] = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
@@ -460,6 +463,18 @@ __global__ void k_conv_ring_refresh(LinArgs a) {
     const ACT *X = (const ACT *)a.qkv + (size_t)b * a.T * Cc;
     for (int t = max(0, a.T - K); t < a.T; t++)
         ring[(size_t)((pos0 + t) % K) * Cc + ch] = act_ld(X, (size_t)t * Cc + ch);
+}
+
+// what the tcgen05 scan expects of a Y that another conv wrote: v times its write gate, q, k and that rounded to tf32
+__global__ void __launch_bounds__(256) k_scan_inputs(LinArgs a, float *Y, const float *be, size_t n4) {
+    const int qd = a.nk * a.dk, Cc = 2 * qd + a.nv * a.dv;
+    for (size_t e = blockIdx.x * 256ull + threadIdx.x; e < n4; e += gridDim.x * 256ull) {
+        const int ch = (int)(e * 4 % Cc);
+        const float s = ch < 2 * qd ? 1.0f : be[e * 4 / Cc * a.nv + (ch - 2 * qd) / a.dv];
+        float4 y = reinterpret_cast<float4 *>(Y)[e];
+        y.x = tf32_rna(s * y.x); y.y = tf32_rna(s * y.y); y.z = tf32_rna(s * y.z); y.w = tf32_rna(s * y.w);
+        reinterpret_cast<float4 *>(Y)[e] = y;
+    }
 }
 
 // per (token, key head): 1/sqrt(sum q^2 + eps), 1/sqrt(sum k^2 + eps);
@@ -718,13 +733,6 @@ __global__ void __launch_bounds__(256, 1) k_linear_prefill_chunk128(LinArgs a, c
 // host entry points
 // =============================================================================
 
-// Kernel bring-up aid, not part of the public interface: when set, the tcgen05 scan copies the first
-// chunk's intermediate tiles (KS, U, QS, PU; [128][64] floats each per (sequence, head)) there.
-static float *g_delta_scan_dump = nullptr;
-extern "C" void ornith_cuda_debug_delta_scan_dump(float *dev) { g_delta_scan_dump = dev; }
-long long *g_delta_scan_trace = nullptr;
-extern "C" void ornith_cuda_debug_delta_scan_trace(long long *dev) { g_delta_scan_trace = dev; }
-
 static ornith_status check_linear(const ornith_cuda_linear_layer *l, const ornith_cuda_linear_state *st) {
     if (!l || !st || l->nk <= 0 || l->nv <= 0 || l->dk <= 0 || l->dv <= 0 || l->nv % l->nk ||
         l->conv_k < 1 || l->conv_k > 9 || !l->conv_w || !l->a_coef || !l->dt_bias || !l->norm_w ||
@@ -857,7 +865,7 @@ ornith_status ornith_cuda_linear_attn_prefill(const ornith_cuda_linear_layer *l,
                 else    k_conv4_silu_prefill<float, true, true><<<g, 128, 0, cs>>>(x, Y, rq, rk, t_begin, t_end);
                 return orn_check_launch("k_conv4_silu_prefill");
             };
-            return launch_linear_prefill_tc5(x, n_seq, act_dtype, Y, rq, rk, nullptr, nullptr, &front, blocks, g_delta_scan_dump, s);
+            return launch_linear_prefill_tc5(x, n_seq, act_dtype, Y, rq, rk, nullptr, nullptr, &front, blocks, s);
         }
         else if (bf && tc)  k_conv4_silu_prefill<__nv_bfloat16, true, false><<<cgrid, 128, 0, s>>>(x, Y, nullptr, nullptr, 0, T);
         else if (bf)   k_conv4_silu_prefill<__nv_bfloat16, false, false><<<cgrid, 128, 0, s>>>(x, Y, nullptr, nullptr, 0, T);
@@ -881,7 +889,12 @@ ornith_status ornith_cuda_linear_attn_prefill(const ornith_cuda_linear_layer *l,
     dim3 grid(l->nv, n_seq);
     if (l->dk == 128 && l->dv == 128) {
         // default: tf32 tensor-core scan; ORNITH_CUDA_PREFILL_FP32=1 keeps every product in fp32
-        if (tc5) return launch_linear_prefill_tc5(x, n_seq, act_dtype, Y, rq, rk, la, be, nullptr, blocks, g_delta_scan_dump, s);
+        if (tc5) {
+            const size_t n4 = n_tok * Cc / 4;
+            k_scan_inputs<<<(unsigned)(n4 / 256 + 1 < 4096 ? n4 / 256 + 1 : 4096), 256, 0, s>>>(x, Y, be, n4);
+            ORN_TRY(orn_check_launch("k_scan_inputs"));
+            return launch_linear_prefill_tc5(x, n_seq, act_dtype, Y, rq, rk, la, be, nullptr, blocks, s);
+        }
         if (tc) return launch_linear_prefill_tc(x, n_seq, act_dtype, Y, rq, rk, la, be, blocks, s);
         if (chunk >= 32) return bf ? launch_chunk<32, __nv_bfloat16>(x, grid, Y, rq, rk, la, be, s)
                                    : launch_chunk<32, float>(x, grid, Y, rq, rk, la, be, s);

@@ -112,6 +112,11 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, ui
     asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n}\n"
                  ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(id), "r"(acc) : "memory");
 }
+// both operands in shared memory
+__device__ __forceinline__ void mma_tf32_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t id, uint32_t acc) {
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}\n"
+                 ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(id), "r"(acc) : "memory");
+}
 // the mbarrier gets one arrival when every tcgen05 operation this thread issued so far is complete
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -159,6 +164,17 @@ __device__ __forceinline__ void tmem_ld8x2_wait(uint32_t ta, float (&a)[8], uint
                  "tcgen05.wait::ld.sync.aligned;"
                  : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7]), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]), "=f"(b[4]), "=f"(b[5]), "=f"(b[6]), "=f"(b[7])
                  : "r"(ta), "r"(tb) : "memory");
+}
+// 32 lanes x 16 columns of two tiles as fragments of 16 lanes x 256 bits: thread 4 g + j gets of each tile, at index
+// 8 m + 4 h + 2 i + c, lane 16 h + 8 i + g, column 8 m + 2 j + c.
+__device__ __forceinline__ void tmem_ld_16x256_wait(uint32_t ta, float (&a)[16], uint32_t tb, float (&b)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %8, %9, %10, %11}, [%32];\n"
+                 "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%4, %5, %6, %7, %12, %13, %14, %15}, [%33];\n"
+                 "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%16, %17, %18, %19, %24, %25, %26, %27}, [%34];\n"
+                 "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%20, %21, %22, %23, %28, %29, %30, %31}, [%35];\n"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7]), "=f"(a[8]), "=f"(a[9]), "=f"(a[10]), "=f"(a[11]), "=f"(a[12]), "=f"(a[13]), "=f"(a[14]), "=f"(a[15]), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]), "=f"(b[4]), "=f"(b[5]), "=f"(b[6]), "=f"(b[7]), "=f"(b[8]), "=f"(b[9]), "=f"(b[10]), "=f"(b[11]), "=f"(b[12]), "=f"(b[13]), "=f"(b[14]), "=f"(b[15])
+                 : "r"(ta), "r"(ta + (16u << 16)), "r"(tb), "r"(tb + (16u << 16)) : "memory");
 }
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&r)[32]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "

@@ -342,3 +342,33 @@ def test_tensor_copy_conv_matches_the_plain_conv(monkeypatch, bf16):
     for a, b in zip(got, ref):
         assert (a == b).all()
     assert np.isfinite(got[1]).all() and np.abs(got[1]).max() > 0
+
+
+@pytest.mark.parametrize("nk,nv,grouped,T,bf16,shifted", [
+    (2, 2, False, 1, False, ""), (2, 6, False, 63, True, ""), (2, 6, True, 64, False, "z"), (1, 5, False, 65, True, "z"),
+    (1, 9, True, 130, False, ""), (2, 4, False, 130, True, "qkv"), (2, 4, True, 65, False, "qkv")])
+def test_scan_head_counts_and_unaligned_tensors(oracle, nk, nv, grouped, T, bf16, shifted):
+    """Value heads per key head on both sides of the preparation's batch of four, chunk edges, z and out off the 16-byte
+    grid (loaded and stored by the threads instead of tensor copies), qkv off it (another conv in front of the scan)."""
+    import torch
+    from ornithology_b200 import device as D
+    layer, kw = linear_case(50 + nv, nk=nk, nv=nv, head_map=O.HEADMAP_GROUPED if grouped else O.HEADMAP_TILED)
+    dl = device_linear(layer, kw)
+    dt, B = torch.bfloat16 if bf16 else torch.float32, 2
+    seqs = [linear_inputs(500 + b, layer, T, bf16) for b in range(B)]
+
+    def place(x, off):                                     # the same values, `off` elements behind a 256-byte boundary
+        buf = torch.empty(x.numel() + off, dtype=dt, device="cuda")
+        buf[off:] = x.to("cuda", dt).flatten()
+        return buf[off:].view(x.shape)
+
+    qkv, a, bm, z = (place(torch.from_numpy(np.stack([s[i] for s in seqs])), 1 if shifted == n else 0) for i, n in enumerate(("qkv", "a", "b", "z")))
+    out = place(torch.zeros(B, T, layer.vd), 1 if shifted == "z" else 0)
+    st = D.LinearState(dl, B)
+    pos = torch.zeros(B, dtype=torch.int32, device="cuda")
+    D.linear_attn_prefill(dl, st, pos, qkv, a, bm, z, T, chunk=64, out=out)
+    for b in range(B):
+        S = np.zeros((layer.nv, 128, 128), np.float32); buf = np.zeros(3 * layer.cc, np.float32)
+        ref = oracle.linear_attn_prefill(layer, S, buf, *seqs[b], chunk=64)
+        assert rel_err(out[b].float().cpu().numpy(), ref) < (TOL_BF16_IO if bf16 else TOL)
+        assert rel_err(st.S[b].cpu().numpy(), S) < TOL
