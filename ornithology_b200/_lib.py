@@ -152,6 +152,7 @@ SYMBOLS = {
 }
 
 _lib = None
+_fast = None
 
 
 class BackendError(RuntimeError):
@@ -175,6 +176,21 @@ def load() -> C.CDLL:
             fn.argtypes = args
     _lib = lib
     return lib
+
+
+def fast():
+    """The entry points whose arguments are integers and pointers only, as attributes without their `ornith_cuda_` prefix, called by
+    way of the _fastcall module: tensors, bytes, integers and None go in as they are."""
+    global _fast
+    if _fast is None:
+        from types import SimpleNamespace
+        from . import _fastcall
+        lib = load()
+        _fast = SimpleNamespace(**{
+            name[len("ornith_cuda_"):]: _fastcall.Function(C.cast(getattr(lib, name), vp).value, int(res is _SZ))
+            for name, (res, args) in SYMBOLS.items()
+            if name.startswith("ornith_cuda_") and res in (_I, _SZ) and args is not None and all(a in (vp, _I, _SZ) for a in args)})
+    return _fast
 
 
 def check(status: int, what: str = "") -> None:

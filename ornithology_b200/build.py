@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 PKG = os.path.dirname(os.path.abspath(__file__))
@@ -19,6 +20,8 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libornith_cuda.so")
+FASTCALL_SRC = os.path.join(CSRC, "py", "fastcall.c")
+FASTCALL = os.path.join(PKG, "_fastcall.so")          # the Python module that calls into the library (_lib.py)
 INCLUDE = os.path.join(ROOT, "include")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -40,10 +43,10 @@ def sources():
 
 
 def _stale() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(FASTCALL):
         return True
     t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(INCLUDE, "ornith_cuda.h")]
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [FASTCALL_SRC, os.path.join(INCLUDE, "ornith_cuda.h")]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
@@ -79,6 +82,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run([nvcc, "-shared", "-o", LIB, *objs, "-lpthread"], capture_output=True, text=True)
     if r.returncode:
         raise RuntimeError(f"link failed:\n{r.stderr}")
+    r = subprocess.run(["gcc", "-O2", "-std=gnu11", "-fPIC", "-shared", "-Wall", "-I", sysconfig.get_paths()["include"], FASTCALL_SRC,
+                        "-o", FASTCALL], capture_output=True, text=True)
+    if r.returncode:
+        raise RuntimeError(f"gcc failed on fastcall.c:\n{r.stderr}")
     with open(os.path.join(OBJ, "ptxas.log"), "w") as fh:
         for f, t in logs.items():
             fh.write(f"==== {f}\n{t}\n")

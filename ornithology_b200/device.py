@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import struct
 
 import numpy as np
 import torch
@@ -24,9 +25,9 @@ __all__ = ["FullLayer", "KvBatch", "LinearLayer", "LinearState", "full_attn_step
            "ACT_F32", "ACT_BF16", "KV_F32", "KV_INT8_HEAD", "KV_Q8_0", "HEADMAP_TILED", "HEADMAP_GROUPED"]
 
 
-# A decode step of one chat is a dozen calls of a few microseconds of GPU work each, so what a call costs on the host counts:
-# pointers and streams go to ctypes as plain integers, and outputs come from new_empty (12 -> 8 us a call; one token's
-# projections of four layers, 16 calls that the host bounds, 178 -> 98 us).
+# A decode step of one chat is a dozen calls of a few microseconds of GPU work each, so what a call costs on the host counts: the
+# calls of a step go through _lib.fast(), descriptions of weights are packed instead of built field by field, and outputs come
+# from new_empty with plain sizes.
 def _ptr(t):
     return None if t is None else t.data_ptr()
 
@@ -196,12 +197,14 @@ class QWeight:
 
 def q8k_image(x, n_in, image=None):
     """x [T][n_in] -> the Q8_K image the integer products read; one image serves every projection of the same input."""
-    lib = _lib.load()
+    f = _lib.fast()
     T = x.numel() // n_in
-    need = lib.ornith_cuda_matmul_q_scratch(GGML_Q8_0, T, n_in)
+    need = f.matmul_q_scratch(GGML_Q8_0, T, n_in)
     if image is None or image.numel() < need:
         image = torch.empty(need, dtype=torch.uint8, device=x.device)
-    check(lib.ornith_cuda_q8k_image(_ptr(x), _act(x), T, n_in, _ptr(image), image.numel(), _stream()), "q8k_image")
+    st = f.q8k_image(x, _act(x), T, n_in, image, image.numel(), _stream())
+    if st:
+        check(st, "q8k_image")
     return image
 
 
@@ -224,14 +227,22 @@ def matmul_q(w: QWeight, x, out=None, image=None, T=None, out_dtype=None):
     return out
 
 
+_QPROJ = [None] + [struct.Struct("@" + "iPiP" * n) for n in range(1, 9)]      # n x ornith_cuda_qproj: type, rows, n_out, output
+
+
 def matmul_q_group(ws, image, T, outs=None, out_dtype=None):
     """Several projections of the same (already quantised) input in one launch per weight type; returns the outputs."""
-    lib = _lib.load()
+    f = _lib.fast()
     if outs is None:
         outs = [torch.empty(T, w.n_out, dtype=out_dtype or torch.float32, device=image.device) for w in ws]
-    arr = (_lib.CudaQproj * len(ws))(*[(w.wtype, w.bytes.data_ptr(), w.n_out, o.data_ptr()) for w, o in zip(ws, outs)])
-    check(lib.ornith_cuda_matmul_q_group(C.addressof(arr), len(ws), ws[0].n_in, _ptr(image), int(T), _act(outs[0]), _stream()),
-          "matmul_q_group")
+    n = len(ws)
+    fields = []
+    for w, o in zip(ws, outs):
+        fields += (w.wtype, w.bytes.data_ptr(), w.n_out, o.data_ptr())
+    packed = (_QPROJ[n] if 0 < n < len(_QPROJ) else struct.Struct("@" + "iPiP" * n)).pack(*fields)
+    st = f.matmul_q_group(packed, n, ws[0].n_in, image, int(T), _act(outs[0]), _stream())
+    if st:
+        check(st, "matmul_q_group")
     return outs
 
 
@@ -321,35 +332,36 @@ class LinearState:
 
 def full_attn_step(layer: FullLayer, kv: KvBatch, kv_len, qproj, k, v, out=None, rope_pos=None, max_len=None):
     """One decode token per sequence through a full-attention layer (between the projections)."""
-    lib = _lib.load()
+    f = _lib.fast()
     B = kv.n_seq
     act = _act(qproj)
     if out is None:
-        out = qproj.new_empty((B, layer.nh * layer.hd))
+        out = qproj.new_empty(B, layer.nh * layer.hd)
     if max_len is None:
         max_len = int(kv_len.max().item()) + 1
-    need = lib.ornith_cuda_full_attn_step_scratch(C.byref(layer.c), B, int(max_len))
+    c = C.addressof(layer.c)
+    need = f.full_attn_step_scratch(c, B, int(max_len))
     scr = layer.scratch.get(need, qproj.device)
-    check(lib.ornith_cuda_full_attn_step(C.byref(layer.c), C.byref(kv.c), _ptr(kv_len), _ptr(rope_pos),
-                                         _ptr(qproj), _ptr(k), _ptr(v), _ptr(out), act, int(max_len),
-                                         _ptr(scr), scr.numel(), _stream()), "full_attn_step")
+    st = f.full_attn_step(c, C.addressof(kv.c), kv_len, rope_pos, qproj, k, v, out, act, int(max_len), scr, scr.numel(), _stream())
+    if st:
+        check(st, "full_attn_step")
     return out
 
 
 def full_attn_prefill(layer: FullLayer, kv: KvBatch, kv_len, qproj, k, v, T, out=None, rope_pos=None, max_len=None):
     """T new tokens per sequence; `max_len` bounds kv_len[b] + T (default: the largest capacity)."""
-    lib = _lib.load()
+    f = _lib.fast()
     if max_len is None:
         max_len = max(kv.capacities)
     B = kv.n_seq
     act = _act(qproj)
     if out is None:
-        out = qproj.new_empty((B, T, layer.nh * layer.hd))
-    need = lib.ornith_cuda_full_attn_prefill_scratch(C.byref(layer.c), B, int(T), int(max_len))
+        out = qproj.new_empty(B, T, layer.nh * layer.hd)
+    c = C.addressof(layer.c)
+    need = f.full_attn_prefill_scratch(c, B, int(T), int(max_len))
     scr = layer.scratch.get(need, qproj.device)
-    check(lib.ornith_cuda_full_attn_prefill(C.byref(layer.c), C.byref(kv.c), _ptr(kv_len), _ptr(rope_pos),
-                                            _ptr(qproj), _ptr(k), _ptr(v), _ptr(out), act, int(T), int(max_len),
-                                            _ptr(scr), scr.numel(), _stream()), "full_attn_prefill")
+    check(f.full_attn_prefill(c, C.addressof(kv.c), kv_len, rope_pos, qproj, k, v, out, act, int(T), int(max_len), scr, scr.numel(),
+                              _stream()), "full_attn_prefill")
     return out
 
 
@@ -361,32 +373,32 @@ def kv_append(layer: FullLayer, kv: KvBatch, kv_len, k, v, T=1, rope_pos=None):
 
 def linear_attn_step(layer: LinearLayer, st: LinearState, pos, qkv, a, b, z, out=None):
     """One decode token per sequence through a gated delta-net layer (between the projections)."""
-    lib = _lib.load()
     act = _act(qkv)
     B = st.n_seq
     if out is None:
-        out = qkv.new_empty((B, layer.vd))
-    check(lib.ornith_cuda_linear_attn_step(C.byref(layer.c), C.byref(st.c), _ptr(pos), _ptr(qkv), _ptr(a),
-                                           _ptr(b), _ptr(z), _ptr(out), act, B, _stream()), "linear_attn_step")
+        out = qkv.new_empty(B, layer.vd)
+    status = _lib.fast().linear_attn_step(C.addressof(layer.c), C.addressof(st.c), pos, qkv, a, b, z, out, act, B, _stream())
+    if status:
+        check(status, "linear_attn_step")
     return out
 
 
 def linear_attn_prefill(layer: LinearLayer, st: LinearState, pos, qkv, a, b, z, T, chunk=32, out=None):
-    lib = _lib.load()
+    f = _lib.fast()
     act = _act(qkv)
     B = st.n_seq
     if out is None:
-        out = qkv.new_empty((B, T, layer.vd))
-    need = lib.ornith_cuda_linear_attn_prefill_scratch(C.byref(layer.c), B, int(T))
+        out = qkv.new_empty(B, T, layer.vd)
+    c = C.addressof(layer.c)
+    need = f.linear_attn_prefill_scratch(c, B, int(T))
     scr = layer.scratch.get(need, qkv.device)
-    check(lib.ornith_cuda_linear_attn_prefill(C.byref(layer.c), C.byref(st.c), _ptr(pos), _ptr(qkv), _ptr(a),
-                                              _ptr(b), _ptr(z), _ptr(out), act, B, int(T), int(chunk),
-                                              _ptr(scr), scr.numel(), _stream()), "linear_attn_prefill")
+    check(f.linear_attn_prefill(c, C.addressof(st.c), pos, qkv, a, b, z, out, act, B, int(T), int(chunk), scr, scr.numel(), _stream()),
+          "linear_attn_prefill")
     return out
 
 
 def advance(counters: torch.Tensor, delta=1):
-    check(_lib.load().ornith_cuda_advance(_ptr(counters), counters.numel(), int(delta), _stream()), "advance")
+    check(_lib.fast().advance(counters, counters.numel(), int(delta), _stream()), "advance")
 
 
 def q8_0_encode(x: torch.Tensor) -> torch.Tensor:

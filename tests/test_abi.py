@@ -153,3 +153,21 @@ def test_projection_sizing_and_no_gpu_behaviour(lib):
         p = _lib.CudaQproj(8, None, 64, None)
         assert lib.ornith_cuda_matmul_q_group(C.byref(p), 1, 2048, None, 4, 0, None) != 0
         assert lib.ornith_cuda_matmul_q(8, None, 2048, 64, None, 0, 4, None, 0, None, 0, None) != 0
+
+
+def test_fast_calls_pass_what_ctypes_passes(lib):
+    """The _fastcall callables against ctypes, on host-only entry points: sizes beyond 32 bits, null pointers, packed structs, errors."""
+    import struct
+    from ornithology_b200 import _lib
+    f = _lib.fast()
+    for args in ((8, 64, 4096), (14, 1 << 20, 8192), (3, 1, 256)):
+        assert f.matmul_q_scratch(*args) == lib.ornith_cuda_matmul_q_scratch(*args)
+    rows = struct.pack("@3i", 4096, 512, 512)
+    arr = (C.c_int * 3)(4096, 512, 512)
+    assert f.matmul_q_tile_tokens(14, 2048, rows, 3, 777) == lib.ornith_cuda_matmul_q_tile_tokens(14, 2048, C.addressof(arr), 3, 777)
+    assert f.matmul_q_tile_tokens(14, 2048, None, 3, 777) == -1
+    with pytest.raises(AttributeError):
+        f.matmul_q_scratch(8, 64, 1.5)
+    with pytest.raises(TypeError):
+        f.matmul_q_scratch(*range(17))
+    assert not hasattr(f, "rope_inv_freq")                 # takes a float: ctypes only
