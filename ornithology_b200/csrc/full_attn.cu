@@ -705,7 +705,7 @@ static long long head_groups(const ornith_cuda_full_layer *l, int n_seq) {
 }
 // Scratch of one decode step: query rows, one arrival counter per (sequence, head), then the partials.
 //   SPLIT_TC  a tensor-core kernel with splits of tps_mma tokens serves the cache;
-//   BALANCED  the Q8_0 raw-fragment kernel with its own schedule: a fixed number of partial slots per head;
+//   BALANCED  the Q8_0 tcgen05 kernel with its own schedule: a fixed number of partial slots per head;
 //   ANY       the size query, which does not see the cache: the larger of the two, with the CUDA-core kernel's
 //             fixed 512- or 128-token splits covered as well.  A step served by the CUDA-core kernel needs this too.
 enum DecodePath { PATH_ANY, PATH_SPLIT_TC, PATH_BALANCED };
@@ -714,7 +714,7 @@ static size_t step_need(const ornith_cuda_full_layer *l, int n_seq, int max_len,
               nsplit = (max_len + t - 1) / t;
     size_t rows = (size_t)n_seq * l->n_heads * nsplit;
     if (path != PATH_SPLIT_TC && l->n_kv_heads > 0 && l->n_heads % l->n_kv_heads == 0) {
-        const size_t bal = (size_t)l->n_heads * gqa_decode_q8_raw_slots(l->n_kv_heads, l->n_heads, n_seq, max_len,
+        const size_t bal = (size_t)l->n_heads * gqa_decode_q8_slots(l->n_kv_heads, l->n_heads, n_seq, max_len,
                                                                          gqa_decode_range_floor(l->n_kv_heads, l->n_heads, n_seq, max_len, short_ranges));
         rows = path == PATH_BALANCED ? bal : (bal > rows ? bal : rows);
     }
@@ -728,7 +728,7 @@ static size_t step_need(const ornith_cuda_full_layer *l, int n_seq, int max_len,
 static DecodePath decode_path(const ornith_cuda_full_layer *l, const ornith_cuda_kv *kv) {
     if (force_generic_decode()) return PATH_ANY;
     const KvView v = make_view(kv);
-    if (gqa_decode_q8_raw_balanced(v, l->n_heads)) return PATH_BALANCED;
+    if (gqa_decode_q8_balanced(v, l->n_heads)) return PATH_BALANCED;
     return (gqa_decode_q8_mma_supported(v, l->n_heads) || gqa_decode_f32_tc_supported(v, l->n_heads) ||
             gqa_decode_i8_raw_supported(v, l->n_heads)) ? PATH_SPLIT_TC : PATH_ANY;
 }
@@ -832,7 +832,7 @@ ornith_status ornith_cuda_full_attn_step(const ornith_cuda_full_layer *l, const 
     int nsplit_used;
     if (gqa_decode_q8_mma_supported(d.kv, nh) && !force_generic_decode()) {
         d.tokens_per_split = tps_mma; d.nsplit = nsplit_used = (max_len + tps_mma - 1) / tps_mma;
-        if (path == PATH_BALANCED) d.nsplit = nsplit_used = gqa_decode_q8_raw_slots(l->n_kv_heads, nh, B, max_len, d.range_floor);
+        if (path == PATH_BALANCED) d.nsplit = nsplit_used = gqa_decode_q8_slots(l->n_kv_heads, nh, B, max_len, d.range_floor);
         ORN_TRY(launch_gqa_decode_q8_mma(d, B, st, &merged));
     } else if (gqa_decode_f32_tc_supported(d.kv, nh) && !force_generic_decode()) {
         d.tokens_per_split = tps_mma; d.nsplit = nsplit_used = (max_len + tps_mma - 1) / tps_mma;

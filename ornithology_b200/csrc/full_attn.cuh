@@ -28,14 +28,15 @@ bool gqa_decode_q8_mma_supported(const KvView &kv, int nh);
 // *merged is set when the launched kernel did the merge itself (a.group_ctr given and supported).
 ornith_status launch_gqa_decode_q8_mma(const DecodeArgs &a, int n_seq, cudaStream_t st, bool *merged);
 
-// Variant for groups of up to 8 query heads that builds its MMA fragments straight
+// Variant with a grid of fixed splits that builds its mma.sync fragments straight
 // from the staged raw rows (gqa_decode_q8_raw.cu).
 ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a, int n_seq, cudaStream_t st, bool *merged);
-// Whether a step over this cache is served by that kernel with its balanced schedule (token ranges of equal
-// length found on the device instead of a grid of fixed splits), and then how many partial slots per head its
-// scratch needs: a.nsplit = gqa_decode_q8_raw_slots(...) and a.part laid out [head][slot][hd + 2].
-bool gqa_decode_q8_raw_balanced(const KvView &kv, int nh);
-int gqa_decode_q8_raw_slots(int nkv, int nh, int n_seq, int max_len, int range_floor);
+// Whether a step over this cache is served by the tcgen05 kernel (gqa_decode_q8_tc5.cu; up to 16 heads per KV head) with its balanced
+// schedule (token ranges of equal length found on the device instead of a grid of fixed splits), and then how many partial slots per
+// head its scratch needs: a.nsplit = gqa_decode_q8_slots(...) and a.part laid out [head][slot][hd + 2].  It merges its partials itself.
+bool gqa_decode_q8_balanced(const KvView &kv, int nh);
+int gqa_decode_q8_slots(int nkv, int nh, int n_seq, int max_len, int range_floor);
+ornith_status launch_gqa_decode_q8_tc5(const DecodeArgs &a, int n_seq, cudaStream_t st);
 // the fewest tiles of a range: the long ones need the fewest partials, the short ones spread small batches further
 int gqa_decode_range_floor(int nkv, int nh, int n_seq, int max_len, bool short_ranges);
 

@@ -549,8 +549,7 @@ bool gqa_decode_q8_mma_supported(const KvView &kv, int nh) {
            ((uintptr_t)kv.K % 16) == 0 && ((uintptr_t)kv.V % 16) == 0;
 }
 
-// ORNITH_CUDA_DECODE_VARIANT: unset = the raw-fragment kernel (groups of 9-16 heads as two CTAs of 8 heads per KV
-// head: 0.51 of HBM bandwidth at 32 query / 2 KV heads against 0.40 for the f16-tile kernel); tile = the variant
+// ORNITH_CUDA_DECODE_VARIANT: unset = the tcgen05 kernel (gqa_decode_q8_tc5.cu has the measurements); tile = the variant
 // that decodes V into an f16 tile; mma = the f16-tile kernel for groups of 9-16 heads
 static int decode_variant() {
     static int variant = -1;
@@ -558,8 +557,8 @@ static int decode_variant() {
     return variant;
 }
 
-// ORNITH_CUDA_DECODE_SCHED=grid keeps the grid of fixed splits for the raw-fragment kernel (A/B comparison)
-bool gqa_decode_q8_raw_balanced(const KvView &kv, int nh) {
+// ORNITH_CUDA_DECODE_SCHED=grid: the raw-fragment kernel and its grid of fixed splits (A/B comparison)
+bool gqa_decode_q8_balanced(const KvView &kv, int nh) {
     static int grid_sched = -1;
     if (grid_sched < 0) { const char *e = getenv("ORNITH_CUDA_DECODE_SCHED"); grid_sched = (e && e[0] == 'g') ? 1 : 0; }
     if (grid_sched || !gqa_decode_q8_mma_supported(kv, nh)) return false;
@@ -568,6 +567,10 @@ bool gqa_decode_q8_raw_balanced(const KvView &kv, int nh) {
 
 ornith_status launch_gqa_decode_q8_mma(const DecodeArgs &a, int n_seq, cudaStream_t st, bool *merged) {
     *merged = false;
+    if (gqa_decode_q8_balanced(a.kv, a.nh)) {
+        *merged = true;
+        return launch_gqa_decode_q8_tc5(a, n_seq, st);
+    }
     static bool configured_dev[ORN_MAX_DEVICES] = {};
     bool &configured = configured_dev[orn_device_index()];
     if (!configured) {

@@ -197,47 +197,13 @@ __device__ __forceinline__ void store_chunk(float *Ow, const float (&acc)[4], in
     Ow[(2 * j + 1) * HD + dim + 1] = acc[3];
 }
 
-// Tiles (16 tokens) a decode step reads for sequence b: its context plus the token being appended; nothing for a
-// sequence whose cache is full (the step leaves it alone).
-__device__ __forceinline__ int seq_tiles(const DecodeArgs &a, int b) {
-    const int len0 = a.kv_len[b];
-    const int cap = (int)(a.kv.seq_off[b + 1] - a.kv.seq_off[b]);
-    return len0 >= cap ? 0 : (len0 + TILE) / TILE;
-}
-
-// Inclusive prefix sum of v over the 128 threads of the CTA; *total = the sum.  wt: 4 ints of shared memory.
-__device__ __forceinline__ int block_scan128(int v, int *wt, int *total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) wt[warp] = incl;
-    __syncthreads();
-    int add = 0, tot = 0;
-#pragma unroll
-    for (int w = 0; w < NWARP; w++) { const int x = wt[w]; if (w < warp) add += x; tot += x; }
-    __syncthreads();
-    *total = tot;
-    return incl + add;
-}
-
-// BALANCED = false: one CTA per (head group, split of tokens_per_split tokens, sequence); grid (groups, nsplit, n_seq).
-// BALANCED = true:  grid (groups, ranges).  The 16-token tiles of all sequences, laid end to end, are cut into
-//   gridDim.y ranges of equal length (found on the device from kv_len: the host never learns the contexts), and a
-//   CTA walks the pieces of the sequences that fall into its range, one partial per piece.  Every CTA is resident
-//   at once and all of them stream the same number of rows, so no SM runs dry before the others; a sequence
-//   shorter than a range costs one partial, a longer one as many as the ranges it touches.  The CTAs of the head
-//   groups that share the same rows (blockIdx.x) walk the same range side by side.
-template <bool BALANCED>
+// One CTA per (head group, split of tokens_per_split tokens, sequence); grid (groups, nsplit, n_seq).
 __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, const __grid_constant__ CUtensorMap map_k,
                                                               const __grid_constant__ CUtensorMap map_v, int tensor_copies) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ float m_s[NWARP][8], l_s[NWARP][8];
     __shared__ __align__(8) unsigned long long bars[NWARP][2];
-    __shared__ int pipe_failed, last_one, scan_s[NWARP], found_s[2];
+    __shared__ int pipe_failed, last_one;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // the next layer's front-end kernel may become resident now; it waits for this grid before it does anything
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -264,96 +230,20 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
     // matrices 2,3 = chunk c + 1
     const uint32_t lane_off = ((lane & 7) + ((lane >> 3) & 1) * 8) * ROWB + (lane >> 4) * 16;
 
-    // ---- the range of this CTA (kv_len and seq_off are not written by the kernel in front, so this runs before
-    //      the wait on it) ------------------------------------------------------------------------------------
-    // the walk's state lives in shared memory (the tile loop needs every register): sequence b, index of its first
-    // tile, next tile to read, end of the range, range length
-    __shared__ int walk_s[9];                                    // [5..8]: sequence, slot, first slot and partial count of the current piece
-    if (BALANCED) {
-        // Ranges are cut in units of cost: a tile costs 1, and every sequence is charged a.piece_cost extra units in
-        // front of its first tile for the fixed work of a piece (query fragments, restart of the copy pipeline,
-        // partial write), so a CTA that walks pieces of several sequences gets fewer tiles.
-        const int pad = a.piece_cost;
-        int pos, range_end, W, total = 0, mine_n = 0, mine_incl = 0;
-        for (int b0 = 0; b0 < a.n_seq; b0 += 128) {
-            const int n = b0 + tid < a.n_seq ? seq_tiles(a, b0 + tid) : 0;
-            int t;
-            const int incl = block_scan128(n ? n + pad : 0, scan_s, &t);
-            if (b0 == 0) { mine_n = n; mine_incl = incl; }           // kept for the search below when the batch is one pass
-            total += t;
-        }
-        // range length: an equal share, but no shorter than the floor (see gqa_decode_range_floor)
-        W = max((total + (int)gridDim.y - 1) / (int)gridDim.y, a.range_floor);
-        pos = (int)blockIdx.y * W;
-        range_end = min(total, pos + W);
-        if (pos >= total) { asm volatile("griddepcontrol.wait;\n" ::: "memory"); return; }
-        // the sequence whose units hold `pos`
-        if (a.n_seq <= 128) {
-            const int cost = mine_n ? mine_n + pad : 0;
-            if (mine_incl - cost <= pos && pos < mine_incl) { found_s[0] = tid; found_s[1] = mine_incl - cost; }
-        } else {
-            int running = 0;
-            for (int b0 = 0; b0 < a.n_seq; b0 += 128) {
-                const int n = b0 + tid < a.n_seq ? seq_tiles(a, b0 + tid) : 0, cost = n ? n + pad : 0;
-                int t;
-                const int incl = running + block_scan128(cost, scan_s, &t);
-                if (incl - cost <= pos && pos < incl) { found_s[0] = b0 + tid; found_s[1] = incl - cost; }
-                running += t;
-                if (running > pos) break;
-            }
-        }
-        __syncthreads();
-        if (tid == 0) { walk_s[0] = found_s[0]; walk_s[1] = found_s[1]; walk_s[2] = pos; walk_s[3] = range_end; walk_s[4] = W; }
-        __syncthreads();
-    }
-
     uint32_t phase = 0;                                           // tiles this warp has consumed: parity of its two barriers
-    bool pipe_ok = true, waited = false;
-    for (bool first_piece = true;; first_piece = false) {
-        // ---- next piece: tiles [tile_lo, tile_hi) of sequence b --------------------------------------------------
-        int tile_lo, tile_hi, slot, slot0, nlive, len0, b;
-        if (BALANCED) {
-            if (!first_piece) __syncthreads();                    // everybody has read the state of the previous piece
-            b = walk_s[0];
-            int seq_first = walk_s[1], pos = walk_s[2];
-            const int range_end = walk_s[3], W = walk_s[4];
-            if (pos >= range_end) break;
-            const int pad = a.piece_cost;
-            int nb = seq_tiles(a, b);
-            // units of sequence b: [seq_first, seq_first + pad + nb); pos < total, so b stays inside the batch
-            while (nb == 0 || seq_first + pad + nb <= pos) { seq_first += nb ? nb + pad : 0; b++; nb = seq_tiles(a, b); }
-            const int real0 = seq_first + pad;                    // unit of the sequence's first tile
-            tile_lo = max(pos - real0, 0);
-            tile_hi = min(nb, range_end - real0);
-            if (tile_hi <= tile_lo) break;                        // the range ends inside the charge in front of sequence b
-            len0 = a.kv_len[b];
-            const int c_first = real0 / W;
-            slot0 = c_first + b;                                  // (range, sequence) pairs in walking order: range + sequence is unique
-            slot = (int)blockIdx.y + b;
-            nlive = (real0 + nb - 1) / W - c_first + 1;           // ranges that hold a piece of this sequence
-            __syncthreads();                                      // everybody has read the old state
-            if (tid == 0) {
-                walk_s[0] = b; walk_s[1] = seq_first; walk_s[2] = seq_first + a.piece_cost + tile_hi;
-                walk_s[5] = b; walk_s[6] = slot; walk_s[7] = slot0; walk_s[8] = nlive;
-            }
-        } else {
-            if (!first_piece) break;
-            b = blockIdx.z;
-            len0 = a.kv_len[b];
-            // A CTA that leaves early still has to wait for the grid in front (programmatic dependent launch):
-            // a grid whose CTAs all returned without waiting would retire, and let the next kernel in the
-            // stream start, before the append kernel has finished.
-            if (len0 >= (int)(a.kv.seq_off[b + 1] - a.kv.seq_off[b])) { asm volatile("griddepcontrol.wait;\n" ::: "memory"); return; }
-            const int tps_tiles = a.tokens_per_split / TILE, nb = (len0 + TILE) / TILE;
-            slot = blockIdx.y; slot0 = 0;
-            tile_lo = slot * tps_tiles;
-            tile_hi = min(nb, tile_lo + tps_tiles);
-            nlive = min(a.nsplit, (len0 + a.tokens_per_split) / a.tokens_per_split);     // splits with t0 < L
-        }
+    bool pipe_ok = true;
+    const int b = blockIdx.z, slot = blockIdx.y, len0 = a.kv_len[b];
+    // A CTA that leaves early still has to wait for the grid in front (programmatic dependent launch):
+    // a grid whose CTAs all returned without waiting would retire, and let the next kernel in the
+    // stream start, before the append kernel has finished.
+    if (len0 >= (int)(a.kv.seq_off[b + 1] - a.kv.seq_off[b])) { asm volatile("griddepcontrol.wait;\n" ::: "memory"); return; }
+    const int tps_tiles = a.tokens_per_split / TILE, tile_lo = slot * tps_tiles, tile_hi = min((len0 + TILE) / TILE, tile_lo + tps_tiles);
+    const int nlive = min(a.nsplit, (len0 + a.tokens_per_split) / a.tokens_per_split);     // splits with t0 < L
+    {
         const int64_t base = a.kv.seq_off[b];
         const int L = len0 + 1;
         const int t0 = tile_lo * TILE, t1 = min(L, tile_hi * TILE);
-        if (!BALANCED && t0 >= L) {
+        if (t0 >= L) {
             asm volatile("griddepcontrol.wait;\n" ::: "memory");
             float *pd = a.part + (((size_t)b * a.nh + (size_t)head0) * a.nsplit + slot) * (HD + 2);
             const size_t part_stride = (size_t)a.nsplit * (HD + 2);
@@ -365,26 +255,24 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
         // start of the pool
         int rem = t1 - t0 - warp * TILE, tok_abs = (int)base + t0 + warp * TILE;
 
-        // ---- per-warp staging slots (K rows, V rows): zero them (skipped tail rows must stay finite; the slots
-        //      also held the warp's output tile of the piece before).  K of the next tile is requested as soon as
+        // ---- per-warp staging slots (K rows, V rows): zero them (skipped tail rows must stay finite).  K of the next tile is requested as soon as
         //      the score loop is done with the slot, V right after the value loop.  The first tile is requested
         //      before anything else so that its latency hides behind the query prologue; under programmatic
         //      dependent launch that happens while the append kernel of this call may still be running, so only
         //      for tiles that end before the row it appends (token len0).
-        if (!BALANCED && !first_piece) __syncthreads();           // (BALANCED: the barriers of the walk above already separate the pieces)
         {
             uint4 *z = reinterpret_cast<uint4 *>(wbase);
             for (int i = lane; i < WARP_BYTES / 16; i += 32) z[i] = make_uint4(0u, 0u, 0u, 0u);
             fence_proxy_async();                                  // generic-proxy zeros before async-proxy copies
             __syncwarp();
         }
-        const bool first_issued = pipe_ok && rem > 0 && (waited || t0 + (warp + 1) * TILE <= len0);
+        const bool first_issued = rem > 0 && t0 + (warp + 1) * TILE <= len0;
         if (first_issued) {
             issue_rows16(rawK, barK, a.kv.K, nkv, rem, lane, mk, kvh, tok_abs);
             issue_rows16(rawV, barV, a.kv.V, nkv, rem, lane, mv, kvh, tok_abs);
         }
         // everything below reads what the append kernel of this call wrote (query rows, the new K/V row, zeroed counters)
-        if (!waited) { asm volatile("griddepcontrol.wait;\n" ::: "memory"); waited = true; }
+        asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
         // ---- query group -> B fragments in stream order: lane (head r, quarter j), k-step c
         //      holds q at the dims of elements 8c+2j and 8c+2j+1 (zeros where the stream has a scale)
@@ -539,13 +427,9 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
             lA += __shfl_xor_sync(0xffffffffu, lA, sft);
             lB += __shfl_xor_sync(0xffffffffu, lB, sft);
         }
-        if (BALANCED) {                                               // (published by the barrier behind the query fragments)
-            const volatile int *w = walk_s;
-            b = w[5]; slot = w[6]; slot0 = w[7]; nlive = w[8];
-        }
-        // partials: BALANCED [head][slot], else [sequence][head][split]; a.nsplit = partial slots per head
+        // partials [sequence][head][split]; a.nsplit = partial slots per head
         const size_t part_stride = (size_t)a.nsplit * (HD + 2);     // next head
-        float *part_g = a.part + (BALANCED ? (size_t)head0 * a.nsplit : ((size_t)b * a.nh + (size_t)head0) * a.nsplit) * (HD + 2);
+        float *part_g = a.part + (((size_t)b * a.nh + (size_t)head0) * a.nsplit) * (HD + 2);
         float *part0 = part_g + (size_t)slot * (HD + 2);
         float *Ow = reinterpret_cast<float *>(smem + QS_BYTES + warp * WARP_BYTES);   // [8 heads][256] f32 over this warp's slots
         store_chunk<0>(Ow, o[0], r, j);   store_chunk<1>(Ow, o[1], r, j);   store_chunk<2>(Ow, o[2], r, j);
@@ -583,7 +467,7 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
                 part[2 + d] = acc * (1.0f / 256.0f) + poison;
             }
         }
-        if (a.group_ctr == nullptr) continue;                         // (only without BALANCED: the combine kernel merges)
+        if (a.group_ctr == nullptr) return;                           // (the combine kernel merges)
 
         // ---- fused merge: the last CTA of this (sequence, head group) to get here combines the group's partials
         //      (reference: src/ornith_attn.c:131-148 normalisation, src/ornith_rforward.c:450 gate).  Nobody waits:
@@ -595,7 +479,7 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
             last_one = (atomicAdd(ctr, 1) == nlive - 1);
         }
         __syncthreads();
-        if (!last_one) continue;
+        if (!last_one) return;
         __threadfence();
         // 16 threads per head, all heads at once: thread (h, q) owns the float2 columns q + 16 k of head h.
         // Partials of other SMs are read past L1.  Four partials' rows are in flight per thread at a time.
@@ -614,7 +498,7 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_q8_raw(DecodeArgs a, cons
                                   : make_float2(act_ld((const float *)a.qproj, at), act_ld((const float *)a.qproj, at + 1));
             }
             const unsigned hm = 0xffffu << (lane & 16);           // this half-warp (the other half may belong to no head)
-            const float *ph = part_g + (size_t)slot0 * (HD + 2) + h * part_stride;   // first partial of head h
+            const float *ph = part_g + h * part_stride;   // first partial of head h
             const float2 ml0 = q < nlive ? __ldcg(reinterpret_cast<const float2 *>(ph + (size_t)q * (HD + 2))) : make_float2(0.0f, 0.0f);
             float M = ml0.y > 0.0f ? ml0.x : -INFINITY;
             for (int s = q + 16; s < nlive; s += 16) {
@@ -707,44 +591,13 @@ bool q8_rows_map(CUtensorMap *m, const void *pool, int nkv) {
 
 }  // namespace
 
-// ranges of the balanced schedule: one per resident CTA of a head-group column (4 CTAs on each of 148 SMs), fewer when
-// the batch is too small for ranges of at least floor_w tiles (same rule as in the kernel)
-static int balanced_ranges(int nkv, int nh, int n_seq, int max_len, int floor_w) {
-    const int X = nkv * ((nh / nkv + 7) / 8);
-    const long long tiles = (max_len + TILE - 1) / TILE;
-    const long long by_work = ((long long)n_seq * tiles + floor_w - 1) / floor_w, cap = 592 / X > 0 ? 592 / X : 1;
-    return (int)(by_work < cap ? (by_work > 0 ? by_work : 1) : cap);
-}
-// By the longest context the call allows.  The last CTA of a sequence merges its partials alone: past ~32 of them that
-// outweighs the gain of a shorter range.  Short ranges: 16 tiles (four per warp) are halved while at most 16 partials
-// result (below 8 tiles, two per warp, the fixed work of a piece is all there is), and only while the long ones give fewer
-// than 100 CTAs.  224 batches of 1 to 64 sequences of 25 to 3000 tokens, 35B, one group of four layers, time with long ranges /
-// with short ones by CTAs of the long form: below 40 1.08, 40 to 60 1.06, 60 to 100 1.04; from 100 up 0.997 to 1.013 in the
-// mean and single batches down to 0.92 (20 sequences of 3000: 107.5 us long, 113.7 short).
-int gqa_decode_range_floor(int nkv, int nh, int n_seq, int max_len, bool short_ranges) {
-    const int tiles = (max_len + TILE - 1) / TILE, w16 = (tiles + 15) / 16, w32 = (tiles + 31) / 32, w_long = w32 > 16 ? w32 : 16;
-    const int X = nkv * ((nh / nkv + 7) / 8);
-    if (!short_ranges || w16 > 16 || X * balanced_ranges(nkv, nh, n_seq, max_len, w_long) >= 100) return w_long;
-    return w16 < 8 ? 8 : w16;
-}
-int gqa_decode_q8_raw_slots(int nkv, int nh, int n_seq, int max_len, int range_floor) {
-    return balanced_ranges(nkv, nh, n_seq, max_len, range_floor) + n_seq;
-}
-
 ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a_in, int n_seq, cudaStream_t st, bool *merged) {
     DecodeArgs a = a_in;
     *merged = a.group_ctr != nullptr;
-    const bool balanced = gqa_decode_q8_raw_balanced(a.kv, a.nh);
-    if (balanced && !a.group_ctr) {
-        orn_record_error("k_gqa_decode_q8_raw: the balanced schedule merges its partials itself and needs the arrival counters");
-        return ORNITH_ERR_FORMAT;
-    }
     static bool configured_dev[ORN_MAX_DEVICES] = {};
     bool &configured = configured_dev[orn_device_index()];
     if (!configured) {
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_gqa_decode_q8_raw<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               SMEM_BYTES), "gqa decode smem opt-in"));
-        ORN_TRY(orn_check(cudaFuncSetAttribute(k_gqa_decode_q8_raw<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        ORN_TRY(orn_check(cudaFuncSetAttribute(k_gqa_decode_q8_raw, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                SMEM_BYTES), "gqa decode smem opt-in"));
         configured = true;
     }
@@ -757,11 +610,7 @@ ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a_in, int n_seq, cudaSt
     const int X = a.kv.nkv * ((a.nh / a.kv.nkv + 7) / 8);
     a.n_seq = n_seq;
     a.status = orn_status_word();
-    static int piece_cost = -1;                                   // ORNITH_CUDA_DECODE_PIECE_COST=<tiles>: see the kernel
-    if (piece_cost < 0) { const char *e = getenv("ORNITH_CUDA_DECODE_PIECE_COST"); piece_cost = e ? atoi(e) : 4; if (piece_cost < 0 || piece_cost > 15) piece_cost = 4; }
-    a.piece_cost = piece_cost;
     dim3 grid(X, a.nsplit, n_seq);
-    if (balanced) grid = dim3(X, balanced_ranges(a.kv.nkv, a.nh, n_seq, a.max_len, a.range_floor), 1);
     // may start while the append kernel in front of it still runs: it waits (griddepcontrol.wait) before it reads that kernel's output
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = dim3(128); cfg.dynamicSmemBytes = SMEM_BYTES; cfg.stream = st;
@@ -769,6 +618,5 @@ ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a_in, int n_seq, cudaSt
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    if (balanced) return orn_check(cudaLaunchKernelEx(&cfg, k_gqa_decode_q8_raw<true>, a, mk, mv, tensor_copies), "k_gqa_decode_q8_raw");
-    return orn_check(cudaLaunchKernelEx(&cfg, k_gqa_decode_q8_raw<false>, a, mk, mv, tensor_copies), "k_gqa_decode_q8_raw");
+    return orn_check(cudaLaunchKernelEx(&cfg, k_gqa_decode_q8_raw, a, mk, mv, tensor_copies), "k_gqa_decode_q8_raw");
 }

@@ -504,3 +504,58 @@ def test_scratch_of_the_long_ranges_is_still_enough():
     assert step(need) == 0
     assert rel_err(out.cpu().numpy(), ref.cpu().numpy()) < 1e-3          # the same sums in another order, f16 operands
     assert step(need - 256) != 0
+
+
+@pytest.mark.parametrize("nh,nkv,row_copies", [(2, 2, "0"), (16, 2, "0"), (18, 2, "0"), (32, 2, "0"), (24, 3, "0"), (16, 2, "1")])
+def test_q8_decode_edges(oracle, monkeypatch, nh, nkv, row_copies):
+    """Q8_0 decode around the units (16 tokens), copies (32), halves (64) and tiles (128) of the tcgen05 kernel, 1 to 16 heads to a
+    KV head (their score columns come in 8s), a full cache in the middle, rows copied one by one.  TOL: f16 rounding (2^-11) of q, K, V
+    and the probabilities, against the largest output."""
+    import torch
+    from ornithology_b200 import device as D
+    monkeypatch.setenv("ORNITH_CUDA_DECODE_ROW_COPIES", row_copies)
+    layer = full_case(40 + nh, nh=nh, nkv=nkv)
+    dl = device_full(layer)
+    ctx = [0, 15, 16, 31, 63, 64, 9, 127, 128, 129, 300]
+    caps = [c + 2 for c in ctx]
+    caps[6] = ctx[6]
+    T = max(ctx)
+    dm, om = _modes("q8_0")
+    kv = D.KvBatch(dm, nkv, layer.hd, caps)
+    QP, K, V = zip(*[full_inputs(400 + b, layer, T + 2) for b in range(len(ctx))])
+    z = torch.zeros(len(ctx), dtype=torch.int32, device="cuda")
+    to = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    D.kv_append(dl, kv, z, to(np.stack([k[:T] for k in K])), to(np.stack([v[:T] for v in V])), T=T)
+    okvs = []
+    for b, c in enumerate(ctx):
+        okvs.append(oracle.kv(max(caps[b], 1), nkv, layer.hd, om))
+        if c:
+            oracle.full_attn_prefill(layer, okvs[b], 0, QP[b][:c], K[b][:c], V[b][:c])
+    kv_len = torch.tensor(ctx, dtype=torch.int32, device="cuda")
+    for s in range(2):
+        at = lambda x: to(np.stack([x[b][ctx[b] + s] for b in range(len(ctx))]))
+        out = D.full_attn_step(dl, kv, kv_len, at(QP), at(K), at(V), max_len=max(caps)).cpu().numpy()
+        for b, c in enumerate(ctx):
+            if c + s < caps[b]:
+                ref = oracle.full_attn_step(layer, okvs[b], c + s, QP[b][c + s], K[b][c + s], V[b][c + s])
+                assert rel_err(out[b], ref) < TOL, (s, b)
+        D.advance(kv_len)
+
+
+def test_q8_decode_many_short_sequences(oracle):
+    """650 sequences of one or two tokens on 8 KV heads: 36 to a CTA, more than its list of merges left for the end holds (32)."""
+    import torch
+    from ornithology_b200 import device as D
+    layer = full_case(60, nh=8, nkv=8)
+    dl = device_full(layer)
+    n = 650
+    dm, om = _modes("q8_0")
+    kv = D.KvBatch(dm, 8, layer.hd, [2] * n)
+    okvs = [oracle.kv(2, 8, layer.hd, om) for _ in range(n)]
+    kv_len = torch.zeros(n, dtype=torch.int32, device="cuda")
+    for s in range(2):
+        QP, K, V = full_inputs(600 + s, layer, n)
+        out = D.full_attn_step(dl, kv, kv_len, *[torch.from_numpy(x).cuda() for x in (QP, K, V)], max_len=2).cpu().numpy()
+        for b in range(n):
+            assert rel_err(out[b], oracle.full_attn_step(layer, okvs[b], s, QP[b], K[b], V[b])) < TOL, (s, b)
+        D.advance(kv_len)
