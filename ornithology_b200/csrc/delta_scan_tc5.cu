@@ -395,7 +395,9 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
 //               32-byte swizzle atoms (a K-major tf32 operand must lie in 16-byte atoms, so K is copied twice)
 //   warp 25     one lane issues the tcgen05.mma of the chain and Q S^T
 //   warp 26     one lane issues those of P U: behind the state update in one stream they kept the issuing lane from the next chunk
-//   warp 27     one lane issues the copies of z and of the outputs, and asks L2 for what comes two chunks later
+//   warp 27     one lane issues the copies of z and of the outputs, and asks L2 for what comes two chunks later (without such
+//               copies warp 24 asks: a lane that nothing waits for must not follow the scan by the parity of a barrier, which may
+//               go round unseen)
 // Tensor memory, 512 columns: two states of 128 (chunk n reads number n & 1; the other takes the decayed copy and then the
 // update), K S^T / w rk U, the accumulator and then operand U, Q S^T, P U.
 // A product that reads what an earlier product of another shape accumulated (the state, K S^T) is only issued after a wait on that
@@ -560,13 +562,30 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     __syncthreads();
     bool ok = true;
 
+    constexpr int TZ = (int)sizeof(ACT), CZ = 128 / TZ;   // tiles of z: their number, their channels
+    const bool tiles = TILE && !(SEG && kind);            // z and the outputs by tensor copies
+    const unsigned char *rec0 = a.rec + (((size_t)b * a.nv + hv) * a.rec_chunks + (SEG ? c0 : 0)) * (size_t)REC_BYTES;
+    auto l2_2d = [&](int x, int y) {
+        asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&map_ym), "r"(x), "r"(y) : "memory");
+    };
+    auto ahead = [&](int n) {                                     // (K and Q rows are shared by the value heads of a key head)
+        if (n >= N) return;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rec0 + (size_t)n * REC_BYTES), "r"((uint32_t)REC_BYTES) : "memory");
+        for (int sl = 0; sl < 4; sl++) l2_2d(2 * qd + hv * 128 + 32 * sl, b * a.T + (c0 + n) * C);
+        if (tiles)
+            for (int t = 0; t < TZ; t++)
+                asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
+                             ::"l"(&map_z), "r"(hv * 128 + t * CZ), "r"((c0 + n) * C), "r"(b) : "memory");
+    };
+
     if (warp == W_TMA) {
         // ================= producer =================
         if (elect_one()) {
             asm volatile("griddepcontrol.wait;\n" ::: "memory");     // everything that comes through here is written by the kernels in front
             const int yrow0 = b * a.T + c0 * C;                       // row of this CTA's first token
-            const unsigned char *rec0 = a.rec + (((size_t)b * a.nv + hv) * a.rec_chunks + (SEG ? c0 : 0)) * (size_t)REC_BYTES;
+            if (!tiles) ahead(1);
             for (int n = 0; n < N && ok; n++) {
+                if (!tiles) ahead(n + 2);                                 // (behind the waits of the chunk before)
                 const unsigned char *r = rec0 + (size_t)n * REC_BYTES;
                 const int y = yrow0 + n * C;
                 auto refill = [&](int s, uint32_t bytes) {                // the buffer is free: its next contents are announced
@@ -893,33 +912,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     }
     if (warp == W_IO) {
         // ================= z, outputs, L2 =================
-        if (elect_one()) {
+        if (tiles && elect_one()) {
             asm volatile("griddepcontrol.wait;\n" ::: "memory");
-            constexpr int TZ = (int)sizeof(ACT), CZ = 128 / TZ;           // tiles of z: their number, their channels
-            const bool out = TILE && !(SEG && kind);
-            const unsigned char *rec0 = a.rec + (((size_t)b * a.nv + hv) * a.rec_chunks + (SEG ? c0 : 0)) * (size_t)REC_BYTES;
-            auto l2_2d = [&](int x, int y) {
-                asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&map_ym), "r"(x), "r"(y) : "memory");
-            };
-            auto ahead = [&](int n) {                                     // (K and Q rows are shared by the value heads of a key head)
-                if (n >= N) return;
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rec0 + (size_t)n * REC_BYTES), "r"((uint32_t)REC_BYTES) : "memory");
-                for (int sl = 0; sl < 4; sl++) l2_2d(2 * qd + hv * 128 + 32 * sl, b * a.T + (c0 + n) * C);
-                if (out)
-                    for (int t = 0; t < TZ; t++)
-                        asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
-                                     ::"l"(&map_z), "r"(hv * 128 + t * CZ), "r"((c0 + n) * C), "r"(b) : "memory");
-            };
             auto load_z = [&](int n) {
                 mbar_expect_tx(su32(&bars.full_z), (uint32_t)(C * 128 * TZ));
                 for (int t = 0; t < TZ; t++)
                     tma_load_3d(base + SM_Z + t * 8192, &map_z, hv * 128 + t * CZ, (c0 + n) * C, b, su32(&bars.full_z));
             };
             ahead(1);
-            if (out) load_z(0);
+            load_z(0);
             for (int n = 0; n < N && ok; n++) {
                 ahead(n + 2);
-                if (!out) { ok = mbar_wait_parked(su32(&bars.ks_done), (uint32_t)n & 1u); continue; }      // (no faster than the scan)
                 ok = mbar_wait_parked(su32(&bars.empty_z), (uint32_t)n & 1u);
                 if (ok && n + 1 < N) load_z(n + 1);
                 if (TZ == 2 && ok) {

@@ -372,3 +372,32 @@ def test_scan_head_counts_and_unaligned_tensors(oracle, nk, nv, grouped, T, bf16
         ref = oracle.linear_attn_prefill(layer, S, buf, *seqs[b], chunk=64)
         assert rel_err(out[b].float().cpu().numpy(), ref) < (TOL_BF16_IO if bf16 else TOL)
         assert rel_err(st.S[b].cpu().numpy(), S) < TOL
+
+
+@pytest.mark.parametrize("segments,bf16", [(1, True), (1, False), (3, True)])
+def test_scan_without_output_copies_ends_with_clean_status(monkeypatch, segments, bf16):
+    """CTAs of the scan whose z and outputs are no tensor copies (off the 16-byte grid; runs from zero and from the identity): no
+    wait of theirs may depend on how far another lane of the CTA has got.  50 chunks: no wait gave up, and the single run has the
+    same bits as with the copies."""
+    import torch
+    from ornithology_b200 import _lib, device as D
+    layer, kw = linear_case(43, nk=2, nv=4)
+    dl = device_linear(layer, kw)
+    T, dt = 3200, torch.bfloat16 if bf16 else torch.float32
+    qkv, a, bm, z = (_t(x, dt)[None] for x in linear_inputs(430, layer, T, bf16))
+
+    def run(n_seg, off):
+        monkeypatch.setenv("ORNITH_CUDA_DELTA_SEGMENTS", str(n_seg))
+        buf = torch.empty(2, T * layer.vd + 8, dtype=dt, device="cuda")
+        zz, out = (b[off:off + T * layer.vd].view(1, T, layer.vd) for b in buf)
+        zz.copy_(z)
+        st = D.LinearState(dl, 1)
+        D.linear_attn_prefill(dl, st, torch.zeros(1, dtype=torch.int32, device="cuda"), qkv, a, bm, zz, T, out=out)
+        torch.cuda.synchronize()
+        assert _lib.load().ornith_cuda_poll_status() == 0
+        return out.float().cpu().numpy(), st.S.cpu().numpy()
+
+    ref, got = run(1, 0), run(segments, 1 if segments == 1 else 0)
+    if segments == 1:
+        assert (ref[0] == got[0]).all() and (ref[1] == got[1]).all()
+    assert rel_err(got[0], ref[0]) < (TOL_BF16_IO if bf16 else TOL) and rel_err(got[1], ref[1]) < TOL
