@@ -1255,7 +1255,11 @@ ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dty
         orn_record_error("delta scan: %d sequences x %d tokens exceed the tensor-map coordinates", n_seq, x.T);
         return ORNITH_ERR_UNSUPPORTED;
     }
-    const DeltaPlan p = delta_plan(x.nv, n_seq, x.T);
+    DeltaPlan p = delta_plan(x.nv, n_seq, x.T);
+    // the finishing pass behind several runs reads z and the norm's weights and writes the outputs four values at a time: a call
+    // with any of them off that grid is one run, whose records take no more scratch
+    const uintptr_t four = act_dtype == ORNITH_ACT_BF16 ? 8 : 16;
+    if (p.n_seg > 1 && (((uintptr_t)x.z | (uintptr_t)x.out) % four || (uintptr_t)x.norm_w % 16)) p.n_seg = 1;
     static bool configured_dev[ORN_MAX_DEVICES] = {};
     bool &configured = configured_dev[orn_device_index()];
     if (!configured) {

@@ -401,3 +401,27 @@ def test_scan_without_output_copies_ends_with_clean_status(monkeypatch, segments
     if segments == 1:
         assert (ref[0] == got[0]).all() and (ref[1] == got[1]).all()
     assert rel_err(got[0], ref[0]) < (TOL_BF16_IO if bf16 else TOL) and rel_err(got[1], ref[1]) < TOL
+
+
+@pytest.mark.parametrize("bf16,shifted", [(True, 1), (True, 4), (False, 1), (False, 2)])
+def test_runs_of_unaligned_tensors(monkeypatch, bf16, shifted):
+    """Few heads, z and out `shifted` elements off a 16-byte boundary: the finishing pass of several runs works on four values at
+    a time, so such a call is one run unless four of its values still lie on their own boundary (4 of bf16)."""
+    import torch
+    from ornithology_b200 import device as D
+    layer, kw = linear_case(44, nk=2, nv=4)
+    dl = device_linear(layer, kw)
+    T, dt = 1600, torch.bfloat16 if bf16 else torch.float32
+    qkv, a, bm, z = (_t(x, dt)[None] for x in linear_inputs(440, layer, T, bf16))
+
+    def run(n_seg, off):
+        monkeypatch.setenv("ORNITH_CUDA_DELTA_SEGMENTS", str(n_seg))
+        buf = torch.empty(2, T * layer.vd + 8, dtype=dt, device="cuda")
+        zz, out = (b[off:off + T * layer.vd].view(1, T, layer.vd) for b in buf)
+        zz.copy_(z)
+        st = D.LinearState(dl, 1)
+        D.linear_attn_prefill(dl, st, torch.zeros(1, dtype=torch.int32, device="cuda"), qkv, a, bm, zz, T, out=out)
+        return out.float().cpu().numpy(), st.S.cpu().numpy()
+
+    ref, got = run(3 if bf16 and shifted == 4 else 1, 0), run(3, shifted)
+    assert (got[0] == ref[0]).all() and (got[1] == ref[1]).all()
