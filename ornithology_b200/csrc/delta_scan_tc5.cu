@@ -63,6 +63,11 @@ __device__ __forceinline__ int tri_at(int i, int l) { return (l & 32) * 64 + (i 
 __device__ __forceinline__ float tf32r(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
 __device__ __forceinline__ float tf32q(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
 
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
 __device__ __forceinline__ void mma_tf32_sync(float (&d)[4], const float (&a)[4], float b0, float b1) {
     asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -199,8 +204,8 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
         mbar_init_fence();
         mbar_expect_tx(su32(&rows_in), 65536u);
         for (int sl = 0; sl < 4; sl++) {
-            tma_load_2d(su32(sm.u.t.K) + sl * 8192, &map_y, qd + kh * 128 + 32 * sl, (int)tok0, su32(&rows_in));
-            tma_load_2d(su32(sm.u.t.Q) + sl * 8192, &map_y, kh * 128 + 32 * sl, (int)tok0, su32(&rows_in));
+            tma_load_3d(su32(sm.u.t.K) + sl * 8192, &map_y, qd + kh * 128 + 32 * sl, t0, b, su32(&rows_in));
+            tma_load_3d(su32(sm.u.t.Q) + sl * 8192, &map_y, kh * 128 + 32 * sl, t0, b, su32(&rows_in));
         }
     }
     if (tid < C) {
@@ -290,7 +295,7 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
                     mma_tf32_sync(gq[t], qa[1], r[2], r[3]);
                 }
         }
-        if (n < C) {                                      // rows past the end are another sequence's: whatever they hold, they count as zero
+        if (n < C) {                                      // rows past the end are zeros, which count for nothing whatever they meet
 #pragma unroll
             for (int t = 0; t < 3; t++)
 #pragma unroll
@@ -476,10 +481,6 @@ __device__ __forceinline__ uint32_t ld_raw(const __nv_bfloat16 *p, size_t i) { r
 __device__ __forceinline__ float cvt_raw(const float *, uint32_t r) { return __uint_as_float(r); }
 __device__ __forceinline__ float cvt_raw(const __nv_bfloat16 *, uint32_t r) { return __uint_as_float(r << 16); }
 
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
-}
 // this thread's stores to shared memory, seen by the tensor copy a thread issues after a barrier
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -565,36 +566,33 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     constexpr int TZ = (int)sizeof(ACT), CZ = 128 / TZ;   // tiles of z: their number, their channels
     const bool tiles = TILE && !(SEG && kind);            // z and the outputs by tensor copies
     const unsigned char *rec0 = a.rec + (((size_t)b * a.nv + hv) * a.rec_chunks + (SEG ? c0 : 0)) * (size_t)REC_BYTES;
-    auto l2_2d = [&](int x, int y) {
-        asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(&map_ym), "r"(x), "r"(y) : "memory");
+    auto l2_rows = [&](const CUtensorMap *map, int x, int t) {
+        asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(x), "r"(t), "r"(b) : "memory");
     };
     auto ahead = [&](int n) {                                     // (K and Q rows are shared by the value heads of a key head)
         if (n >= N) return;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rec0 + (size_t)n * REC_BYTES), "r"((uint32_t)REC_BYTES) : "memory");
-        for (int sl = 0; sl < 4; sl++) l2_2d(2 * qd + hv * 128 + 32 * sl, b * a.T + (c0 + n) * C);
+        for (int sl = 0; sl < 4; sl++) l2_rows(&map_ym, 2 * qd + hv * 128 + 32 * sl, (c0 + n) * C);
         if (tiles)
-            for (int t = 0; t < TZ; t++)
-                asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
-                             ::"l"(&map_z), "r"(hv * 128 + t * CZ), "r"((c0 + n) * C), "r"(b) : "memory");
+            for (int t = 0; t < TZ; t++) l2_rows(&map_z, hv * 128 + t * CZ, (c0 + n) * C);
     };
 
     if (warp == W_TMA) {
         // ================= producer =================
         if (elect_one()) {
             asm volatile("griddepcontrol.wait;\n" ::: "memory");     // everything that comes through here is written by the kernels in front
-            const int yrow0 = b * a.T + c0 * C;                       // row of this CTA's first token
             if (!tiles) ahead(1);
             for (int n = 0; n < N && ok; n++) {
                 if (!tiles) ahead(n + 2);                                 // (behind the waits of the chunk before)
                 const unsigned char *r = rec0 + (size_t)n * REC_BYTES;
-                const int y = yrow0 + n * C;
+                const int t0 = (c0 + n) * C;                              // (rows past the sequence's last token arrive as zeros)
                 auto refill = [&](int s, uint32_t bytes) {                // the buffer is free: its next contents are announced
                     if (n >= 1) ok = ok && mbar_wait_parked(su32(&bars.empty[s]), (uint32_t)(n - 1) & 1u);
                     if (ok) mbar_expect_tx(su32(&bars.full[s]), bytes);
                     return ok;
                 };
                 auto rows = [&](int dst, const CUtensorMap *map, int x, int s) {
-                    for (int sl = 0; sl < 4; sl++) tma_load_2d(base + dst + sl * 8192, map, x + 32 * sl, y, su32(&bars.full[s]));
+                    for (int sl = 0; sl < 4; sl++) tma_load_3d(base + dst + sl * 8192, map, x + 32 * sl, t0, b, su32(&bars.full[s]));
                 };
                 auto part = [&](int dst, int off, uint32_t bytes, int s) { bulk_load(base + dst, r + off, bytes, su32(&bars.full[s])); };
                 if (!refill(B_K, 32768u)) break;
@@ -1118,24 +1116,11 @@ int delta_seg_plan(int nv, int n_seq, int n_chunks, int *seg_chunks) {
     return p;
 }
 
-// [rows][cols] f32, boxes of 32 columns x box_rows rows; 128-byte swizzle, in 16-byte or in 32-byte atoms
-ornith_status f32_rows_map(CUtensorMap *m, const void *basep, uint64_t cols, uint64_t rows, uint32_t box_rows, bool atom32) {
-    OrnTensorMapEncodeFn enc = orn_tensor_map_encoder();
-    if (!enc) { orn_record_error("delta scan: cuTensorMapEncodeTiled is not available"); return (ornith_status)ORNITH_ERR_BACKEND; }
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)cols * 4};
-    cuuint32_t box[2] = {32, box_rows};
-    cuuint32_t es[2] = {1, 1};
-    const CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void *>(basep), dims, strides, box, es,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           atom32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) { orn_record_error("delta scan: cuTensorMapEncodeTiled failed (%d)", (int)r); return (ornith_status)ORNITH_ERR_BACKEND; }
-    return ORNITH_OK;
-}
-
-// [n_seq][T][width] activations: boxes of 128 bytes of channels x `rows` tokens of one sequence, 128-byte swizzle
-ornith_status act_rows_map(CUtensorMap *m, const void *basep, bool bf, uint64_t width, uint64_t T, uint64_t n_seq, uint32_t rows) {
+// [n_seq][T][width] values: boxes of 128 bytes of channels x `rows` tokens of one sequence, 128-byte swizzle.  The sequences are a
+// dimension of their own: rows of a box behind a sequence's last token arrive as zeros and not as the next one's first tokens, whose
+// infinities the products would spread over the chunk (0 x Inf).
+ornith_status rows_map(CUtensorMap *m, const void *basep, bool bf, uint64_t width, uint64_t T, uint64_t n_seq, uint32_t rows,
+                       CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
     OrnTensorMapEncodeFn enc = orn_tensor_map_encoder();
     if (!enc) { orn_record_error("delta scan: cuTensorMapEncodeTiled is not available"); return (ornith_status)ORNITH_ERR_BACKEND; }
     const uint64_t row = width * (bf ? 2 : 4);
@@ -1144,7 +1129,7 @@ ornith_status act_rows_map(CUtensorMap *m, const void *basep, bool bf, uint64_t 
     cuuint32_t box[3] = {bf ? 64u : 32u, rows, 1};
     cuuint32_t es[3] = {1, 1, 1};
     const CUresult r = enc(m, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(basep), dims, strides, box, es,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { orn_record_error("delta scan: cuTensorMapEncodeTiled failed (%d)", (int)r); return (ornith_status)ORNITH_ERR_BACKEND; }
     return ORNITH_OK;
@@ -1277,12 +1262,12 @@ ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dty
     // z and the outputs travel by tensor copies where their rows lie on 16-byte boundaries (the row length always is a multiple)
     const bool tile = ((uintptr_t)x.z % 16) == 0 && ((uintptr_t)x.out % 16) == 0;
     CUtensorMap my, mym, mz, mo;
-    ORN_TRY(f32_rows_map(&my, Y, (uint64_t)Cc, (uint64_t)n_seq * x.T, C, false));
-    ORN_TRY(f32_rows_map(&mym, Y, (uint64_t)Cc, (uint64_t)n_seq * x.T, C, true));
+    ORN_TRY(rows_map(&my, Y, false, (uint64_t)Cc, (uint64_t)x.T, (uint64_t)n_seq, C));
+    ORN_TRY(rows_map(&mym, Y, false, (uint64_t)Cc, (uint64_t)x.T, (uint64_t)n_seq, C, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B));
     mz = mo = my;
     if (tile) {
-        ORN_TRY(act_rows_map(&mz, x.z, bf, (uint64_t)x.nv * 128, (uint64_t)x.T, (uint64_t)n_seq, C));
-        ORN_TRY(act_rows_map(&mo, x.out, bf, (uint64_t)x.nv * 128, (uint64_t)x.T, (uint64_t)n_seq, 16));
+        ORN_TRY(rows_map(&mz, x.z, bf, (uint64_t)x.nv * 128, (uint64_t)x.T, (uint64_t)n_seq, C));
+        ORN_TRY(rows_map(&mo, x.out, bf, (uint64_t)x.nv * 128, (uint64_t)x.T, (uint64_t)n_seq, 16));
     }
     unsigned char *rec = (unsigned char *)work;
     const size_t slot_bytes = (size_t)units * p.per * REC_BYTES;

@@ -425,3 +425,26 @@ def test_runs_of_unaligned_tensors(monkeypatch, bf16, shifted):
 
     ref, got = run(3 if bf16 and shifted == 4 else 1, 0), run(3, shifted)
     assert (got[0] == ref[0]).all() and (got[1] == ref[1]).all()
+
+
+@pytest.mark.parametrize("bf16,where", [(False, "v"), (True, "v"), (False, "k"), (True, "q")])
+def test_sequences_of_a_batch_stay_apart(bf16, where):
+    """65 tokens: the second chunk's tiles reach 63 rows past the sequence's last token.  Infinities in the first tokens of the next
+    sequence leave this one as it is alone, bit for bit."""
+    import torch
+    from ornithology_b200 import device as D
+    layer, kw = linear_case(45, nk=2, nv=4)
+    dl = device_linear(layer, kw)
+    T, dt = 65, torch.bfloat16 if bf16 else torch.float32
+    seqs = [linear_inputs(450 + b, layer, T, bf16) for b in range(2)]
+    first = {"q": 0, "k": layer.qd, "v": 2 * layer.qd}[where]
+    seqs[1][0][:3, first:first + 256] = np.inf
+
+    def run(n):
+        st = D.LinearState(dl, n)
+        pos = torch.zeros(n, dtype=torch.int32, device="cuda")
+        out = D.linear_attn_prefill(dl, st, pos, *[_t(np.stack([s[i] for s in seqs[:n]]), dt) for i in range(4)], T)
+        return out[0].float().cpu().numpy(), st.S[0].cpu().numpy()
+
+    alone, beside = run(1), run(2)
+    assert (alone[0] == beside[0]).all() and (alone[1] == beside[1]).all() and np.isfinite(alone[0]).all()
