@@ -14,7 +14,7 @@
 // owns 128 adjacent channels (one q or k head when the channel is a q/k channel, so the sums of squares of a head
 // are warp sums) and a run of 16 (bf16) or 8 (f32) tokens, which it walks with a sliding window of 4 rows.  The
 // first tile of a sequence takes its history from the conv ring instead.  Same arithmetic as k_conv4_silu_prefill's
-// tensor-core form: fused multiply-adds in tap order, hardware-exponential SiLU, v times its write gate, all rounded to tf32.
+// tensor-core form: fused multiply-adds in tap order, hardware-exponential SiLU, q and k rounded to tf32, v times its write gate in f32.
 #include <cuda.h>
 #include <cuda_bf16.h>
 
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(128, CT_CTAS) k_conv4_silu_prefill_tma(LinArgs
                 pairs(h[0], x0); pairs(h[1], x1); pairs(h[2], x2);
             }
             const bool qk = ch < 2 * qd;                  // warp-uniform: a warp covers 128 channels = one head
-            // v channels leave as beta v, what the chunk's products take, rounded to tf32: lane i has the write gate of token i
+            // v channels leave as beta v, what the scan takes: lane i has the write gate of token i
             float beta = 0.0f;
             if (!qk && lane < TPT && tfirst + lane < a.T)
                 beta = sigmoid_f(act_ld((const ACT *)a.b, ((size_t)b * a.T + tfirst + lane) * a.nv + (ch - 2 * qd) / 128));
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(128, CT_CTAS) k_conv4_silu_prefill_tma(LinArgs
                         float4 y;
                         unpack2(y2[0], &y.x, &y.y);
                         unpack2(y2[1], &y.z, &y.w);
-                        y.x = tf32_round(y.x); y.y = tf32_round(y.y); y.z = tf32_round(y.z); y.w = tf32_round(y.w);
+                        if (QK) { y.x = tf32_round(y.x); y.y = tf32_round(y.y); y.z = tf32_round(y.z); y.w = tf32_round(y.w); }
                         if (WHOLE || i8 + i < left) *reinterpret_cast<float4 *>(Yp) = y;
                         Yp += Cc;
                         if (QK) ss[i] = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
@@ -241,7 +241,7 @@ ornith_status launch_t(const LinArgs &x, int n_seq, float *Y, float *rq, float *
 
 }  // namespace
 
-// conv + SiLU of tokens t_begin .. t_end - 1 of every sequence into Y (q, k and beta v, rounded to tf32), inverse norms into rq / rk.
+// conv + SiLU of tokens t_begin .. t_end - 1 of every sequence into Y (q and k rounded to tf32, beta v), inverse norms into rq / rk.
 // *handled = false (and ORNITH_OK) when the shape cannot be addressed by a tensor copy: the caller takes the plain kernel.
 ornith_status launch_conv4_silu_prefill_tma(const LinArgs &x, int n_seq, int act_dtype, float *Y, float *rq, float *rk,
                                             int t_begin, int t_end, cudaStream_t s, bool *handled) {

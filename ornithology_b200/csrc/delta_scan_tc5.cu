@@ -10,23 +10,27 @@
 // inverse norms rk_i, rq_i, G_i the running sum of the log-decay inside the chunk, p_i = exp(G_i),
 // Gamma_ij = exp(G_i - G_j), w_j = Gamma_63,j:
 //   M = diag(beta) strictLower(Gamma o Khat Khat^T),  A = (I + M)^-1,  P = lower(Gamma o Qhat Khat^T)
-//   U = A (beta V) + A' (K S^T),  A' = -A diag(beta p rk)
+//   T = beta V - diag(beta p rk) (K S^T),  U = A T
 //   O = diag(p rq) (Q S^T) + P U
 //   S <- p_63 S + sum_j (w_j rk_j u_j) k_j^T
 // (Khat, Qhat the normalised rows; the norms are folded into the per-token factors so that the
-// tensor cores read the K / Q tiles straight from the conv output; its v channels are stored as beta V.)  A, A', P and
+// tensor cores read the K / Q tiles straight from the conv output; its v channels are stored as beta V, in f32.)  A, P and
 // the per-token factors do not depend on the state: k_delta_prep produces them for all chunks at once.
 //
 // k_delta_scan_tc5, one CTA per (value head, sequence), keeps everything transposed, dv on the
 // 128 tensor-memory lanes:
 //   (K S^T)^T = S K^T             M128 N64  K128   A operand = the state itself (tensor memory)
 //   (Q S^T)^T = S Q^T             M128 N64  K128   the same
-//   U^T  = (beta V)^T A^T + (K S^T)^T A'^T   M128 N64 K64 twice   A operands = the beta V tile (shared memory, MN-major) and
-//                                                the accumulator K S^T as it is
+//   U^T  = T^T A^T                M128 N64  K64    A operand = T^T, formed in f32 and rounded once
 //   S'  = p_63 S + (w rk U)^T K   M128 N128 K64    A operand = (w rk U)^T; B = the K tile, MN-major
 //   (PU)^T = U^T P^T              M128 N64  K64    A operand = U^T
 // so the fp32 state never leaves tensor memory during a prompt: it is the accumulator of the
 // update and, read as tf32 (low mantissa bits ignored), the A operand of the next chunk.
+//
+// T is a difference, small where the state already holds what is written (keys that come again, slow decay), and its error
+// enters the state: it is formed in f32 from f32 terms, rounded to nearest, and meets one rounded A.  As
+// U = A (beta V) + A' (K S^T), A' = -A diag(beta p rk), with both matrices and both terms rounded on their own, a token repeated
+// 1000 times left the state 3.5e-3 off (largest error over largest value; so 3.1e-4), where independent rows show nothing of it.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -44,15 +48,13 @@ constexpr int C = 64;                                   // tokens per chunk
 constexpr float LOG2E_F = 1.4426950408889634f;
 // What the preparation leaves for one (value head, chunk), in the layouts the scan's copies need: every part is one
 // contiguous bulk copy.
-//   A, A', P   lower triangular: columns 0..31 of 64 rows, then columns 32..63 of rows 32..63; rows of 128 bytes, 128-byte swizzle
+//   A, P    lower triangular: columns 0..31 of 64 rows, then columns 32..63 of rows 32..63; rows of 128 bytes, 128-byte swizzle
 //           (a K-major B operand)
-//   factors    w rk (64), p rq (64), p_63
-constexpr int REC_A = 0, REC_AK = 12288, REC_P = 24576, REC_F = 36864, REC_BYTES = 37632;
-constexpr uint32_t TRI_BYTES = 12288, FAC_BYTES = 2 * C * 4 + 16;
-// The tensor core drops the 13 low mantissa bits of the state and of K S^T when it reads them, which takes 2^-11 / (2 ln 2) =
-// 3.52e-4 off a value on average (mantissas spread evenly over their logarithm).  A' and p rq scale that back.
-constexpr float S_DROP = 1.0f + 3.52e-4f;
-static_assert(REC_F + (int)FAC_BYTES <= REC_BYTES && REC_BYTES % 256 == 0, "record layout");
+//   factors    w rk (64), p rq (64), p_63 and 3 more, -beta p rk (64)
+constexpr int REC_A = 0, REC_P = 12288, REC_F = 24576, REC_BYTES = 25600;
+constexpr uint32_t TRI_BYTES = 12288, FAC_BYTES = (3 * C + 4) * 4;
+constexpr int F_W = 0, F_PQ = C, F_PEND = 2 * C, F_BPK = 2 * C + 4;
+static_assert(REC_F + (int)FAC_BYTES <= REC_BYTES && REC_BYTES % 256 == 0 && FAC_BYTES % 16 == 0, "record layout");
 // float index of element (i, l) of such a triangle
 __device__ __forceinline__ int tri_at(int i, int l) { return (l & 32) * 64 + (i - (l & 32)) * 32 + (((((l & 31) >> 2) ^ (i & 7)) << 2) | (l & 3)); }
 
@@ -214,7 +216,6 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
     }
     // gates of the heads m0 .. m0 + 3: thread (head, token); running sums of the log-decay over the chunk
     const int gh = tid >> 6, pt = tid & 63;
-    float bpk = 0.0f;                                     // -beta p rk of the thread's (head, token)
     auto gates = [&](int m0) {
         float gg = 0.0f, bb = 0.0f;
         if (m0 + gh < nvk && pt < n) {
@@ -242,10 +243,10 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
         if (m0 + gh < nvk) {
             float *f = reinterpret_cast<float *>(p.rec + (((size_t)b * a.nv + head_of(m0 + gh)) * p.rec_chunks + blockIdx.x) * REC_BYTES + REC_F);
             const float gend = sm.gend[gh], pp = expf(gg);
-            f[pt] = expf(gend - gg) * sm.rk[pt];
-            f[C + pt] = pp * sm.rq[pt] * S_DROP;
-            if (pt < 4) f[2 * C + pt] = expf(gend);
-            bpk = -bb * pp * sm.rk[pt] * (S_DROP * S_DROP);
+            f[F_W + pt] = expf(gend - gg) * sm.rk[pt];
+            f[F_PQ + pt] = pp * sm.rq[pt];
+            if (pt < 4) f[F_PEND + pt] = expf(gend);
+            f[F_BPK + pt] = -bb * pp * sm.rk[pt];
         }
     };
     gates(0);
@@ -367,23 +368,20 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
             }
         }
         __syncthreads();
-        sm.be[gh][pt] = bpk;                              // (beta has been read for the last time)
         if ((w >> 1) < heads) invert_diagonal(sm.u.M[w >> 1], w & 1, lane);
         __syncthreads();
 #pragma unroll 1
         for (int h = w >> 2; h < heads; h += 2) {         // two teams of four warps
             float *M = sm.u.M[h];
             invert_below(M, w & 3, lane, 1 + (w >> 2));
-            // A and -A diag(beta p rk), rounded to tf32: columns 0..31 of the rows 16 x .., then columns 32..63 of rows 32 + 16 (x - 4) ..
+            // A, rounded to tf32: columns 0..31 of the rows 16 x .., then columns 32..63 of rows 32 + 16 (x - 4) ..
             const int t = tid & 127, pc = t & 7, r = t >> 3;
             const float *ms = M + r * 64 + ((pc ^ swz(r & 7)) << 2);
             float *Ag = reinterpret_cast<float *>(rec_of(h) + REC_A) + r * 32 + ((pc ^ (r & 7)) << 2);
-            const float4 s0 = *reinterpret_cast<const float4 *>(&sm.be[h][4 * pc]), s1 = *reinterpret_cast<const float4 *>(&sm.be[h][32 + 4 * pc]);
 #pragma unroll
             for (int x = 0; x < 6; x++) {
-                const float4 v = *reinterpret_cast<const float4 *>(ms + (x < 4 ? x * 1024 : (x - 2) * 1024 + 32)), s = x < 4 ? s0 : s1;
+                const float4 v = *reinterpret_cast<const float4 *>(ms + (x < 4 ? x * 1024 : (x - 2) * 1024 + 32));
                 *reinterpret_cast<float4 *>(Ag + x * 512) = make_float4(tf32q(v.x), tf32q(v.y), tf32q(v.z), tf32q(v.w));
-                *reinterpret_cast<float4 *>(Ag + x * 512 + (REC_AK - REC_A) / 4) = make_float4(tf32q(v.x * s.x), tf32q(v.y * s.y), tf32q(v.z * s.z), tf32q(v.w * s.w));
             }
         }
     }
@@ -392,25 +390,25 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
 // =============================================================================
 // sequential part: one CTA per (value head, sequence)
 // =============================================================================
-//   warps 0-7   chain: the decayed copy of the state, then U as the operands of the two products behind it; two threads per lane (row
-//               of S)
+//   warps 0-7   chain: T from K S^T and beta V, the decayed copy of the state, then U as the operands of the two products behind it;
+//               two threads per lane (row of S)
 //   warps 8-23  output, off the chain: O, per-token RMSNorm over the head, SiLU(z) gate, store
 //   warp 24     one lane issues the copies of the chunk's operands: one buffer each, refilled as soon as the product that reads it is
-//               complete, which is most of a chunk before its next use.  K and beta V rows that serve as MN-major operands come in
-//               32-byte swizzle atoms (a K-major tf32 operand must lie in 16-byte atoms, so K is copied twice)
+//               complete, which is most of a chunk before its next use.  K rows that serve as an MN-major operand come in 32-byte swizzle
+//               atoms (a K-major tf32 operand must lie in 16-byte atoms, so K is copied twice)
 //   warp 25     one lane issues the tcgen05.mma of the chain and Q S^T
 //   warp 26     one lane issues those of P U: behind the state update in one stream they kept the issuing lane from the next chunk
 //   warp 27     one lane issues the copies of z and of the outputs, and asks L2 for what comes two chunks later (without such
 //               copies warp 24 asks: a lane that nothing waits for must not follow the scan by the parity of a barrier, which may
 //               go round unseen)
 // Tensor memory, 512 columns: two states of 128 (chunk n reads number n & 1; the other takes the decayed copy and then the
-// update), K S^T / w rk U, the accumulator and then operand U, Q S^T, P U.
-// A product that reads what an earlier product of another shape accumulated (the state, K S^T) is only issued after a wait on that
+// update), K S^T / T / w rk U, the accumulator and then operand U, Q S^T, P U.
+// A product that reads what an earlier product of another shape accumulated (the state) is only issued after a wait on that
 // one's commit: the pipe does not order them, and issued back to back the read came too early.
-// What bounds it: the chain of a chunk, K S^T (530 cycles), its commit, A' K S^T (260), its commit, the pass over U (about 600), the
-// update (530), its commit; Q S^T, beta V's product and P U run beside those waits, and the copies, one period ahead, take up to 1.7 us
-// when the passes in front of the next slab share the memory.  4.0k to 4.3k cycles a chunk (64 chunks x 64 heads alone 220 -> 145 us; with
-// T = beta V - (beta p rk) K S^T made by the chain warps between the first two products 5.5k, with z loaded by the output warps 6.2k).
+// What bounds it: the chain of a chunk, K S^T (530 cycles), its commit, the pass over T (about 500: beta V is in registers by then),
+// A T (260), its commit, the pass over U (about 600), the update (530), its commit; Q S^T and P U run beside those waits, and the copies, one
+// period ahead, take up to 1.7 us when the passes in front of the next slab share the memory.  4.9k cycles a chunk (64 chunks x 64 heads
+// alone 220 -> 168 us; with beta V read from shared memory behind K S^T 5.5k, with z loaded by the output warps 6.2k).
 // The output warps have as long for a chunk.  So they read their tiles as 16 x 256-bit fragments, a thread holding 4 rows of 4 tokens
 // (the sum of squares over the head is three shuffle levels on 4 values; as one row of 16 tokens it was five levels on 16),
 // arithmetic goes in pairs, and z and bf16 outputs pass through shared memory by tensor copies, read and written as transposed
@@ -420,19 +418,19 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
 constexpr int W_TMA = 24, W_MMA = 25, W_PU = 26, W_IO = 27, NTHREADS = 28 * 32;
 constexpr int TM_S = 0, TM_X = 256, TM_U = 320, TM_QS = 384, TM_PU = 448, TM_COLS = 512;   // tensor-memory columns
 constexpr int NFAC = 4;
-constexpr int SM_K = 0, SM_V = 32768, SM_Q = 65536, SM_KM = 98304;
-// the two A tiles whole (64 x 64): their upper right quarter is zeroed once and never written again
-constexpr int SM_AV = 131072, SM_AK = SM_AV + 16384, SM_P = SM_AK + 16384;
+constexpr int SM_K = 0, SM_V = 32768, SM_Q = 65536, SM_KM = 98304;   // (beta V: 64 rows of 128, not swizzled)
+// the A tile whole (64 x 64): its upper right quarter is zeroed once and never written again
+constexpr int SM_A = 131072, SM_P = SM_A + 16384;
 constexpr int SM_F = SM_P + (int)TRI_BYTES;             // NFAC x factors
 constexpr int SM_Z = (SM_F + NFAC * (int)FAC_BYTES + 1023) / 1024 * 1024;   // z of a chunk: 64 x 128 activations (bf16 or f32)
 constexpr int SM_O = SM_Z + 16384;                      // bf16 outputs of a chunk on their way out (f32 ones are stored by the threads)
 constexpr int SCAN_SMEM = SM_Z + 32768 + 1024;          // + alignment slack
 static_assert(SCAN_SMEM + 4096 <= 227 * 1024, "with the static part: the shared memory of an SM");
 
-enum { B_K, B_V, B_AK, B_Q, B_KM, B_P, NBUF };          // operand buffers (B_V: beta V and A)
+enum { B_K, B_V, B_A, B_Q, B_KM, B_P, NBUF };           // operand buffers
 struct ScanBars {
     unsigned long long full[NBUF], empty[NBUF], full_f[NFAC], red[2][4], o_full[4], o_free[4];
-    unsigned long long ks_done, u_done, wu_ready, u_ready, s_done, pu_done, qs_done, o_read, full_z, empty_z;
+    unsigned long long ks_done, t_ready, u_done, wu_ready, u_ready, s_done, pu_done, qs_done, o_read, full_z, empty_z;
 };
 
 struct ScanArgs {
@@ -496,6 +494,7 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t 
 template <typename ACT, bool SEG, bool TILE>
 __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_constant__ CUtensorMap map_y,
                                                                const __grid_constant__ CUtensorMap map_ym,
+                                                               const __grid_constant__ CUtensorMap map_v,
                                                                const __grid_constant__ CUtensorMap map_z,
                                                                const __grid_constant__ CUtensorMap map_o, ScanArgs a) {
     extern __shared__ unsigned char smraw[];
@@ -516,20 +515,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     unsigned char *gbase = smraw + (base - su32(smraw));
 
     if (tid == 0) {
-        for (int s = 0; s < NBUF; s++) { mbar_init(su32(&bars.full[s]), 1); mbar_init(su32(&bars.empty[s]), 1); }
+        for (int s = 0; s < NBUF; s++) { mbar_init(su32(&bars.full[s]), 1); mbar_init(su32(&bars.empty[s]), s == B_V ? 8 : 1); }
         for (int s = 0; s < NFAC; s++) mbar_init(su32(&bars.full_f[s]), 1);
         for (int s = 0; s < 2; s++)
             for (int g = 0; g < 4; g++) mbar_init(su32(&bars.red[s][g]), 4);
         for (int g = 0; g < 4; g++) { mbar_init(su32(&bars.o_full[g]), 4); mbar_init(su32(&bars.o_free[g]), 1); }
-        mbar_init(su32(&bars.ks_done), 1); mbar_init(su32(&bars.u_done), 1);
+        mbar_init(su32(&bars.ks_done), 1); mbar_init(su32(&bars.t_ready), 8); mbar_init(su32(&bars.u_done), 1);
         mbar_init(su32(&bars.wu_ready), 8); mbar_init(su32(&bars.u_ready), 8); mbar_init(su32(&bars.s_done), 1);
         mbar_init(su32(&bars.pu_done), 1); mbar_init(su32(&bars.qs_done), 1); mbar_init(su32(&bars.o_read), 16);
         mbar_init(su32(&bars.full_z), 1); mbar_init(su32(&bars.empty_z), 16);
         mbar_init_fence();
     }
     if (warp == W_MMA) tmem_alloc(&tmem_slot, TM_COLS);
-    for (int e = tid; e < 512; e += NTHREADS)             // rows 0..31, columns 32..63 of both A tiles
-        *reinterpret_cast<float4 *>(gbase + (e < 256 ? SM_AV : SM_AK) + 8192 + (e & 255) * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (tid < 256)                                        // rows 0..31, columns 32..63 of A
+        *reinterpret_cast<float4 *>(gbase + SM_A + 8192 + tid * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
     fence_async();
     fence_before();
     __syncthreads();
@@ -572,7 +571,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     auto ahead = [&](int n) {                                     // (K and Q rows are shared by the value heads of a key head)
         if (n >= N) return;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(rec0 + (size_t)n * REC_BYTES), "r"((uint32_t)REC_BYTES) : "memory");
-        for (int sl = 0; sl < 4; sl++) l2_rows(&map_ym, 2 * qd + hv * 128 + 32 * sl, (c0 + n) * C);
+        l2_rows(&map_v, 2 * qd + hv * 128, (c0 + n) * C);
         if (tiles)
             for (int t = 0; t < TZ; t++) l2_rows(&map_z, hv * 128 + t * CZ, (c0 + n) * C);
     };
@@ -600,13 +599,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 // (the readers of the factors of chunk n - 4 are done: K S^T of chunk n - 1 was behind them)
                 mbar_expect_tx(su32(&bars.full_f[n % NFAC]), FAC_BYTES);
                 bulk_load(base + SM_F + n % NFAC * FAC_BYTES, r + REC_F, FAC_BYTES, su32(&bars.full_f[n % NFAC]));
-                if (!refill(B_V, 32768u + TRI_BYTES)) break;
-                rows(SM_V, &map_ym, 2 * qd + hv * 128, B_V);
-                part(SM_AV, REC_A, 8192u, B_V);
-                part(SM_AV + 8192 + 4096, REC_A + 8192, 4096u, B_V);
-                if (!refill(B_AK, TRI_BYTES)) break;
-                part(SM_AK, REC_AK, 8192u, B_AK);
-                part(SM_AK + 8192 + 4096, REC_AK + 8192, 4096u, B_AK);
+                if (!refill(B_V, 32768u)) break;
+                tma_load_3d(base + SM_V, &map_v, 2 * qd + hv * 128, t0, b, su32(&bars.full[B_V]));
+                if (!refill(B_A, TRI_BYTES)) break;
+                part(SM_A, REC_A, 8192u, B_A);
+                part(SM_A + 8192 + 4096, REC_A + 8192, 4096u, B_A);
                 if (!refill(B_Q, 32768u)) break;
                 rows(SM_Q, &map_y, kh * 128, B_Q);
                 if (!refill(B_KM, 32768u)) break;
@@ -618,7 +615,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
     } else if (warp == W_MMA) {
         // ================= every tcgen05.mma =================
         if (elect_one()) {
-            constexpr uint32_t ID_64 = idesc(2, 64, false), ID_SU = idesc(2, 128, true), ID_V = ID_64 | (1u << 15);
+            constexpr uint32_t ID_64 = idesc(2, 64, false), ID_SU = idesc(2, 128, true);
             auto full = [&](int s, int n) { return mbar_wait(su32(&bars.full[s]), (uint32_t)n & 1u); };
             auto empty = [&](int s) { mma_commit(su32(&bars.empty[s])); };
             auto times_state = [&](uint32_t d, uint32_t S, uint32_t tile) {       // D[dv][token] = sum_dk S[dv][dk] tile[token][dk]
@@ -628,32 +625,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             // what a product needs beside the result it follows is waited for ahead of that result
             for (int n = 0; n < N; n++) {
                 const uint32_t S = tmem + TM_S + 128 * (n & 1), S2 = tmem + TM_S + 128 * ((n & 1) ^ 1);
-                ok = full(B_K, n) && full(B_V, n) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u));
+                ok = full(B_K, n) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u));
                 if (!ok) break;
                 fence_after();
                 times_state(tmem + TM_X, S, base + SM_K);                         // (K S^T)^T
                 mma_commit(su32(&bars.ks_done));
                 empty(B_K);
-                // U^T = (beta V)^T A^T + (K S^T)^T A'^T; U of the chunk before is an operand no more
-                ok = n == 0 || mbar_wait(su32(&bars.pu_done), (uint32_t)(n - 1) & 1u);
-                if (!ok) break;
-                const bool with_v = !(SEG && kind == 2);
-                if (with_v) {
-#pragma unroll
-                    for (int ks = 0; ks < 8; ks++)
-                        mma_tf32_ss(tmem + TM_U, smem_desc_mn32(base + SM_V + ks * 1024, 8192, 512),
-                                    smem_desc(base + SM_AV + (ks >> 2) * 8192 + (ks & 3) * 32, 16, 1024), ID_V, ks > 0);
-                }
-                empty(B_V);
-                ok = full(B_AK, n) && mbar_wait(su32(&bars.ks_done), (uint32_t)n & 1u);
+                // U^T = T^T A^T; U of the chunk before is an operand no more
+                ok = full(B_A, n) && (n == 0 || mbar_wait(su32(&bars.pu_done), (uint32_t)(n - 1) & 1u)) && mbar_wait(su32(&bars.t_ready), (uint32_t)n & 1u);
                 if (!ok) break;
                 fence_after();
 #pragma unroll
                 for (int ks = 0; ks < 8; ks++)
-                    mma_tf32_ts(tmem + TM_U, tmem + TM_X + 8 * ks, smem_desc(base + SM_AK + (ks >> 2) * 8192 + (ks & 3) * 32, 16, 1024), ID_64,
-                                ks > 0 || with_v);
+                    mma_tf32_ts(tmem + TM_U, tmem + TM_X + 8 * ks, smem_desc(base + SM_A + (ks >> 2) * 8192 + (ks & 3) * 32, 16, 1024), ID_64, ks > 0);
                 mma_commit(su32(&bars.u_done));
-                empty(B_AK);
+                empty(B_A);
                 // the tiles Q S^T and P U of the chunk before have been read
                 ok = full(B_Q, n) && (n == 0 || mbar_wait(su32(&bars.o_read), (uint32_t)(n - 1) & 1u));
                 if (!ok) break;
@@ -692,38 +678,60 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             }
         }
     } else if (warp < 8) {
-        // ================= chain: the decayed state, U =================
+        // ================= chain: T, the decayed state, U =================
         const uint32_t X = lane_t + TM_X + 32 * half, U = lane_t + TM_U + 32 * half;
+        const float *bv = reinterpret_cast<const float *>(gbase + SM_V) + 32 * half * 128 + row;     // beta V of token 32 half + i: bv[128 i]
         for (int n = 0; n < N; n++) {
             const float *fac = reinterpret_cast<const float *>(gbase + SM_F + (n % NFAC) * FAC_BYTES);
             const uint32_t S = lane_t + TM_S + 128 * (n & 1) + 64 * half, S2 = lane_t + TM_S + 128 * ((n & 1) ^ 1) + 64 * half;
             ok = mbar_wait(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u));
             if (!ok) break;
             fence_after();
-            float x[32];
-            {   // the other state = p_63 S, while the tensor core reads S (the update is accumulated onto it)
-                const float pend = fac[2 * C];
+            float x[32], v[32];
+            // the other state = p_63 S, while the tensor core reads S (the update is accumulated onto it): a half beside K S^T, a half
+            // beside A T
+            const float pend = fac[F_PEND];
+            auto decay = [&](int cc) {
                 const f32x2 p2 = pack2(pend, pend);
-#pragma unroll 1
-                for (int cc = 0; cc < 2; cc++) {
-                    tmem_ld32_wait(S + 32 * cc, x);
+                tmem_ld32_wait(S + 32 * cc, x);
 #pragma unroll
-                    for (int i = 0; i < 32; i += 2) { const f32x2 y = mul2(p2, pack2(x[i], x[i + 1])); unpack2(y, &x[i], &x[i + 1]); }
-                    tmem_st32(S2 + 32 * cc, x);
-                }
+                for (int i = 0; i < 32; i += 2) { const f32x2 y = mul2(p2, pack2(x[i], x[i + 1])); unpack2(y, &x[i], &x[i + 1]); }
+                tmem_st32(S2 + 32 * cc, x);
+            };
+            decay(0);
+            ok = mbar_wait(su32(&bars.full[B_V]), (uint32_t)n & 1u);
+            if (!ok) break;
+#pragma unroll
+            for (int i = 0; i < 32; i++) v[i] = SEG && kind == 2 ? 0.0f : bv[128 * i];
+            ok = mbar_wait(su32(&bars.ks_done), (uint32_t)n & 1u);
+            if (!ok) break;
+            fence_after();
+            tmem_ld32_wait(X, x);                                        // (K S^T)^T
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {                            // T^T over it
+                const float4 b4 = *reinterpret_cast<const float4 *>(fac + F_BPK + 32 * half + i);    // -beta p rk
+                unpack2(fma2(pack2(b4.x, b4.y), pack2(x[i], x[i + 1]), pack2(v[i], v[i + 1])), &x[i], &x[i + 1]);
+                unpack2(fma2(pack2(b4.z, b4.w), pack2(x[i + 2], x[i + 3]), pack2(v[i + 2], v[i + 3])), &x[i + 2], &x[i + 3]);
             }
+#pragma unroll
+            for (int i = 0; i < 32; i++) x[i] = tf32q(x[i]);
+            tmem_st32(X, x);
+            tmem_wait_st();
+            fence_before();
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(su32(&bars.t_ready)); mbar_arrive(su32(&bars.empty[B_V])); }
+            decay(1);
             ok = mbar_wait(su32(&bars.u_done), (uint32_t)n & 1u);
             if (!ok) break;
             fence_after();
             tmem_ld32_wait(U, x);                                        // U^T
-            fac += 32 * half;
-            // (w rk U)^T over (K S^T)^T first: the state update waits for it
+            // (w rk U)^T over T^T first: the state update waits for it
 #pragma unroll
             for (int hh = 0; hh < 4; hh++) {                             // 8 tokens at a time
                 float f[8];
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
-                    const float4 w4 = *reinterpret_cast<const float4 *>(fac + 8 * hh + 4 * i);   // w rk
+                    const float4 w4 = *reinterpret_cast<const float4 *>(fac + F_W + 32 * half + 8 * hh + 4 * i);   // w rk
                     const float *t = x + 8 * hh + 4 * i;
                     const f32x2 t0 = mul2(pack2(w4.x, w4.y), pack2(t[0], t[1])), t1 = mul2(pack2(w4.z, w4.w), pack2(t[2], t[3]));
                     unpack2(t0, f + 4 * i, f + 4 * i + 1);
@@ -822,12 +830,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             fence_after();
             float x[16];                                                 // O = p rq QS + P U
             {
-                const float *pq = reinterpret_cast<const float *>(gbase + SM_F + (n % NFAC) * FAC_BYTES) + C + 16 * grp + 2 * j;
+                const float *pq = reinterpret_cast<const float *>(gbase + SM_F + (n % NFAC) * FAC_BYTES) + F_PQ + 16 * grp + 2 * j;
                 float q[16];
                 tmem_ld_16x256_wait(t_qs, q, t_pu, x);
                 const float2 pa = *reinterpret_cast<const float2 *>(pq), pb = *reinterpret_cast<const float2 *>(pq + 8);
-                const float back = SEG && kind == 2 && n == 0 ? 1.0f / S_DROP : 1.0f;        // (the identity loses nothing when read)
-                const f32x2 p2[2] = {pack2(pa.x * back, pa.y * back), pack2(pb.x * back, pb.y * back)};
+                const f32x2 p2[2] = {pack2(pa.x, pa.y), pack2(pb.x, pb.y)};
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) unpack2(fma2(p2[i >> 3], pack2(q[i], q[i + 1]), pack2(x[i], x[i + 1])), &x[i], &x[i + 1]);
             }
@@ -1094,8 +1101,8 @@ __global__ void __launch_bounds__(128, 2) k_delta_seg_finish(ScanArgs a) {
 
 // How many runs the prompt is cut into: only when the heads alone would leave most SMs idle (2 P - 1 CTAs per head), with at least 16
 // chunks per run, and not into two: every run but the first is scanned twice and finished by two more kernels.  us, one run | the
-// best cut: 32 heads x 4096 tokens 219 | 245, 8192 402 | 427; 16 heads x 1024 tokens 60 | 97, 4096 187 | 190, 8192 350 | 296;
-// 8 heads x 2048 92 | 110, 4096 166 | 146, 32768 1206 | 527.  ORNITH_CUDA_DELTA_SEGMENTS=<n> forces a count (1 = off).
+// best cut: 32 heads x 4096 tokens 239 | 272, 8192 458 | 491; 16 heads x 1024 tokens 66 | 105, 4096 221 | 215, 8192 420 | 354;
+// 8 heads x 2048 101 | 117, 4096 192 | 166, 32768 1397 | 653.  ORNITH_CUDA_DELTA_SEGMENTS=<n> forces a count (1 = off).
 int delta_seg_plan(int nv, int n_seq, int n_chunks, int *seg_chunks) {
     int p = 1;
     const char *e = getenv("ORNITH_CUDA_DELTA_SEGMENTS");
@@ -1116,17 +1123,17 @@ int delta_seg_plan(int nv, int n_seq, int n_chunks, int *seg_chunks) {
     return p;
 }
 
-// [n_seq][T][width] values: boxes of 128 bytes of channels x `rows` tokens of one sequence, 128-byte swizzle.  The sequences are a
+// [n_seq][T][width] values: boxes of 128 bytes of channels (or `channels`) x `rows` tokens of one sequence, 128-byte swizzle.  The sequences are a
 // dimension of their own: rows of a box behind a sequence's last token arrive as zeros and not as the next one's first tokens, whose
 // infinities the products would spread over the chunk (0 x Inf).
 ornith_status rows_map(CUtensorMap *m, const void *basep, bool bf, uint64_t width, uint64_t T, uint64_t n_seq, uint32_t rows,
-                       CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
+                       CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B, uint32_t channels = 0) {
     OrnTensorMapEncodeFn enc = orn_tensor_map_encoder();
     if (!enc) { orn_record_error("delta scan: cuTensorMapEncodeTiled is not available"); return (ornith_status)ORNITH_ERR_BACKEND; }
     const uint64_t row = width * (bf ? 2 : 4);
     cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)T, (cuuint64_t)n_seq};
     cuuint64_t strides[2] = {(cuuint64_t)row, (cuuint64_t)(row * T)};
-    cuuint32_t box[3] = {bf ? 64u : 32u, rows, 1};
+    cuuint32_t box[3] = {channels ? channels : bf ? 64u : 32u, rows, 1};
     cuuint32_t es[3] = {1, 1, 1};
     const CUresult r = enc(m, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void *>(basep), dims, strides, box, es,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -1197,9 +1204,9 @@ ornith_status slab_pipe_ready(SlabPipe &p) {
 }  // namespace
 
 // Slabs of the prompt; 1 = no pipeline (ORNITH_CUDA_DELTA_SLABS overrides).  The scan of up to half as many heads as SMs leaves the
-// passes in front of it room; each slab costs a start of the scan.  us at 1 | 2 | 3 | 4 | 8 slabs: 64 heads x 4096 tokens 257 | 268 | 274 |
-// 278 | 315, 8192 490 | 465 | 473 | 495 | 515, 16384 948 | 885 | 903 | 920 | 986, 32768 1925 | 1750 | 1755 | 1725 | 1877; 32 heads x 8192
-// 414 | 402 | 405 | 427, 16384 801 | 747 | 731 | 714; 128 heads x 8192 790 | 824 | 934 | 961 | 1029.
+// passes in front of it room; each slab costs a start of the scan.  us at 1 | 2 | 3 | 4 | 8 slabs: 64 heads x 4096 tokens 281 | 275 | 286 |
+// 286 | 322, 8192 546 | 499 | 490 | 496 | 525, 16384 1062 | 944 | 908 | 898 | 932, 32768 2155 | 1848 | 1810 | 1772 | 1813; 32 heads x 8192
+// 493 | 462 | 457 | 488, 16384 885 | 809 | 796 | 810; 128 heads x 8192 749 | 737 | 794 | 833 | 956.
 static int slab_plan(int heads, int n_chunks, int n_seg) {
     if (n_seg > 1 || heads > 148) return 1;
     int n = heads <= 74 ? min(4, 1 + n_chunks / 128) : 1;
@@ -1223,7 +1230,7 @@ ornith_status release_delta_slab_pipe() {
     return orn_check(e, "delta scan stream destroy");
 }
 
-using ScanKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ScanArgs);
+using ScanKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, ScanArgs);
 static ScanKernel scan_kernel(bool bf, bool seg, bool tile) {
     static const ScanKernel k[8] = {k_delta_scan_tc5<float, false, false>, k_delta_scan_tc5<__nv_bfloat16, false, false>,
                                     k_delta_scan_tc5<float, true, false>,  k_delta_scan_tc5<__nv_bfloat16, true, false>,
@@ -1261,9 +1268,10 @@ ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dty
     const bool bf = act_dtype == ORNITH_ACT_BF16;
     // z and the outputs travel by tensor copies where their rows lie on 16-byte boundaries (the row length always is a multiple)
     const bool tile = ((uintptr_t)x.z % 16) == 0 && ((uintptr_t)x.out % 16) == 0;
-    CUtensorMap my, mym, mz, mo;
+    CUtensorMap my, mym, mv, mz, mo;
     ORN_TRY(rows_map(&my, Y, false, (uint64_t)Cc, (uint64_t)x.T, (uint64_t)n_seq, C));
     ORN_TRY(rows_map(&mym, Y, false, (uint64_t)Cc, (uint64_t)x.T, (uint64_t)n_seq, C, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B));
+    ORN_TRY(rows_map(&mv, Y, false, (uint64_t)Cc, (uint64_t)x.T, (uint64_t)n_seq, C, CU_TENSOR_MAP_SWIZZLE_NONE, 128));
     mz = mo = my;
     if (tile) {
         ORN_TRY(rows_map(&mz, x.z, bf, (uint64_t)x.nv * 128, (uint64_t)x.T, (uint64_t)n_seq, C));
@@ -1300,8 +1308,8 @@ ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dty
         sa.rec = rec + slot * slot_bytes; sa.c_begin = cb; sa.c_count = cn;
         dim3 grid((unsigned)x.nv, (unsigned)n_seq);
         if (chained)
-            return orn_check(orn_launch_dependent(scan_kernel(bf, false, tile), grid, dim3(NTHREADS), SCAN_SMEM, ss, my, mym, mz, mo, sa), "k_delta_scan_tc5");
-        scan_kernel(bf, false, tile)<<<grid, NTHREADS, SCAN_SMEM, ss>>>(my, mym, mz, mo, sa);
+            return orn_check(orn_launch_dependent(scan_kernel(bf, false, tile), grid, dim3(NTHREADS), SCAN_SMEM, ss, my, mym, mv, mz, mo, sa), "k_delta_scan_tc5");
+        scan_kernel(bf, false, tile)<<<grid, NTHREADS, SCAN_SMEM, ss>>>(my, mym, mv, mz, mo, sa);
         return orn_check_launch("k_delta_scan_tc5");
     };
 
@@ -1343,7 +1351,7 @@ ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dty
     // few heads: the runs of the prompt side by side, then the carry over the runs and the finishing pass
     ORN_TRY(prep(0, p.n_chunks, 0, front != nullptr));
     dim3 grid((unsigned)x.nv, (unsigned)n_seq, (unsigned)(2 * a.n_seg - 1));
-    scan_kernel(bf, true, tile)<<<grid, NTHREADS, SCAN_SMEM, s>>>(my, mym, mz, mo, a);
+    scan_kernel(bf, true, tile)<<<grid, NTHREADS, SCAN_SMEM, s>>>(my, mym, mv, mz, mo, a);
     ORN_TRY(orn_check_launch("k_delta_scan_tc5 (runs)"));
     k_delta_seg_carry<<<dim3((unsigned)x.nv, (unsigned)n_seq, 16), 128, 0, s>>>(a);
     ORN_TRY(orn_check_launch("k_delta_seg_carry"));

@@ -421,9 +421,9 @@ __global__ void __launch_bounds__(128) k_conv4_silu_prefill(LinArgs a, float *Y,
 #undef ORN_CONV4
         if (FAST && ch < 2 * qd) {                        // q and k feed tf32 tensor-core products: round once, here
             y.x = tf32_rna(y.x); y.y = tf32_rna(y.y); y.z = tf32_rna(y.z); y.w = tf32_rna(y.w);
-        } else if (NORMS) {                               // the tcgen05 scan's v channels: beta v, rounded to tf32
+        } else if (NORMS) {                               // the tcgen05 scan's v channels: beta v
             const float bt = sigmoid_f(act_ld((const ACT *)a.b, ((size_t)b * a.T + t0 + i) * a.nv + (ch - 2 * qd) / 128));
-            y.x = tf32_rna(bt * y.x); y.y = tf32_rna(bt * y.y); y.z = tf32_rna(bt * y.z); y.w = tf32_rna(bt * y.w);
+            y.x *= bt; y.y *= bt; y.z *= bt; y.w *= bt;
         }
         *reinterpret_cast<float4 *>(Y + ((size_t)b * a.T + t0 + i) * Cc + ch) = y;
         if (NORMS) ss[i] = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);
@@ -465,14 +465,17 @@ __global__ void k_conv_ring_refresh(LinArgs a) {
         ring[(size_t)((pos0 + t) % K) * Cc + ch] = act_ld(X, (size_t)t * Cc + ch);
 }
 
-// what the tcgen05 scan expects of a Y that another conv wrote: v times its write gate, q, k and that rounded to tf32
+// what the tcgen05 scan expects of a Y that another conv wrote: q and k rounded to tf32, v times its write gate
 __global__ void __launch_bounds__(256) k_scan_inputs(LinArgs a, float *Y, const float *be, size_t n4) {
     const int qd = a.nk * a.dk, Cc = 2 * qd + a.nv * a.dv;
     for (size_t e = blockIdx.x * 256ull + threadIdx.x; e < n4; e += gridDim.x * 256ull) {
         const int ch = (int)(e * 4 % Cc);
-        const float s = ch < 2 * qd ? 1.0f : be[e * 4 / Cc * a.nv + (ch - 2 * qd) / a.dv];
         float4 y = reinterpret_cast<float4 *>(Y)[e];
-        y.x = tf32_rna(s * y.x); y.y = tf32_rna(s * y.y); y.z = tf32_rna(s * y.z); y.w = tf32_rna(s * y.w);
+        if (ch < 2 * qd) { y.x = tf32_rna(y.x); y.y = tf32_rna(y.y); y.z = tf32_rna(y.z); y.w = tf32_rna(y.w); }
+        else {
+            const float s = be[e * 4 / Cc * a.nv + (ch - 2 * qd) / a.dv];
+            y.x *= s; y.y *= s; y.z *= s; y.w *= s;
+        }
         reinterpret_cast<float4 *>(Y)[e] = y;
     }
 }

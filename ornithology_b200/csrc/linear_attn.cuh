@@ -34,8 +34,8 @@ ornith_status launch_linear_prefill_tc(const LinArgs &x, int n_seq, int act_dtyp
                                        cudaStream_t s);
 
 // The same scan on the 5th-generation tensor cores (delta_scan_tc5.cu): tcgen05.mma in tf32 with the
-// state in tensor memory, operands staged by TMA, 64-token chunks.  Y must hold q, k and beta v (v times its write
-// gate), rounded to tf32 (the convs of this path do that, k_scan_inputs after another); work = linear_prefill_tc5_work_bytes() bytes;
+// state in tensor memory, operands staged by TMA, 64-token chunks.  Y must hold q and k rounded to tf32 and
+// beta v (v times its write gate; the convs of this path do that, k_scan_inputs after another); work = linear_prefill_tc5_work_bytes() bytes;
 // la = be = nullptr: the gates are computed from the layer's a / b inputs.
 //
 // With a front (the causal conv of a token range, as a launch the caller provides) the chunk preparation that ends the

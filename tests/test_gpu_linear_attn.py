@@ -448,3 +448,54 @@ def test_sequences_of_a_batch_stay_apart(bf16, where):
 
     alone, beside = run(1), run(2)
     assert (alone[0] == beside[0]).all() and (alone[1] == beside[1]).all() and np.isfinite(alone[0]).all()
+
+
+def _delta_rule_64(kw, nk, nv, S, before, qkv, a, b, z):
+    """The layer's definition in 64 bits: conv over `before` (3 rows) and qkv, then the recurrence, norm and gate."""
+    T, sig = len(qkv), lambda x: 1.0 / (1.0 + np.exp(-x))
+    x = np.concatenate([before, qkv]).astype(np.float64)
+    y = sum(x[j:j + T] * kw["conv_w"][:, j].astype(np.float64) for j in range(4))
+    y = (y * sig(y)).reshape(T, 2 * nk + nv, 128)
+    unit = lambda r: r / np.sqrt((r * r).sum(-1, keepdims=True) + 1e-6)
+    q, k, v = unit(y[:, np.arange(nv) % nk]), unit(y[:, nk + np.arange(nv) % nk]), y[:, 2 * nk:]
+    alpha = np.exp(kw["a_coef"].astype(np.float64) * np.log1p(np.exp(a.astype(np.float64) + kw["dt_bias"])))
+    beta, o = sig(b.astype(np.float64)), np.empty((T, nv, 128))
+    for t in range(T):
+        S = S * alpha[t, :, None, None]
+        u = beta[t, :, None] * (v[t] - (S @ k[t, :, :, None])[..., 0])
+        S = S + u[..., None] * k[t, :, None]
+        o[t] = (S @ q[t, :, :, None])[..., 0]
+    o *= 128 ** -0.5
+    o *= kw["norm_w"].astype(np.float64) / np.sqrt((o * o).mean(-1, keepdims=True) + 1e-6)
+    z = z.astype(np.float64).reshape(T, nv, 128)
+    return (o * z * sig(z)).reshape(T, -1), S, x[-3:]
+
+
+@pytest.mark.parametrize("period", [1, 2, 8])
+@pytest.mark.parametrize("form,T", [("plain", 1000), ("slabs", 1000), ("3 runs", 3100), ("runs by the rule", 3100)])
+def test_repeated_rows_with_slow_decay(monkeypatch, form, T, period):
+    """Keys that come again while the state decays slowly: what is written is a small difference of large terms.  Two calls, the
+    second with the state of the first.  With the difference formed in f32 and rounded once the state is at most 5.3e-4 off
+    (the state's reading in tf32: its low bits dropped, 3.5e-4 on average) and the outputs behind the first chunk 1.3e-3; with its two terms
+    rounded apart the state was 1.2e-3 to 3.5e-3 off.  49 chunks and 4 heads: the rule takes 3 runs."""
+    import torch
+    from ornithology_b200 import device as D
+    env = {"plain": ("1", "1"), "slabs": ("1", "3"), "3 runs": ("3", "1"), "runs by the rule": ("", "")}[form]
+    monkeypatch.setenv("ORNITH_CUDA_DELTA_SEGMENTS", env[0])
+    monkeypatch.setenv("ORNITH_CUDA_DELTA_SLABS", env[1])
+    nk, nv = 2, 4
+    layer, kw = linear_case(46, nk=nk, nv=nv)
+    kw["a_coef"] = np.full(nv, -0.005, np.float32)
+    dl = device_linear(layer, kw)
+    g = np.random.default_rng(460)
+    qkv = g.standard_normal((period, layer.cc)).astype(np.float32)[np.arange(T) % period]
+    a, b, z = np.full((T, nv), -1.5, np.float32), np.full((T, nv), 2.2, np.float32), g.standard_normal((T, layer.vd)).astype(np.float32)
+    st = D.LinearState(dl, 1)
+    pos = torch.zeros(1, dtype=torch.int32, device="cuda")
+    S, before = np.zeros((nv, 128, 128)), np.zeros((3, layer.cc))
+    for call in range(2):
+        out = D.linear_attn_prefill(dl, st, pos, *[_t(x)[None] for x in (qkv, a, b, z)], T)
+        D.advance(pos, T)
+        ref, S, before = _delta_rule_64(kw, nk, nv, S, before, qkv, a, b, z)
+        assert rel_err(out.cpu().numpy()[0, 64:], ref[64:]) < 1.6e-3, call
+        assert rel_err(st.S.cpu().numpy()[0], S) < 8e-4, call
