@@ -33,7 +33,6 @@ __device__ __forceinline__ void tile_copy(uint32_t dst, const CUtensorMap *map, 
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(col), "r"(row) : "memory");
 }
-__device__ __forceinline__ float tf32_round(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
 
 __device__ __forceinline__ float4 ld_row4(const unsigned char *row, int ch_local, const __nv_bfloat16 *) {
     const uint2 u = *reinterpret_cast<const uint2 *>(row + ch_local * 2);
@@ -157,7 +156,7 @@ __global__ void __launch_bounds__(128, CT_CTAS) k_conv4_silu_prefill_tma(LinArgs
                         float4 y;
                         unpack2(y2[0], &y.x, &y.y);
                         unpack2(y2[1], &y.z, &y.w);
-                        if (QK) { y.x = tf32_round(y.x); y.y = tf32_round(y.y); y.z = tf32_round(y.z); y.w = tf32_round(y.w); }
+                        if (QK) { y.x = tf32r(y.x); y.y = tf32r(y.y); y.z = tf32r(y.z); y.w = tf32r(y.w); }
                         if (WHOLE || i8 + i < left) *reinterpret_cast<float4 *>(Yp) = y;
                         Yp += Cc;
                         if (QK) ss[i] = (y.x * y.x + y.y * y.y) + (y.z * y.z + y.w * y.w);

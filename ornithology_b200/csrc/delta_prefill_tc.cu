@@ -39,12 +39,6 @@ constexpr uint32_t BLK_BYTES = BLK_FLOATS * 4;
 constexpr int TILE_FLOATS = TC * LDK;                     // one chunk of normalised k (or q) rows, padded as in shared memory
 constexpr uint32_t TILE_BYTES = TILE_FLOATS * 4;
 
-__device__ __forceinline__ float tf32r(float x) {
-    uint32_t u;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(u) : "f"(x));
-    return __uint_as_float(u);
-}
-
 // D(16x8) += A(16x8) B(8x8).  Fragment owners, g = lane / 4, j = lane % 4:
 //   a0 (g, j) a1 (g+8, j) a2 (g, j+4) a3 (g+8, j+4);  b0 (k=j, n=g) b1 (k=j+4, n=g);
 //   d0 (g, 2j) d1 (g, 2j+1) d2 (g+8, 2j) d3 (g+8, 2j+1).
@@ -218,10 +212,6 @@ __device__ __forceinline__ void ldsm4(float (&r)[4], uint32_t addr) {
                  : "=r"(x0), "=r"(x1), "=r"(x2), "=r"(x3) : "r"(addr));
     r[0] = __uint_as_float(x0); r[1] = __uint_as_float(x1); r[2] = __uint_as_float(x2); r[3] = __uint_as_float(x3);
 }
-// Round to tf32 for an MMA operand in one integer add (finite inputs): the tensor core
-// ignores the 13 low mantissa bits, so adding half a tf32 ulp to the magnitude first
-// turns its truncation into round-to-nearest (ties away from zero).
-__device__ __forceinline__ float tf32q(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
 // store into another CTA of the cluster; the 4 bytes are credited to that CTA's mbarrier,
 // and are visible to whoever sees the phase complete
 __device__ __forceinline__ void st_async_f32(uint32_t addr, float v, uint32_t bar) {

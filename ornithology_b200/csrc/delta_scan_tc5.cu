@@ -58,13 +58,6 @@ static_assert(REC_F + (int)FAC_BYTES <= REC_BYTES && REC_BYTES % 256 == 0 && FAC
 // float index of element (i, l) of such a triangle
 __device__ __forceinline__ int tri_at(int i, int l) { return (l & 32) * 64 + (i - (l & 32)) * 32 + (((((l & 31) >> 2) ^ (i & 7)) << 2) | (l & 3)); }
 
-// Round to tf32 (nearest, ties away from zero; finite inputs) with integer arithmetic: cvt.rna.tf32.f32 runs at
-// the special-function rate, a sixteenth of this.  tf32r gives a clean tf32 value (low 13 mantissa bits zero) for
-// operands that are stored; tf32q only adds the half ulp, for operands that go straight to the tensor core, which
-// ignores the low bits.
-__device__ __forceinline__ float tf32r(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
-__device__ __forceinline__ float tf32q(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
-
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, int x, int y, int z, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
@@ -681,6 +674,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
         // ================= chain: T, the decayed state, U =================
         const uint32_t X = lane_t + TM_X + 32 * half, U = lane_t + TM_U + 32 * half;
         const float *bv = reinterpret_cast<const float *>(gbase + SM_V) + 32 * half * 128 + row;     // beta V of token 32 half + i: bv[128 i]
+        const float quiet_nan = __int_as_float(0x7fc00000);              // (as tf32, too)
         for (int n = 0; n < N; n++) {
             const float *fac = reinterpret_cast<const float *>(gbase + SM_F + (n % NFAC) * FAC_BYTES);
             const uint32_t S = lane_t + TM_S + 128 * (n & 1) + 64 * half, S2 = lane_t + TM_S + 128 * ((n & 1) ^ 1) + 64 * half;
@@ -703,6 +697,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             if (!ok) break;
 #pragma unroll
             for (int i = 0; i < 32; i++) v[i] = SEG && kind == 2 ? 0.0f : bv[128 * i];
+            // A beta v or a factor that is no finite number makes this row's U NaN.  The roundings below would hide it (-0 for NaN, see
+            // tf32q; a minimum for each of the 96 took 4 % of the prefill), so it is looked for here, beside K S^T, and written
+            // below.  What is no number in the state or in A shows in Q S^T or in P U anyway.
+            bool bad = __any_sync(0xffffffffu, 0.0f * fac[F_BPK + 32 * half + lane] != 0.0f);
+            {
+                f32x2 z = 0;
+                float z0, z1;
+#pragma unroll
+                for (int i = 0; i < 32; i += 2) z = fma2(pack2(v[i], v[i + 1]), 0, z);
+                unpack2(z, &z0, &z1);
+                bad = bad || z0 + z1 != 0.0f;
+            }
             ok = mbar_wait(su32(&bars.ks_done), (uint32_t)n & 1u);
             if (!ok) break;
             fence_after();
@@ -714,7 +720,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 unpack2(fma2(pack2(b4.z, b4.w), pack2(x[i + 2], x[i + 3]), pack2(v[i + 2], v[i + 3])), &x[i + 2], &x[i + 3]);
             }
 #pragma unroll
-            for (int i = 0; i < 32; i++) x[i] = tf32q(x[i]);
+            for (int i = 0; i < 32; i++) x[i] = tf32q_finite(x[i]);
             tmem_st32(X, x);
             tmem_wait_st();
             fence_before();
@@ -738,7 +744,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                     unpack2(t1, f + 4 * i + 2, f + 4 * i + 3);
                 }
 #pragma unroll
-                for (int i = 0; i < 8; i++) f[i] = tf32q(f[i]);
+                for (int i = 0; i < 8; i++) f[i] = tf32q_finite(f[i]);
+                if (hh == 0 && bad) f[0] = quiet_nan;
                 tmem_st8(X + 8 * hh, f);
             }
             tmem_wait_st();
@@ -746,7 +753,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             __syncwarp();
             if (lane == 0) mbar_arrive(su32(&bars.wu_ready));
 #pragma unroll
-            for (int i = 0; i < 32; i++) x[i] = tf32q(x[i]);
+            for (int i = 0; i < 32; i++) x[i] = tf32q_finite(x[i]);
+            if (bad) x[0] = quiet_nan;
             tmem_st32(U, x);                                             // tf32 U^T over the accumulator
             tmem_wait_st();
             fence_before();

@@ -376,8 +376,6 @@ __global__ void __launch_bounds__(128) k_conv_silu_prefill(LinArgs a, float *Y) 
 constexpr int CONV4_TOK = ORN_CONV4_TOK;      // 8 tokens (+ 3 of history) per thread: ~80 registers, 24 warps per SM; 16 tokens took 128
                                               // registers (16 warps per SM) and the kernel waited on its loads (200 us per 8192 tokens x 12288 channels)
 
-// nearest tf32 value (ties away from zero, finite inputs), in integer arithmetic
-__device__ __forceinline__ float tf32_rna(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xFFFFE000u); }
 // NORMS (needs dk = 128, so that the 32 threads of a warp own exactly one q or k head): the kernel also leaves the
 // inverse L2 norms 1/sqrt(sum x^2 + 1e-6) of the q and k rows it produces in rq / rk [token][key head], which saves
 // the pass of k_linear_prep over the image (reference: ot_l2norm_eps, src/ornith_tensor.c:155-160).
@@ -420,7 +418,7 @@ __global__ void __launch_bounds__(128) k_conv4_silu_prefill(LinArgs a, float *Y,
         ORN_CONV4(x, w[0], bias.x); ORN_CONV4(y, w[1], bias.y); ORN_CONV4(z, w[2], bias.z); ORN_CONV4(w, w[3], bias.w);
 #undef ORN_CONV4
         if (FAST && ch < 2 * qd) {                        // q and k feed tf32 tensor-core products: round once, here
-            y.x = tf32_rna(y.x); y.y = tf32_rna(y.y); y.z = tf32_rna(y.z); y.w = tf32_rna(y.w);
+            y.x = tf32r(y.x); y.y = tf32r(y.y); y.z = tf32r(y.z); y.w = tf32r(y.w);
         } else if (NORMS) {                               // the tcgen05 scan's v channels: beta v
             const float bt = sigmoid_f(act_ld((const ACT *)a.b, ((size_t)b * a.T + t0 + i) * a.nv + (ch - 2 * qd) / 128));
             y.x *= bt; y.y *= bt; y.z *= bt; y.w *= bt;
@@ -471,7 +469,7 @@ __global__ void __launch_bounds__(256) k_scan_inputs(LinArgs a, float *Y, const 
     for (size_t e = blockIdx.x * 256ull + threadIdx.x; e < n4; e += gridDim.x * 256ull) {
         const int ch = (int)(e * 4 % Cc);
         float4 y = reinterpret_cast<float4 *>(Y)[e];
-        if (ch < 2 * qd) { y.x = tf32_rna(y.x); y.y = tf32_rna(y.y); y.z = tf32_rna(y.z); y.w = tf32_rna(y.w); }
+        if (ch < 2 * qd) { y.x = tf32r(y.x); y.y = tf32r(y.y); y.z = tf32r(y.z); y.w = tf32r(y.w); }
         else {
             const float s = be[e * 4 / Cc * a.nv + (ch - 2 * qd) / a.dv];
             y.x *= s; y.y *= s; y.z *= s; y.w *= s;

@@ -57,6 +57,14 @@ ornith_status launch_linear_prefill_tc5(const LinArgs &x, int n_seq, int act_dty
                                         const float *rk, const float *la, const float *be, const TC5Front *front,
                                         float *work, cudaStream_t s);
 
+// Round to tf32 (nearest, ties away from zero) with integer arithmetic: cvt.rna.tf32.f32 runs at the special-function rate, a
+// sixteenth of this.  tf32q only adds the half ulp, for operands that go straight to the tensor core, which ignores the 13 low
+// mantissa bits; tf32r leaves them zero.  The minimum keeps NaN what it is: arithmetic gives 0x7fffffff, of which the addition alone
+// (tf32q_finite) makes -0.
+__device__ __forceinline__ float tf32q(float x) { return __int_as_float(min(__float_as_int(x), 0x7fffefff) + 0x1000); }
+__device__ __forceinline__ float tf32r(float x) { return __uint_as_float(__float_as_uint(tf32q(x)) & 0xFFFFE000u); }
+__device__ __forceinline__ float tf32q_finite(float x) { return __int_as_float(__float_as_int(x) + 0x1000); }
+
 __device__ __forceinline__ float4 lds128(const float *p) {        // not hoisted: keeps k/q out of registers
     float4 v;
     asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];\n"

@@ -499,3 +499,34 @@ def test_repeated_rows_with_slow_decay(monkeypatch, form, T, period):
         ref, S, before = _delta_rule_64(kw, nk, nv, S, before, qkv, a, b, z)
         assert rel_err(out.cpu().numpy()[0, 64:], ref[64:]) < 1.6e-3, call
         assert rel_err(st.S.cpu().numpy()[0], S) < 8e-4, call
+
+
+@pytest.mark.parametrize("where,bad", [("v", np.nan), ("v", np.inf), ("k", np.nan), ("q", np.nan)])
+def test_what_is_no_number_shows(where, bad):
+    """A value that is no number at token 70: the heads it belongs to give NaN from there on (a q: for the four tokens its conv
+    reaches), with their state; other heads, and these in the chunks before, keep their bits."""
+    import torch
+    from ornithology_b200 import device as D
+    layer, kw = linear_case(47, nk=2, nv=4)
+    dl = device_linear(layer, kw)
+    T = 200
+    qkv, a, b, z = linear_inputs(470, layer, T)
+
+    def run(x):
+        st = D.LinearState(dl, 1)
+        pos = torch.zeros(1, dtype=torch.int32, device="cuda")
+        out = D.linear_attn_prefill(dl, st, pos, *[_t(y)[None] for y in (x, a, b, z)], T)
+        return out.cpu().numpy().reshape(T, 4, 128), st.S.cpu().numpy()[0]
+
+    ref, S = run(qkv)
+    qkv[70, {"q": 128, "k": layer.qd + 128, "v": 2 * layer.qd + 128}[where] + 5] = bad      # key head 1, or value head 1
+    got, S_bad = run(qkv)
+    hit = [1] if where == "v" else [1, 3]                             # value heads of key head 1 (tiled)
+    kept = [h for h in range(4) if h not in hit]
+    assert (got[:, kept] == ref[:, kept]).all() and (S_bad[kept] == S[kept]).all()
+    assert (got[:64, hit] == ref[:64, hit]).all()
+    assert np.isnan(got[70:74 if where == "q" else T, hit]).all()
+    if where == "q":
+        assert (got[74:, hit] == ref[74:, hit]).all() and (S_bad == S).all()
+    else:
+        assert all(np.isnan(S_bad[h]).any() for h in hit)
