@@ -155,9 +155,11 @@ ornith_status ornith_cuda_sync(void *stream);
 /* The same check without waiting: reads and clears the current device's status word. */
 ornith_status ornith_cuda_poll_status(void);
 /* Every wait inside the kernels (on an mbarrier, for a copy or a tensor-core result) is bounded.
- * This runs a one-thread kernel that waits `polls` polls on a barrier nobody arrives on, and checks
- * that the wait comes back and is reported: the expected return value is ORNITH_ERR_BACKEND with
- * the status word set; ORNITH_ERR_FORMAT means the give-up path did not work.  Nothing faults. */
+ * This runs a small kernel in which a thread waits `polls` polls on a barrier nobody arrives on, and
+ * a warp, half of it for two polls, on one that completes later; it checks that the first wait comes
+ * back and is reported and that the second gives up in every lane: the expected return value is
+ * ORNITH_ERR_BACKEND with the status word set; ORNITH_ERR_FORMAT means the give-up path did not work.
+ * Nothing faults. */
 ornith_status ornith_cuda_selftest_wait_timeout(int polls);
 /* Allocation hook (host-side failure injection; reference: the OOM checks of the init functions,
  * src/ornith_attn.c:32-46): when set, every device allocation the library makes — ornith_cuda_malloc,

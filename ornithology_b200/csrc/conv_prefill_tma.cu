@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(128, CT_CTAS) k_conv4_silu_prefill_tma(LinArgs
         const int tile = (int)tile_l, stage = k % CT_NST;
         const int cb = tile % c.n_cblk, tt = (tile / c.n_cblk) % c.n_ttile, b = tile / (c.n_cblk * c.n_ttile);
         const int t0 = c.t_begin + tt * CT_TOK, ch = cb * CH + ch_local;
-        if (ok && !tc5::mbar_wait(su32(&bars[stage]), (uint32_t)(k / CT_NST) & 1u)) { ok = false; failed = 1; }
+        if (ok && !tc5::mbar_wait_warp(su32(&bars[stage]), (uint32_t)(k / CT_NST) & 1u)) { ok = false; failed = 1; }
         if (ok && ch < Cc) {
             const unsigned char *rows = smem + stage * CT_STAGE + (grp * TPT) * CT_ROWB;    // row i = token t0 + grp TPT - 3 + i
             float4 w[4];                                  // w[q] = taps of channel ch + q

@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
                 if (a.T - 4 + i >= 0) ring[(size_t)((pos0 + a.T - 4 + i) & 3) * Cc + ch] = v[i];
         }
     }
-    if (!mbar_wait(su32(&rows_in), 0u)) report_timeout(p.status, ORN_WAIT_DELTA_SCAN);
+    if (!mbar_wait_warp(su32(&rows_in), 0u)) report_timeout(p.status, ORN_WAIT_DELTA_SCAN);
 
     // Gram tiles: warp w has the rows 16 mt .. of K and of Q and up to three groups of 8 columns from nt0 on (20 such groups lie on
     // or below the diagonal)
@@ -423,7 +423,7 @@ static_assert(SCAN_SMEM + 4096 <= 227 * 1024, "with the static part: the shared 
 enum { B_K, B_V, B_A, B_Q, B_KM, B_P, NBUF };           // operand buffers
 struct ScanBars {
     unsigned long long full[NBUF], empty[NBUF], full_f[NFAC], red[2][4], o_full[4], o_free[4];
-    unsigned long long ks_done, t_ready, u_done, wu_ready, u_ready, s_done, pu_done, qs_done, o_read, full_z, empty_z;
+    unsigned long long ks_done, t_ready, u_done, wu_ready, u_ready, s_done, pu_done, qs_done, o_read, full_z, empty_z, drained[2];
 };
 
 struct ScanArgs {
@@ -472,6 +472,9 @@ __device__ __forceinline__ uint32_t ld_raw(const __nv_bfloat16 *p, size_t i) { r
 __device__ __forceinline__ float cvt_raw(const float *, uint32_t r) { return __uint_as_float(r); }
 __device__ __forceinline__ float cvt_raw(const __nv_bfloat16 *, uint32_t r) { return __uint_as_float(r << 16); }
 
+// A warp that leaves its loop when a wait gives up does so with all its lanes: each reads the clock for itself, and those that stay
+// would miss the others at the next collective instruction.  One vote where a role may leave: a vote for every wait took 1.5 % more.
+__device__ __forceinline__ bool all_lanes(bool ok) { return __all_sync(0xffffffffu, ok); }
 // this thread's stores to shared memory, seen by the tensor copy a thread issues after a barrier
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
@@ -516,6 +519,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
         mbar_init(su32(&bars.ks_done), 1); mbar_init(su32(&bars.t_ready), 8); mbar_init(su32(&bars.u_done), 1);
         mbar_init(su32(&bars.wu_ready), 8); mbar_init(su32(&bars.u_ready), 8); mbar_init(su32(&bars.s_done), 1);
         mbar_init(su32(&bars.pu_done), 1); mbar_init(su32(&bars.qs_done), 1); mbar_init(su32(&bars.o_read), 16);
+        for (int s = 0; s < 2; s++) mbar_init(su32(&bars.drained[s]), 1);
         mbar_init(su32(&bars.full_z), 1); mbar_init(su32(&bars.empty_z), 16);
         mbar_init_fence();
     }
@@ -573,6 +577,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
         // ================= producer =================
         if (elect_one()) {
             asm volatile("griddepcontrol.wait;\n" ::: "memory");     // everything that comes through here is written by the kernels in front
+            int announced = 0, factors = 0;
             if (!tiles) ahead(1);
             for (int n = 0; n < N && ok; n++) {
                 if (!tiles) ahead(n + 2);                                 // (behind the waits of the chunk before)
@@ -580,7 +585,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 const int t0 = (c0 + n) * C;                              // (rows past the sequence's last token arrive as zeros)
                 auto refill = [&](int s, uint32_t bytes) {                // the buffer is free: its next contents are announced
                     if (n >= 1) ok = ok && mbar_wait_parked(su32(&bars.empty[s]), (uint32_t)(n - 1) & 1u);
-                    if (ok) mbar_expect_tx(su32(&bars.full[s]), bytes);
+                    if (ok) { mbar_expect_tx(su32(&bars.full[s]), bytes); announced++; }
                     return ok;
                 };
                 auto rows = [&](int dst, const CUtensorMap *map, int x, int s) {
@@ -592,6 +597,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 // (the readers of the factors of chunk n - 4 are done: K S^T of chunk n - 1 was behind them)
                 mbar_expect_tx(su32(&bars.full_f[n % NFAC]), FAC_BYTES);
                 bulk_load(base + SM_F + n % NFAC * FAC_BYTES, r + REC_F, FAC_BYTES, su32(&bars.full_f[n % NFAC]));
+                factors++;
                 if (!refill(B_V, 32768u)) break;
                 tma_load_3d(base + SM_V, &map_v, 2 * qd + hv * 128, t0, b, su32(&bars.full[B_V]));
                 if (!refill(B_A, TRI_BYTES)) break;
@@ -603,6 +609,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 rows(SM_KM, &map_ym, qd + kh * 128, B_KM);
                 if (!refill(B_P, TRI_BYTES)) break;
                 part(SM_P, REC_P, TRI_BYTES, B_P);
+            }
+            if (!ok) {                                                    // the copies asked for land before the CTA goes
+                for (int s = 0; s < NBUF && s < announced; s++) (void)mbar_wait(su32(&bars.full[s]), (uint32_t)((announced + NBUF - 1 - s) / NBUF - 1) & 1u);
+                for (int s = 0; s < NFAC && s < factors; s++) (void)mbar_wait(su32(&bars.full_f[s]), (uint32_t)((factors + NFAC - 1 - s) / NFAC - 1) & 1u);
             }
         }
     } else if (warp == W_MMA) {
@@ -649,6 +659,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 mma_commit(su32(&bars.s_done));
                 empty(B_KM);
             }
+            if (!ok) {                                                    // nothing may be multiplied when the tensor memory goes back
+                mma_commit(su32(&bars.drained[0]));
+                (void)mbar_wait(su32(&bars.drained[0]), 0u);
+            }
         }
     } else if (warp == W_PU) {
         // ================= (P U)^T =================
@@ -669,6 +683,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 mma_commit(su32(&bars.pu_done));
                 mma_commit(su32(&bars.empty[B_P]));
             }
+            if (!ok) {
+                mma_commit(su32(&bars.drained[1]));
+                (void)mbar_wait(su32(&bars.drained[1]), 0u);
+            }
         }
     } else if (warp < 8) {
         // ================= chain: T, the decayed state, U =================
@@ -678,7 +696,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
         for (int n = 0; n < N; n++) {
             const float *fac = reinterpret_cast<const float *>(gbase + SM_F + (n % NFAC) * FAC_BYTES);
             const uint32_t S = lane_t + TM_S + 128 * (n & 1) + 64 * half, S2 = lane_t + TM_S + 128 * ((n & 1) ^ 1) + 64 * half;
-            ok = mbar_wait(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u));
+            ok = all_lanes(mbar_wait(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u)));
             if (!ok) break;
             fence_after();
             float x[32], v[32];
@@ -693,8 +711,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 tmem_st32(S2 + 32 * cc, x);
             };
             decay(0);
-            ok = mbar_wait(su32(&bars.full[B_V]), (uint32_t)n & 1u);
-            if (!ok) break;
+            ok = mbar_wait(su32(&bars.full[B_V]), (uint32_t)n & 1u);         // (where it gives up the warp reads on, and stops below)
 #pragma unroll
             for (int i = 0; i < 32; i++) v[i] = SEG && kind == 2 ? 0.0f : bv[128 * i];
             // A beta v or a factor that is no finite number makes this row's U NaN.  The roundings below would hide it (-0 for NaN, see
@@ -709,7 +726,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 unpack2(z, &z0, &z1);
                 bad = bad || z0 + z1 != 0.0f;
             }
-            ok = mbar_wait(su32(&bars.ks_done), (uint32_t)n & 1u);
+            ok = all_lanes(ok && mbar_wait(su32(&bars.ks_done), (uint32_t)n & 1u));
             if (!ok) break;
             fence_after();
             tmem_ld32_wait(X, x);                                        // (K S^T)^T
@@ -727,7 +744,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             __syncwarp();
             if (lane == 0) { mbar_arrive(su32(&bars.t_ready)); mbar_arrive(su32(&bars.empty[B_V])); }
             decay(1);
-            ok = mbar_wait(su32(&bars.u_done), (uint32_t)n & 1u);
+            ok = all_lanes(mbar_wait(su32(&bars.u_done), (uint32_t)n & 1u));
             if (!ok) break;
             fence_after();
             tmem_ld32_wait(U, x);                                        // U^T
@@ -761,7 +778,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             __syncwarp();
             if (lane == 0) mbar_arrive(su32(&bars.u_ready));
         }
-        ok = ok && mbar_wait(su32(&bars.s_done), (uint32_t)(N - 1) & 1u);
+        ok = all_lanes(ok && mbar_wait(su32(&bars.s_done), (uint32_t)(N - 1) & 1u));
         fence_after();
 #pragma unroll 1
         for (int cc = 0; cc < 2; cc++) {                                 // the state goes home
@@ -799,7 +816,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 // the gate factors of this chunk, while the tensor core still works on it: norm weight x SiLU(z)
                 if (TILE) {
                     ok = mbar_wait_parked(su32(&bars.full_z), (uint32_t)n & 1u);
-                    if (!ok) break;
 #pragma unroll
                     for (int m = 0; m < 2; m++) {
                         if (sizeof(ACT) == 2) {
@@ -832,8 +848,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                     unpack2(mul2(mul2(z2, pack2(w, w)), pack2(rcp_fast(e0), rcp_fast(e1))), &zr[i], &zr[i + 1]);
                 }
             }
-            ok = mbar_wait_parked(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && mbar_wait_parked(su32(&bars.qs_done), (uint32_t)n & 1u) &&
-                 mbar_wait_parked(su32(&bars.pu_done), (uint32_t)n & 1u);
+            ok = all_lanes(ok && mbar_wait_parked(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && mbar_wait_parked(su32(&bars.qs_done), (uint32_t)n & 1u) &&
+                           mbar_wait_parked(su32(&bars.pu_done), (uint32_t)n & 1u));
             if (!ok) break;
             fence_after();
             float x[16];                                                 // O = p rq QS + P U
@@ -881,7 +897,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(su32(&bars.red[s][grp]));
-            ok = mbar_wait_parked(su32(&bars.red[s][grp]), (uint32_t)(n >> 1) & 1u);
+            if (TILE_O && n >= 1) ok = mbar_wait_parked(su32(&bars.o_free[grp]), (uint32_t)(n - 1) & 1u);      // the group's rows of the chunk before have left
+            ok = all_lanes(ok && mbar_wait_parked(su32(&bars.red[s][grp]), (uint32_t)(n >> 1) & 1u));
             if (!ok) break;
             const float4 r4 = *reinterpret_cast<const float4 *>(&red[s][grp][8 * (lane >> 4) + 2 * j + ((lane >> 3) & 1)][0]);
             const float ss = a.out_scale * a.out_scale * ((r4.x + r4.y) + (r4.z + r4.w));
@@ -892,8 +909,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
 #pragma unroll
             for (int i = 0; i < 16; i += 2) unpack2(mul2(mul2(pack2(x[i], x[i + 1]), i2[i >> 3]), pack2(zr[i], zr[i + 1])), &x[i], &x[i + 1]);
             if (TILE_O) {
-                if (n >= 1) ok = mbar_wait_parked(su32(&bars.o_free[grp]), (uint32_t)(n - 1) & 1u);     // the group's rows of the chunk before have left
-                if (!ok) break;
 #pragma unroll
                 for (int m = 0; m < 2; m++) {
                     uint32_t r[4];
@@ -934,10 +949,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             };
             ahead(1);
             load_z(0);
+            int loads = 1;
             for (int n = 0; n < N && ok; n++) {
                 ahead(n + 2);
                 ok = mbar_wait_parked(su32(&bars.empty_z), (uint32_t)n & 1u);
-                if (ok && n + 1 < N) load_z(n + 1);
+                if (ok && n + 1 < N) { load_z(n + 1); loads++; }
                 if (TZ == 2 && ok) {
                     for (int g = 0; g < 4 && ok; g++) {
                         ok = mbar_wait_parked(su32(&bars.o_full[g]), (uint32_t)n & 1u);
@@ -954,6 +970,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                     for (int g = 0; g < 4; g++) mbar_arrive(su32(&bars.o_free[g]));
                 }
             }
+            if (!ok) (void)mbar_wait(su32(&bars.full_z), (uint32_t)(loads - 1) & 1u);
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");    // shared memory outlives the copies
         }
     }

@@ -53,10 +53,10 @@ constexpr int W_V = 8, W_SM = 16, W_LD = 20, W_MMA = 22, NT = 23 * 32;
 constexpr int NMERGE = 32;
 constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
-struct Bars {
+struct __align__(16) Bars {
     unsigned long long raw_full[NSLOT], raw_empty[NSLOT];
     unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], s_empty[2], p_full[2], p_empty[2];
-    unsigned long long q_full, o_free;
+    unsigned long long q_full, o_free, drained;
 };
 
 // Units a step reads for sequence b: its context and the token being appended; none for a sequence whose cache is full (it is left alone).
@@ -119,6 +119,10 @@ __device__ __forceinline__ void decode_half(uint32_t half, uint32_t keep, SINK s
 
 // (the parked wait starts with the clock, 160 cycles that most waits here do not need)
 __device__ __forceinline__ bool wait_for(uint32_t bar, uint32_t parity) { return mbar_try(bar, parity) || mbar_wait_parked(bar, parity); }
+// Lanes give up each for itself, by its own reading of the clock.  So no lane leaves its warp when a wait did: those that stayed would
+// miss it at the next collective instruction.  The warp goes on without waiting and passes nothing on (the loaders, who must not copy
+// over a slot in use, leave together).  Votes at the waits themselves took 1 % of the batches of 256 x 8192 tokens.
+__device__ __forceinline__ bool all_lanes(bool ok) { return __all_sync(0xffffffffu, ok); }
 // Operand B with the heads contiguous: rows of 16 heads (32 bytes) a token, 32-byte swizzle (16-byte piece c of row r at c ^ (r >> 2 & 1))
 __device__ __forceinline__ uint64_t p_desc(uint32_t saddr) {
     return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(256 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)6 << 61);
@@ -246,7 +250,7 @@ __global__ void __launch_bounds__(NT, 1) k_gqa_decode_q8_tc5(DecodeArgs a, const
             mbar_init(su32(&bars.s_full[s]), 1); mbar_init(su32(&bars.s_empty[s]), 4);
             mbar_init(su32(&bars.p_full[s]), 4); mbar_init(su32(&bars.p_empty[s]), 1);
         }
-        mbar_init(su32(&bars.q_full), 4); mbar_init(su32(&bars.o_free), 4);
+        mbar_init(su32(&bars.q_full), 4); mbar_init(su32(&bars.o_free), 4); mbar_init(su32(&bars.drained), 1);
         mbar_init_fence();
         merge_n = 0;
     }
@@ -273,7 +277,7 @@ __global__ void __launch_bounds__(NT, 1) k_gqa_decode_q8_tc5(DecodeArgs a, const
             for (int t = p.t0; t < p.t1 && ok; t += TILE, T++)
                 for (int i = 0; i < 4 && ok; i++) {
                     const int s = 8 * kv + (T & 1) * 4 + i, tok = t + i * SLOT, valid = max(0, min(SLOT, p.t1 - tok));
-                    if (T >= 2) ok = wait_for(su32(&bars.raw_empty[s]), (uint32_t)((T >> 1) - 1) & 1u);
+                    if (T >= 2) ok = all_lanes(wait_for(su32(&bars.raw_empty[s]), (uint32_t)((T >> 1) - 1) & 1u));
                     if (!ok) break;
                     const uint32_t bar = su32(&bars.raw_full[s]), dst = base + SM_RAW + s * SLOT_BYTES;
                     if (valid == SLOT && tensor_copies) {
@@ -296,13 +300,12 @@ __global__ void __launch_bounds__(NT, 1) k_gqa_decode_q8_tc5(DecodeArgs a, const
         // Warps 0-3 have dims 0..127 of 32 rows each, warps 4-7 dims 128..255.
         const int q = warp & 3, hf = warp >> 2;
         int T = 0;
-        while (ok && next_piece(a, w, range, p)) {
-            for (int t = p.t0; t < p.t1 && ok; t += TILE, T++) {
+        while (next_piece(a, w, range, p)) {
+            for (int t = p.t0; t < p.t1; t += TILE, T++) {
                 const int g = T & 1, slot = 4 * g + q;
                 const uint32_t kt = tmem + ((uint32_t)(32 * q) << 16) + TM_K + 128 * g + 64 * hf;
-                if (T >= 2) ok = wait_for(su32(&bars.k_empty[g]), (uint32_t)((T >> 1) - 1) & 1u);
+                if (T >= 2) ok = ok && wait_for(su32(&bars.k_empty[g]), (uint32_t)((T >> 1) - 1) & 1u);
                 ok = ok && wait_for(su32(&bars.raw_full[slot]), (uint32_t)(T >> 1) & 1u);
-                if (!ok) break;
                 fence_after();
                 if (t + 32 * q < p.t1) {                             // (rows past the end: whatever their scores are, they are masked)
                     float o[32];
@@ -313,8 +316,7 @@ __global__ void __launch_bounds__(NT, 1) k_gqa_decode_q8_tc5(DecodeArgs a, const
                     tmem_wait_st();
                 }
                 fence_before();
-                __syncwarp();
-                if (lane == 0) { mbar_arrive(su32(&bars.k_full[g])); mbar_arrive(su32(&bars.raw_empty[slot])); }
+                if (all_lanes(ok) && lane == 0) { mbar_arrive(su32(&bars.k_full[g])); mbar_arrive(su32(&bars.raw_empty[slot])); }
             }
         }
     } else if (warp < W_SM) {
@@ -325,11 +327,10 @@ __global__ void __launch_bounds__(NT, 1) k_gqa_decode_q8_tc5(DecodeArgs a, const
         const int th = (warp - W_V) >> 2, r = 2 * th + ((warp >> 1) & 1), hf = (lane >> 3) & 1, row = (warp & 1) * 16 + (lane >> 4) * 8 + (lane & 7), token = 32 * r + row;
         const uint32_t vt = base + SM_V + th * 32768 + hf * 16384 + (token & 63) * 128;
         int T = 0;
-        while (ok && next_piece(a, w, range, p)) {
-            for (int t = p.t0; t < p.t1 && ok; t += TILE, T++) {
+        while (next_piece(a, w, range, p)) {
+            for (int t = p.t0; t < p.t1; t += TILE, T++) {
                 const int slot = 8 + (T & 1) * 4 + r;
-                ok = wait_for(su32(&bars.raw_full[slot]), (uint32_t)(T >> 1) & 1u);
-                if (!ok) break;
+                ok = ok && wait_for(su32(&bars.raw_full[slot]), (uint32_t)(T >> 1) & 1u);
                 // the first 64 dims stay in registers while the value product of the tile before still reads the buffer
                 // a row past the end becomes zeros (a probability of zero must not meet anything but a number)
                 uint32_t o[NST];
@@ -343,7 +344,7 @@ __global__ void __launch_bounds__(NT, 1) k_gqa_decode_q8_tc5(DecodeArgs a, const
                         if (i == NST - 1) {
 #pragma unroll
                             for (int k = 0; k < NST; k++) asm volatile("" : "+r"(o[k]));     // (decoded here, not after the wait)
-                            if (T >= 1) ok = wait_for(su32(&bars.v_empty[th]), (uint32_t)(T - 1) & 1u);
+                            if (T >= 1) ok = ok && wait_for(su32(&bars.v_empty[th]), (uint32_t)(T - 1) & 1u);
 #pragma unroll
                             for (int c = 0; c < NST / 4; c++) put(c, o + 4 * c);
                         }
@@ -353,8 +354,7 @@ __global__ void __launch_bounds__(NT, 1) k_gqa_decode_q8_tc5(DecodeArgs a, const
                     if ((i & 3) == 3) put(i >> 2, o);
                 });
                 fence_async();
-                __syncwarp();
-                if (lane == 0) { mbar_arrive(su32(&bars.raw_empty[slot])); mbar_arrive(su32(&bars.v_full[th])); }
+                if (all_lanes(ok) && lane == 0) { mbar_arrive(su32(&bars.raw_empty[slot])); mbar_arrive(su32(&bars.v_full[th])); }
             }
         }
     } else if (warp == W_MMA) {
@@ -400,6 +400,10 @@ __global__ void __launch_bounds__(NT, 1) k_gqa_decode_q8_tc5(DecodeArgs a, const
                 }
                 if (ok) values(T - 1, T - 1 == T0);                  // ahead of the wait for the next piece's queries
                 n++;
+            }
+            if (!ok) {                                               // nothing may be multiplied when the tensor memory goes back
+                mma_commit(su32(&bars.drained));
+                (void)wait_for(su32(&bars.drained), 0u);
             }
         }
     } else {

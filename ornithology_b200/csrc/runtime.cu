@@ -140,15 +140,31 @@ OrnTensorMapEncodeFn orn_tensor_map_encoder() {
 
 // A kernel whose only job is to wait, a few polls long, on an mbarrier nobody arrives on: the wait
 // helper of the tensor-core kernels must come back, report through the status word, and leave the
-// context usable.  Nothing is in flight when it gives up.
-__global__ void k_wait_selftest(unsigned int *status, int polls, int *gave_up) {
-    __shared__ unsigned long long bar;
+// context usable.  Then by a whole warp on one that completes 50 ms later, half of its lanes with a
+// limit of two polls: all of them must give up.  Nothing is in flight when they do.  *result: 1 for
+// the first wait, 2 for the second.
+__global__ void __launch_bounds__(64) k_wait_selftest(unsigned int *status, int polls, int *result) {
+    __shared__ unsigned long long bar[2];
     if (threadIdx.x == 0) {
-        tc5::mbar_init(tc5::su32(&bar), 1);
+        for (unsigned long long &b : bar) tc5::mbar_init(tc5::su32(&b), 1);
         tc5::mbar_init_fence();
-        const bool ok = tc5::mbar_wait(tc5::su32(&bar), 0, polls);
-        if (!ok) tc5::report_timeout(status, ORN_WAIT_SELFTEST);
-        *gave_up = ok ? 0 : 1;
+    }
+    __syncthreads();
+    if (threadIdx.x == 32) {
+        const unsigned long long t0 = tc5::global_ns();
+        for (int i = 0; i < (1 << 20) && tc5::global_ns() - t0 < 50000000ull; i++) __nanosleep(1000);
+        tc5::mbar_arrive(tc5::su32(&bar[1]));
+    }
+    if (threadIdx.x < 32) {
+        bool ok = true;
+        if (threadIdx.x == 0) {
+            ok = tc5::mbar_wait(tc5::su32(&bar[0]), 0, polls);
+            if (!ok) tc5::report_timeout(status, ORN_WAIT_SELFTEST);
+        }
+        __syncwarp();
+        const bool all = tc5::mbar_wait_warp(tc5::su32(&bar[1]), 0, threadIdx.x & 1 ? 2 : 1 << 24);
+        const bool none = __ballot_sync(0xffffffffu, all) == 0;
+        if (threadIdx.x == 0) *result = (ok ? 0 : 1) + (none ? 2 : 0);
     }
 }
 
@@ -186,12 +202,12 @@ ornith_status ornith_cuda_selftest_wait_timeout(int polls) {
     int *flag = nullptr;
     ORN_TRY(orn_check(cudaMalloc((void **)&flag, sizeof(int)), "selftest flag"));
     int gave_up = -1;
-    k_wait_selftest<<<1, 32>>>(status, polls, flag);
+    k_wait_selftest<<<1, 64>>>(status, polls, flag);
     ornith_status st = orn_check_launch("k_wait_selftest");
     if (st == ORNITH_OK) st = orn_check(cudaMemcpy(&gave_up, flag, sizeof(int), cudaMemcpyDeviceToHost), "selftest read-back");
     (void)cudaFree(flag);
     if (st != ORNITH_OK) return st;
-    if (gave_up != 1) { orn_record_error("wait self-test: the wait did not give up (%d)", gave_up); return ORNITH_ERR_FORMAT; }
+    if (gave_up != 3) { orn_record_error("wait self-test: a wait did not give up, or not in all lanes of its warp (%d)", gave_up); return ORNITH_ERR_FORMAT; }
     st = take_status_word();                       // must report the give-up
     if (st == ORNITH_OK && status) { orn_record_error("wait self-test: the status word stayed clear"); return ORNITH_ERR_FORMAT; }
     return st == ORNITH_OK ? (ornith_status)ORNITH_ERR_BACKEND : st;   // the expected outcome is ORNITH_ERR_BACKEND

@@ -64,6 +64,11 @@ __device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity) 
     }
     return false;
 }
+// The same by a whole warp, which it leaves converged and of one opinion: each lane reads the clock for itself, and where a barrier
+// completes around the limit some would give up, leave their loop and be missed by the warp's next collective instruction.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int limit = 1 << 24) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit));
+}
 // Status word of a launch (device-visible host memory, zero when all is well): a wait that
 // gave up leaves a non-zero code there; the host reads it at its next synchronisation.
 __device__ __forceinline__ void report_timeout(unsigned int *status, unsigned int code) {
