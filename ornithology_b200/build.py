@@ -21,7 +21,9 @@ CSRC = os.path.join(PKG, "csrc")
 OBJ = os.path.join(PKG, "build")
 LIB = os.path.join(PKG, "libornith_cuda.so")
 FASTCALL_SRC = os.path.join(CSRC, "py", "fastcall.c")
-FASTCALL = os.path.join(PKG, "_fastcall.so")          # the Python module that calls into the library (_lib.py)
+# the Python module that calls into the library (_lib.py), for the Python that builds it; where that has no headers _lib.py does without
+FASTCALL = os.path.join(PKG, "_fastcall" + sysconfig.get_config_var("EXT_SUFFIX"))
+PY_INCLUDE = sysconfig.get_paths()["include"]
 INCLUDE = os.path.join(ROOT, "include")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -42,8 +44,12 @@ def sources():
     return cu, c
 
 
+def _has_python_headers() -> bool:
+    return os.path.exists(os.path.join(PY_INCLUDE, "Python.h"))
+
+
 def _stale() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(FASTCALL):
+    if not os.path.exists(LIB) or (_has_python_headers() and not os.path.exists(FASTCALL)):
         return True
     t = os.path.getmtime(LIB)
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [FASTCALL_SRC, os.path.join(INCLUDE, "ornith_cuda.h")]
@@ -53,7 +59,7 @@ def _stale() -> bool:
 def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not _stale():
         return LIB
-    extra = os.environ.get("ORNITH_NVCC_EXTRA", "").split()       # e.g. -DORNITH_SCAN_TRACE for kernel bring-up
+    extra = os.environ.get("ORNITH_NVCC_EXTRA", "").split()       # further -D definitions
     os.makedirs(OBJ, exist_ok=True)
     nvcc = _nvcc()
     cu, c = sources()
@@ -82,10 +88,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
     r = subprocess.run([nvcc, "-shared", "-o", LIB, *objs, "-lpthread"], capture_output=True, text=True)
     if r.returncode:
         raise RuntimeError(f"link failed:\n{r.stderr}")
-    r = subprocess.run(["gcc", "-O2", "-std=gnu11", "-fPIC", "-shared", "-Wall", "-I", sysconfig.get_paths()["include"], FASTCALL_SRC,
-                        "-o", FASTCALL], capture_output=True, text=True)
-    if r.returncode:
-        raise RuntimeError(f"gcc failed on fastcall.c:\n{r.stderr}")
+    if _has_python_headers():
+        r = subprocess.run(["gcc", "-O2", "-std=gnu11", "-fPIC", "-shared", "-Wall", "-I", PY_INCLUDE, FASTCALL_SRC, "-o", FASTCALL],
+                           capture_output=True, text=True)
+        if r.returncode:
+            raise RuntimeError(f"gcc failed on fastcall.c:\n{r.stderr}")
     with open(os.path.join(OBJ, "ptxas.log"), "w") as fh:
         for f, t in logs.items():
             fh.write(f"==== {f}\n{t}\n")

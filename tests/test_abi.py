@@ -155,19 +155,36 @@ def test_projection_sizing_and_no_gpu_behaviour(lib):
         assert lib.ornith_cuda_matmul_q(8, None, 2048, 64, None, 0, 4, None, 0, None, 0, None) != 0
 
 
-def test_fast_calls_pass_what_ctypes_passes(lib):
-    """The _fastcall callables against ctypes, on host-only entry points: sizes beyond 32 bits, null pointers, packed structs, errors."""
+@pytest.mark.parametrize("module", [True, False])
+def test_fast_calls_pass_what_ctypes_passes(lib, monkeypatch, module):
+    """The callables of _lib.fast(), with the _fastcall module and without it, against ctypes, on host-only entry points: sizes
+    beyond 32 bits, null pointers, packed structs, whole numbers of every kind (as values, never as addresses), errors."""
     import struct
+    import sys
+    import numpy as np
+    import torch
     from ornithology_b200 import _lib
+    monkeypatch.setattr(_lib, "_fast", None)
+    if not module:
+        import ornithology_b200
+        monkeypatch.delattr(ornithology_b200, "_fastcall", raising=False)
+        monkeypatch.setitem(sys.modules, "ornithology_b200._fastcall", None)      # importing it raises ImportError
     f = _lib.fast()
+    assert type(f.matmul_q_scratch).__name__ == ("Function" if module else "function")
     for args in ((8, 64, 4096), (14, 1 << 20, 8192), (3, 1, 256)):
         assert f.matmul_q_scratch(*args) == lib.ornith_cuda_matmul_q_scratch(*args)
+    want = lib.ornith_cuda_matmul_q_scratch(8, 64, 4096)
+    for whole in (np.int64, np.int32, torch.tensor, lambda n: torch.tensor([n])):
+        assert f.matmul_q_scratch(8, 64, whole(4096)) == lib.ornith_cuda_matmul_q_scratch(8, 64, whole(4096)) == want > 0
     rows = struct.pack("@3i", 4096, 512, 512)
     arr = (C.c_int * 3)(4096, 512, 512)
     assert f.matmul_q_tile_tokens(14, 2048, rows, 3, 777) == lib.ornith_cuda_matmul_q_tile_tokens(14, 2048, C.addressof(arr), 3, 777)
+    assert f.matmul_q_tile_tokens(14, 2048, torch.tensor([4096, 512, 512], dtype=torch.int32), 3, 777) == f.matmul_q_tile_tokens(14, 2048, rows, 3, 777)
     assert f.matmul_q_tile_tokens(14, 2048, None, 3, 777) == -1
-    with pytest.raises(AttributeError):
-        f.matmul_q_scratch(8, 64, 1.5)
-    with pytest.raises(TypeError):
-        f.matmul_q_scratch(*range(17))
+    for bad in (1.5, None, "6", b"6"):
+        with pytest.raises((TypeError, C.ArgumentError)):
+            f.matmul_q_scratch(8, 64, bad)
+    for n in (0, 2, 4, 17):
+        with pytest.raises(TypeError):
+            f.matmul_q_scratch(*range(n))
     assert not hasattr(f, "rope_inv_freq")                 # takes a float: ctypes only
