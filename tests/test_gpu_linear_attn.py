@@ -222,14 +222,15 @@ def test_segment_parallel_scan_against_oracle(oracle, monkeypatch, segments, bf1
     """Few heads: the prompt is cut into runs that are scanned side by side (from a zero state and from the identity),
     stitched by a carry over the runs and a finishing product.  2000 tokens (a ragged last chunk), 4 key / 8 value
     heads, two calls with the state carried; segments = 0 leaves the choice to the library (8 heads: 9 runs wanted,
-    3 possible at 8 chunks per run).  Outputs and final state against the CPU scan."""
+    3 possible at 16 chunks per run in 3100 tokens, which have the bits of 3 forced runs and not of one).  Outputs and
+    final state against the CPU scan."""
     import torch
     from ornithology_b200 import device as D
     if segments:
         monkeypatch.setenv("ORNITH_CUDA_DELTA_SEGMENTS", str(segments))
     layer, kw = linear_case(41, nk=4, nv=8)
     dl = device_linear(layer, kw)
-    T1, T2 = 1500, 500
+    T1, T2 = 1500 if segments else 3100, 500
     QKV, A, Bm, Z = linear_inputs(410, layer, T1 + T2, bf16)
     S = np.zeros((layer.nv, 128, 128), np.float32); buf = np.zeros(3 * layer.cc, np.float32)
     st = D.LinearState(dl, 1)
@@ -242,6 +243,13 @@ def test_segment_parallel_scan_against_oracle(oracle, monkeypatch, segments, bf1
         out = D.linear_attn_prefill(dl, st, pos, _t(QKV[sl], dt)[None], _t(A[sl], dt)[None], _t(Bm[sl], dt)[None], _t(Z[sl], dt)[None], n, chunk=64)
         assert rel_err(out.float().cpu().numpy()[0], ref) < tol, t0
         assert rel_err(st.S.cpu().numpy()[0], S) < TOL, t0
+        if segments == 0 and t0 == 0:                      # the library's choice, known by its bits
+            for forced, same in (("3", True), ("1", False)):
+                with monkeypatch.context() as m:
+                    m.setenv("ORNITH_CUDA_DELTA_SEGMENTS", forced)
+                    other = D.LinearState(dl, 1)
+                    o2 = D.linear_attn_prefill(dl, other, pos, _t(QKV[sl], dt)[None], _t(A[sl], dt)[None], _t(Bm[sl], dt)[None], _t(Z[sl], dt)[None], n, chunk=64)
+                    assert bool((o2 == out).all()) == same, forced
         D.advance(pos, n)
 
 
@@ -267,9 +275,9 @@ def test_64_head_prefill_is_reproducible():
             assert (got[0] == first[0]).all() and (got[1] == first[1]).all(), rep
 
 
-@pytest.mark.parametrize("T,pos0", [(4096 + 37, 0), (8192, 2)])
+@pytest.mark.parametrize("T,pos0", [(8192 + 37, 0), (8192, 2)])
 def test_slab_pipeline_matches_the_single_launch(monkeypatch, T, pos0):
-    """Long prompts with one wave of heads run conv + chunk preparation of the next slab beside the scan of
+    """Long prompts (128 chunks and more) with one wave of heads run conv + chunk preparation of the next slab beside the scan of
     the current one (two streams, events).  The slabs hand the state over in f32 exactly as the chunks of a
     single launch do, so outputs, state and conv history must be bit-identical to the unpipelined form, on a
     ragged length, with a non-empty history, and when a second call follows at once on the same stream."""
