@@ -87,7 +87,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm(
 // What most kernels of the chains do first: wait for the kernel in front (whose results they read and whose inputs they may
 // overwrite), then let the one behind take its place on the SMs.  A step of one chat is a dozen kernels of a few
 // microseconds; without this each pays its launch latency after the end of the one before.  Not so, on purpose:
-// k_gqa_decode_q8_raw and k_linear_decode_ring release the kernel behind them at once (it must wait before all else) and
+// k_gqa_decode_q8_tc5 and k_linear_decode_ring release the kernel behind them at once (it must wait before all else) and
 // wait themselves only before they read what the kernel in front wrote; k_conv4_silu_prefill_tma, itself launched plainly,
 // releases at once too; the projection kernels, the tcgen05 scan and the tcgen05 GQA prefill wait only where they first touch
 // such data and release nothing before their end; the int8 decode kernel is launched plainly.

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(128) k_full_prep(PrepArgs a) {
     const int hd = a.kv.hd, nkv = a.kv.nkv, nh = a.nh;
     // Launched as a programmatic dependent of the kernel in front of it (the layer before): resident when that kernel
     // ends, and waiting for its end before anything else.  After that a decode kernel launched behind this one may
-    // begin its prologue (it streams cache rows early, and waits for this grid before it reads its output).
+    // begin its prologue (the Q8_0 one finds its ranges; it waits for this grid before it asks for any row).
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (a.group_ctr)
@@ -728,9 +728,8 @@ static size_t step_need(const ornith_cuda_full_layer *l, int n_seq, int max_len,
 static DecodePath decode_path(const ornith_cuda_full_layer *l, const ornith_cuda_kv *kv) {
     if (force_generic_decode()) return PATH_ANY;
     const KvView v = make_view(kv);
-    if (gqa_decode_q8_balanced(v, l->n_heads)) return PATH_BALANCED;
-    return (gqa_decode_q8_mma_supported(v, l->n_heads) || gqa_decode_f32_tc_supported(v, l->n_heads) ||
-            gqa_decode_i8_raw_supported(v, l->n_heads)) ? PATH_SPLIT_TC : PATH_ANY;
+    if (gqa_decode_q8_supported(v, l->n_heads)) return PATH_BALANCED;
+    return (gqa_decode_f32_tc_supported(v, l->n_heads) || gqa_decode_i8_raw_supported(v, l->n_heads)) ? PATH_SPLIT_TC : PATH_ANY;
 }
 
 template <typename ACT>
@@ -828,13 +827,12 @@ ornith_status ornith_cuda_full_attn_step(const ornith_cuda_full_layer *l, const 
     d.group_ctr = group_ctr; d.qproj = qproj; d.out = out; d.gated = l->gated; d.act_dtype = act_dtype;
     d.n_seq = B; d.max_len = max_len; d.status = nullptr; d.piece_cost = 0;
     d.range_floor = path == PATH_BALANCED ? gqa_decode_range_floor(l->n_kv_heads, nh, B, max_len, short_ranges) : 0;
-    bool merged = false;
     int nsplit_used;
-    if (gqa_decode_q8_mma_supported(d.kv, nh) && !force_generic_decode()) {
-        d.tokens_per_split = tps_mma; d.nsplit = nsplit_used = (max_len + tps_mma - 1) / tps_mma;
-        if (path == PATH_BALANCED) d.nsplit = nsplit_used = gqa_decode_q8_slots(l->n_kv_heads, nh, B, max_len, d.range_floor);
-        ORN_TRY(launch_gqa_decode_q8_mma(d, B, st, &merged));
-    } else if (gqa_decode_f32_tc_supported(d.kv, nh) && !force_generic_decode()) {
+    if (path == PATH_BALANCED) {
+        d.tokens_per_split = 0; d.nsplit = gqa_decode_q8_slots(l->n_kv_heads, nh, B, max_len, d.range_floor);
+        return launch_gqa_decode_q8_tc5(d, B, st);
+    }
+    if (gqa_decode_f32_tc_supported(d.kv, nh) && !force_generic_decode()) {
         d.tokens_per_split = tps_mma; d.nsplit = nsplit_used = (max_len + tps_mma - 1) / tps_mma;
         ORN_TRY(launch_gqa_decode_f32_tc(d, B, st));
     } else if (gqa_decode_i8_raw_supported(d.kv, nh) && !force_generic_decode()) {
@@ -852,7 +850,6 @@ ornith_status ornith_cuda_full_attn_step(const ornith_cuda_full_layer *l, const 
         ORN_TRY(orn_check_launch("k_gqa_decode_generic"));
     }
 
-    if (merged) return ORNITH_OK;
     CombineArgs c;
     c.kv = d.kv; c.kv_len = kv_len; c.part = part; c.qproj = qproj; c.out = out;
     c.nh = nh; c.nsplit = nsplit_used; c.gated = l->gated; c.tokens_per_split = d.tokens_per_split;

@@ -10,37 +10,29 @@ struct DecodeArgs {
     float *part;                         // [n_seq][nh][nsplit][hd + 2]: m, l, o[hd]
     int nh, nsplit, tokens_per_split;
     float scale;
-    // Fused merge (kernels that support it; group_ctr == nullptr leaves the merge to k_gqa_combine): the last CTA
-    // of a (sequence, head group) to finish merges the group's partials, applies the output gate and stores.
-    int *group_ctr;                      // [n_seq][grid.x] arrival counters, zero when the kernel starts
+    // Fused merge (the Q8_0 kernel): the last CTA of a (sequence, KV head) to finish merges the group's partials, applies the
+    // output gate and stores.
+    int *group_ctr;                      // [n_seq][n_kv_heads] arrival counters, zero when the kernel starts
     const void *qproj;                   // gate = second half of each head's projection row (gated != 0)
     void *out;
     int gated, act_dtype;
     int n_seq, max_len;                  // batch size and the call's bound on any context after the append
-    int range_floor;                     // balanced schedule: the fewest tiles of a range (gqa_decode_range_floor)
-    int piece_cost;                      // balanced schedule: tiles charged per sequence for the fixed work of a piece
+    int range_floor;                     // Q8_0 kernel: the fewest units of 16 tokens of a range (gqa_decode_range_floor)
+    int piece_cost;                      // Q8_0 kernel: units charged per sequence for the fixed work of a piece
     unsigned int *status;                // device status word (a bounded wait that gave up sets ORN_WAIT_DECODE), or NULL
 };
 
-// Tensor-core split-K decode over Q8_0 rows, head_dim 256, up to 16 query heads
-// per KV head.  Writes the same partials as the generic kernel.
-bool gqa_decode_q8_mma_supported(const KvView &kv, int nh);
-// *merged is set when the launched kernel did the merge itself (a.group_ctr given and supported).
-ornith_status launch_gqa_decode_q8_mma(const DecodeArgs &a, int n_seq, cudaStream_t st, bool *merged);
-
-// Variant with a grid of fixed splits that builds its mma.sync fragments straight
-// from the staged raw rows (gqa_decode_q8_raw.cu).
-ornith_status launch_gqa_decode_q8_raw(const DecodeArgs &a, int n_seq, cudaStream_t st, bool *merged);
-// Whether a step over this cache is served by the tcgen05 kernel (gqa_decode_q8_tc5.cu; up to 16 heads per KV head) with its balanced
-// schedule (token ranges of equal length found on the device instead of a grid of fixed splits), and then how many partial slots per
-// head its scratch needs: a.nsplit = gqa_decode_q8_slots(...) and a.part laid out [head][slot][hd + 2].  It merges its partials itself.
-bool gqa_decode_q8_balanced(const KvView &kv, int nh);
+// Decode over Q8_0 rows on the tcgen05 tensor cores (gqa_decode_q8_tc5.cu), head_dim 256, up to 16 query heads per KV head, token ranges of
+// equal length found on the device.  It merges its partials itself: a.nsplit = gqa_decode_q8_slots(...) slots per head,
+// a.part laid out [head][slot][hd + 2].
+bool gqa_decode_q8_supported(const KvView &kv, int nh);
 int gqa_decode_q8_slots(int nkv, int nh, int n_seq, int max_len, int range_floor);
 ornith_status launch_gqa_decode_q8_tc5(const DecodeArgs &a, int n_seq, cudaStream_t st);
-// the fewest tiles of a range: the long ones need the fewest partials, the short ones spread small batches further
+// the fewest units of a range: the long ones need the fewest partials, the short ones spread small batches further
 int gqa_decode_range_floor(int nkv, int nh, int n_seq, int max_len, bool short_ranges);
 
-// The same for int8-per-head rows (gqa_decode_i8_raw.cu), up to 8 query heads per KV head.
+// Split-K decode over int8-per-head rows (gqa_decode_i8_raw.cu), up to 16 query heads per KV head.  Writes the same partials as the
+// generic kernel.
 bool gqa_decode_i8_raw_supported(const KvView &kv, int nh);
 ornith_status launch_gqa_decode_i8_raw(const DecodeArgs &a, int n_seq, cudaStream_t st);
 

@@ -1,6 +1,6 @@
 // gqa_decode_i8_raw.cu — split-K GQA decode over int8-per-head rows (the engine's own quantised
 // cache: 256 codes per row and one f32 scale per row in a side array), groups of up to 16 query
-// heads (two CTAs of 8 heads beyond 8), head_dim 256.  The structure is that of the Q8_0 kernel (gqa_decode_q8_raw.cu).
+// heads (two CTAs of 8 heads beyond 8), head_dim 256.
 //
 // Replaces the attend half of ornith_gqa_step for kv->quantized caches (reference:
 // src/ornith_attn.c:111-148, codec src/ornith_attn.c:24-47).

@@ -5,7 +5,7 @@
 // the output gate (src/ornith_rforward.c:450).
 //
 // What bounds it: the rows from memory on long contexts, a piece's fixed chain (queries, first rows, products, partial, merge) on short
-// ones.  A warp that builds mma.sync fragments from the raw rows (gqa_decode_q8_raw.cu, which ran here before) issues a dozen
+// ones.  A warp that builds mma.sync fragments from the raw rows (the kernel that ran here before) issues a dozen
 // instructions per 16-byte piece for every 8 heads and was bound by that: 0.72 of the memory rate with 8 heads to a KV head, 0.43 with
 // 16, whose rows it converted twice.  Here a row is converted once, whatever the number of heads, and the products cost no issue
 // slots.  One CTA per SM walks a range of the batch's rows, 128 tokens (a tile) at a time:
@@ -624,13 +624,14 @@ int gqa_decode_q8_slots(int nkv, int nh, int n_seq, int max_len, int range_floor
     return balanced_ranges(nkv, nh, n_seq, max_len, range_floor) + n_seq;
 }
 
+bool gqa_decode_q8_supported(const KvView &kv, int nh) {
+    return kv.mode == ORNITH_KV_Q8_0 && kv.hd == HD && nh % kv.nkv == 0 && nh / kv.nkv <= 16 &&
+           ((uintptr_t)kv.K % 16) == 0 && ((uintptr_t)kv.V % 16) == 0;
+}
+
 ornith_status launch_gqa_decode_q8_tc5(const DecodeArgs &a_in, int n_seq, cudaStream_t st) {
     DecodeArgs a = a_in;
     const int G = a.nh / a.kv.nkv;
-    if (!a.group_ctr) {
-        orn_record_error("k_gqa_decode_q8_tc5: the kernel merges its partials itself and needs the arrival counters");
-        return ORNITH_ERR_FORMAT;
-    }
     static bool configured_dev[ORN_MAX_DEVICES] = {};
     bool &configured = configured_dev[orn_device_index()];
     if (!configured) {
