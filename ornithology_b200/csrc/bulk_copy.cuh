@@ -25,6 +25,9 @@ __device__ __forceinline__ bool bc_mbar_wait(uint32_t bar, uint32_t parity) {
         if (bc_mbar_try_wait(bar, parity)) return true;
     return false;
 }
+// The same by a whole warp, whose lanes go on or give up together: those that stayed would miss the others at the warp's next
+// collective instruction.
+__device__ __forceinline__ bool bc_mbar_wait_warp(uint32_t bar, uint32_t parity) { return __all_sync(0xffffffffu, bc_mbar_wait(bar, parity)); }
 // dst, src 16-byte aligned, bytes a multiple of 16
 __device__ __forceinline__ void bc_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n"

@@ -472,8 +472,9 @@ __device__ __forceinline__ uint32_t ld_raw(const __nv_bfloat16 *p, size_t i) { r
 __device__ __forceinline__ float cvt_raw(const float *, uint32_t r) { return __uint_as_float(r); }
 __device__ __forceinline__ float cvt_raw(const __nv_bfloat16 *, uint32_t r) { return __uint_as_float(r << 16); }
 
-// A warp that leaves its loop when a wait gives up does so with all its lanes: each reads the clock for itself, and those that stay
-// would miss the others at the next collective instruction.  One vote where a role may leave: a vote for every wait took 1.5 % more.
+// Lanes give up each for itself, by its own reading of the clock, and those that stayed in a loop would miss the others at the warp's next
+// collective instruction.  So a chain warp goes on without waiting when a wait gave up, and passes nothing on; an output warp
+// leaves with all its lanes.  Votes at the chain's waits took 1.5 %.
 __device__ __forceinline__ bool all_lanes(bool ok) { return __all_sync(0xffffffffu, ok); }
 // this thread's stores to shared memory, seen by the tensor copy a thread issues after a barrier
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -696,8 +697,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
         for (int n = 0; n < N; n++) {
             const float *fac = reinterpret_cast<const float *>(gbase + SM_F + (n % NFAC) * FAC_BYTES);
             const uint32_t S = lane_t + TM_S + 128 * (n & 1) + 64 * half, S2 = lane_t + TM_S + 128 * ((n & 1) ^ 1) + 64 * half;
-            ok = all_lanes(mbar_wait(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u)));
-            if (!ok) break;
+            ok = ok && mbar_wait(su32(&bars.full_f[n % NFAC]), (uint32_t)(n / NFAC) & 1u) && (n == 0 || mbar_wait(su32(&bars.s_done), (uint32_t)(n - 1) & 1u));
             fence_after();
             float x[32], v[32];
             // the other state = p_63 S, while the tensor core reads S (the update is accumulated onto it): a half beside K S^T, a half
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 tmem_st32(S2 + 32 * cc, x);
             };
             decay(0);
-            ok = mbar_wait(su32(&bars.full[B_V]), (uint32_t)n & 1u);         // (where it gives up the warp reads on, and stops below)
+            ok = ok && mbar_wait(su32(&bars.full[B_V]), (uint32_t)n & 1u);
 #pragma unroll
             for (int i = 0; i < 32; i++) v[i] = SEG && kind == 2 ? 0.0f : bv[128 * i];
             // A beta v or a factor that is no finite number makes this row's U NaN.  The roundings below would hide it (-0 for NaN, see
@@ -726,8 +726,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
                 unpack2(z, &z0, &z1);
                 bad = bad || z0 + z1 != 0.0f;
             }
-            ok = all_lanes(ok && mbar_wait(su32(&bars.ks_done), (uint32_t)n & 1u));
-            if (!ok) break;
+            ok = ok && mbar_wait(su32(&bars.ks_done), (uint32_t)n & 1u);
             fence_after();
             tmem_ld32_wait(X, x);                                        // (K S^T)^T
 #pragma unroll
@@ -741,11 +740,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             tmem_st32(X, x);
             tmem_wait_st();
             fence_before();
-            __syncwarp();
-            if (lane == 0) { mbar_arrive(su32(&bars.t_ready)); mbar_arrive(su32(&bars.empty[B_V])); }
+            if (all_lanes(ok) && lane == 0) { mbar_arrive(su32(&bars.t_ready)); mbar_arrive(su32(&bars.empty[B_V])); }
             decay(1);
-            ok = all_lanes(mbar_wait(su32(&bars.u_done), (uint32_t)n & 1u));
-            if (!ok) break;
+            ok = ok && mbar_wait(su32(&bars.u_done), (uint32_t)n & 1u);
             fence_after();
             tmem_ld32_wait(U, x);                                        // U^T
             // (w rk U)^T over T^T first: the state update waits for it
@@ -767,18 +764,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) k_delta_scan_tc5(const __grid_con
             }
             tmem_wait_st();
             fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(su32(&bars.wu_ready));
+            if (all_lanes(ok) && lane == 0) mbar_arrive(su32(&bars.wu_ready));
 #pragma unroll
             for (int i = 0; i < 32; i++) x[i] = tf32q_finite(x[i]);
             if (bad) x[0] = quiet_nan;
             tmem_st32(U, x);                                             // tf32 U^T over the accumulator
             tmem_wait_st();
             fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(su32(&bars.u_ready));
+            if (all_lanes(ok) && lane == 0) mbar_arrive(su32(&bars.u_ready));
         }
-        ok = all_lanes(ok && mbar_wait(su32(&bars.s_done), (uint32_t)(N - 1) & 1u));
+        ok = ok && mbar_wait(su32(&bars.s_done), (uint32_t)(N - 1) & 1u);
         fence_after();
 #pragma unroll 1
         for (int cc = 0; cc < 2; cc++) {                                 // the state goes home

@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(128, 3) k_gqa_decode_f32_tc(DecodeArgs a) {
     for (uint32_t n = 0; it < ntiles; it += NWARP, n++) {
         const int tok0 = t0 + it * TILE;
         const bool more = it + NWARP < ntiles;
-        if (!bc_mbar_wait(barK, n & 1)) { (void)bc_mbar_wait(barV, n & 1); pipe_ok = false; break; }
+        if (!bc_mbar_wait_warp(barK, n & 1)) { (void)bc_mbar_wait(barV, n & 1); pipe_ok = false; break; }
 
         // ---- S = Q K^T: 32 k-steps of 8 dims in two accumulator chains ----------------------
         float s0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, s1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(128, 3) k_gqa_decode_f32_tc(DecodeArgs a) {
         const float pb0 = tf32q((j & 1) ? v01 : v00), pb1 = tf32q((j & 1) ? v11 : v10);
 
         // ---- O^T += V^T P^T: 16 m-tiles of 16 dims, one k-step of 8 tokens -------------------
-        if (!bc_mbar_wait(barV, n & 1)) { if (more) (void)bc_mbar_wait(barK, (n + 1) & 1); pipe_ok = false; break; }
+        if (!bc_mbar_wait_warp(barV, n & 1)) { if (more) (void)bc_mbar_wait(barK, (n + 1) & 1); pipe_ok = false; break; }
         const float *vlo = Vt + j * LDVT + g, *vhi = Vt + (j + 4) * LDVT + g;
 #pragma unroll
         for (int mt = 0; mt < 16; mt++)

@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_i8_raw(DecodeArgs a) {
     for (uint32_t n = 0; it < ntiles; it += NWARP, n++) {
         const int tok0 = t0 + it * TILE;
         const bool more = it + NWARP < ntiles;
-        if (!mbar_wait(barK, n & 1)) {
+        if (!__all_sync(0xffffffffu, mbar_wait(barK, n & 1))) {      // (the lanes of a warp give up together)
             (void)mbar_wait(barV, n & 1);                         // bounded chance for the other copy to drain
             pipe_ok = false;
             break;
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(128, 4) k_gqa_decode_i8_raw(DecodeArgs a) {
         const uint32_t pb1 = movmatrix_trans(pack_h2(x10 * w1, x11 * w1));
 
         // ---- O^T += V^T P^T: one m-tile per chunk ---------------------------------------------
-        if (!mbar_wait(barV, n & 1)) {
+        if (!__all_sync(0xffffffffu, mbar_wait(barV, n & 1))) {
             if (more) (void)mbar_wait(barK, (n + 1) & 1);
             pipe_ok = false;
             break;

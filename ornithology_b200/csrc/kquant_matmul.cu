@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(NWARP * 32, (CTAS_PER_SM<TYPE, KS, MT>)) k_mat
 #pragma unroll
         for (int t = 0; t < MT; t++) term[t][0] = term[t][1] = term[t][2] = term[t][3] = 0.0f;
         if (seg < a.nseg) {
-            if (ok && !tc5::mbar_wait(smem_u32(&bars[seg % nstage]), (uint32_t)(seg / nstage) & 1u)) { ok = false; failed = 1; }
+            if (ok && !tc5::mbar_wait_warp(smem_u32(&bars[seg % nstage]), (uint32_t)(seg / nstage) & 1u)) { ok = false; failed = 1; }
             if (ok && active) {
                 smem_ptr stage = smem + (size_t)(seg % nstage) * stage_bytes;
                 smem_ptr wrow0 = stage + (wr * 16 + g) * BOX + ((seg * BLOCK) & 15);

@@ -68,7 +68,7 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
 }
 // bounded wait (poll limit and 2 s of wall time)
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return tc5::mbar_wait(bar, parity); }
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) { return tc5::mbar_wait_warp(bar, parity); }
 __device__ __forceinline__ void tensor_copy_rows(uint32_t dst, const CUtensorMap *map, int word0, int row0, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n"
                  ::"r"(dst), "l"(map), "r"(bar), "r"(word0), "r"(row0) : "memory");
