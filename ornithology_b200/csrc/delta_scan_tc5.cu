@@ -81,7 +81,7 @@ __device__ __forceinline__ void mma_tf32_sync(float (&d)[4], const float (&a)[4]
 // What the former kernel spent its 25k to 35k cycles a chunk on was waiting: shared-memory loads behind stores that might alias them,
 // a broadcast load to every two multiply-adds, gate inputs and rows fetched one dependent load after the other.  Here the
 // loads of a phase are issued together and nothing but M goes through shared memory: 22k to 27k cycles, two CTAs to an SM; 4096 tokens of
-// 64 heads 85 -> 68 us.  It is bound by latency (issue 0.4, shared-memory pipe 0.5).  Measured and not kept: the products of the
+// 64 heads 85 -> 68 us.  It is bound by latency and shared memory (issue 0.42, shared-memory pipe 0.77).  Measured and not kept: the products of the
 // inverse on the tensor cores in three tf32 terms (60 us, but A then differs in the last places from what f32 gives); three
 // CTAs to an SM (75 us, spills); persistent CTAs that request the next item's rows early (71 us).
 //
@@ -400,8 +400,8 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
 // one's commit: the pipe does not order them, and issued back to back the read came too early.
 // What bounds it: the chain of a chunk, K S^T (530 cycles), its commit, the pass over T (about 500: beta V is in registers by then),
 // A T (260), its commit, the pass over U (about 600), the update (530), its commit; Q S^T and P U run beside those waits, and the copies, one
-// period ahead, take up to 1.7 us when the passes in front of the next slab share the memory.  4.9k cycles a chunk (64 chunks x 64 heads
-// alone 220 -> 168 us; with beta V read from shared memory behind K S^T 5.5k, with z loaded by the output warps 6.2k).
+// period ahead, take up to 1.7 us when the passes in front of the next slab share the memory.  5.3k cycles a chunk (64 chunks x 64 heads
+// alone 220 -> 180 us; with beta V read from shared memory behind K S^T 5.5k, with z loaded by the output warps 6.2k).
 // The output warps have as long for a chunk.  So they read their tiles as 16 x 256-bit fragments, a thread holding 4 rows of 4 tokens
 // (the sum of squares over the head is three shuffle levels on 4 values; as one row of 16 tokens it was five levels on 16),
 // arithmetic goes in pairs, and z and bf16 outputs pass through shared memory by tensor copies, read and written as transposed

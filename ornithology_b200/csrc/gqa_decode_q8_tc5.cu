@@ -603,9 +603,9 @@ bool rows_map(CUtensorMap *m, const void *pool, int nkv) {
 
 }  // namespace
 
-// Ranges the scratch is made for: four to an SM and 8 heads, fewer when the batch is too small for ranges of at least floor_w units (same
-// rule as in the kernel).  The kernel has one CTA per SM and uses at most a quarter of them on large batches; callers hold scratch of
-// this size.
+// Ranges the scratch is made for: four to an SM and 8 heads (what an earlier kernel had resident), fewer when the batch is too small for ranges
+// of at least floor_w units (same rule as in the kernel).  This kernel has one CTA per SM and uses at most a quarter of them on
+// large batches; callers hold scratch of this size, and the rule below counts in it.
 static int balanced_ranges(int nkv, int nh, int n_seq, int max_len, int floor_w) {
     const int X = nkv * ((nh / nkv + 7) / 8);
     const long long tiles = (max_len + UNIT - 1) / UNIT;
@@ -614,6 +614,10 @@ static int balanced_ranges(int nkv, int nh, int n_seq, int max_len, int floor_w)
 }
 // By the longest context the call allows: ranges of at least 16 units (two tiles) and at most ~32 partials to a sequence, which the last CTA
 // merges alone.  Short ranges (one tile, at most 16 partials) only while the long ones are fewer than 100: beyond that the SMs are busy.
+// us of a step's attention, this rule | long ranges only | short ones always: 35B, 1 sequence of 256 tokens 13.0 | 13.8 | 13.0, of 2048 17.0 | 16.0 |
+// 17.0, of 4096 17.8 | 17.8 | 18.3, of 32768 30.1 | 30.1 | 39.0; 2 of 1024 15.3 | 19.5 | 15.2; 4 of 256 18.9 | 21.0 | 19.0, of 16384 29.2 |
+// 29.3 | 33.4; 8 of 1024 20.1 | 21.2 | 20.1, of 2048 23.4 | 23.3 | 19.4 (the line of 100 is not the best there), of 8192 28.8 | 28.7 | 28.6;
+// 397B, 1 of 32768 35.8 | 35.7 | 43.5, 2 of 1024 18.3 | 23.8 | 18.3, 8 of 2048 29.9 | 29.8 | 24.0.
 int gqa_decode_range_floor(int nkv, int nh, int n_seq, int max_len, bool short_ranges) {
     const int tiles = (max_len + UNIT - 1) / UNIT, w16 = (tiles + 15) / 16, w32 = (tiles + 31) / 32, w_long = w32 > 16 ? w32 : 16;
     const int X = nkv * ((nh / nkv + 7) / 8);

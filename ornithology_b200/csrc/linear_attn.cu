@@ -337,7 +337,7 @@ __global__ void k_conv_ring_image(float *ring, float *image, int K, int C, int p
 constexpr int CONV_TOK = 32;             // tokens walked by one thread
 
 // Y[tok][ch] = SiLU(conv) as f32.  grid (Cc/128, T/CONV_TOK, n_seq).  The ring is
-// only read here; the new history is stored afterwards (k_conv_ring_refresh; on the tcgen05 path k_delta_prep64).
+// only read here; the new history is stored afterwards (k_conv_ring_refresh; on the tcgen05 path k_delta_prep).
 template <typename ACT>
 __global__ void __launch_bounds__(128) k_conv_silu_prefill(LinArgs a, float *Y) {
     const int qd = a.nk * a.dk, Cc = 2 * qd + a.nv * a.dv, K = a.conv_k;

@@ -11,7 +11,7 @@ __device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvt
 // One lane of a converged warp, for the roles that one thread plays.  Not `lane == 0`: behind a branch that the compiler
 // cannot see to be taken by one thread, every tcgen05.mma is wrapped in code that makes its operands uniform, and a
 // thread then issues one product per 47 to 67 cycles; behind the election it is the tensor pipe that bounds (tf32
-// M128 N64 K8: 33 cycles, N128: 65, N256: 129).
+// M128 N64 K8: 33 cycles, N128: 65, N256: 129).  (Faster products are not always a faster kernel: see k_matmul_kq_tc5.)
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
