@@ -258,7 +258,11 @@ __global__ void __launch_bounds__(256, 2) k_delta_prep(const __grid_constant__ C
                 if (a.T - 4 + i >= 0) ring[(size_t)((pos0 + a.T - 4 + i) & 3) * Cc + ch] = v[i];
         }
     }
-    if (!mbar_wait_warp(su32(&rows_in), 0u)) report_timeout(p.status, ORN_WAIT_DELTA_SCAN);
+    if (!mbar_wait_warp(su32(&rows_in), 0u)) {            // A and P become NaN; the copies land before the CTA goes
+        report_timeout(p.status, ORN_WAIT_DELTA_SCAN);
+        sm.rk[lane] = sm.rk[32 + lane] = NAN;
+        (void)mbar_wait_warp(su32(&rows_in), 0u);
+    }
 
     // Gram tiles: warp w has the rows 16 mt .. of K and of Q and up to three groups of 8 columns from nt0 on (20 such groups lie on
     // or below the diagonal)
